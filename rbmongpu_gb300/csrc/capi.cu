@@ -55,7 +55,7 @@ int deep_log_psi(const rbmg_psi* psi, int count, const uint64_t* d_spins, uint64
 struct Workspace {
     DevBuf sample_spins, eloc, logpsi, logpsi_p, T, U, X, Tp, weights, coef1, coef2, coef3, omega, pr, nn;
     DevBuf partial, block_scratch, sums, acc_O, acc_EO, acc_Ek, acc_wO, acc_pO, block_max, zsum;
-    DevBuf smat, smean, okrows, sshift, splanes, serror, sout;
+    DevBuf smat, smean, spart, okrows, sshift, splanes, serror, sout;
     DevBuf acc_B, eabs2, lsums, rw, rwc, acc_C2, acc_C3;
     DevBuf fqa_qa, fqa_r, fqa_flip, fqa_lpf, fqa_lp, fqa_out;   // free-quantum-axis terms of the HSD
 };
@@ -2196,11 +2196,12 @@ extern "C" int rbmg_s_matrix(const rbmg_psi* psi, rbmg_ensemble* ens, int flags,
     // centred: every row is shifted by the first chunk's mean row (in FP64) before the FP32
     // products, so that the covariance is not the small difference of two large sums
     RBMG_CK(W.sshift.ensure(sizeof(double2) * L));
+    if (centered) RBMG_CK(W.spart.ensure(sm_mean_bytes(L)));
     bool have_shift = false;
     auto with_shift = [&](SmSource& a) -> cudaError_t {
         if (!centered) return cudaSuccess;
         if (!have_shift) {
-            const cudaError_t e = launch_sm_row_mean(a, W.sshift.as<double2>(), stream());
+            const cudaError_t e = launch_sm_row_mean(a, W.sshift.as<double2>(), W.spart.as<double2>(), stream());
             if (e != cudaSuccess) return e;
             have_shift = true;
         }
@@ -2221,12 +2222,12 @@ extern "C" int rbmg_s_matrix(const rbmg_psi* psi, rbmg_ensemble* ens, int flags,
             e = launch_sm_tc_accumulate(a, W.smat.as<double2>(), W.splanes.p, W.serror.as<int>(), &nlaunch, sms,
                                         stream());
         } else {
-            e = launch_sm_accumulate(a, W.smat.as<double2>(), nullptr, sms, stream());
+            e = launch_sm_accumulate(a, W.smat.as<double2>(), sms, stream());
             nlaunch++;
         }
         if (e != cudaSuccess || !centered) return e;
         nlaunch++;
-        return launch_sm_mean(a, W.smean.as<double2>(), stream());
+        return launch_sm_mean(a, W.smean.as<double2>(), W.spart.as<double2>(), stream());
     };
     // CUDA events around every accumulation launch (rbmg_s_matrix_timing)
     std::vector<cudaEvent_t> ev;

@@ -23,6 +23,7 @@ namespace {
 
 constexpr int kT = 64;          // tile edge
 constexpr int kS = 16;          // samples per shared-memory stage
+constexpr int kSmMeanSlices = 64;
 constexpr int kFlush = 1024;    // samples accumulated in FP32 before the FP64 update
 
 __global__ void __launch_bounds__(256) sm_herk_kernel(SmSource a, double2* __restrict__ S, int nt, int slice,
@@ -115,26 +116,57 @@ __global__ void __launch_bounds__(256) sm_herk_kernel(SmSource a, double2* __res
     }
 }
 
-// mean[k] += sum_s w_s (F[s][k] - shift[k]) (FP64); assign: mean[k] = the sum * scale
-__global__ void sm_mean_kernel(SmSource a, double2* mean, int assign, double scale) {
+// partial[z][k] = sum over slice z of the samples of w_s (F[s][k] - shift[k]) (FP64).  One
+// thread per column walks its slice: a column's loads depend on nothing, but a thread keeps
+// only a few in flight, so the samples are cut into enough slices to fill the GPU (one slice
+// of 4096 samples on 16 blocks took 1760 us at L = 1980, 64 slices take 130 us).
+__global__ void sm_mean_kernel(SmSource a, int per_slice, double2* partial) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.L) return;
     SmSource u = a;
     u.weighted = 0;
     const SmElem e = sm_elem_of(u, k);
     double sr = 0.0, si = 0.0;
-    for (int s = 0; s < a.count; s++) {
-        const float2 v = sm_load_f(u, e, s, k);
-        const double c = a.weighted ? a.w[s] : 1.0;
-        sr += c * v.x;
-        si += c * v.y;
-    }
-    if (assign) {
-        mean[k] = make_double2(sr * scale, si * scale);
+    const int s0 = blockIdx.y * per_slice, s1 = min(a.count, s0 + per_slice);
+    if (a.kind == 0 && !a.shift && !a.weighted) {
+        // the elements are FP32 values with a sign: no FP64 step but the sum (FP64 instructions
+        // and conversions are most of this kernel's time)
+#pragma unroll 4
+        for (int s = s0; s < s1; s++) {
+            float2 v = a.T[static_cast<long>(s) * a.Mpad + e.j];
+            if (e.i >= 0) {
+                const uint64_t word = a.enumerate ? ((e.i >> 6) == 0 ? a.enum_base + static_cast<uint64_t>(s) : 0ull)
+                                                  : a.spins[static_cast<long>(s) * a.nw + (e.i >> 6)];
+                if (!((word >> (e.i & 63)) & 1ull)) v = make_float2(-v.x, -v.y);
+            }
+            sr += static_cast<double>(v.x);
+            si += static_cast<double>(v.y);
+        }
     } else {
-        mean[k].x += sr;
-        mean[k].y += si;
+#pragma unroll 4
+        for (int s = s0; s < s1; s++) {
+            const float2 v = sm_load_f(u, e, s, k);
+            const double c = a.weighted ? a.w[s] : 1.0;
+            sr += c * v.x;
+            si += c * v.y;
+        }
     }
+    partial[static_cast<long>(blockIdx.y) * a.L + k] = make_double2(sr, si);
+}
+
+// mean[k] += the slices' sums in order; assign: mean[k] = their sum * scale
+__global__ void sm_mean_finish_kernel(int L, int slices, const double2* partial, double2* mean, int assign,
+                                      double scale) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= L) return;
+    double sr = 0.0, si = 0.0;
+#pragma unroll 8
+    for (int z = 0; z < slices; z++) {
+        const double2 v = partial[static_cast<long>(z) * L + k];
+        sr += v.x;
+        si += v.y;
+    }
+    mean[k] = assign ? make_double2(sr * scale, si * scale) : make_double2(mean[k].x + sr, mean[k].y + si);
 }
 
 // out[off + r][off + c] = S[r][c] / Z with the lower triangle mirrored from the upper and
@@ -166,7 +198,7 @@ __global__ void sm_finish_kernel(int L, const double2* __restrict__ S, const dou
 
 }  // namespace
 
-cudaError_t launch_sm_accumulate(const SmSource& a, double2* S, double2* mean, int num_sms, cudaStream_t st) {
+cudaError_t launch_sm_accumulate(const SmSource& a, double2* S, int num_sms, cudaStream_t st) {
     if (a.count <= 0) return cudaSuccess;
     const int nt = (a.L + kT - 1) / kT;
     const int upper = nt * (nt + 1) / 2;
@@ -178,23 +210,32 @@ cudaError_t launch_sm_accumulate(const SmSource& a, double2* S, double2* mean, i
     const int slice = (a.count + split - 1) / split;
     const dim3 grid(nt * nt, split);
     sm_herk_kernel<<<grid, 256, 0, st>>>(a, S, nt, slice, split > 1);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess || !mean) return e;
-    return launch_sm_mean(a, mean, st);
-}
-
-cudaError_t launch_sm_mean(const SmSource& a, double2* mean, cudaStream_t st) {
-    if (a.count <= 0) return cudaSuccess;
-    sm_mean_kernel<<<(a.L + 127) / 128, 128, 0, st>>>(a, mean, 0, 1.0);
     return cudaGetLastError();
 }
 
-cudaError_t launch_sm_row_mean(const SmSource& a, double2* out, cudaStream_t st) {
+// slices of at least 16 samples, at most kSmMeanSlices
+static cudaError_t sm_mean(const SmSource& a, double2* mean, double2* partial, int assign, double scale,
+                           cudaStream_t st) {
+    const int per = std::max(16, (a.count + kSmMeanSlices - 1) / kSmMeanSlices);
+    const int slices = (a.count + per - 1) / per;
+    const dim3 grid((a.L + 127) / 128, slices);
+    sm_mean_kernel<<<grid, 128, 0, st>>>(a, per, partial);
+    sm_mean_finish_kernel<<<grid.x, 128, 0, st>>>(a.L, slices, partial, mean, assign, scale);
+    return cudaGetLastError();
+}
+
+size_t sm_mean_bytes(int L) { return sizeof(double2) * kSmMeanSlices * static_cast<size_t>(L); }
+
+cudaError_t launch_sm_mean(const SmSource& a, double2* mean, double2* partial, cudaStream_t st) {
+    return a.count <= 0 ? cudaSuccess : sm_mean(a, mean, partial, 0, 1.0, st);
+}
+
+cudaError_t launch_sm_row_mean(const SmSource& a, double2* out, double2* partial, cudaStream_t st) {
+    if (a.count <= 0) return cudaSuccess;
     SmSource u = a;
     u.weighted = 0;
     u.shift = nullptr;
-    sm_mean_kernel<<<(a.L + 127) / 128, 128, 0, st>>>(u, out, 1, 1.0 / static_cast<double>(a.count));
-    return cudaGetLastError();
+    return sm_mean(u, out, partial, 1, 1.0 / static_cast<double>(a.count), st);
 }
 
 cudaError_t launch_sm_finish(int L, const double2* S, const double2* mean, double inv_z, int centered,

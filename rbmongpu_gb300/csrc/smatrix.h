@@ -25,12 +25,13 @@ struct SmSource {
 };
 
 // S [L][L] += sum_s c_s G_s^T conj(G_s) on the upper tiles, G_s = F_s - shift (c_s = w_s
-// when weighted, else 1); mean [L] += sum_s c_s G_s when mean is not null
-cudaError_t launch_sm_accumulate(const SmSource& src, double2* S, double2* mean, int num_sms, cudaStream_t st);
-// mean [L] += sum_s c_s G_s alone
-cudaError_t launch_sm_mean(const SmSource& src, double2* mean, cudaStream_t st);
+// when weighted, else 1)
+cudaError_t launch_sm_accumulate(const SmSource& src, double2* S, int num_sms, cudaStream_t st);
+// mean [L] += sum_s c_s G_s; partial: sm_mean_bytes(L) of scratch
+size_t sm_mean_bytes(int L);
+cudaError_t launch_sm_mean(const SmSource& src, double2* mean, double2* partial, cudaStream_t st);
 // out [L] = sum_s F_s / count (unweighted, unshifted): the shift of a centred S matrix
-cudaError_t launch_sm_row_mean(const SmSource& src, double2* out, cudaStream_t st);
+cudaError_t launch_sm_row_mean(const SmSource& src, double2* out, double2* partial, cudaStream_t st);
 // the same products on the tensor cores (smatrix_tc.cu): BF16 hi / mid / lo operand planes
 // of the chunk in `planes` (sm_tc_planes_bytes(L, count) bytes), one operand pass and one
 // persistent MMA launch on num_sms CTAs (counted into *launches); a tensor-core wait that
