@@ -57,6 +57,7 @@ struct Workspace {
     DevBuf partial, block_scratch, sums, acc_O, acc_EO, acc_Ek, acc_wO, acc_pO, block_max, zsum;
     DevBuf smat, smean, spart, okrows, sshift, splanes, serror, sout;
     DevBuf acc_B, eabs2, lsums, rw, rwc, acc_C2, acc_C3;
+    DevBuf tab64, tab64_p;   // spin-group sums of psi's and psi''s FP64 weights
     DevBuf fqa_qa, fqa_r, fqa_flip, fqa_lpf, fqa_lp, fqa_out;   // free-quantum-axis terms of the HSD
 };
 
@@ -164,7 +165,24 @@ static int rbm_upload64(const rbmg_psi* p) {
     return RBMG_OK;
 }
 
-static Rbm64 rbm64(const rbmg_psi* p) { return Rbm64{p->N, p->M, p->dW64.as<double2>(), p->db64.as<double2>()}; }
+static Rbm64 rbm64(const rbmg_psi* p) {
+    return Rbm64{p->N, p->M, p->dW64.as<double2>(), p->db64.as<double2>(), nullptr};
+}
+
+// The FP64 parameters for a pass over `count` configurations, with the table of spin-group
+// sums formed in `tab` on the calling thread's stream where it pays.  A call of log psi with
+// and without the table: N = 12, M = 24: 37 / 35 us at 256 configurations, 38 / 36 at 1024,
+// 39 / 49 at 2048; N = 36, M = 75: 36 / 51 us at 64 (the chain of N additions shows even
+// where the GPU is idle), 117 / 326 at 8192; N = 75, M = 150: 51 / 109 at 64, 209 / 963 at
+// 8192
+static int rbm64_for(const rbmg_psi* p, uint64_t count, DevBuf& tab, Rbm64* out) {
+    *out = rbm64(p);
+    if (count < 2048 && p->N < 24) return RBMG_OK;
+    RBMG_CK(tab.ensure(rbm_table64_bytes(p->N, p->M)));
+    RBMG_CK(launch_rbm_table64(*out, tab.as<double2>(), stream()));
+    out->tab = tab.as<double2>();
+    return RBMG_OK;
+}
 
 extern "C" int rbmg_psi_create(int N, int M, const double* alpha, const double* beta, const double* b,
                                const double* W, double prefactor, int free_quantum_axis, rbmg_psi** out) {
@@ -620,7 +638,7 @@ extern "C" int rbmg_ensemble_destroy(rbmg_ensemble* ens) {
 
 // ====================================================================== sample streams
 static int rbm_upload64(const rbmg_psi* p);
-static Rbm64 rbm64(const rbmg_psi* p);
+static int rbm64_for(const rbmg_psi* p, uint64_t count, DevBuf& tab, Rbm64* out);
 
 namespace rbmg {
 
@@ -658,7 +676,10 @@ static int psi_log_psi_dev(const rbmg_psi* psi, int count, const uint64_t* d_spi
         Rbm64 nopp{};
         nopp.N = psi->N;
         nopp.M = psi->M;
-        RBMG_CK(launch_rbm_hsd64(::rbm64(psi), nopp, none, L, stream()));
+        Rbm64 P;
+        const int rt = ::rbm64_for(psi, static_cast<uint64_t>(count), ws().tab64, &P);
+        if (rt != RBMG_OK) return rt;
+        RBMG_CK(launch_rbm_hsd64(P, nopp, none, L, stream()));
         return RBMG_OK;
     }
     return deep_log_psi(psi, count, d_spins, enum_base, enumerate, d_out, stream());
@@ -1714,7 +1735,11 @@ extern "C" int rbmg_hsd_gradient(const rbmg_psi* psi, const rbmg_psi* pp, const 
                 L.spins = c.spins;
                 L.eloc = W.eloc.as<double2>();
                 L.dlogpsi = W.logpsi_p.as<double2>();
-                RBMG_CK(launch_rbm_hsd64(rbm64(psi), rbm64(pp), od, L, stream()));
+                Rbm64 P, PP;
+                int rr = rbm64_for(psi, static_cast<uint64_t>(c.count), W.tab64, &P);
+                if (rr == RBMG_OK) rr = rbm64_for(pp, static_cast<uint64_t>(c.count), W.tab64_p, &PP);
+                if (rr != RBMG_OK) return rr;
+                RBMG_CK(launch_rbm_hsd64(P, PP, od, L, stream()));
             } else {
                 const int rr = deep_hsd64_chunk(psi, pp, op, c, W.eloc.as<double2>(), W.logpsi_p.as<double2>(),
                                                 stream());
@@ -1999,6 +2024,12 @@ extern "C" int rbmg_hsd_distance_2nd_order(const rbmg_psi* psi, const rbmg_psi* 
         RBMG_CK(W.omega.ensure(sizeof(double2) * c.count));
         RBMG_CK(W.pr.ensure(sizeof(double2) * c.count));
         RBMG_CK(W.nn.ensure(sizeof(double2) * c.count));
+        Rbm64 P{}, PP{};
+        if (psi->kind == 0) {
+            int rr = rbm64_for(psi, static_cast<uint64_t>(c.count), W.tab64, &P);
+            if (rr == RBMG_OK) rr = rbm64_for(pp, static_cast<uint64_t>(c.count), W.tab64_p, &PP);
+            if (rr != RBMG_OK) return rr;
+        }
         for (int which = 0; which < 2; which++) {
             double2* e = which == 0 ? W.eloc.as<double2>() : W.coef2.as<double2>();
             if (psi->kind == 0) {
@@ -2009,7 +2040,7 @@ extern "C" int rbmg_hsd_distance_2nd_order(const rbmg_psi* psi, const rbmg_psi* 
                 L.spins = c.spins;
                 L.eloc = e;
                 L.dlogpsi = W.logpsi_p.as<double2>();
-                RBMG_CK(launch_rbm_hsd64(rbm64(psi), rbm64(pp), which == 0 ? od : od2, L, stream()));
+                RBMG_CK(launch_rbm_hsd64(P, PP, which == 0 ? od : od2, L, stream()));
             } else {
                 const int rr = deep_hsd64_chunk(psi, pp, which == 0 ? op : op2, c, e, W.logpsi_p.as<double2>(),
                                                 stream());

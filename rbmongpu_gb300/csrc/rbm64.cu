@@ -19,20 +19,54 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
     return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 
-// include/quantum_state/psi_functions.hpp:49-57 in FP64
-__device__ __forceinline__ double2 lc64(double2 z) {
-    const double s = z.x > 0.0 ? 1.0 : -1.0;
-    double2 t = make_double2(s * 3.746646023906276 + z.x, z.y);
-    t = cmul(z, t);
-    t.x += 7.771429504240965;
-    t = cmul(z, t);
-    t.x += s * 10.2180213465;
-    t = cmul(z, t);
-    t.x += 9.19376335670885;
-    const double2 num = make_double2(5.49914721954 - s * 2.16564366435 * z.x, -s * 2.16564366435 * z.y);
-    const double den = t.x * t.x + t.y * t.y;
-    const double qr = (num.x * t.x + num.y * t.y) / den, qi = (num.y * t.x - num.x * t.y) / den;
-    return make_double2(s * 0.9003320053750442 * z.x + qr - 0.598139, s * 0.9003320053750442 * z.y + qi);
+// The rational log-cosh (include/quantum_state/psi_functions.hpp:49-57) in FP64, kept open as
+// f + C = A u + n / D(u): u = sign(Re z) z, n / D = (nr + i ni) inv.  FP64 instructions issue
+// at 1/64 of the FP32 rate and are all that these kernels wait for, so they are counted: the
+// quartic with real coefficients runs on u's trace 2p and norm |u|^2 (11 operations against
+// 13 of the complex Horner scheme), the sign is folded in by integer operations, and one
+// reciprocal serves both parts: the hardware's estimate (at least 19 bits) and one cubic step
+// r (1 + e + e^2), e = 1 - den r, which leaves e^3 < 2^-57.  32 FP64 operations with the
+// difference and its sum, against 61 with two divisions.
+constexpr double kLcC = 0.598139;
+constexpr double kLcA = 0.9003320053750442;
+
+struct Lc64 {
+    double p, q, nr, ni, inv;
+    __device__ __forceinline__ double2 open() const { return make_double2(fma(kLcA, p, nr * inv), fma(kLcA, q, ni * inv)); }
+    // d += (f + C) - g
+    __device__ __forceinline__ void add_difference(double2 g, double2& d) const {
+        d.x += fma(kLcA, p, fma(nr, inv, -g.x));
+        d.y += fma(kLcA, q, fma(ni, inv, -g.y));
+    }
+};
+
+__device__ __forceinline__ double rcp64(double den) {
+    // |D|^2 overflows for |z| > 1e38 only; the clamp keeps 0 rather than NaN there, as a
+    // division does
+    const int hi = min(__double2hiint(den), 0x7FD00000);
+    den = __hiloint2double(hi, __double2loint(den));
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(den));
+    const double e = fma(-den, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+
+__device__ __forceinline__ Lc64 lc64(double2 z) {
+    // sign = z.x > 0 ? 1 : -1 (positive doubles are positive integers; zero counts as -1)
+    const long long flip = __double_as_longlong(z.x) > 0 ? 0ll : static_cast<long long>(0x8000000000000000ull);
+    Lc64 f;
+    f.p = __longlong_as_double(__double_as_longlong(z.x) ^ flip);
+    f.q = __longlong_as_double(__double_as_longlong(z.y) ^ flip);
+    const double r = f.p + f.p, n = fma(f.q, f.q, f.p * f.p);
+    const double b3 = r + 3.746646023906276;
+    const double b2 = fma(r, b3, 7.771429504240965 - n);
+    const double b1 = fma(r, b2, fma(-n, b3, 10.2180213465));
+    const double dr = fma(f.p, b1, fma(-n, b2, 9.19376335670885)), di = f.q * b1;
+    const double ur = fma(-2.16564366435, f.p, 5.49914721954), ui = -2.16564366435 * f.q;
+    f.nr = fma(ur, dr, ui * di);
+    f.ni = fma(ui, dr, -(ur * di));
+    f.inv = rcp64(fma(dr, dr, di * di));
+    return f;
 }
 
 __device__ __forceinline__ double2 warp_sum64(double2 v) {
@@ -46,9 +80,95 @@ __device__ __forceinline__ double2 warp_sum64(double2 v) {
 
 __device__ __forceinline__ bool spin_up(const uint64_t* s, int i) { return (s[i >> 6] >> (i & 63)) & 1ull; }
 
-// shared memory per warp: theta[M], f[M] (double2 each).  op.S = 0 skips the local
-// energy and PP.W = null skips log psi'; with both it is the FP64 log psi pass that the
-// exact-summation weights and the psi vector use.
+// six consecutive spins of a configuration, from spin 6 g on
+__device__ __forceinline__ int spin_group(const uint64_t* s, int g, int N) {
+    const int i = kTab64Spins * g, w = i >> 6, sh = i & 63;
+    uint64_t v = s[w] >> sh;
+    if (sh > 64 - kTab64Spins && w + 1 < kMaxWords) v |= s[w + 1] << (64 - sh);
+    return static_cast<int>(v & ((1u << min(kTab64Spins, N - i)) - 1u));
+}
+
+// tab[g][m][j] = sum over the spins i of group g of +-W[i][j], signs by the bits of m; group 0
+// carries b[j].  An angle is then one entry per six spins (2 FP64 additions for 12).
+__global__ void table64_kernel(Rbm64 P, double2* tab) {
+    const int groups = (P.N + kTab64Spins - 1) / kTab64Spins;
+    const long total = static_cast<long>(groups) * kTab64Size * P.M;
+    for (long e = blockIdx.x * 256L + threadIdx.x; e < total; e += static_cast<long>(gridDim.x) * 256) {
+        const int j = static_cast<int>(e % P.M);
+        const int m = static_cast<int>(e / P.M) % kTab64Size, g = static_cast<int>(e / P.M / kTab64Size);
+        double2 a = g == 0 ? P.b[j] : make_double2(0.0, 0.0);
+        for (int i = kTab64Spins * g; i < min(P.N, kTab64Spins * (g + 1)); i++) {
+            const double2 w = P.W[static_cast<long>(i) * P.M + j];
+            const double sg = (m >> (i - kTab64Spins * g)) & 1 ? 1.0 : -1.0;
+            a.x = fma(sg, w.x, a.x);
+            a.y = fma(sg, w.y, a.y);
+        }
+        tab[e] = a;
+    }
+}
+
+__device__ __forceinline__ double2 angle64(const Rbm64& P, const uint64_t* s, int j) {
+    if (P.tab) {
+        double2 a = make_double2(0.0, 0.0);
+        const int groups = (P.N + kTab64Spins - 1) / kTab64Spins;
+#pragma unroll 2
+        for (int g = 0; g < groups; g++) {
+            const double2 t = P.tab[(static_cast<long>(g) * kTab64Size + spin_group(s, g, P.N)) * P.M + j];
+            a.x += t.x;
+            a.y += t.y;
+        }
+        return a;
+    }
+    double2 a = P.b[j];
+    for (int i = 0; i < P.N; i++) {
+        const double2 w = P.W[static_cast<long>(i) * P.M + j];
+        if (spin_up(s, i)) { a.x += w.x; a.y += w.y; }
+        else { a.x -= w.x; a.y -= w.y; }
+    }
+    return a;
+}
+
+// coefficient and phase of string n on the configuration s
+__device__ __forceinline__ double2 string_factor64(const OpDev& op, int n, const uint64_t* s) {
+    int parity = 0;
+    for (int k = 0; k < kMaxWords; k++) parity += __popcll(op.zmask[n * kMaxWords + k] & ~s[k]);
+    const double2 c = op.coef[n];
+    const int yp = op.ypow[n] & 3;
+    const double2 r = yp == 0 ? c : (yp == 1 ? make_double2(c.y, -c.x) : (yp == 2 ? make_double2(-c.x, -c.y)
+                                                                                : make_double2(-c.y, c.x)));
+    return (parity & 1) ? make_double2(-r.x, -r.y) : r;
+}
+
+// The warp's sums of eight complex values a lane, in one folding butterfly: lanes 4 u .. 4 u + 3
+// receive the sum of value u (9 complex additions a lane against 40 of eight butterflies)
+__device__ __forceinline__ double2 warp_fold8(double2 (&d)[8], int lane) {
+#pragma unroll
+    for (int half = 4, off = 16; half >= 1; half >>= 1, off >>= 1) {
+        const bool up = (lane & off) != 0;
+#pragma unroll
+        for (int i = 0; i < half; i++) {
+            const double2 send = up ? d[i] : d[i + half], keep = up ? d[i + half] : d[i];
+            d[i].x = keep.x + __shfl_xor_sync(0xffffffffu, send.x, off);
+            d[i].y = keep.y + __shfl_xor_sync(0xffffffffu, send.y, off);
+        }
+    }
+#pragma unroll
+    for (int off = 2; off >= 1; off >>= 1) {
+        d[0].x += __shfl_xor_sync(0xffffffffu, d[0].x, off);
+        d[0].y += __shfl_xor_sync(0xffffffffu, d[0].y, off);
+    }
+    return d[0];
+}
+
+// One warp per configuration, its lanes over the hidden units.  Shared memory per warp:
+// theta[M], f[M] + C (double2 each).  op.S = 0 skips the local energy and PP.W = null skips
+// log psi'; with both it is the FP64 log psi pass that the exact-summation weights and the psi
+// vector use.  Bound: the FP64 pipe.  The off-diagonal strings are taken eight at a time
+// (their lane sums folded together), and their exp, cos and sin 32 at a time, one string per
+// lane, so that no FP64 instruction repeats in the 32 lanes what one could do: N = 16, M = 32
+// over 2^16 configurations (one pass with log psi', one for the weights) takes 2670 us,
+// 9350 us with one string at a time in all lanes; 1.8 ms is the issue time of the strings'
+// activations alone.
 __global__ void rbm_hsd64_kernel(Rbm64 P, Rbm64 PP, OpDev op, Hsd64Launch L) {
     extern __shared__ double2 smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -63,78 +183,91 @@ __global__ void rbm_hsd64_kernel(Rbm64 P, Rbm64 PP, OpDev op, Hsd64Launch L) {
         const uint64_t idx = L.enum_base + static_cast<uint64_t>(t);
         s[0] = N >= 64 ? idx : (idx & ((1ull << N) - 1ull));
     } else {
-        for (int k = 0; k < nw; k++) s[k] = L.spins[t * nw + k];
+#pragma unroll
+        for (int k = 0; k < kMaxWords; k++)
+            if (k < nw) s[k] = L.spins[t * nw + k];
     }
     double2 lp = make_double2(0.0, 0.0);
     for (int j = lane; j < M; j += 32) {
-        double2 a = P.b[j];
-        for (int i = 0; i < N; i++) {
-            const double2 w = P.W[static_cast<long>(i) * M + j];
-            if (spin_up(s, i)) { a.x += w.x; a.y += w.y; }
-            else { a.x -= w.x; a.y -= w.y; }
-        }
+        const double2 a = angle64(P, s, j);
+        const double2 v = lc64(a).open();
         th[j] = a;
-        f[j] = lc64(a);
-        lp.x += f[j].x;
-        lp.y += f[j].y;
+        f[j] = v;
+        lp.x += v.x - kLcC;
+        lp.y += v.y;
     }
     lp = warp_sum64(lp);
     __syncwarp();
     // local energy (include/operator/Operator.hpp:90-115) with per-angle differences
-    double er = 0.0, ei = 0.0;
-    for (int n = 0; n < op.S; n++) {
-        int parity = 0;
-        for (int k = 0; k < nw; k++) parity += __popcll(op.zmask[n * kMaxWords + k] & ~s[k]);
-        const double sg = (parity & 1) ? -1.0 : 1.0;
-        const double2 c0 = op.coef[n];
-        const int yp = op.ypow[n] & 3;
-        double2 cf = yp == 0 ? c0 : (yp == 1 ? make_double2(c0.y, -c0.x) : (yp == 2 ? make_double2(-c0.x, -c0.y)
-                                                                                  : make_double2(-c0.y, c0.x)));
-        cf.x *= sg;
-        cf.y *= sg;
-        const int nf = op.nflip[n];
-        if (nf == 0) {
-            er += cf.x;
-            ei += cf.y;
-            continue;
-        }
-        const int off = op.flip_off[n];
-        double2 d = make_double2(0.0, 0.0);
-        for (int j = lane; j < M; j += 32) {
-            double2 a = th[j];
-            for (int q = 0; q < nf; q++) {
-                const int site = op.flip_sites[off + q];
-                const double2 w = P.W[static_cast<long>(site) * M + j];
-                const double two_s = spin_up(s, site) ? -2.0 : 2.0;
-                a.x += two_s * w.x;
-                a.y += two_s * w.y;
-            }
-            const double2 g = lc64(a);
-            d.x += g.x - f[j].x;
-            d.y += g.y - f[j].y;
-        }
-        d = warp_sum64(d);
-        const double m = exp(d.x);
-        const double2 x = make_double2(m * cos(d.y), m * sin(d.y));
-        er += cf.x * x.x - cf.y * x.y;
-        ei += cf.x * x.y + cf.y * x.x;
+    double2 e = make_double2(0.0, 0.0);
+    for (int n = lane; n < op.S; n += 32) {
+        if (op.nflip[n] != 0) continue;
+        const double2 cf = string_factor64(op, n, s);
+        e.x += cf.x;
+        e.y += cf.y;
     }
+    const int strings = op.S > 0 ? op.num_offdiag : 0;
+    for (int q0 = 0; q0 < strings; q0 += 32) {
+        double2 mine = make_double2(0.0, 0.0);   // log psi(s'_n) - log psi(s) of string q0 + lane
+        for (int b = 0; b < 4 && q0 + 8 * b < strings; b++) {
+            double2 d[8];
+            int site[8], flips[8];
+            double two_s[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                d[u] = make_double2(0.0, 0.0);
+                const int n = op.offdiag[min(q0 + 8 * b + u, strings - 1)];
+                flips[u] = op.nflip[n];
+                site[u] = op.flip_off[n];
+                const int first = op.flip_sites[site[u]];
+                two_s[u] = spin_up(s, first) ? -2.0 : 2.0;
+                if (flips[u] == 1) site[u] = first;
+            }
+            for (int j = lane; j < M; j += 32) {
+                const double2 a0 = th[j], f0 = f[j];
+#pragma unroll
+                for (int u = 0; u < 8; u++) {
+                    double2 a = a0;
+                    if (flips[u] == 1) {
+                        const double2 w = P.W[static_cast<long>(site[u]) * M + j];
+                        a.x = fma(two_s[u], w.x, a.x);
+                        a.y = fma(two_s[u], w.y, a.y);
+                    } else {
+                        for (int k = 0; k < flips[u]; k++) {
+                            const int i = op.flip_sites[site[u] + k];
+                            const double2 w = P.W[static_cast<long>(i) * M + j];
+                            const double sg = spin_up(s, i) ? -2.0 : 2.0;
+                            a.x = fma(sg, w.x, a.x);
+                            a.y = fma(sg, w.y, a.y);
+                        }
+                    }
+                    lc64(a).add_difference(f0, d[u]);
+                }
+            }
+            const double2 sum = warp_fold8(d, lane);
+            const double vx = __shfl_sync(0xffffffffu, sum.x, 4 * (lane & 7));
+            const double vy = __shfl_sync(0xffffffffu, sum.y, 4 * (lane & 7));
+            if (lane >> 3 == b) mine = make_double2(vx, vy);
+        }
+        if (q0 + lane < strings) {
+            const double2 cf = string_factor64(op, op.offdiag[q0 + lane], s);
+            const double m = exp(mine.x);
+            double sn, cs;
+            sincos(mine.y, &sn, &cs);
+            const double2 x = make_double2(m * cs, m * sn);
+            e.x += cf.x * x.x - cf.y * x.y;
+            e.y += cf.x * x.y + cf.y * x.x;
+        }
+    }
+    if (op.S > 0) e = warp_sum64(e);
     // log psi'(s) - log psi(s), angle by angle
     double2 dl = make_double2(0.0, 0.0);
-    for (int j = lane; PP.W && j < M; j += 32) {
-        double2 a = PP.b[j];
-        for (int i = 0; i < N; i++) {
-            const double2 w = PP.W[static_cast<long>(i) * M + j];
-            if (spin_up(s, i)) { a.x += w.x; a.y += w.y; }
-            else { a.x -= w.x; a.y -= w.y; }
-        }
-        const double2 g = lc64(a);
-        dl.x += g.x - f[j].x;
-        dl.y += g.y - f[j].y;
+    if (PP.W) {
+        for (int j = lane; j < M; j += 32) lc64(angle64(PP, s, j)).add_difference(f[j], dl);
+        dl = warp_sum64(dl);
     }
-    dl = warp_sum64(dl);
     if (lane == 0) {
-        if (L.eloc) L.eloc[t] = make_double2(er, ei);
+        if (L.eloc) L.eloc[t] = e;
         if (L.logpsi) L.logpsi[t] = lp;
         if (L.dlogpsi) L.dlogpsi[t] = dl;
     }
@@ -283,6 +416,16 @@ cudaError_t launch_fqa_grad(int count, int N, const uint64_t* spins, uint64_t en
                             const double2* c, const double2* r, const double* qa, double2* out, cudaStream_t st) {
     if (count <= 0) return cudaSuccess;
     fqa_grad_kernel<<<2 * N, 256, 0, st>>>(count, N, spins, enum_base, enumerate, c, r, qa, out);
+    return cudaGetLastError();
+}
+
+size_t rbm_table64_bytes(int N, int M) {
+    return sizeof(double2) * static_cast<size_t>((N + kTab64Spins - 1) / kTab64Spins) * kTab64Size * M;
+}
+
+cudaError_t launch_rbm_table64(const Rbm64& P, double2* tab, cudaStream_t st) {
+    const long total = static_cast<long>(rbm_table64_bytes(P.N, P.M) / sizeof(double2));
+    table64_kernel<<<static_cast<int>(std::min(4096L, (total + 255) / 256)), 256, 0, st>>>(P, tab);
     return cudaGetLastError();
 }
 

@@ -13,7 +13,13 @@ struct Rbm64 {
     int N, M;
     const double2* W;   // [N][M]
     const double2* b;   // [M]
+    const double2* tab; // sums of W over groups of spins (launch_rbm_table64), or null
 };
+
+// spins per table group and sign patterns of a group
+constexpr int kTab64Spins = 6, kTab64Size = 1 << kTab64Spins;
+size_t rbm_table64_bytes(int N, int M);
+cudaError_t launch_rbm_table64(const Rbm64& P, double2* tab, cudaStream_t st);
 
 struct Hsd64Launch {
     int count;
