@@ -53,7 +53,7 @@ int deep_log_psi(const rbmg_psi* psi, int count, const uint64_t* d_spins, uint64
 // ---------------------------------------------------------------- workspace
 // Grow-only scratch buffers shared by all calls on this thread's device.
 struct Workspace {
-    DevBuf sample_spins, eloc, logpsi, logpsi_p, T, U, X, Tp, weights, coef1, coef2, coef3, omega, pr, nn;
+    DevBuf sample_spins, eloc, logpsi, logpsi_p, T, U, X, theta, en, vpart, Tp, weights, coef1, coef2, coef3, omega, pr, nn;
     DevBuf partial, block_scratch, sums, acc_O, acc_EO, acc_Ek, acc_wO, acc_pO, block_max, zsum;
     DevBuf smat, smean, spart, okrows, sshift, splanes, serror, sout;
     DevBuf acc_B, eabs2, lsums, rw, rwc, acc_C2, acc_C3;
@@ -410,6 +410,16 @@ static int op_compile(rbmg_operator* op) {
                 if ((flips[w] >> bpos) & 1ull) op->flip_sites.push_back(64 * w + bpos);
         op->nflip[n] = static_cast<int>(op->flip_sites.size()) - op->flip_off[n];
         if (op->nflip[n] > 0) op->offdiag_slot[n] = op->num_offdiag++;
+    }
+    {
+        std::vector<char> seen(64 * kMaxWords, 0);
+        op->single_flips = op->num_offdiag > 0;
+        for (int n = 0; n < op->S && op->single_flips; n++) {
+            if (op->nflip[n] == 0) continue;
+            char& site = seen[op->flip_sites[op->flip_off[n]]];
+            if (op->nflip[n] > 1 || site) op->single_flips = false;
+            site = 1;
+        }
     }
     if (op->flip_sites.empty()) op->flip_sites.push_back(0);
     auto up = [](DevBuf& d, const void* h, size_t bytes) -> cudaError_t {
@@ -1269,8 +1279,20 @@ static int ev_gradient_sums(const rbmg_psi* psi, const rbmg_operator* op, rbmg_e
             }
             RBMG_CK(W.T.ensure(sizeof(float2) * c.count * psi->Mpad));
             RBMG_CK(W.U.ensure(sizeof(float2) * c.count * psi->Mpad));
-            RBMG_CK(W.X.ensure(sizeof(float2) * std::max<size_t>(1, size_t(c.count) * op->num_offdiag * psi->Mpad)));
+            // a transverse field (each string one site's own): the strings' terms e_n are formed
+            // first, then U and the V sums from the stored angles; otherwise e_n tanh(theta''_n)
+            // of every string and sample is stored.  The fluctuation gradient's second V sum has
+            // the stored form only
+            const bool single = op->single_flips && !fluct;
             EstLaunch L{};
+            if (single) {
+                RBMG_CK(W.theta.ensure(sizeof(float2) * c.count * psi->Mpad));
+                RBMG_CK(W.en.ensure(sizeof(float2) * size_t(c.count) * op->num_offdiag));
+                L.theta = W.theta.as<float2>();
+                L.en = W.en.as<float2>();
+            } else {
+                RBMG_CK(W.X.ensure(sizeof(float2) * std::max<size_t>(1, size_t(c.count) * op->num_offdiag * psi->Mpad)));
+            }
             L.count = c.count;
             L.enum_base = c.enum_base;
             L.spins = c.spins;
@@ -1286,6 +1308,27 @@ static int ev_gradient_sums(const rbmg_psi* psi, const rbmg_operator* op, rbmg_e
             RBMG_CK(launch_coef(c.count, c.weights, nullptr, 1.0, W.coef1.as<double2>(), stream()));
             RBMG_CK(launch_coef(c.count, c.weights, W.eloc.as<double2>(), 1.0, W.coef2.as<double2>(), stream(),
                                 make_double2(E0.real(), E0.imag())));
+            if (single) {
+                RBMG_CK(W.vpart.ensure(grad_vectors_bytes(c.count, N, psi->M, kSplits)));
+                GradVectors G{};
+                G.count = c.count;
+                G.N = N;
+                G.nw = nw;
+                G.M = psi->M;
+                G.Mpad = psi->Mpad;
+                G.spins = c.spins;
+                G.enum_base = c.enum_base;
+                G.enumerate = c.enumerate;
+                G.w = c.weights;
+                G.W = psi->dW.as<float2>();
+                G.theta = L.theta;
+                G.T = L.T;
+                G.en = L.en;
+                G.U = W.U.as<float2>();
+                G.e_shift = make_float2(static_cast<float>(E0.real()), static_cast<float>(E0.imag()));
+                G.site_ptr = op->d_site_ptr.as<int>();
+                RBMG_CK(launch_grad_vectors(G, od, W.acc_Ek.as<double2>(), W.vpart.as<double2>(), kSplits, stream()));
+            }
             double2* part = W.partial.as<double2>();
             RBMG_CK(launch_outer_reduce(c.count, N, nw, psi->M, c.spins, c.enum_base, c.enumerate,
                                         W.coef1.as<double2>(), W.T.as<float2>(), psi->Mpad, 0,
@@ -1296,10 +1339,11 @@ static int ev_gradient_sums(const rbmg_psi* psi, const rbmg_operator* op, rbmg_e
             RBMG_CK(launch_outer_reduce(c.count, N, nw, psi->M, c.spins, c.enum_base, c.enumerate,
                                         W.coef1.as<double2>(), W.U.as<float2>(), psi->Mpad, 0,
                                         W.acc_Ek.as<double2>(), part, kSplits, stream()));
-            RBMG_CK(launch_vterm_reduce(c.count, N, nw, psi->M, psi->Mpad, c.spins, c.enum_base, c.enumerate,
-                                        c.weights, W.X.as<float2>(), op->num_offdiag, op->d_site_ptr.as<int>(),
-                                        op->d_site_slots.as<int>(), W.acc_Ek.as<double2>(), part, kSplits,
-                                        stream()));
+            if (!single)
+                RBMG_CK(launch_vterm_reduce(c.count, N, nw, psi->M, psi->Mpad, c.spins, c.enum_base, c.enumerate,
+                                            c.weights, W.X.as<float2>(), op->num_offdiag, op->d_site_ptr.as<int>(),
+                                            op->d_site_slots.as<int>(), W.acc_Ek.as<double2>(), part, kSplits,
+                                            stream()));
             if (adjoint) {
                 RBMG_CK(launch_outer_reduce(c.count, N, nw, psi->M, c.spins, c.enum_base, c.enumerate,
                                             W.coef2.as<double2>(), W.T.as<float2>(), psi->Mpad, 0,

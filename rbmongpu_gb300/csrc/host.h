@@ -143,6 +143,7 @@ struct rbmg_operator {
     std::vector<uint64_t> zmask;
     int num_offdiag = 0;
     int max_site = -1;
+    bool single_flips = false;   // every off-diagonal string flips one site, no two the same
     rbmg::DevBuf d_coef, d_coef32, d_site1, d_next1, d_ypow, d_zmask, d_nflip, d_flip_off, d_flip_sites, d_slot;
     rbmg::DevBuf d_offdiag;
     // per-site CSR of the off-diagonal slots whose string flips the site (E_k term)

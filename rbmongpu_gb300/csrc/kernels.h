@@ -91,6 +91,10 @@ struct EstLaunch {
     double2* logpsi_prime;      // [count]
     float2* Tp;                 // [count][Mpad'] tanh of psi' angles
     double2 e_shift;            // U is stored as U - e_shift * T (centred E_k sums)
+    // EST_GRADVEC of a single-flip operator: the angles and the off-diagonal strings' terms in
+    // place of U and X, which launch_grad_vectors forms (null: the general form above)
+    float2* theta;              // [count][Mpad]
+    float2* en;                 // [count][num_offdiag]
 };
 
 // PsiDeep net on the device (include/quantum_state/PsiDeep.hpp:38-84): per layer the

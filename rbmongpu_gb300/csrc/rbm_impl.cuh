@@ -745,6 +745,116 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) rbm_est_kernel(RbmDev P, 
 }
 
 // ---------------------------------------------------------------------------
+// The gradient's per-sample pass for an operator whose off-diagonal strings flip one site each
+// (EstLaunch::en): T = tanh(theta), the angles, every string's term e_n and the local energy.
+// One warp per configuration, lanes over the hidden units, as rbm_est_kernel; bound by the FP32
+// pipe.  Eight strings at a time, two of them in the halves of each packed operation, and their
+// lane sums folded in one butterfly; the exponentials of 32 strings run in the 32 lanes at once
+// (they took as long as a unit's activation in every lane before).  Each string's arithmetic
+// and the order of the energy's sum are rbm_est_kernel's, so the values are the same.
+// N = 64, M = 128, 64 + 128 strings, 4096 samples: 70 us, and 178 us for launch_grad_vectors,
+// against 263 us of rbm_est_kernel and 354 us of the sums over its stored terms.
+// ---------------------------------------------------------------------------
+template <int K, int NW>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock) rbm_grad_terms_kernel(RbmDev P, OpDev op, EstLaunch L) {
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const long t = static_cast<long>(blockIdx.x) * kWarpsPerBlock + wib;
+    __shared__ float2 terms_sm[kWarpsPerBlock][32];
+    if (t >= L.count) return;
+    float2* terms = terms_sm[wib];
+    Spins<NW> s;
+    if (L.flags & EST_ENUMERATE) {
+        const uint64_t idx = L.enum_base + static_cast<uint64_t>(t);
+        s.w[0] = P.N >= 64 ? idx : (idx & ((1ull << P.N) - 1ull));
+#pragma unroll
+        for (int k = 1; k < NW; k++) s.w[k] = 0;
+    } else {
+#pragma unroll
+        for (int k = 0; k < NW; k++) s.w[k] = L.spins[t * NW + k];
+    }
+    float tr[K], ti[K];
+    float2 f[K];
+    rbm_refresh(P, s, tr, ti, lane);
+    const long row = t * P.Mpad + lane;
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        float2 th;
+        lc_tanh_approx(tr[k], ti[k], f[k], th);
+        L.T[row + 32 * k] = th;
+        L.theta[row + 32 * k] = make_float2(tr[k], ti[k]);
+    }
+    // lanes 0 and 1: the compensated sums of the terms' real and imaginary parts (KahanC)
+    float ks = 0.0f, kc = 0.0f;
+    for (int n0 = 0; n0 < op.S; n0 += 32) {
+        const int n = n0 + lane;
+        const bool live = n < op.S;
+        const float2 cf = live ? string_factor(op, n, s) : make_float2(0.0f, 0.0f);
+        const bool flips = live && op.nflip[n] != 0;
+        const unsigned off = __ballot_sync(0xffffffffu, flips);
+        const int rank = __popc(off & ((1u << lane) - 1u));
+        float2 d = make_float2(0.0f, 0.0f);
+        unsigned m = off;
+        for (int b = 0; m; b++) {
+            const float2* wrow[8];
+            float two_s[8];
+            int site = 0;
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                if (m) {
+                    site = op.flip_sites[op.flip_off[n0 + __ffs(m) - 1]];
+                    m &= m - 1;
+                }
+                two_s[u] = s.up(site) ? -2.0f : 2.0f;
+                wrow[u] = P.W + static_cast<long>(site) * P.Mpad + lane;
+            }
+            pair_t pr[4], pi[4];
+#pragma unroll
+            for (int v = 0; v < 4; v++) pr[v] = pi[v] = splat2(0.0f);
+#pragma unroll
+            for (int k = 0; k < K; k++) {
+#pragma unroll
+                for (int v = 0; v < 4; v++) {
+                    const float2 wa = __ldg(wrow[2 * v] + 32 * k), wb = __ldg(wrow[2 * v + 1] + 32 * k);
+                    const pair_t ts = pk2(two_s[2 * v], two_s[2 * v + 1]);
+                    const Pair2 g = lc_c2_approx(fma2(ts, pk2(wa.x, wb.x), splat2(tr[k])),
+                                                 fma2(ts, pk2(wa.y, wb.y), splat2(ti[k])));
+                    pr[v] = add2(pr[v], sub2(g.re, splat2(f[k].x)));
+                    pi[v] = add2(pi[v], sub2(g.im, splat2(f[k].y)));
+                }
+            }
+            float2 part[8];
+#pragma unroll
+            for (int v = 0; v < 4; v++) {
+                up2(pr[v], part[2 * v].x, part[2 * v + 1].x);
+                up2(pi[v], part[2 * v].y, part[2 * v + 1].y);
+            }
+            const float2 sum = warp_fold8(part, lane);
+            const float dx = __shfl_sync(0xffffffffu, sum.x, 4 * (rank & 7));
+            const float dy = __shfl_sync(0xffffffffu, sum.y, 4 * (rank & 7));
+            if (rank >> 3 == b) d = make_float2(dx, dy);
+        }
+        float2 e = cf;
+        if (flips) {
+            e = string_term(cf, d);
+            L.en[t * op.num_offdiag + op.offdiag_slot[n]] = e;
+        }
+        terms[lane] = e;
+        __syncwarp();
+        const int cnt = min(32, op.S - n0);
+        if (lane < 2) {
+            const float* v = reinterpret_cast<const float*>(terms) + lane;
+            for (int i = 0; i < cnt; i++) {
+                const float y = __fsub_rn(v[2 * i], kc), z = __fadd_rn(ks, y);
+                kc = __fsub_rn(__fsub_rn(z, ks), y);
+                ks = z;
+            }
+        }
+        __syncwarp();
+    }
+    if (lane < 2) reinterpret_cast<double*>(L.eloc + t)[lane] = static_cast<double>(ks) - static_cast<double>(kc);
+}
+
+// ---------------------------------------------------------------------------
 // Local energies only (the measurement of a chain step, Operator.hpp:90-115), the lanes
 // over the strings: one warp per configuration; its angles
 // and f(theta) sit in the warp's shared-memory slice, and every lane evaluates the whole
@@ -939,6 +1049,16 @@ cudaError_t rbm_est_launch_k(const RbmDev& P, const OpDev* op, const RbmDev* PP,
             case 2: rbm_eloc_t_kernel<K, 2><<<grid, block, 0, st>>>(P, o, L); break;
             case 3: rbm_eloc_t_kernel<K, 3><<<grid, block, 0, st>>>(P, o, L); break;
             case 4: rbm_eloc_t_kernel<K, 4><<<grid, block, 0, st>>>(P, o, L); break;
+            default: return cudaErrorInvalidValue;
+        }
+        return cudaGetLastError();
+    }
+    if (L.en) {
+        switch (nw) {
+            case 1: rbm_grad_terms_kernel<K, 1><<<grid, block, 0, st>>>(P, o, L); break;
+            case 2: rbm_grad_terms_kernel<K, 2><<<grid, block, 0, st>>>(P, o, L); break;
+            case 3: rbm_grad_terms_kernel<K, 3><<<grid, block, 0, st>>>(P, o, L); break;
+            case 4: rbm_grad_terms_kernel<K, 4><<<grid, block, 0, st>>>(P, o, L); break;
             default: return cudaErrorInvalidValue;
         }
         return cudaGetLastError();

@@ -4,6 +4,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "kernels.h"
+
 namespace rbmg {
 
 constexpr int kMaxSeries = 6;
@@ -25,6 +27,26 @@ cudaError_t launch_vterm_reduce(int count, int N, int nw, int M, int Mpad, const
                                 int enumerate, const double* w, const float2* X, int num_offdiag,
                                 const int* site_ptr, const int* site_slots, double2* out, double2* partial,
                                 int max_splits, cudaStream_t st, const double2* cw = nullptr);
+// U [count][Mpad] (EstLaunch) and the V sums of launch_vterm_reduce for an operator whose
+// off-diagonal strings flip one site each, no two the same, from the strings' terms `en`
+// [count][num_offdiag] and the angles `theta` [count][Mpad]; partial: grad_vectors_bytes
+struct GradVectors {
+    int count, N, nw, M, Mpad;
+    const uint64_t* spins;
+    uint64_t enum_base;
+    int enumerate;
+    const double* w;
+    const float2* W;      // [N][Mpad]
+    const float2* theta;
+    const float2* T;      // [count][Mpad] tanh(theta)
+    const float2* en;
+    float2* U;
+    float2 e_shift;       // U is stored as U - e_shift T
+    const int* site_ptr;  // [N + 1]
+};
+size_t grad_vectors_bytes(int count, int N, int M, int max_splits);
+cudaError_t launch_grad_vectors(const GradVectors& g, const OpDev& op, double2* out, double2* partial, int max_splits,
+                                cudaStream_t st);
 // sums[q] += sum_s w[s] v_q[s]; block_scratch: kSumBlocks * kMaxSeries double2
 cudaError_t launch_weighted_sums(int count, const double* w, const SeriesSet& set, double2* block_scratch,
                                  double2* sums, cudaStream_t st);

@@ -4,6 +4,7 @@
 // most 32 samples, accumulated in FP64, then per-block partials combined by a
 // second kernel in block order.  No floating-point atomics, so results are
 // bit-reproducible run to run.
+#include "device_math.cuh"
 #include "kernels.h"
 #include "reduce.h"
 
@@ -153,6 +154,193 @@ __global__ void vterm_kernel(int count, int N, int nw, int M, int Mpad, const ui
     if (warp == 0 && i == 0 && j < M) {
         const long plane = static_cast<long>(1 + N) * M;
         partial[blockIdx.z * plane + j] = make_double2(0.0, 0.0);   // row 0 carries no V term
+    }
+}
+
+// U and the V sums of a single-flip operator from the angles and the terms e_n (GradVectors).
+// tanh(theta'') is evaluated again here instead of being stored by the pass that forms the e_n:
+// per sample and string that is a second activation of every unit against 16 bytes written and
+// read (268 MB a 4096-sample chunk at N = 64, M = 128).
+// Warp q of the block takes samples z per_split + q + 8 k of split z (k < 32 of chunk c), its
+// lanes 32 hidden units: vterm_kernel's FP32 groups, summed in its order.  The strings go by
+// eight in the operator's order, so that every U_j is the same ordered sum; a block's terms and
+// signs are staged in shared memory, two samples side by side for the packed operations.  A
+// thread holds eight V sums; its samples' U are in shared memory between blocks of strings.
+// Bound by the FP32 pipe (57 lane operations per sample, string and unit; 42 % busy) and the
+// latency of the staging: 178 us a chunk, against 354 us of vterm_kernel on stored terms.
+constexpr int kGvStrings = 8, kGvTile = 8, kGvWarps = 8;
+
+// ONE: a lane of the general pass holds one hidden unit (Mpad = 32); its compiled form joins the
+// other product of Im(e tanh) into an FMA than with more units, and so does this one.
+template <bool ONE>
+__global__ void __launch_bounds__(32 * kGvWarps) grad_vectors_kernel(GradVectors g, OpDev op, int per_split,
+                                                                     int chunks, int cap, double2* partial) {
+    extern __shared__ __align__(16) unsigned char gv_smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int pairs = cap / 2;
+    // [warp][string][pair] (ex0, ex1, ey0, ey1) and (2 s'0, 2 s'1, g0, g1)
+    float4* stA = reinterpret_cast<float4*>(gv_smem) + warp * 2 * kGvStrings * pairs;
+    float4* stB = stA + kGvStrings * pairs;
+    float2* red = reinterpret_cast<float2*>(reinterpret_cast<float4*>(gv_smem) + kGvWarps * 2 * kGvStrings * pairs);
+    pair_t* us = reinterpret_cast<pair_t*>(red + kGvStrings * kGvWarps * 32) + warp * 2 * pairs * 32 + lane;
+    const int j = blockIdx.x * 32 + lane;
+    const int z = blockIdx.y / chunks, c = blockIdx.y - z * chunks;
+    const int s_end = min(g.count, (z + 1) * per_split);
+    const int s0 = z * per_split + warp + 8 * 32 * c;
+    const int cnt = s0 < s_end ? min(32, (s_end - s0 + 7) / 8) : 0;   // sample k of the warp: s0 + 8 k
+    for (int q = 0; q < pairs; q++) us[(2 * q) * 32] = us[(2 * q + 1) * 32] = splat2(0.0f);
+    const int nw = g.nw;
+    auto word = [&](int s, int k) -> uint64_t {
+        if (!g.enumerate) return k < nw ? g.spins[static_cast<long>(s) * nw + k] : 0ull;
+        if (k != 0) return 0ull;
+        const uint64_t idx = g.enum_base + static_cast<uint64_t>(s);
+        return g.N >= 64 ? idx : (idx & ((1ull << g.N) - 1ull));
+    };
+    auto load = [&](const float2* a, int k) {
+        return k < cnt ? a[static_cast<long>(s0 + 8 * k) * g.Mpad + j] : make_float2(0.0f, 0.0f);
+    };
+    double2* out = partial + static_cast<long>(blockIdx.y) * (1 + g.N) * g.M;
+    for (int i = warp; i <= g.N; i += kGvWarps)   // the rows no string writes
+        if (j < g.M && (i == 0 || g.site_ptr[i - 1] == g.site_ptr[i])) out[static_cast<long>(i) * g.M + j] = make_double2(0.0, 0.0);
+    for (int n0 = 0; n0 < op.S;) {
+        // up to eight consecutive strings of one kind
+        const bool diag = op.nflip[n0] == 0;
+        int nb = 1;
+        while (nb < kGvStrings && n0 + nb < op.S && (op.nflip[n0 + nb] == 0) == diag) nb++;
+        __syncwarp();
+        for (int e = lane; e < kGvStrings * 2 * pairs; e += 32) {
+            const int u = e % kGvStrings, k = e / kGvStrings, n = n0 + u;
+            float2 en = make_float2(0.0f, 0.0f);
+            float ts = 0.0f, gw = 0.0f;
+            if (u < nb && k < cnt) {
+                const int s = s0 + 8 * k;
+                if (diag) {
+                    // string_factor of this sample
+                    int parity = 0;
+                    for (int q = 0; q < nw; q++) parity += __popcll(op.zmask[n * kMaxWords + q] & ~word(s, q));
+                    const float2 cf = op.coef32[n];
+                    const int yp = op.ypow[n] & 3;
+                    en = yp == 0 ? cf : (yp == 1 ? make_float2(cf.y, -cf.x)
+                                                 : (yp == 2 ? make_float2(-cf.x, -cf.y) : make_float2(-cf.y, cf.x)));
+                    if (parity & 1) en = make_float2(-en.x, -en.y);
+                } else {
+                    const int site = op.flip_sites[op.flip_off[n]];
+                    const bool up = (word(s, site >> 6) >> (site & 63)) & 1ull;
+                    en = g.en[static_cast<long>(s) * op.num_offdiag + op.offdiag_slot[n]];
+                    ts = up ? -2.0f : 2.0f;
+                    gw = (up ? 1.0f : -1.0f) * (g.w ? static_cast<float>(g.w[s]) : 1.0f);
+                }
+            }
+            float* a = reinterpret_cast<float*>(stA + u * pairs + (k >> 1)) + (k & 1);
+            float* b = reinterpret_cast<float*>(stB + u * pairs + (k >> 1)) + (k & 1);
+            a[0] = en.x;
+            a[2] = en.y;
+            b[0] = ts;
+            b[2] = gw;
+        }
+        __syncwarp();
+        if (diag) {
+            for (int k0 = 0; k0 < cnt; k0 += kGvTile) {
+#pragma unroll
+                for (int v = 0; v < kGvTile / 2; v++) {
+                    const int q = (k0 >> 1) + v;
+                    if (q >= pairs) break;
+                    const float2 a0 = load(g.T, 2 * q), a1 = load(g.T, 2 * q + 1);
+                    const pair_t tx = pk2(a0.x, a1.x), ty = pk2(a0.y, a1.y);
+                    const pair_t nty = mul2(splat2(-1.0f), ty);
+                    pair_t ur = us[(2 * q) * 32], ui = us[(2 * q + 1) * 32];
+                    for (int u = 0; u < nb; u++) {
+                        const float4 e = stA[u * pairs + q];
+                        const pair_t ex = pk2(e.x, e.y), ey = pk2(e.z, e.w);
+                        ur = add2(ur, fma2(ex, tx, mul2(ey, nty)));
+                        ui = add2(ui, fma2(ex, ty, mul2(ey, tx)));
+                    }
+                    us[(2 * q) * 32] = ur;
+                    us[(2 * q + 1) * 32] = ui;
+                }
+            }
+        } else {
+            float2 w[kGvStrings], V[kGvStrings];
+#pragma unroll
+            for (int u = 0; u < kGvStrings; u++) {
+                w[u] = make_float2(0.0f, 0.0f);
+                V[u] = make_float2(0.0f, 0.0f);
+                if (u < nb)
+                    w[u] = __ldg(g.W + static_cast<long>(op.flip_sites[op.flip_off[n0 + u]]) * g.Mpad + j);
+            }
+            for (int k0 = 0; k0 < cnt; k0 += kGvTile) {
+                pair_t tr[kGvTile / 2], ti[kGvTile / 2], ur[kGvTile / 2], ui[kGvTile / 2];
+#pragma unroll
+                for (int v = 0; v < kGvTile / 2; v++) {
+                    const int q = min((k0 >> 1) + v, pairs - 1);
+                    const float2 a0 = load(g.theta, k0 + 2 * v), a1 = load(g.theta, k0 + 2 * v + 1);
+                    tr[v] = pk2(a0.x, a1.x);
+                    ti[v] = pk2(a0.y, a1.y);
+                    ur[v] = us[(2 * q) * 32];
+                    ui[v] = us[(2 * q + 1) * 32];
+                }
+#pragma unroll
+                for (int u = 0; u < kGvStrings; u++) {
+                    if (u >= nb) break;
+                    const pair_t wx = splat2(w[u].x), wy = splat2(w[u].y);
+#pragma unroll
+                    for (int v = 0; v < kGvTile / 2; v++) {
+                        const int q = min((k0 >> 1) + v, pairs - 1);
+                        const float4 e = stA[u * pairs + q], b = stB[u * pairs + q];
+                        const pair_t ts = pk2(b.x, b.y);
+                        const Pair2 h = tanh2_approx(fma2(ts, wx, tr[v]), fma2(ts, wy, ti[v]));
+                        const pair_t ex = pk2(e.x, e.y), ey = pk2(e.z, e.w);
+                        const pair_t vx = fma2(ex, h.re, mul2(splat2(-1.0f), mul2(ey, h.im)));
+                        const pair_t vy = ONE ? fma2(ex, h.im, mul2(ey, h.re)) : fma2(ey, h.re, mul2(ex, h.im));
+                        ur[v] = add2(ur[v], vx);
+                        ui[v] = add2(ui[v], vy);
+                        if (k0 + 2 * v < cnt) {
+                            float x0, x1, y0, y1;
+                            up2(vx, x0, x1);
+                            up2(vy, y0, y1);
+                            V[u].x = fmaf(b.z, x0, V[u].x);
+                            V[u].y = fmaf(b.z, y0, V[u].y);
+                            V[u].x = fmaf(b.w, x1, V[u].x);
+                            V[u].y = fmaf(b.w, y1, V[u].y);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int v = 0; v < kGvTile / 2; v++) {
+                    const int q = (k0 >> 1) + v;
+                    if (q < pairs) {
+                        us[(2 * q) * 32] = ur[v];
+                        us[(2 * q + 1) * 32] = ui[v];
+                    }
+                }
+            }
+            __syncthreads();   // the previous block's sums have been read
+#pragma unroll
+            for (int u = 0; u < kGvStrings; u++) red[(u * kGvWarps + warp) * 32 + lane] = V[u];
+            __syncthreads();
+            if (warp < nb && j < g.M) {
+                double2 t = make_double2(0.0, 0.0);
+                for (int q = 0; q < kGvWarps; q++) {
+                    const float2 v = red[(warp * kGvWarps + q) * 32 + lane];
+                    t.x += v.x;
+                    t.y += v.y;
+                }
+                const int site = op.flip_sites[op.flip_off[n0 + warp]];
+                out[static_cast<long>(1 + site) * g.M + j] = t;
+            }
+        }
+        n0 += nb;
+    }
+    const float shx = g.e_shift.x, shy = g.e_shift.y;
+    for (int k = 0; k < cnt; k++) {
+        const float2 t = load(g.T, k);
+        float x[2], y[2];
+        up2(us[(2 * (k >> 1)) * 32], x[0], x[1]);
+        up2(us[(2 * (k >> 1) + 1) * 32], y[0], y[1]);
+        float2 u = make_float2(x[k & 1], y[k & 1]);
+        u.x -= __fmaf_rn(shx, t.x, -__fmul_rn(shy, t.y));
+        u.y -= __fmaf_rn(shx, t.y, __fmul_rn(shy, t.x));
+        g.U[static_cast<long>(s0 + 8 * k) * g.Mpad + j] = u;
     }
 }
 
@@ -318,6 +506,41 @@ cudaError_t launch_vterm_reduce(int count, int N, int nw, int M, int Mpad, const
                                        site_ptr, site_slots, partial, per_split);
     const long elems = static_cast<long>(1 + N) * M;
     finish_splits_kernel<<<grid_for(elems), 256, 0, st>>>(elems, splits, partial, out, -2.0);
+    return cudaGetLastError();
+}
+
+// vterm_kernel's split of the samples, and chunks of 32 samples a warp
+static void grad_vectors_shape(int count, int max_splits, int* per_split, int* splits, int* chunks, int* cap) {
+    *per_split = max(64, (count + max_splits - 1) / max_splits);
+    *splits = (count + *per_split - 1) / *per_split;
+    const int per_warp = (*per_split + 7) / 8;
+    *chunks = (per_warp + 31) / 32;
+    *cap = min(32, (per_warp + 1) / 2 * 2);
+}
+
+size_t grad_vectors_bytes(int count, int N, int M, int max_splits) {
+    int per_split, splits, chunks, cap;
+    grad_vectors_shape(count, max_splits, &per_split, &splits, &chunks, &cap);
+    return sizeof(double2) * static_cast<size_t>(splits) * chunks * (1 + N) * M;
+}
+
+cudaError_t launch_grad_vectors(const GradVectors& g, const OpDev& op, double2* out, double2* partial, int max_splits,
+                                cudaStream_t st) {
+    if (g.count <= 0) return cudaSuccess;
+    int per_split, splits, chunks, cap;
+    grad_vectors_shape(g.count, max_splits, &per_split, &splits, &chunks, &cap);
+    const size_t sm = sizeof(float4) * kGvWarps * kGvStrings * cap + sizeof(float2) * kGvStrings * kGvWarps * 32 +
+                      sizeof(pair_t) * kGvWarps * 32 * cap;
+    const auto kernel = g.Mpad == 32 ? grad_vectors_kernel<true> : grad_vectors_kernel<false>;
+    if (sm > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   static_cast<int>(sm));
+        if (e != cudaSuccess) return e;
+    }
+    const dim3 grid(g.Mpad / 32, splits * chunks);
+    kernel<<<grid, 32 * kGvWarps, sm, st>>>(g, op, per_split, chunks, cap, partial);
+    const long elems = static_cast<long>(1 + g.N) * g.M;
+    finish_splits_kernel<<<grid_for(elems), 256, 0, st>>>(elems, splits * chunks, partial, out, -2.0);
     return cudaGetLastError();
 }
 
