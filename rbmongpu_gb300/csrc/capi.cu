@@ -1238,7 +1238,7 @@ static int ev_gradient_sums(const rbmg_psi* psi, const rbmg_operator* op, rbmg_e
         r = op_site_lists(const_cast<rbmg_operator*>(op), N);
         if (r != RBMG_OK) return r;
         per_sample = sizeof(float2) * psi->Mpad * (2 + op->num_offdiag) + 64;
-        RBMG_CK(W.partial.ensure(sizeof(double2) * kSplits * (1 + N) * psi->M));
+        RBMG_CK(W.partial.ensure(sizeof(double2) * kMaxOuter * kSplits * (1 + N) * psi->M));
     }
     const size_t max_chunk = psi->kind == 0 ? std::max<size_t>(256, (size_t(512) << 20) / per_sample) : 4096;
     // The sums are centred on E0, the mean local energy of the first chunk:
@@ -1330,43 +1330,39 @@ static int ev_gradient_sums(const rbmg_psi* psi, const rbmg_operator* op, rbmg_e
                 RBMG_CK(launch_grad_vectors(G, od, W.acc_Ek.as<double2>(), W.vpart.as<double2>(), kSplits, stream()));
             }
             double2* part = W.partial.as<double2>();
-            RBMG_CK(launch_outer_reduce(c.count, N, nw, psi->M, c.spins, c.enum_base, c.enumerate,
-                                        W.coef1.as<double2>(), W.T.as<float2>(), psi->Mpad, 0,
-                                        W.acc_O.as<double2>(), part, kSplits, stream()));
-            RBMG_CK(launch_outer_reduce(c.count, N, nw, psi->M, c.spins, c.enum_base, c.enumerate,
-                                        W.coef2.as<double2>(), W.T.as<float2>(), psi->Mpad, 1,
-                                        W.acc_EO.as<double2>(), part, kSplits, stream()));
-            RBMG_CK(launch_outer_reduce(c.count, N, nw, psi->M, c.spins, c.enum_base, c.enumerate,
-                                        W.coef1.as<double2>(), W.U.as<float2>(), psi->Mpad, 0,
-                                        W.acc_Ek.as<double2>(), part, kSplits, stream()));
+            // the sums over T, together: O, and (E - E0) O* or, for the adjoint, C2 and C3
+            OuterSet sums_t{}, sums_u{};
+            sums_t.add(W.coef1.as<double2>(), 0, W.acc_O.as<double2>());
+            if (adjoint) {
+                RBMG_CK(W.coef3.ensure(sizeof(double2) * c.count));
+                RBMG_CK(launch_coef_real(c.count, c.weights, W.eloc.as<double2>(), E0.real(), W.coef3.as<double2>(),
+                                         stream()));
+                sums_t.add(W.coef2.as<double2>(), 0, W.acc_C2.as<double2>());
+                sums_t.add(W.coef3.as<double2>(), 1, W.acc_C3.as<double2>());
+            } else {
+                sums_t.add(W.coef2.as<double2>(), 1, W.acc_EO.as<double2>());
+            }
+            RBMG_CK(launch_outer_reduce(c.count, N, nw, psi->M, c.spins, c.enum_base, c.enumerate, sums_t,
+                                        W.T.as<float2>(), psi->Mpad, part, kSplits, stream()));
+            sums_u.add(W.coef1.as<double2>(), 0, W.acc_Ek.as<double2>());
+            if (fluct) {
+                RBMG_CK(W.coef3.ensure(sizeof(double2) * c.count));
+                RBMG_CK(launch_coef_conj(c.count, c.weights, W.eloc.as<double2>(), make_double2(E0.real(), E0.imag()),
+                                         W.coef3.as<double2>(), stream()));
+                sums_u.add(W.coef3.as<double2>(), 0, W.acc_B.as<double2>());
+            }
+            RBMG_CK(launch_outer_reduce(c.count, N, nw, psi->M, c.spins, c.enum_base, c.enumerate, sums_u,
+                                        W.U.as<float2>(), psi->Mpad, part, kSplits, stream()));
             if (!single)
                 RBMG_CK(launch_vterm_reduce(c.count, N, nw, psi->M, psi->Mpad, c.spins, c.enum_base, c.enumerate,
                                             c.weights, W.X.as<float2>(), op->num_offdiag, op->d_site_ptr.as<int>(),
                                             op->d_site_slots.as<int>(), W.acc_Ek.as<double2>(), part, kSplits,
                                             stream()));
-            if (adjoint) {
-                RBMG_CK(launch_outer_reduce(c.count, N, nw, psi->M, c.spins, c.enum_base, c.enumerate,
-                                            W.coef2.as<double2>(), W.T.as<float2>(), psi->Mpad, 0,
-                                            W.acc_C2.as<double2>(), part, kSplits, stream()));
-                RBMG_CK(W.coef3.ensure(sizeof(double2) * c.count));
-                RBMG_CK(launch_coef_real(c.count, c.weights, W.eloc.as<double2>(), E0.real(), W.coef3.as<double2>(),
-                                         stream()));
-                RBMG_CK(launch_outer_reduce(c.count, N, nw, psi->M, c.spins, c.enum_base, c.enumerate,
-                                            W.coef3.as<double2>(), W.T.as<float2>(), psi->Mpad, 1,
-                                            W.acc_C3.as<double2>(), part, kSplits, stream()));
-            }
-            if (fluct) {
-                RBMG_CK(W.coef3.ensure(sizeof(double2) * c.count));
-                RBMG_CK(launch_coef_conj(c.count, c.weights, W.eloc.as<double2>(), make_double2(E0.real(), E0.imag()),
-                                         W.coef3.as<double2>(), stream()));
-                RBMG_CK(launch_outer_reduce(c.count, N, nw, psi->M, c.spins, c.enum_base, c.enumerate,
-                                            W.coef3.as<double2>(), W.U.as<float2>(), psi->Mpad, 0,
-                                            W.acc_B.as<double2>(), part, kSplits, stream()));
+            if (fluct)
                 RBMG_CK(launch_vterm_reduce(c.count, N, nw, psi->M, psi->Mpad, c.spins, c.enum_base, c.enumerate,
                                             nullptr, W.X.as<float2>(), op->num_offdiag, op->d_site_ptr.as<int>(),
                                             op->d_site_slots.as<int>(), W.acc_B.as<double2>(), part, kSplits,
                                             stream(), W.coef3.as<double2>()));
-            }
         }
         SeriesSet set{};
         set.n = 1;
@@ -1857,9 +1853,10 @@ extern "C" int rbmg_hsd_gradient(const rbmg_psi* psi, const rbmg_psi* pp, const 
                 L.logpsi_prime = W.logpsi.as<double2>();
                 L.Tp = W.T.as<float2>();
                 RBMG_CK(launch_rbm_estimate(pd, nullptr, &pd, L, stream()));
-                RBMG_CK(launch_outer_reduce(cnt, N, nw, pp->M, L.spins, L.enum_base, enumerate,
-                                            W.coef1.as<double2>() + base, W.T.as<float2>(), pp->Mpad, 1,
-                                            W.acc_wO.as<double2>(), W.partial.as<double2>(), kSplits, stream()));
+                OuterSet set{};
+                set.add(W.coef1.as<double2>() + base, 1, W.acc_wO.as<double2>());
+                RBMG_CK(launch_outer_reduce(cnt, N, nw, pp->M, L.spins, L.enum_base, enumerate, set,
+                                            W.T.as<float2>(), pp->Mpad, W.partial.as<double2>(), kSplits, stream()));
             }
         } else {
             const int rr = deep_hsd_okreduce(pp, passes == 2 ? pass : -1, count, sp, 0, enumerate,
@@ -1990,9 +1987,10 @@ extern "C" int rbmg_kl_gradient(const rbmg_psi* psi, const rbmg_psi* pp, rbmg_en
             L.logpsi_prime = W.logpsi_p.as<double2>();
             L.Tp = W.T.as<float2>();
             RBMG_CK(launch_rbm_estimate(pd, nullptr, &pd, L, stream()));
-            RBMG_CK(launch_outer_reduce(cnt, N, nw, pp->M, L.spins, L.enum_base, enumerate,
-                                        W.coef1.as<double2>() + base, W.T.as<float2>(), pp->Mpad, 1,
-                                        W.acc_wO.as<double2>(), W.partial.as<double2>(), kSplits, stream()));
+            OuterSet set{};
+            set.add(W.coef1.as<double2>() + base, 1, W.acc_wO.as<double2>());
+            RBMG_CK(launch_outer_reduce(cnt, N, nw, pp->M, L.spins, L.enum_base, enumerate, set, W.T.as<float2>(),
+                                        pp->Mpad, W.partial.as<double2>(), kSplits, stream()));
         }
     } else {
         const int rr = deep_hsd_okreduce(pp, -1, count, sp, 0, enumerate, W.coef1.as<double2>(),

@@ -16,11 +16,24 @@ struct SeriesSet {
     const double2* v[kMaxSeries];
 };
 
-// out[r][j] += sum_s c[s] f(A[s][j]) g_r(s), g_0 = 1, g_{1+i} = s_i; f = conj if conj_a.
-// partial: scratch of max_splits * (1+N) * M double2.
+// up to kMaxOuter sums over the same rows A: out_q[r][j] += sum_s c_q[s] f_q(A[s][j]) g_r(s),
+// g_0 = 1, g_{1+i} = s_i; f_q = conj if conj_q.  partial: scratch of
+// n * max_splits * (1+N) * M double2.
+constexpr int kMaxOuter = 3;
+struct OuterSet {
+    int n;
+    const double2* c[kMaxOuter];
+    int conj[kMaxOuter];
+    double2* out[kMaxOuter];
+    void add(const double2* coef, int conjugate, double2* sum) {
+        c[n] = coef;
+        conj[n] = conjugate;
+        out[n++] = sum;
+    }
+};
 cudaError_t launch_outer_reduce(int count, int N, int nw, int M, const uint64_t* spins, uint64_t enum_base,
-                                int enumerate, const double2* c, const float2* A, int lda, int conj_a, double2* out,
-                                double2* partial, int max_splits, cudaStream_t st);
+                                int enumerate, const OuterSet& set, const float2* A, int lda, double2* partial,
+                                int max_splits, cudaStream_t st);
 // out[1+i][j] += -2 sum_s w[s] s_i sum_{slots of site i} X[s][slot][j]; with cw the per-sample
 // coefficient is the complex cw[s] (w ignored)
 cudaError_t launch_vterm_reduce(int count, int N, int nw, int M, int Mpad, const uint64_t* spins, uint64_t enum_base,
