@@ -79,6 +79,7 @@ struct rbmg_psi {
     int M = 0, Mpad = 0;
     std::vector<rbmg::cplx> b, W;
     rbmg::DevBuf dW, db, dWq, dbq;     // complex64 rows, and the sampler's paired copies (kernels.h)
+    rbmg::DevBuf dWg, dbg;             // paired copies of the grouped sampler (RbmDev::Wg)
     rbmg::DevBuf dWt;                  // W transposed, units paired [Mpad / 2][N] (RbmDev::Wt4)
     rbmg::DevBuf dWtc;                 // W as BF16 hi / mid / lo tensor-core operands (angles_tc.cu), if supported
     rbmg::DevBuf tc_error;             // set when a tensor-core pass of this psi gave up waiting
@@ -103,7 +104,8 @@ struct rbmg_psi {
     rbmg::RbmDev rbm_dev() const {
         return rbmg::RbmDev{N, M, Mpad, static_cast<const float2*>(dW.p), static_cast<const float2*>(db.p),
                             static_cast<const float4*>(dWq.p), static_cast<const float4*>(dbq.p),
-                            static_cast<const float4*>(dWt.p)};
+                            static_cast<const float4*>(dWt.p), static_cast<const float4*>(dWg.p),
+                            static_cast<const float4*>(dbg.p)};
     }
 };
 

@@ -45,6 +45,20 @@ __global__ void rbm_pairs_kernel(int N, int Mpad, int KP, const float2* W, const
     (row < N ? Wq[idx] : bq[rem]) = make_float4(a.x, c.x, a.y, c.y);
 }
 
+// Wg [N][K H][G], bg [K H][G] (kernels.h); row N is the bias
+__global__ void rbm_group_pairs_kernel(int N, int Mpad, int G, const float2* W, const float2* b, float4* Wg,
+                                       float4* bg) {
+    const long idx = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int per_row = Mpad / 2;
+    if (idx >= static_cast<long>(N + 1) * per_row) return;
+    const int row = static_cast<int>(idx / per_row), rem = static_cast<int>(idx - static_cast<long>(row) * per_row);
+    const int g = rem % G, pp = rem / G, H = 16 / G;
+    const int j0 = 32 * (pp / H) + 2 * G * (pp % H) + g;
+    const float2* src = row < N ? W + static_cast<long>(row) * Mpad : b;
+    const float2 a = src[j0], c = src[j0 + G];
+    (row < N ? Wg[idx] : bg[rem]) = make_float4(a.x, c.x, a.y, c.y);
+}
+
 // Wt4 [Mpad / 2][N]: entry (p, i) = (x_j, x_j+4, y_j, y_j+4) of W[i], j = 8 (p / 4) + p % 4
 __global__ void rbm_transpose_kernel(int N, int Mpad, const float2* W, float4* Wt4) {
     const long idx = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -56,11 +70,16 @@ __global__ void rbm_transpose_kernel(int N, int Mpad, const float2* W, float4* W
 }
 
 cudaError_t launch_rbm_pairs(int N, int Mpad, const float2* W, const float2* b, float4* Wq, float4* bq,
-                             float4* Wt, cudaStream_t st) {
+                             float4* Wt, float4* Wg, float4* bg, cudaStream_t st) {
     const int KP = (Mpad / 32 + 1) / 2;
     const long n = static_cast<long>(N + 1) * KP * 32;
     rbm_pairs_kernel<<<static_cast<int>((n + 255) / 256), 256, 0, st>>>(N, Mpad, KP, W, b, Wq, bq);
     cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    const long q = static_cast<long>(N + 1) * (Mpad / 2);
+    rbm_group_pairs_kernel<<<static_cast<int>((q + 255) / 256), 256, 0, st>>>(N, Mpad, rbm_group(Mpad / 32), W, b, Wg,
+                                                                              bg);
+    e = cudaGetLastError();
     if (e != cudaSuccess || !Wt) return e;
     const long m = static_cast<long>(N) * (Mpad / 2);
     rbm_transpose_kernel<<<static_cast<int>((m + 255) / 256), 256, 0, st>>>(N, Mpad, W, Wt);

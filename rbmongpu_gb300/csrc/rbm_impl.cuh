@@ -620,6 +620,175 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, 6) rbm_mc_smem_kernel(Rbm
     }
 }
 
+// ---------------------------------------------------------------------------
+// The sampler with several walkers per warp: G lanes share a walker (rbm_group), each with
+// PP = 16 K / G pairs of hidden units.  What a proposal does once per walker -- the random words,
+// the site, the last steps of the lane sum, the exponential, the test -- was 65 % of the warp's
+// instructions at K = 4 (273 a proposal, 96 of them activations) and now serves 32 / G walkers.
+// Lane g holds what lanes g, g + G, g + 2 G, ... of the one-walker kernel hold: their partial
+// sums stay apart until they meet in the order of its butterfly (offsets 16, 8, ... down to G
+// within the lane, the rest by shuffles), so angles, sums and decisions are the same bit for bit.
+// Bound by the FP32 pipe (16384 walkers: its floor is half of the time) and, with few walkers,
+// by one proposal's latency.  Microseconds a sweep with one walker a warp and grouped: N = 24,
+// M = 24: 12 / 10 at 16 walkers, 29 / 13 at 4096, 92 / 32 at 16384; N = 32, M = 64: 16 / 13,
+// 38 / 24, 124 / 76; N = 64, M = 128: 33 / 32, 97 / 72, 344 / 233.  Blocks of one, two or four
+// warps and keeping the proposed angles measured alike; G = 8 at K = 2 and 4 (G = 4 at K = 1)
+// was slower up to 4096 walkers (K = 4: 33 / 57 at 16, 97 / 75) and gained 6 % at 16384.
+// ---------------------------------------------------------------------------
+template <int K, int G, int NW, bool SZ>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, 4) rbm_mc_group_kernel(RbmDev P, McLaunch L) {
+    constexpr int H = 16 / G, PP = K * H, PW = 32 / G;   // PW walkers per warp
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, g = lane % G;
+    const int w0 = (blockIdx.x * kWarpsPerBlock + wib) * PW;
+    if (w0 >= L.B) return;
+    const int w = min(w0 + lane / G, L.B - 1);
+    const bool live = w0 + lane / G < L.B;   // a group past the end repeats the last walker, unwritten
+    __shared__ uint4 words_sm[kWarpsPerBlock][32];
+    GroupRng<G> rng;
+    const uint64_t nmagic = fastmod_magic(static_cast<uint32_t>(P.N));
+    Spins<NW> s;
+    {
+        uint64_t start = L.rng_index[w];
+        if (L.init) {
+            WalkerRng r;   // the lanes of a group draw the same words, groups go their own way
+            r.init(L.seed, L.walker_base + static_cast<uint32_t>(w), start);
+#pragma unroll
+            for (int k = 0; k < NW; k++) s.w[k] = 0;
+            if (SZ) s.w[0] = draw_n_over_k(r, P.N, static_cast<unsigned>((L.sector + P.N) / 2));
+            else draw_spins(r, P.N, s);
+            start = r.index;
+        } else {
+#pragma unroll
+            for (int k = 0; k < NW; k++) s.w[k] = L.spins[static_cast<long>(w) * NW + k];
+        }
+        __syncwarp();
+        rng.init(L.seed, L.walker_base + static_cast<uint32_t>(w), start, words_sm[wib] + (lane - g), g);
+    }
+    pair_t tr[PP], ti[PP], re[PP];
+    unsigned long long acc = 0, props = 0;
+    const int total_sweeps = L.n_therm + L.n_samples * L.sweeps_per_sample;
+    int sample = 0;
+    for (int sw = 0; sw < total_sweeps; sw++) {
+        // angles from the spins
+#pragma unroll
+        for (int p = 0; p < PP; p++) {
+            const float4 b = __ldg(P.bg + p * G + g);
+            tr[p] = pk2(b.x, b.y);
+            ti[p] = pk2(b.z, b.w);
+        }
+        const float4* row = P.Wg + g;
+        for (int i = 0; i < P.N; i++, row += PP * G) {
+            const pair_t sg = splat2(s.up(i) ? 1.0f : -1.0f);
+#pragma unroll
+            for (int p = 0; p < PP; p++) {
+                const float4 v = __ldg(row + p * G);
+                tr[p] = fma2(sg, pk2(v.x, v.y), tr[p]);   // sg = +-1: the products are exact
+                ti[p] = fma2(sg, pk2(v.z, v.w), ti[p]);
+            }
+        }
+#pragma unroll
+        for (int p = 0; p < PP; p++) re[p] = lc_re2(tr[p], ti[p]);
+        for (int prop = 0; prop < P.N; prop++) {
+            rng.ensure(2, g);
+            const int site = static_cast<int>(fastmod(rng.peek(), nmagic, static_cast<uint32_t>(P.N)));
+            rng.pos++;
+            Spins<NW> s2 = s;
+            s2.flip(site);
+            const bool first_new = s2.up(site);
+            const pair_t t0 = splat2(first_new ? 2.0f : -2.0f);
+            const float4* row0 = P.Wg + static_cast<long>(site) * PP * G + g;
+            pair_t t1 = t0;
+            const float4* row1 = row0;
+            if (SZ) {
+                // the partner: drawn until its spin equals the first site's new one
+                int sec = site;
+                bool found = false;
+                for (int guard = 0; guard < (1 << 20) && __any_sync(0xffffffffu, !found); guard++) {
+                    rng.ensure(1, g);
+                    if (!found) {
+                        const int c = static_cast<int>(fastmod(rng.peek(), nmagic, static_cast<uint32_t>(P.N)));
+                        rng.pos++;
+                        if ((c == site ? first_new : s.up(c)) == first_new) {
+                            sec = c;
+                            found = true;
+                        }
+                    }
+                }
+                s2.flip(sec);
+                t1 = splat2(s2.up(sec) ? 2.0f : -2.0f);
+                row1 = P.Wg + static_cast<long>(sec) * PP * G + g;
+                rng.ensure(1, g);
+            }
+            pair_t part[H], fnew[PP];
+#pragma unroll
+            for (int h = 0; h < H; h++) part[h] = splat2(0.0f);
+#pragma unroll
+            for (int p = 0; p < PP; p++) {
+                const float4 v = __ldg(row0 + p * G);
+                pair_t nr = fma2(t0, pk2(v.x, v.y), tr[p]), ni = fma2(t0, pk2(v.z, v.w), ti[p]);
+                if (SZ) {
+                    const float4 u = __ldg(row1 + p * G);
+                    nr = fma2(t1, pk2(u.x, u.y), nr);
+                    ni = fma2(t1, pk2(u.z, u.w), ni);
+                }
+                fnew[p] = lc_re2(nr, ni);
+                part[p % H] = add2(part[p % H], sub2(fnew[p], re[p]));
+            }
+            // the butterfly of the one-walker kernel: lanes l and l ^ off, off = 16, 8, 4, 2, 1
+#pragma unroll
+            for (int half = H / 2; half >= 1; half >>= 1)
+#pragma unroll
+                for (int h = 0; h < half; h++) part[h] = add2(part[h], part[h + half]);
+            float d0, d1;
+            up2(part[0], d0, d1);
+            float delta = __fadd_rn(d0, d1);
+#pragma unroll
+            for (int off = G / 2; off >= 1; off >>= 1)
+                delta = __fadd_rn(delta, __shfl_xor_sync(0xffffffffu, delta, off));
+            bool accept = delta > 0.0f;
+            if (!accept) {
+                const float u = __fmul_rn(static_cast<float>((rng.peek() >> 8) + 1u), 5.9604644775390625e-8f);
+                rng.pos++;
+                accept = u <= expf_det(__fmul_rn(2.0f, delta));
+            }
+            if (accept) {
+                s = s2;
+                acc++;
+#pragma unroll
+                for (int p = 0; p < PP; p++) {
+                    const float4 v = __ldg(row0 + p * G);
+                    tr[p] = fma2(t0, pk2(v.x, v.y), tr[p]);
+                    ti[p] = fma2(t0, pk2(v.z, v.w), ti[p]);
+                    if (SZ) {
+                        const float4 u = __ldg(row1 + p * G);
+                        tr[p] = fma2(t1, pk2(u.x, u.y), tr[p]);
+                        ti[p] = fma2(t1, pk2(u.z, u.w), ti[p]);
+                    }
+                    re[p] = fnew[p];
+                }
+            }
+            __syncwarp();
+        }
+        props += P.N;
+        const int done = sw + 1 - L.n_therm;
+        if (done > 0 && done % L.sweeps_per_sample == 0) {
+            const long out = static_cast<long>(L.sample_base + sample) * L.B + w;
+            if (L.sample_spins && g == 0 && live) {
+#pragma unroll
+                for (int k = 0; k < NW; k++) L.sample_spins[out * NW + k] = s.w[k];
+            }
+            sample++;
+        }
+    }
+    if (g == 0 && live) {
+#pragma unroll
+        for (int k = 0; k < NW; k++) L.spins[static_cast<long>(w) * NW + k] = s.w[k];
+        L.rng_index[w] = rng.index();
+        L.accepts[w] += acc;
+        L.proposals[w] += props;
+    }
+}
+
 // Fast-sweep sampler (MonteCarloLoop::set_fast_sweep, MonteCarloLoop.hpp:108-113, 139-151,
 // 162-171): a thermalisation sweep is N mask updates, a sampling sweep one.  The angles are
 // recomputed from the spins every N updates of the thermalisation and at the start of every
@@ -997,22 +1166,16 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) rbm_eloc_t_kernel(RbmDev 
 // ---------------------------------------------------------------------------
 // launchers for this K (instantiated by rbm_k<K>.cu)
 // ---------------------------------------------------------------------------
+// Several walkers per warp: always up to K = 4; at K = 8 (N = 90, M = 250) from 2048 walkers on
+// (66 / 78 us a sweep at 16, 79 / 81 at 1024, 119 / 105 at 2048, 730 / 595 at 16384, one walker
+// a warp / grouped); not above (K = 13, N = 100, M = 400: 158 / 250 at 256, 1251 / 1239 at 16384
+// with the state in shared memory, K = 18: 2425 / 2766 at 16384)
+constexpr bool rbm_grouped(int K, int walkers) { return K <= 4 || (K == 8 && walkers >= 2048); }
+
+// one walker per warp (K > 4)
 template <int K>
-cudaError_t rbm_mc_launch_k(const RbmDev& P, const OpDev* op, const McLaunch& L, cudaStream_t st) {
+cudaError_t rbm_mc_wide_launch_k(const RbmDev& P, const McLaunch& L, dim3 grid, dim3 block, cudaStream_t st) {
     const int nw = (P.N + 63) / 64;
-    const dim3 grid((L.B + kWarpsPerBlock - 1) / kWarpsPerBlock), block(32 * kWarpsPerBlock);
-    (void)op;
-    if (L.fast_tries > 0) {
-        if (L.total_z) return cudaErrorInvalidValue;
-        switch (nw) {
-            case 1: rbm_mc_fast_kernel<K, 1><<<grid, block, 0, st>>>(P, L); break;
-            case 2: rbm_mc_fast_kernel<K, 2><<<grid, block, 0, st>>>(P, L); break;
-            case 3: rbm_mc_fast_kernel<K, 3><<<grid, block, 0, st>>>(P, L); break;
-            case 4: rbm_mc_fast_kernel<K, 4><<<grid, block, 0, st>>>(P, L); break;
-            default: return cudaErrorInvalidValue;
-        }
-        return cudaGetLastError();
-    }
     if (K >= 13 && !L.total_z) {
         constexpr int KP = (K + 1) / 2;
         const size_t sm = sizeof(pair_t) * 4 * KP * 32 * kWarpsPerBlock;
@@ -1033,6 +1196,40 @@ cudaError_t rbm_mc_launch_k(const RbmDev& P, const OpDev* op, const McLaunch& L,
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
+}
+
+template <int K>
+cudaError_t rbm_mc_launch_k(const RbmDev& P, const OpDev* op, const McLaunch& L, cudaStream_t st) {
+    const int nw = (P.N + 63) / 64;
+    const dim3 grid((L.B + kWarpsPerBlock - 1) / kWarpsPerBlock), block(32 * kWarpsPerBlock);
+    (void)op;
+    if (L.fast_tries > 0) {
+        if (L.total_z) return cudaErrorInvalidValue;
+        switch (nw) {
+            case 1: rbm_mc_fast_kernel<K, 1><<<grid, block, 0, st>>>(P, L); break;
+            case 2: rbm_mc_fast_kernel<K, 2><<<grid, block, 0, st>>>(P, L); break;
+            case 3: rbm_mc_fast_kernel<K, 3><<<grid, block, 0, st>>>(P, L); break;
+            case 4: rbm_mc_fast_kernel<K, 4><<<grid, block, 0, st>>>(P, L); break;
+            default: return cudaErrorInvalidValue;
+        }
+        return cudaGetLastError();
+    }
+    if constexpr (K <= 8) {
+        if (rbm_grouped(K, L.B)) {
+            constexpr int G = rbm_group(K), per_block = kWarpsPerBlock * 32 / G;
+            const dim3 blocks((L.B + per_block - 1) / per_block);
+            if (L.total_z && nw != 1) return cudaErrorInvalidValue;
+            if (L.total_z) rbm_mc_group_kernel<K, G, 1, true><<<blocks, block, 0, st>>>(P, L);
+            else if (nw == 1) rbm_mc_group_kernel<K, G, 1, false><<<blocks, block, 0, st>>>(P, L);
+            else if (nw == 2) rbm_mc_group_kernel<K, G, 2, false><<<blocks, block, 0, st>>>(P, L);
+            else if (nw == 3) rbm_mc_group_kernel<K, G, 3, false><<<blocks, block, 0, st>>>(P, L);
+            else if (nw == 4) rbm_mc_group_kernel<K, G, 4, false><<<blocks, block, 0, st>>>(P, L);
+            else return cudaErrorInvalidValue;
+            return cudaGetLastError();
+        }
+    }
+    if constexpr (K > 4) return rbm_mc_wide_launch_k<K>(P, L, grid, block, st);
+    return cudaErrorInvalidValue;
 }
 
 template <int K>
