@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <functional>
 #include <memory>
+#include <type_traits>
 
 #include "device_math.cuh"
 #include "host.h"
@@ -518,7 +519,7 @@ __global__ void col_finish_kernel(int P, int splits, const double2* __restrict__
 // Metropolis for PsiDeep / PsiPair: one CTA per walker, full forward pass per proposal
 // (PsiDeep.hpp:191-194: angles are not updated incrementally; single flips of a complex
 // net move layer 0 incrementally here, and run several walkers per CTA in
-// deep_mc_multi_kernel).  Fast sweep
+// deep_mc_pairs_kernel).  Fast sweep
 // (MonteCarloLoop.hpp:162-171): the proposal flips the AND of fast_tries random
 // configurations, N such updates per thermalisation sweep and one per sampling sweep.
 __global__ void deep_mc_kernel(DeepNetDev n0, DeepNetDev n1, int pair, McLaunch L) {
@@ -645,119 +646,181 @@ __global__ void deep_mc_kernel(DeepNetDev n0, DeepNetDev n1, int pair, McLaunch 
     }
 }
 
-// The same chains as deep_mc_kernel's incremental path (a complex net, single-flip
-// proposals, no pair or translation sums), WPC walkers per CTA: one thread per unit
-// evaluates that unit for all WPC walkers, so each weight and connection index read from
-// L1 serves WPC independent multiply-add chains.  Walker k's Philox stream is drawn by
-// thread k alone (site, uniform, start spins) and published through shared memory; every
-// walker's arithmetic is deep_mc_kernel's, in the same order, so spins, accept counts and
-// stream positions are identical.
-// forward_from_z0 for WPC configurations at once: configuration k's layer-0
-// pre-activations are zof(k)[0 .. size[0]); with STORE its angles and activations go to
-// angles / acts + k * units
-template <int WPC, bool STORE, typename ZOf>
-__device__ __forceinline__ void forward_multi(const DeepNetDev& net, ZOf zof, float2* in, float2* out,
-                                              float2* angles, float2* acts, float2* red, float2 lp[WPC]) {
-    const int t = threadIdx.x;
-    const int width = net.width, size0 = net.size[0], units = net.units;
+// ---------------------------------------------------------------- several configurations a block
+// Two configurations lie side by side, (x0, x1, y0, y1), and every operation is a packed one on
+// both.  A thread evaluates one unit of a layer for NP such pairs: a weight and its connection
+// index are read once for 2 NP multiply-adds, whose inputs are shared by the whole warp where
+// the layer is dense.  Each configuration's sums are forward_once's, in its order.
+struct CPair {
+    pair_t re, im;
+};
+__device__ __forceinline__ CPair ld_pair(const float4* p) {
+    const float4 v = *p;
+    return CPair{pk2(v.x, v.y), pk2(v.z, v.w)};
+}
+__device__ __forceinline__ void st_pair(float4* p, CPair v) {
+    float4 o;
+    up2(v.re, o.x, o.y);
+    up2(v.im, o.z, o.w);
+    *p = o;
+}
+// a += w b for both configurations (cadd(a, cmul(w, b)))
+__device__ __forceinline__ void cmac(CPair& a, float2 w, CPair b) {
+    const pair_t wx = splat2(w.x), wy = splat2(w.y), nwy = splat2(-w.y);
+    a.re = add2(a.re, fma2(wx, b.re, mul2(nwy, b.im)));
+    a.im = add2(a.im, fma2(wx, b.im, mul2(wy, b.re)));
+}
+__device__ __forceinline__ CPair cmul(CPair a, CPair b) {
+    const pair_t nay = mul2(splat2(-1.0f), a.im);
+    return CPair{fma2(a.re, b.re, mul2(nay, b.im)), fma2(a.re, b.im, mul2(a.im, b.re))};
+}
+__device__ __forceinline__ CPair act_pair(CPair z) {
+    const Pair2 y = lc_c2(z.re, z.im);
+    return CPair{y.re, y.im};
+}
+__device__ __forceinline__ CPair dact_pair(CPair z) {
+    float x0, x1, y0, y1;
+    up2(z.re, x0, x1);
+    up2(z.im, y0, y1);
+    const float2 a = tanh_c(x0, y0), b = tanh_c(x1, y1);
+    return CPair{pk2(a.x, b.x), pk2(a.y, b.y)};
+}
+
+constexpr int kPairThreads = 128;   // threads of the kernels below
+
+// sums over the connections of `size` units for `pairs` pairs, NP of them per thread: weight
+// w[c * size + t] of connection c times the input in[.][c] (a dense layer: the input is shared
+// by the warp) or in[.][ci[c * size + t]]; emit(pair, t, sum)
+template <int NP, bool DENSE, typename Emit>
+__device__ __forceinline__ void layer_sums(int size, int conn, const float2* __restrict__ w,
+                                           const int* __restrict__ ci, const float4* in, int in_size, int pairs,
+                                           Emit emit) {
+    const int groups = pairs / NP;
+    for (int item = threadIdx.x; item < size * groups; item += kPairThreads) {
+        const int grp = item / size, t = item - grp * size;
+        const float4* x = in + grp * NP * in_size;
+        CPair a[NP];
 #pragma unroll
-    for (int k = 0; k < WPC; k++) {
-        const float2* zk = zof(k);
-        for (int u = t; u < size0; u += blockDim.x) {
-            const float2 y = act<false>(zk[u]);
-            if (STORE) {
-                angles[k * units + net.begin_angle[0] + u] = zk[u];
-                acts[k * units + net.begin_angle[0] + u] = y;
-            }
-            in[k * width + u] = y;
+        for (int p = 0; p < NP; p++) a[p] = CPair{splat2(0.0f), splat2(0.0f)};
+#pragma unroll 8
+        for (int c = 0; c < conn; c++) {
+            const float2 wv = __ldg(w + c * size + t);
+            const int i = DENSE ? c : __ldg(ci + c * size + t);
+#pragma unroll
+            for (int p = 0; p < NP; p++) cmac(a[p], wv, ld_pair(x + p * in_size + i));
         }
+#pragma unroll
+        for (int p = 0; p < NP; p++) emit(grp * NP + p, t, a[p]);
     }
+}
+
+// pairs per thread: as many as leave work for most threads
+template <int PAIRS, bool DENSE, typename Emit>
+__device__ __forceinline__ void layer_sums_split(int size, int conn, const float2* w, const int* ci, const float4* in,
+                                                 int in_size, Emit emit) {
+    if (PAIRS >= 4 && size >= 64) layer_sums<(PAIRS >= 4 ? 4 : 1), DENSE>(size, conn, w, ci, in, in_size, PAIRS, emit);
+    else if (PAIRS >= 2 && size * PAIRS >= 128)
+        layer_sums<(PAIRS >= 2 ? 2 : 1), DENSE>(size, conn, w, ci, in, in_size, PAIRS, emit);
+    else layer_sums<1, DENSE>(size, conn, w, ci, in, in_size, PAIRS, emit);
+}
+
+// layers 1 .. L - 1 from layer 0's activations in bufs[0]; layer l's activations go to
+// bufs[l & 1], emit(l, pair, t, angle, activation) sees them.  Ends with a barrier.
+template <int PAIRS, typename Emit>
+__device__ __forceinline__ void forward_pairs(const DeepNetDev& net, float4* const (&bufs)[2], Emit emit) {
     __syncthreads();
     for (int l = 1; l < net.L; l++) {
-        const int size = net.size[l], conn = net.conn[l];
-        if (t < size) {
-            const float2* wl = net.w[l];
-            const int* ci = net.cidx[l];
-            float2 a[WPC];
-#pragma unroll
-            for (int k = 0; k < WPC; k++) a[k] = czero<float2>();
-            for (int c = 0; c < conn; c++) {
-                const float2 wv = wl[c * size + t];
-                const int i = ci[c * size + t];
-#pragma unroll
-                for (int k = 0; k < WPC; k++) a[k] = cadd(a[k], cmul(wv, in[k * width + i]));
-            }
-            const float2 bv = net.b[l][t];
-#pragma unroll
-            for (int k = 0; k < WPC; k++) {
-                const float2 z = cadd(a[k], bv);
-                const float2 y = act<false>(z);
-                if (STORE) {
-                    angles[k * units + net.begin_angle[l] + t] = z;
-                    acts[k * units + net.begin_angle[l] + t] = y;
-                }
-                out[k * width + t] = y;
-            }
-        }
+        const int size = net.size[l], conn = net.conn[l], below = net.size[l - 1];
+        const float4* in = bufs[(l - 1) & 1];
+        float4* out = bufs[l & 1];
+        const float2* bias = net.b[l];
+        auto done = [&](int p, int t, CPair a) {
+            const float2 bv = __ldg(bias + t);
+            const CPair z{add2(a.re, splat2(bv.x)), add2(a.im, splat2(bv.y))};
+            const CPair y = act_pair(z);
+            st_pair(out + p * size + t, y);
+            emit(l, p, t, z, y);
+        };
+        if (net.wt[l]) layer_sums_split<PAIRS, true>(size, conn, net.w[l], nullptr, in, below, done);
+        else layer_sums_split<PAIRS, false>(size, conn, net.w[l], net.cidx[l], in, below, done);
         __syncthreads();
-        float2* tmp = in;
-        in = out;
-        out = tmp;
     }
-    // each configuration's block_sum of its terms, in block_sum's order
+}
+
+// sum_j act_j fw_j of one pair by a warp (block_sum's order); every lane receives it
+__device__ __forceinline__ CPair final_sum(const DeepNetDev& net, const float4* in, int lane) {
     const int last = net.size[net.L - 1];
-    const int lane = t & 31, warp = t >> 5, nwarps = (blockDim.x + 31) >> 5;
-    float2 v[WPC];
-#pragma unroll
-    for (int k = 0; k < WPC; k++) {
-        v[k] = t < last ? cmul(in[k * width + t], net.fw[t]) : czero<float2>();
+    CPair r{splat2(0.0f), splat2(0.0f)};
+    for (int q = 0; q < last; q += 32) {
+        CPair v{splat2(0.0f), splat2(0.0f)};
+        if (q + lane < last) {
+            const float2 f = net.fw[q + lane];
+            v = cmul(ld_pair(in + q + lane), CPair{splat2(f.x), splat2(f.y)});
+        }
 #pragma unroll
         for (int off = 16; off >= 1; off >>= 1) {
-            v[k].x += __shfl_xor_sync(0xffffffffu, v[k].x, off);
-            v[k].y += __shfl_xor_sync(0xffffffffu, v[k].y, off);
+            v.re = add2(v.re, __shfl_xor_sync(0xffffffffu, v.re, off));
+            v.im = add2(v.im, __shfl_xor_sync(0xffffffffu, v.im, off));
         }
+        r.re = add2(r.re, v.re);
+        r.im = add2(r.im, v.im);
     }
-    __syncthreads();
-    if (lane == 0)
-#pragma unroll
-        for (int k = 0; k < WPC; k++) red[k * 32 + warp] = v[k];
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < WPC; k++) {
-        float2 r = czero<float2>();
-        for (int q = 0; q < nwarps; q++) r = cadd(r, red[k * 32 + q]);
-        lp[k] = r;
-    }
+    return r;
 }
 
-size_t deep_mc_multi_smem(const DeepNetDev& n, int wpc) {
-    return wpc * (sizeof(float2) * (32 + 2 * n.width + 2 * n.size[0]) + sizeof(uint64_t) * kMaxWords +
-                  2 * sizeof(int));
+// layer 0's pre-activation of unit u moved by a flip of `site` (ts = 2 x the new spin)
+__device__ __forceinline__ float2 move_z0(const DeepNetDev& net, int site, float ts, int u, float2 z) {
+    for (int d = 0; d < net.w0n; d++) {
+        const float2 w = __ldg(net.w0 + (static_cast<long>(d) * net.N + site) * net.size[0] + u);
+        z.x = __fmaf_rn(ts, w.x, z.x);   // ts = +-2: the product is exact
+        z.y = __fmaf_rn(ts, w.y, z.y);
+    }
+    return z;
 }
 
-template <int WPC>
-__global__ void deep_mc_multi_kernel(DeepNetDev n0, McLaunch L) {
+// float4 of the two activation buffers: layers 0 and 2, layer 1
+__host__ __device__ inline int pair_buf(const DeepNetDev& n, int which) {
+    return which == 0 ? (n.L > 2 && n.size[2] > n.size[0] ? n.size[2] : n.size[0]) : (n.L > 1 ? n.size[1] : 0);
+}
+
+size_t deep_mc_pairs_smem(const DeepNetDev& n, int pairs) {
+    return sizeof(float4) * pairs * (n.size[0] + pair_buf(n, 0) + pair_buf(n, 1)) +
+           2 * pairs * (sizeof(uint64_t) * ((n.N + 63) / 64) + 2 * sizeof(int2));
+}
+
+// deep_mc_kernel's single-flip chains (a complex net, no translation sums) for 2 PAIRS walkers
+// a block.  Layer 0's pre-activations are kept per walker and moved by the flipped spin's
+// weights; an accepted move is committed when the next proposal is formed from them.  Walker
+// k's random words, test and counters belong to one lane of the warp that forms its log psi.
+// Bound by the FP32 pipe (six operations a complex multiply-add, in forward_once's order).
+// Seven blocks an SM: 8192 walkers are 6.7 blocks of eight an SM, and with six resident the
+// rest ran after the others (100-200-100-50 net, four sweeps: 67.5 ms with a thread per unit,
+// 54.8 ms with six blocks, 35.8 ms; two units per thread 57, weights fetched ahead of their
+// use into registers 40 to 43).
+template <int PAIRS>
+__global__ void __launch_bounds__(kPairThreads, 7) deep_mc_pairs_kernel(DeepNetDev net, McLaunch L) {
     extern __shared__ __align__(16) unsigned char smem[];
-    const int width = n0.width, size0 = n0.size[0];
-    float2* red = reinterpret_cast<float2*>(smem);                     // [WPC][32]
-    float2* in = red + WPC * 32;                                       // [WPC][width]
-    float2* out = in + WPC * width;                                    // [WPC][width]
-    float2* zb = out + WPC * width;                                    // [WPC][2][size0]
-    uint64_t* s = reinterpret_cast<uint64_t*>(zb + 2 * WPC * size0);   // [WPC][kMaxWords]
-    int* site_sh = reinterpret_cast<int*>(s + WPC * kMaxWords);        // [WPC]
-    int* flag_sh = site_sh + WPC;                                      // [WPC]
-    const int N = n0.N, nw = (N + 63) / 64;
+    constexpr int WPC = 2 * PAIRS;
+    const int size0 = net.size[0], N = net.N, nw = (N + 63) / 64;
+    float4* zs = reinterpret_cast<float4*>(smem);                       // [PAIRS][size0]
+    float4* const bufs[2] = {zs + PAIRS * size0, zs + PAIRS * (size0 + pair_buf(net, 0))};
+    uint64_t* s = reinterpret_cast<uint64_t*>(bufs[1] + PAIRS * pair_buf(net, 1));   // [WPC][nw]
+    int2* moved = reinterpret_cast<int2*>(s + WPC * nw);         // [WPC] accepted move: site, bits of ts (0: none)
+    int2* trial = moved + WPC;                                          // [WPC] proposal
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int first = blockIdx.x * WPC;
-    const int t = threadIdx.x;
-    // thread k < WPC owns walker first + k: its stream, spins updates and counters
-    const int mine = first + t;
-    const bool owner = t < WPC && mine < L.B;
+    // lane r < 2 of warp q < PAIRS owns walker k = 2 q + r
+    const int k_own = 2 * warp + lane;
+    const bool own = warp < PAIRS && lane < 2, owner = own && first + k_own < L.B;
+    const int mine = first + k_own;
     WalkerRng rng;
+    rng.init(L.seed, L.walker_base + static_cast<uint32_t>(mine), owner ? L.rng_index[mine] : 0);
     unsigned long long acc = 0, props = 0;
-    if (t < WPC) {
-        rng.init(L.seed, L.walker_base + static_cast<uint32_t>(mine), owner ? L.rng_index[mine] : 0);
-        uint64_t* sk = s + t * kMaxWords;
-        for (int k = 0; k < kMaxWords; k++) sk[k] = 0;
+    float lpr = 0.0f;
+    int site = 0;
+    if (own) {
+        uint64_t* sk = s + k_own * nw;
+        for (int k = 0; k < nw; k++) sk[k] = 0;
         if (owner) {
             if (L.init) {
                 for (int k = 0; k < nw; k++) {
@@ -771,94 +834,106 @@ __global__ void deep_mc_multi_kernel(DeepNetDev n0, McLaunch L) {
             }
         }
     }
-    float lpr[WPC];
-    float2 nl[WPC], lp0[WPC];
-    int cur = 0;   // bit k: the half of walker k's layer-0 pair that holds its state
+    auto none = [](int, int, int, CPair, CPair) {};
+    // Re log psi of this lane's walker (lanes 0 and 1 of the owning warps)
+    auto log_psi = [&]() {
+        float v0 = 0.0f, v1 = 0.0f;
+        if (warp < PAIRS) {
+            const CPair r = final_sum(net, bufs[(net.L - 1) & 1] + warp * net.size[net.L - 1], lane);
+            up2(r.re, v0, v1);
+        }
+        return lane == 1 ? v1 : v0;
+    };
+    // the owner's next proposal
+    auto propose = [&]() {
+        if (!own) return;
+        float ts = 0.0f;
+        if (owner) {
+            site = static_cast<int>(rng.next() % static_cast<uint32_t>(N));
+            ts = bit_up(s + k_own * nw, site) ? -2.0f : 2.0f;
+        }
+        trial[k_own] = make_int2(site, __float_as_int(ts));
+    };
     const int total = L.n_therm + L.n_samples * L.sweeps_per_sample;
     int sample = 0;
     for (int sw = 0; sw < total; sw++) {
+        __syncthreads();
         // layer 0 and log psi of every state from its spins
+        for (int item = t; item < PAIRS * size0; item += kPairThreads) {
+            const int p = item / size0, u = item - p * size0;
+            const uint64_t *s0 = s + 2 * p * nw, *s1 = s0 + nw;
+            CPair a{splat2(0.0f), splat2(0.0f)};
+            const int conn = net.conn[0];
+#pragma unroll 4
+            for (int c = 0; c < conn; c++) {
+                const float2 w = __ldg(net.w[0] + c * size0 + u);
+                const int i = __ldg(net.cidx[0] + c * size0 + u);
+                const pair_t sg = pk2(bit_up(s0, i) ? 1.0f : -1.0f, bit_up(s1, i) ? 1.0f : -1.0f);
+                a.re = fma2(sg, splat2(w.x), a.re);   // sg = +-1: the products are exact
+                a.im = fma2(sg, splat2(w.y), a.im);
+            }
+            const float2 b = net.b[0][u];
+            const CPair z{add2(a.re, splat2(b.x)), add2(a.im, splat2(b.y))};
+            st_pair(zs + item, z);
+            st_pair(bufs[0] + item, act_pair(z));
+        }
+        forward_pairs<PAIRS>(net, bufs, none);
+        lpr = log_psi();
+        if (own) moved[k_own] = make_int2(0, 0);
+        propose();
         __syncthreads();
-#pragma unroll
-        for (int k = 0; k < WPC; k++) layer0_pre(n0, s + k * kMaxWords, zb + (2 * k + ((cur >> k) & 1)) * size0);
-        __syncthreads();
-        forward_multi<WPC, false>(n0, [&](int k) { return zb + (2 * k + ((cur >> k) & 1)) * size0; }, in, out,
-                                  nullptr, nullptr, red, lp0);
-#pragma unroll
-        for (int k = 0; k < WPC; k++) lpr[k] = lp0[k].x;
         for (int p = 0; p < N; p++) {
-            if (owner) site_sh[t] = static_cast<int>(rng.next() % static_cast<uint32_t>(N));
-            // a proposal's layer 0: its state's moved by the flipped spin's connections
-#pragma unroll
-            for (int k = 0; k < WPC; k++) {
-                const int h = (cur >> k) & 1;
-                const float2* src = zb + (2 * k + h) * size0;
-                float2* dst = zb + (2 * k + 1 - h) * size0;
-                for (int u = t; u < size0; u += blockDim.x) dst[u] = src[u];
-            }
-            __syncthreads();
-#pragma unroll
-            for (int k = 0; k < WPC; k++) {
-                if (first + k >= L.B) continue;
-                const int site = site_sh[k];
-                const float two_s = bit_up(s + k * kMaxWords, site) ? -2.0f : 2.0f;
-                float2* dst = zb + (2 * k + 1 - ((cur >> k) & 1)) * size0;
-                for (int q = n0.sptr[site] + t; q < n0.sptr[site + 1]; q += blockDim.x) {
-                    const int e = n0.sq[q];
-                    const float2 wv = n0.w[0][e];
-                    float2* zz = dst + e % size0;
-                    atomicAdd(&zz->x, two_s * wv.x);
-                    atomicAdd(&zz->y, two_s * wv.y);
+            for (int item = t; item < PAIRS * size0; item += kPairThreads) {
+                const int q = item / size0, u = item - q * size0;
+                float4 z = zs[item];
+                float2 z0 = make_float2(z.x, z.z), z1 = make_float2(z.y, z.w);
+                const int2 m0 = moved[2 * q], m1 = moved[2 * q + 1];
+                if (m0.y | m1.y) {
+                    if (m0.y) z0 = move_z0(net, m0.x, __int_as_float(m0.y), u, z0);
+                    if (m1.y) z1 = move_z0(net, m1.x, __int_as_float(m1.y), u, z1);
+                    zs[item] = make_float4(z0.x, z1.x, z0.y, z1.y);
                 }
+                const int2 p0 = trial[2 * q], p1 = trial[2 * q + 1];
+                z0 = move_z0(net, p0.x, __int_as_float(p0.y), u, z0);
+                z1 = move_z0(net, p1.x, __int_as_float(p1.y), u, z1);
+                st_pair(bufs[0] + item, act_pair(CPair{pk2(z0.x, z1.x), pk2(z0.y, z1.y)}));
             }
-            __syncthreads();
-            forward_multi<WPC, false>(n0, [&](int k) { return zb + (2 * k + 1 - ((cur >> k) & 1)) * size0; }, in,
-                                      out, nullptr, nullptr, red, nl);
-            if (t < WPC) {
-                float mnl = nl[0].x, mlp = lpr[0];
-#pragma unroll
-                for (int k = 1; k < WPC; k++)
-                    if (k == t) {
-                        mnl = nl[k].x;
-                        mlp = lpr[k];
-                    }
+            forward_pairs<PAIRS>(net, bufs, none);
+            const float nl = log_psi();
+            if (own) {
                 bool accept = false;
                 if (owner) {
-                    const float delta = mnl - mlp;
+                    const float delta = nl - lpr;
                     accept = delta > 0.0f;
                     if (!accept) accept = rng.uniform() <= expf_det(2.0f * delta);
                     if (accept) {
-                        const int site = site_sh[t];
-                        s[t * kMaxWords + (site >> 6)] ^= 1ull << (site & 63);
+                        s[k_own * nw + (site >> 6)] ^= 1ull << (site & 63);
+                        lpr = nl;
                         acc++;
                     }
                     props++;
                 }
-                flag_sh[t] = accept ? 1 : 0;
+                moved[k_own] = accept ? trial[k_own] : make_int2(0, 0);
             }
+            propose();
             __syncthreads();
-#pragma unroll
-            for (int k = 0; k < WPC; k++)
-                if (flag_sh[k]) {
-                    lpr[k] = nl[k].x;
-                    cur ^= 1 << k;
-                }
         }
+        if (owner) rng.index--;   // the word of the proposal that the sweep's end leaves undone
         const int done = sw + 1 - L.n_therm;
         if (done > 0 && done % L.sweeps_per_sample == 0) {
             const long row0 = static_cast<long>(L.sample_base + sample) * L.B;
             if (L.sample_spins)
-                for (int i = t; i < WPC * nw; i += blockDim.x) {
+                for (int i = t; i < WPC * nw; i += kPairThreads) {
                     const int k = i / nw, word = i % nw;
-                    if (first + k < L.B) L.sample_spins[(row0 + first + k) * nw + word] = s[k * kMaxWords + word];
+                    if (first + k < L.B) L.sample_spins[(row0 + first + k) * nw + word] = s[k * nw + word];
                 }
             sample++;
         }
     }
     __syncthreads();
-    for (int i = t; i < WPC * nw; i += blockDim.x) {
+    for (int i = t; i < WPC * nw; i += kPairThreads) {
         const int k = i / nw, word = i % nw;
-        if (first + k < L.B) L.spins[static_cast<long>(first + k) * nw + word] = s[k * kMaxWords + word];
+        if (first + k < L.B) L.spins[static_cast<long>(first + k) * nw + word] = s[k * nw + word];
     }
     if (owner) {
         L.rng_index[mine] = rng.index;
@@ -912,6 +987,14 @@ __device__ void backward_deltas(const DeepNetDev& net, Work<V>& w, Emit emit) {
         cur = nxt;
         nxt = tmp;
     }
+}
+
+// a neighbour's term of the local energy, cf psi(s') / psi(s), in FP64.  One function for the
+// kernels below, so that they round alike.
+__device__ __noinline__ double2 neighbour_term(double2 cf, float2 lq, float2 lp) {
+    const double dr = static_cast<double>(lq.x) - lp.x, di = static_cast<double>(lq.y) - lp.y;
+    const double m = exp(dr);
+    return make_double2(m * (cf.x * cos(di) - cf.y * sin(di)), m * (cf.x * sin(di) + cf.y * cos(di)));
 }
 
 // One CTA per sample: E_loc(s) (FP32 passes, FP64 sum), then for every configuration x
@@ -983,9 +1066,7 @@ __global__ void deep_adjoint_kernel(DeepNetDev net, OpDev op, int count, const u
             __syncthreads();
         }
         const float2 lq = forward_from_z0<true>(net, z0n, w);
-        const double dr = static_cast<double>(lq.x) - lp.x, di = static_cast<double>(lq.y) - lp.y;
-        const double m = exp(dr);
-        const double2 e = make_double2(m * (cf.x * cos(di) - cf.y * sin(di)), m * (cf.x * sin(di) + cf.y * cos(di)));
+        const double2 e = neighbour_term(cf, lq, lp);
         eor += e.x;
         eoi += e.y;
         pass(sp, t * xs + q, make_float2(static_cast<float>(ws * e.x), static_cast<float>(ws * e.y)), false);
@@ -1004,193 +1085,225 @@ __global__ void deep_adjoint_kernel(DeepNetDev net, OpDev op, int count, const u
     if (threadIdx.x == 0) eloc[t] = make_double2(er, ei);
 }
 
-// backward_deltas for NB configurations at once (configuration k's angles at angles +
-// k * units, its error buffers at cur / nxt + k * width); emit(k, layer, unit, delta) for
-// k < nb
-template <int NB, typename Emit>
-__device__ void backward_multi(const DeepNetDev& net, const float2* angles, float2* cur, float2* nxt, int nb,
-                               Emit emit) {
-    const int t = threadIdx.x;
-    const int L = net.L, width = net.width, units = net.units;
-    for (int l = L - 1; l >= 0; l--) {
-        const int size = net.size[l];
-        float2 d[NB];
-#pragma unroll
-        for (int k = 0; k < NB; k++) d[k] = czero<float2>();
-        if (t < size) {
-            const int at = net.begin_angle[l] + t;
-            if (l == L - 1) {
-                const float2 f = net.fw[t];
-#pragma unroll
-                for (int k = 0; k < NB; k++) d[k] = cmul(f, dact<false>(angles[k * units + at]));
-            } else {
-                const int nsize = net.size[l + 1];
-                float2 acc[NB];
-#pragma unroll
-                for (int k = 0; k < NB; k++) acc[k] = czero<float2>();
-                const float2* wn = net.w[l + 1];
-                for (int e = net.rptr[l][t]; e < net.rptr[l][t + 1]; e++) {
-                    const int q = net.rq[l][e];
-                    const float2 wv = wn[q];
-                    const int j = q % nsize;
-#pragma unroll
-                    for (int k = 0; k < NB; k++) acc[k] = cadd(acc[k], cmul(wv, nxt[k * width + j]));
-                }
-#pragma unroll
-                for (int k = 0; k < NB; k++) d[k] = cmul(acc[k], dact<false>(angles[k * units + at]));
-            }
-        }
-        __syncthreads();
-        if (t < size)
-#pragma unroll
-            for (int k = 0; k < NB; k++) {
-                cur[k * width + t] = d[k];
-                if (k < nb) emit(k, l, t, d[k]);
-            }
-        __syncthreads();
-        float2* tmp = cur;
-        cur = nxt;
-        nxt = tmp;
-    }
+size_t deep_adjoint_pairs_smem(const DeepNetDev& n, int pairs) {
+    return sizeof(float4) * pairs * (n.units + pair_buf(n, 0) + pair_buf(n, 1)) +
+           sizeof(float2) * (n.size[0] + 4 * pairs) + sizeof(uint64_t) * kMaxWords + 16;
 }
 
-size_t deep_adjoint_multi_smem(const DeepNetDev& n, int nb) {
-    return sizeof(float2) * (nb * (32 + 2 * n.width + 2 * n.units + n.size[0]) + n.size[0]) +
-           sizeof(uint64_t) * (1 + nb) * kMaxWords;
-}
-
-// deep_adjoint_kernel with the off-diagonal neighbours of a sample taken NB at a time: the
-// thread of a unit evaluates it (forward and reverse) for all NB neighbours, so each weight
-// read serves NB chains.  Every configuration's arithmetic and the local energy's order of
-// summation are deep_adjoint_kernel's: the outputs are identical.
-template <int NB>
-__global__ void deep_adjoint_multi_kernel(DeepNetDev net, OpDev op, int count, const uint64_t* spins,
-                                          uint64_t enum_base, int enumerate, const double* weights, int score,
-                                          double2* eloc, float2* acts, float2* dlts, float2* alpha, uint64_t* xspins,
-                                          int xs, float2* dltsO, float2* alphaO) {
+// deep_adjoint_kernel with 2 PAIRS of a sample's off-diagonal neighbours at a time, two in the
+// halves of each packed operation.  Every configuration's arithmetic and the local energy's
+// order of summation are deep_adjoint_kernel's: the outputs are identical.  The neighbours'
+// FP64 exponentials run in the lanes of one warp, once each: in every thread of the block they
+// held the FP64 pipe for 28000 cycles a neighbour on the 100-200-100-50 net, which was the
+// kernel's whole time.  Bound by the FP32 pipe and, at 128 threads, by the layers' barriers.
+// 8192 samples of that net: 70.3 -> 19.4 ms.
+template <int PAIRS>
+__global__ void __launch_bounds__(kPairThreads, 5) deep_adjoint_pairs_kernel(
+    DeepNetDev net, OpDev op, int count, const uint64_t* spins, uint64_t enum_base, int enumerate,
+    const double* weights, int score, double2* eloc, float2* acts, float2* dlts, float2* alpha, uint64_t* xspins,
+    int xs, float2* dltsO, float2* alphaO) {
     extern __shared__ __align__(16) unsigned char smem[];
-    const int width = net.width, size0 = net.size[0], units = net.units;
-    float2* red = reinterpret_cast<float2*>(smem);                   // [NB][32]
-    float2* in = red + NB * 32;                                      // [NB][width]
-    float2* out = in + NB * width;                                   // [NB][width]
-    float2* angles = out + NB * width;                               // [NB][units]
-    float2* actsb = angles + NB * units;                             // [NB][units]
-    float2* z0s = actsb + NB * units;                                // [size0] the sample's layer 0
-    float2* z0n = z0s + size0;                                       // [NB][size0] the neighbours'
-    uint64_t* s = reinterpret_cast<uint64_t*>(z0n + NB * size0);     // [kMaxWords] the sample
-    uint64_t* sp = s + kMaxWords;                                    // [NB][kMaxWords] the neighbours
+    constexpr int NB = 2 * PAIRS;
+    const int size0 = net.size[0], units = net.units;
+    float4* angles = reinterpret_cast<float4*>(smem);                   // [PAIRS][units]
+    float4* const bufs[2] = {angles + PAIRS * units, angles + PAIRS * (units + pair_buf(net, 0))};
+    float2* z0s = reinterpret_cast<float2*>(bufs[1] + PAIRS * pair_buf(net, 1));   // [size0] the sample's layer 0
+    float2* lqs = z0s + size0;                                          // [NB] log psi
+    float2* afs = lqs + NB;                                             // [NB] coefficients of the deltas
+    // 16-byte aligned whatever size0
+    uint64_t* s = reinterpret_cast<uint64_t*>((reinterpret_cast<size_t>(afs + NB) + 15) & ~size_t(15));
     const long t = blockIdx.x;
     if (t >= count) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nw = (net.N + 63) / 64;
     load_config(spins, enum_base, enumerate, t, net.N, s);
-    __syncthreads();
-    layer0_pre(net, s, z0s);
-    __syncthreads();
-    auto self_z = [&](int) { return static_cast<const float2*>(z0s); };
-    float2 lp1[1];
-    forward_multi<1, false>(net, self_z, in, out, nullptr, nullptr, red, lp1);
-    const float2 lp = lp1[0];
-    double er = 0.0, ei = 0.0, eor = 0.0, eoi = 0.0;
-    for (int n = 0; n < op.S; n++) {
-        if (op.nflip[n] != 0) continue;
-        const double2 cf = apply_string(op, n, s, sp);
-        er += cf.x;
-        ei += cf.y;
+    for (int u = tid; u < size0; u += kPairThreads) {
+        float2 a = make_float2(0.0f, 0.0f);
+        for (int c = 0; c < net.conn[0]; c++) {
+            const float2 w = __ldg(net.w[0] + c * size0 + u);
+            const float sg = bit_up(s, __ldg(net.cidx[0] + c * size0 + u)) ? 1.0f : -1.0f;
+            a.x = __fmaf_rn(sg, w.x, a.x);
+            a.y = __fmaf_rn(sg, w.y, a.y);
+        }
+        const float2 b = net.b[0][u];
+        z0s[u] = make_float2(a.x + b.x, a.y + b.y);
     }
+    __syncthreads();
     const double ws = weights ? weights[t] : 1.0;
-    const float wsf = static_cast<float>(ws);
-    int q = 0;   // neighbours done
-    int n = 0;   // next string to scan
-    for (;;) {
-        // the next (up to) NB off-diagonal strings, their neighbours' spins and coefficients
-        double2 cf[NB];
-        int ns[NB];
-        int nb = 0;
-#pragma unroll
-        for (int k = 0; k < NB; k++) {
-            while (n < op.S && op.nflip[n] == 0) n++;
-            ns[k] = -1;
-            cf[k] = make_double2(0.0, 0.0);
-            if (n < op.S) {
-                cf[k] = apply_string(op, n, s, sp + k * kMaxWords);
-                ns[k] = n;
-                nb = k + 1;
-                n++;
+    // log psi of the pairs in the last buffer to lqs
+    auto log_psi = [&](int pairs) {
+        if (warp < pairs) {
+            const CPair r = final_sum(net, bufs[(net.L - 1) & 1] + warp * net.size[net.L - 1], lane);
+            float x0, x1, y0, y1;
+            up2(r.re, x0, x1);
+            up2(r.im, y0, y1);
+            if (lane == 0) {
+                lqs[2 * warp] = make_float2(x0, y0);
+                lqs[2 * warp + 1] = make_float2(x1, y1);
             }
         }
-        if (nb == 0) break;
-        // each neighbour's layer 0: the sample's moved by the flipped spins' connections
-        for (int i = threadIdx.x; i < NB * size0; i += blockDim.x) z0n[i] = z0s[i % size0];
         __syncthreads();
-#pragma unroll
-        for (int k = 0; k < NB; k++) {
-            if (k >= nb) break;
-            const int m = ns[k];
-            for (int f = 0; f < op.nflip[m]; f++) {
-                const int site = op.flip_sites[op.flip_off[m] + f];
-                const float two_s = bit_up(s, site) ? -2.0f : 2.0f;
-                for (int e = net.sptr[site] + threadIdx.x; e < net.sptr[site + 1]; e += blockDim.x) {
-                    const int c = net.sq[e];
-                    const float2 wv = net.w[0][c];
-                    float2* z = z0n + k * size0 + c % size0;
-                    atomicAdd(&z->x, two_s * wv.x);
-                    atomicAdd(&z->y, two_s * wv.y);
+    };
+    // stored forward pass of configurations x0 .. x0 + nb - 1, layer 0 from z0of(pair, u)
+    auto forward = [&](auto pairs_c, auto z0of, long x0, int nb) {
+        constexpr int P = decltype(pairs_c)::value;
+        auto keep = [&](int l, int p, int u, CPair z, CPair y) {
+            const int at = net.begin_angle[l] + u;
+            st_pair(angles + p * units + at, z);
+            float a0, a1, b0, b1;
+            up2(y.re, a0, a1);
+            up2(y.im, b0, b1);
+            float2* row = acts + (x0 + 2 * p) * units + at;
+            if (2 * p < nb) row[0] = make_float2(a0, b0);
+            if (2 * p + 1 < nb) row[units] = make_float2(a1, b1);
+        };
+        for (int item = tid; item < P * size0; item += kPairThreads) {
+            const int p = item / size0, u = item - p * size0;
+            const CPair z = z0of(p, u);
+            const CPair y = act_pair(z);
+            st_pair(bufs[0] + item, y);
+            keep(0, p, u, z, y);
+        }
+        forward_pairs<P>(net, bufs, keep);
+    };
+    // reverse pass: alpha_x delta_l(x) of configurations x0 .. x0 + nb - 1; with self also
+    // w_s delta_l of the sample
+    auto backward = [&](auto pairs_c, long x0, int nb, bool self) {
+        constexpr int P = decltype(pairs_c)::value;
+        const float wsf = static_cast<float>(ws);
+        for (int l = net.L - 1; l >= 0; l--) {
+            const int size = net.size[l];
+            float4* cur = bufs[l & 1];
+            auto done = [&](int p, int u, CPair a) {
+                const int at = net.begin_angle[l] + u;
+                const CPair d = cmul(a, dact_pair(ld_pair(angles + p * units + at)));
+                st_pair(cur + p * size + u, d);
+                float d0x, d1x, d0y, d1y;
+                up2(d.re, d0x, d1x);
+                up2(d.im, d0y, d1y);
+                float2* row = dlts + (x0 + 2 * p) * units + at;
+                if (2 * p < nb) row[0] = cmul(afs[2 * p], make_float2(d0x, d0y));
+                if (2 * p + 1 < nb) row[units] = cmul(afs[2 * p + 1], make_float2(d1x, d1y));
+                if (self && p == 0) dltsO[t * units + at] = make_float2(wsf * d0x, wsf * d0y);
+            };
+            if (l == net.L - 1) {
+                for (int item = tid; item < P * size; item += kPairThreads) {
+                    const int p = item / size, u = item - p * size;
+                    const float2 f = net.fw[u];
+                    done(p, u, CPair{splat2(f.x), splat2(f.y)});
                 }
-                // one site at a time: each unit meets a site once, so the sums do not
-                // depend on the order of the atomic additions
-                __syncthreads();
+            } else {
+                const int above = net.size[l + 1];
+                const float4* nxt = bufs[(l + 1) & 1];
+                if (net.wt[l + 1]) {
+                    layer_sums_split<P, true>(size, above, net.wt[l + 1], nullptr, nxt, above, done);
+                } else {
+                    const float2* wn = net.w[l + 1];
+                    for (int item = tid; item < P * size; item += kPairThreads) {
+                        const int p = item / size, u = item - p * size;
+                        CPair a{splat2(0.0f), splat2(0.0f)};
+                        for (int e = net.rptr[l][u]; e < net.rptr[l][u + 1]; e++) {
+                            const int q = net.rq[l][e];
+                            cmac(a, wn[q], ld_pair(nxt + p * above + q % above));
+                        }
+                        done(p, u, a);
+                    }
+                }
+            }
+            __syncthreads();
+        }
+    };
+    auto self_z = [&](int, int u) {
+        const float2 z = z0s[u];
+        return CPair{splat2(z.x), splat2(z.y)};
+    };
+    const std::integral_constant<int, 1> one;
+    const std::integral_constant<int, PAIRS> all;
+    forward(one, self_z, t * xs, 1);   // the sample's rows are written again with its reverse pass
+    log_psi(1);
+    const float2 lp = lqs[0];
+    // warp 0: the diagonal strings' sum, in order
+    double er = 0.0, ei = 0.0, eor = 0.0, eoi = 0.0;
+    auto factor = [&](int n) {
+        int parity = 0;
+        for (int k = 0; k < kMaxWords; k++) parity += __popcll(op.zmask[n * kMaxWords + k] & ~s[k]);
+        const double sg = (parity & 1) ? -1.0 : 1.0;
+        const double2 c = op.coef[n];
+        const int yp = op.ypow[n] & 3;
+        const double2 r = yp == 0 ? c : (yp == 1 ? make_double2(c.y, -c.x)
+                                                 : (yp == 2 ? make_double2(-c.x, -c.y) : make_double2(-c.y, c.x)));
+        return make_double2(sg * r.x, sg * r.y);
+    };
+    if (warp == 0) {
+        for (int n0 = 0; n0 < op.S; n0 += 32) {
+            const bool diag = n0 + lane < op.S && op.nflip[n0 + lane] == 0;
+            const double2 cf = diag ? factor(n0 + lane) : make_double2(0.0, 0.0);
+            for (unsigned m = __ballot_sync(0xffffffffu, diag); m; m &= m - 1) {
+                er += __shfl_sync(0xffffffffu, cf.x, __ffs(m) - 1);
+                ei += __shfl_sync(0xffffffffu, cf.y, __ffs(m) - 1);
             }
         }
-        float2 lq[NB];
-        forward_multi<NB, true>(net, [&](int k) { return static_cast<const float2*>(z0n + k * size0); }, in, out,
-                                angles, actsb, red, lq);
-        float2 af[NB];
-#pragma unroll
-        for (int k = 0; k < NB; k++) {
-            af[k] = make_float2(0.f, 0.f);
-            if (k < nb) {
-                const double dr = static_cast<double>(lq[k].x) - lp.x, di = static_cast<double>(lq[k].y) - lp.y;
-                const double mg = exp(dr);
-                const double2 e = make_double2(mg * (cf[k].x * cos(di) - cf[k].y * sin(di)),
-                                               mg * (cf[k].x * sin(di) + cf[k].y * cos(di)));
-                eor += e.x;
-                eoi += e.y;
-                af[k] = make_float2(static_cast<float>(ws * e.x), static_cast<float>(ws * e.y));
-            }
-        }
-        // stored activations, spins and weights of the neighbours, then their reverse passes
-        const long x0 = t * xs + q + 1;
-        for (int i = threadIdx.x; i < nb * units; i += blockDim.x)
-            acts[(x0 + i / units) * units + i % units] = actsb[i];
-        for (int i = threadIdx.x; i < nb * nw; i += blockDim.x)
-            xspins[(x0 + i / nw) * nw + i % nw] = sp[(i / nw) * kMaxWords + i % nw];
-        if (threadIdx.x < nb)
-#pragma unroll
-            for (int k = 0; k < NB; k++)
-                if (k == static_cast<int>(threadIdx.x)) alpha[x0 + k] = af[k];
-        backward_multi<NB>(net, angles, in, out, nb, [&](int k, int l, int j, float2 d) {
-            dlts[(x0 + k) * units + net.begin_angle[l] + j] = cmul(af[k], d);
-        });
-        q += nb;
     }
-    er += eor;
-    ei += eoi;
+    for (int q = 0; q < op.num_offdiag; q += NB) {
+        const int nb = min(NB, op.num_offdiag - q);
+        const long x0 = t * xs + q + 1;
+        // a neighbour's layer 0: the sample's moved by the flipped spins, one after the other
+        forward(all, [&](int p, int u) {
+            float2 z[2];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                z[h] = z0s[u];
+                if (2 * p + h >= nb) continue;
+                const int n = op.offdiag[q + 2 * p + h], off = op.flip_off[n];
+                for (int f = 0; f < op.nflip[n]; f++) {
+                    const int site = op.flip_sites[off + f];
+                    z[h] = move_z0(net, site, bit_up(s, site) ? -2.0f : 2.0f, u, z[h]);
+                }
+            }
+            return CPair{pk2(z[0].x, z[1].x), pk2(z[0].y, z[1].y)};
+        }, x0, nb);
+        log_psi(PAIRS);
+        if (warp == 0) {
+            double2 e = make_double2(0.0, 0.0);
+            if (lane < nb) {
+                e = neighbour_term(factor(op.offdiag[q + lane]), lqs[lane], lp);
+                const float2 af = make_float2(static_cast<float>(ws * e.x), static_cast<float>(ws * e.y));
+                afs[lane] = af;
+                alpha[x0 + lane] = af;
+            }
+            for (int k = 0; k < nb; k++) {
+                eor += __shfl_sync(0xffffffffu, e.x, k);
+                eoi += __shfl_sync(0xffffffffu, e.y, k);
+            }
+        }
+        for (int i = tid; i < nb * nw; i += kPairThreads) {
+            const int k = i / nw, word = i - k * nw, n = op.offdiag[q + k];
+            uint64_t v = s[word];
+            for (int f = 0; f < op.nflip[n]; f++) {
+                const int site = op.flip_sites[op.flip_off[n] + f];
+                if ((site >> 6) == word) v ^= 1ull << (site & 63);
+            }
+            xspins[(x0 + k) * nw + word] = v;
+        }
+        __syncthreads();
+        backward(all, x0, nb, false);
+    }
     // the configuration itself last: its coefficient -sum_n e_n (+ 2 E_loc with the
     // sampling term) needs every neighbour's term
-    double2 a = make_double2(-eor, -eoi);
-    if (score) a.x += 2.0 * er;
-    const float2 afs = make_float2(static_cast<float>(ws * a.x), static_cast<float>(ws * a.y));
-    forward_multi<1, true>(net, self_z, in, out, angles, actsb, red, lp1);
     const long xi = t * xs;
-    for (int i = threadIdx.x; i < units; i += blockDim.x) acts[xi * units + i] = actsb[i];
-    if (threadIdx.x < nw) xspins[xi * nw + threadIdx.x] = s[threadIdx.x];
-    if (threadIdx.x == 0) alpha[xi] = afs;
-    backward_multi<1>(net, angles, in, out, 1, [&](int, int l, int j, float2 d) {
-        dlts[xi * units + net.begin_angle[l] + j] = cmul(afs, d);
-        if (score) dltsO[t * units + net.begin_angle[l] + j] = make_float2(wsf * d.x, wsf * d.y);
-    });
-    if (score && threadIdx.x == 0) alphaO[t] = make_float2(wsf, 0.f);
-    if (threadIdx.x == 0) eloc[t] = make_double2(er, ei);
+    if (tid == 0) {
+        er += eor;
+        ei += eoi;
+        double2 a = make_double2(-eor, -eoi);
+        if (score) a.x += 2.0 * er;
+        afs[0] = make_float2(static_cast<float>(ws * a.x), static_cast<float>(ws * a.y));
+        alpha[xi] = afs[0];
+        if (score) alphaO[t] = make_float2(static_cast<float>(ws), 0.f);
+        eloc[t] = make_double2(er, ei);
+    }
+    if (tid < nw) xspins[xi * nw + tid] = s[tid];
+    forward(one, self_z, xi, 1);
+    backward(one, xi, 1, score != 0);
 }
 
 // partial[z][m][n] = sum over the configurations x of split z of D[x][m] * A(x, n), where
@@ -1305,6 +1418,34 @@ static cudaError_t upload(DeepHost* h, const std::vector<T>& v, const T** out) {
     return e;
 }
 
+// dst[at[e]] = src[e]
+__global__ void scatter_entries_kernel(int n, const float2* src, const int* at, float2* dst) {
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) dst[at[e]] = src[e];
+}
+
+// dst[c][r] = src[r][c]
+__global__ void transpose_kernel(int rows, int cols, const float2* src, float2* dst) {
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < rows * cols; e += gridDim.x * blockDim.x)
+        dst[(e % cols) * rows + e / cols] = src[e];
+}
+
+// the layouts formed from the device weights, after an upload or an optimiser step
+int deep_derive(const rbmg_psi* psi) {
+    if (psi->kind == 2) return RBMG_OK;
+    const DeepNetDev& d = psi->deep_dev[0];
+    const int n0 = d.conn[0] * d.size[0];
+    scatter_entries_kernel<<<(n0 + 255) / 256, 256, 0, stream()>>>(n0, d.w[0], d.w0at, const_cast<float2*>(d.w0));
+    RBMG_CK(cudaGetLastError());
+    for (int l = 1; l < d.L; l++) {
+        if (!d.wt[l]) continue;
+        const int n = d.size[l] * d.size[l - 1];
+        transpose_kernel<<<(n + 255) / 256, 256, 0, stream()>>>(d.size[l - 1], d.size[l], d.w[l],
+                                                                const_cast<float2*>(d.wt[l]));
+        RBMG_CK(cudaGetLastError());
+    }
+    return RBMG_OK;
+}
+
 // Device copy of the net(s): part 0 = complex net (PsiDeep) or real part (PsiPair), 1 = imaginary part.
 int deep_upload(rbmg_psi* psi) {
     auto h = std::make_unique<DeepHost>();
@@ -1387,6 +1528,37 @@ int deep_upload(rbmg_psi* psi) {
             RBMG_CK(upload(h.get(), ptr, &d.sptr));
             RBMG_CK(upload(h.get(), q, &d.sq));
         }
+        if (psi->kind != 2) {
+            // layer 0 by spin: a unit's further connections to a spin go to further planes
+            const auto& L0 = psi->layers[0];
+            std::vector<int> at(L0.connections.size());
+            std::vector<int> seen(static_cast<size_t>(psi->N) * L0.size, 0);
+            d.w0n = 1;
+            for (size_t e = 0; e < at.size(); e++) {
+                const size_t cell = static_cast<size_t>(L0.connections[e]) * L0.size + e % L0.size;
+                const int plane = seen[cell]++;
+                d.w0n = std::max(d.w0n, plane + 1);
+                at[e] = static_cast<int>(static_cast<size_t>(plane) * psi->N * L0.size + cell);
+            }
+            RBMG_CK(upload(h.get(), at, &d.w0at));
+            auto w0 = std::make_unique<DevBuf>();
+            const size_t bytes = sizeof(float2) * d.w0n * psi->N * L0.size;
+            RBMG_CK(w0->ensure(bytes));
+            RBMG_CK(cudaMemset(w0->p, 0, bytes));
+            d.w0 = w0->as<float2>();
+            h->bufs.push_back(std::move(w0));
+            for (int l = 1; l < L; l++) {
+                const auto& Ly = psi->layers[l];
+                bool dense = Ly.conn == psi->layers[l - 1].size;
+                for (size_t e = 0; dense && e < Ly.connections.size(); e++)
+                    dense = Ly.connections[e] == e / Ly.size;
+                if (!dense) continue;
+                auto b = std::make_unique<DevBuf>();
+                RBMG_CK(b->ensure(sizeof(float2) * Ly.weights.size()));
+                d.wt[l] = b->as<float2>();
+                h->bufs.push_back(std::move(b));
+            }
+        }
         std::vector<float2> f32(psi->final_weights.size());
         std::vector<double2> f64(psi->final_weights.size());
         for (size_t q = 0; q < f32.size(); q++) {
@@ -1403,6 +1575,11 @@ int deep_upload(rbmg_psi* psi) {
     psi->deep_dev[0] = h->net[0];
     psi->deep_dev[1] = h->net[1];
     psi->deep_host = std::shared_ptr<void>(h.release(), [](void* p) { delete static_cast<DeepHost*>(p); });
+    // the uploads went through the legacy stream, which stream() does not wait for
+    RBMG_CK(cudaStreamSynchronize(cudaStreamLegacy));
+    const int r = deep_derive(psi);
+    if (r != RBMG_OK) return r;
+    RBMG_CK(cudaStreamSynchronize(stream()));
     return RBMG_OK;
 }
 
@@ -1588,32 +1765,32 @@ int deep_adjoint_chunk(const rbmg_psi* psi, const rbmg_operator* op, const Chunk
     const size_t sm = smem_for(net, sizeof(float2), true) + 2 * sizeof(float2) * net.size[0];
     RBMG_CK(set_smem(deep_adjoint_kernel, sm));
     // neighbours per pass of the reverse kernel (RBMG_DEEP_ADJOINT_BATCH = 1, 2, 4 or 8;
-    // default 4), the same outputs
-    int nbatch = 4;
+    // default 8), the same outputs
+    int nbatch = 8;
     if (const char* v = std::getenv("RBMG_DEEP_ADJOINT_BATCH")) nbatch = std::atoi(v);
     if (nbatch != 1 && nbatch != 2 && nbatch != 4 && nbatch != 8)
         return fail(RBMG_EINVAL, "RBMG_DEEP_ADJOINT_BATCH: 1, 2, 4 or 8");
-    const size_t smb = deep_adjoint_multi_smem(net, nbatch);
-    if (nbatch == 2) RBMG_CK(set_smem(deep_adjoint_multi_kernel<2>, smb));
-    if (nbatch == 4) RBMG_CK(set_smem(deep_adjoint_multi_kernel<4>, smb));
-    if (nbatch == 8) RBMG_CK(set_smem(deep_adjoint_multi_kernel<8>, smb));
+    const size_t smb = deep_adjoint_pairs_smem(net, nbatch / 2);
+    if (nbatch == 2) RBMG_CK(set_smem(deep_adjoint_pairs_kernel<1>, smb));
+    if (nbatch == 4) RBMG_CK(set_smem(deep_adjoint_pairs_kernel<2>, smb));
+    if (nbatch == 8) RBMG_CK(set_smem(deep_adjoint_pairs_kernel<4>, smb));
     constexpr int kMaxSplits = 64;
     for (int base = 0; base < c.count; base += chunk) {
         const int cnt = std::min(chunk, c.count - base);
         const uint64_t* sp = c.spins ? c.spins + static_cast<size_t>(base) * nw : nullptr;
         const double* wb = c.weights ? c.weights + base : nullptr;
         if (nbatch == 8)
-            deep_adjoint_multi_kernel<8><<<cnt, threads_for(net), smb, st>>>(
+            deep_adjoint_pairs_kernel<4><<<cnt, kPairThreads, smb, st>>>(
                 net, op->dev(), cnt, sp, c.enum_base + base, c.enumerate, wb, score, d_eloc + base,
                 acts.as<float2>(), dlts.as<float2>(), alpha.as<float2>(), xsp.as<uint64_t>(), xs, dltsO.as<float2>(),
                 alphaO.as<float2>());
         else if (nbatch == 4)
-            deep_adjoint_multi_kernel<4><<<cnt, threads_for(net), smb, st>>>(
+            deep_adjoint_pairs_kernel<2><<<cnt, kPairThreads, smb, st>>>(
                 net, op->dev(), cnt, sp, c.enum_base + base, c.enumerate, wb, score, d_eloc + base,
                 acts.as<float2>(), dlts.as<float2>(), alpha.as<float2>(), xsp.as<uint64_t>(), xs, dltsO.as<float2>(),
                 alphaO.as<float2>());
         else if (nbatch == 2)
-            deep_adjoint_multi_kernel<2><<<cnt, threads_for(net), smb, st>>>(
+            deep_adjoint_pairs_kernel<1><<<cnt, kPairThreads, smb, st>>>(
                 net, op->dev(), cnt, sp, c.enum_base + base, c.enumerate, wb, score, d_eloc + base,
                 acts.as<float2>(), dlts.as<float2>(), alpha.as<float2>(), xsp.as<uint64_t>(), xs, dltsO.as<float2>(),
                 alphaO.as<float2>());
@@ -1699,10 +1876,10 @@ int deep_stream(rbmg_ensemble* e, const rbmg_psi* psi, const rbmg_operator* op, 
     if (const char* v = std::getenv("RBMG_DEEP_WALKERS_PER_BLOCK")) wpc = std::atoi(v);
     if (wpc != 1 && wpc != 2 && wpc != 4 && wpc != 8) return fail(RBMG_EINVAL, "RBMG_DEEP_WALKERS_PER_BLOCK: 1, 2, 4 or 8");
     if (e->fast_sweep_tries != 0 || psi->kind == 2 || n0.ti) wpc = 1;
-    const size_t smm = deep_mc_multi_smem(n0, wpc);
-    if (wpc == 2) RBMG_CK(set_smem(deep_mc_multi_kernel<2>, smm));
-    if (wpc == 4) RBMG_CK(set_smem(deep_mc_multi_kernel<4>, smm));
-    if (wpc == 8) RBMG_CK(set_smem(deep_mc_multi_kernel<8>, smm));
+    const size_t smm = deep_mc_pairs_smem(n0, wpc / 2);
+    if (wpc == 2) RBMG_CK(set_smem(deep_mc_pairs_kernel<1>, smm));
+    if (wpc == 4) RBMG_CK(set_smem(deep_mc_pairs_kernel<2>, smm));
+    if (wpc == 8) RBMG_CK(set_smem(deep_mc_pairs_kernel<4>, smm));
     const int blocks = (B + wpc - 1) / wpc;
     bool first = true;
     for (int row0 = 0; row0 < steps; row0 += rows_per_chunk) {
@@ -1721,11 +1898,11 @@ int deep_stream(rbmg_ensemble* e, const rbmg_psi* psi, const rbmg_operator* op, 
         L.accepts = e->accepts.as<unsigned long long>();
         L.proposals = e->proposals.as<unsigned long long>();
         if (wpc == 2)
-            deep_mc_multi_kernel<2><<<blocks, threads_for(n0), smm, stream()>>>(n0, L);
+            deep_mc_pairs_kernel<1><<<blocks, kPairThreads, smm, stream()>>>(n0, L);
         else if (wpc == 4)
-            deep_mc_multi_kernel<4><<<blocks, threads_for(n0), smm, stream()>>>(n0, L);
+            deep_mc_pairs_kernel<2><<<blocks, kPairThreads, smm, stream()>>>(n0, L);
         else if (wpc == 8)
-            deep_mc_multi_kernel<8><<<blocks, threads_for(n0), smm, stream()>>>(n0, L);
+            deep_mc_pairs_kernel<4><<<blocks, kPairThreads, smm, stream()>>>(n0, L);
         else
             deep_mc_kernel<<<B, threads_for(n0), sm, stream()>>>(n0, n1, psi->kind == 2, L);
         RBMG_CK(cudaGetLastError());

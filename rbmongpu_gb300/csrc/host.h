@@ -116,6 +116,8 @@ namespace rbmg {
 int psi_sync_host(const rbmg_psi* psi);
 int psi_master_ensure(rbmg_psi* psi);
 int psi_scatter(rbmg_psi* psi, const double2* packed);
+// deep.cu: the layouts of a deep net that are derived from its device weights
+int deep_derive(const rbmg_psi* psi);
 // capi.cu: the energy gradient formed on the device, d_grad [P]; energy to value[2]
 int ev_gradient_device(const rbmg_psi* psi, const rbmg_operator* op, rbmg_ensemble* ens, double2* d_grad,
                        double* value);

@@ -124,6 +124,14 @@ struct DeepNetDev {
     // sq[sptr[i] .. sptr[i + 1]) (the single-flip update of its pre-activations)
     const int* sptr;
     const int* sq;
+    // derived from the weights (deep_derive; complex nets): layer 0's weights as w0n planes of
+    // [N][size[0]] (plane d: a unit's d-th connection to the spin, zero where there is none),
+    // entry e of w[0] at w0at[e]; per dense layer l >= 1 (connection c is unit c of the layer
+    // below) its weights transposed, wt[l] [size[l]][size[l - 1]], null otherwise
+    const float2* w0;
+    const int* w0at;
+    int w0n;
+    const float2* wt[3];
 };
 
 // ---- launchers (return cudaError_t) ----

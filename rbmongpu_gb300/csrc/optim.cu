@@ -294,7 +294,7 @@ int psi_scatter(rbmg_psi* psi, const double2* packed) {
     const dim3 grid(std::min(blocks_of(maxc, 256), 64), t.n);
     deep_scatter_kernel<<<grid, 256, 0, stream()>>>(packed, t);
     RBMG_CK(cudaGetLastError());
-    return RBMG_OK;
+    return deep_derive(psi);
 }
 
 }  // namespace rbmg
