@@ -1306,77 +1306,195 @@ __global__ void __launch_bounds__(kPairThreads, 5) deep_adjoint_pairs_kernel(
     backward(one, xi, 1, score != 0);
 }
 
-// partial[z][m][n] = sum over the configurations x of split z of D[x][m] * A(x, n), where
-// D[x][m] = D[x * ldd + m] and A(x, n) = A[x * lda + n] (A_ACTS), +-1 for spin n of the
-// spin row xsp + x * xld (A_SPINS) or 1 (A_ONES).  FP32 products and sums within a split,
-// FP64 partials.
-enum : int { A_ACTS = 0, A_SPINS = 1, A_ONES = 2 };
-template <int AMODE>
-__global__ void __launch_bounds__(256) adj_cgemm_kernel(int K, int M, int Nn, const float2* __restrict__ D, int ldd,
-                                                        const float2* __restrict__ A, int lda,
-                                                        const uint64_t* __restrict__ xsp, int xld, int per_split,
-                                                        double2* __restrict__ partial) {
-    __shared__ float2 sD[32][33];
-    __shared__ float2 sA[32][33];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int m0 = blockIdx.x * 32, n0 = blockIdx.y * 32;
-    const int k0 = blockIdx.z * per_split, k1 = min(K, k0 + per_split);
-    float2 acc[2][2];
+// The configurations of a launch lie in parts of `rows` (the last one shorter); a part is cut
+// into at most kAdjSplits splits of equal length, each an FP32 sum in order.  The sums cancel
+// to a small part of their terms (a configuration's against its neighbours'), so the result
+// depends on this order in its leading digits: it does not change with the launch.
+constexpr int kAdjSplits = 64;
+struct AdjSplit {
+    int k0, k1;   // configurations of split z
+};
+__host__ __device__ inline int adj_splits_of(int K) { return K < 512 ? 1 : (K / 256 < kAdjSplits ? K / 256 : kAdjSplits); }
+__host__ __device__ inline int adj_grid_splits(int K, int rows) {
+    return K <= rows ? adj_splits_of(K) : (K + rows - 1) / rows * kAdjSplits;
+}
+__device__ __forceinline__ AdjSplit adj_split(int K, int rows, int z) {
+    const int part = z / kAdjSplits, q = z - part * kAdjSplits;
+    const int n = min(rows, K - part * rows), splits = adj_splits_of(n), per = (n + splits - 1) / splits;
+    const int k0 = part * rows + min(n, q * per);
+    return AdjSplit{k0, part * rows + min(n, q * per + per)};
+}
+
+// partial[z][m][n] = sum over the configurations x of split z of D[x][m] A(x, n), where
+// D[x][m] = D[x * ldd + m] and A(x, n) = A[x * lda + n], or with SPINS +-1 for spin n of the spin
+// row xsp + x * xld; A(x, Nn) = 1, so that column Nn holds the bias sums.  A thread holds 4 x 4
+// (SPINS: 4 x 8) products, so that 16-byte shared loads keep up with the FP32 pipe (2 x 2 with
+// 8-byte loads, and the biases as a product of their own, took 22.5 ms for 8192 samples of the
+// 100-200-100-50 net); stages of 16 configurations arrive by asynchronous copies while the
+// one before is used.  Bound by the FP32 pipe, six operations a product: 11.3 ms.
+constexpr int kAdjStage = 16, kAdjTm = 32;
+
+template <bool SPINS>
+__global__ void __launch_bounds__(128) adj_cgemm_kernel(int K, int rows, int M, int Nn, const float2* __restrict__ D,
+                                                        int ldd, const float2* __restrict__ A, int lda,
+                                                        const uint64_t* __restrict__ xsp, int xld,
+                                                        float2* __restrict__ partial) {
+    constexpr int JN = SPINS ? 8 : 4, TN = 16 * JN;
+    using Elem = std::conditional_t<SPINS, float, float2>;
+    __shared__ __align__(16) float2 sD[2][kAdjStage][kAdjTm];
+    __shared__ __align__(16) Elem sA[2][kAdjStage][TN];
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int m0 = blockIdx.x * kAdjTm, n0 = blockIdx.y * TN;
+    const AdjSplit sp = adj_split(K, rows, blockIdx.z);
+    float2 acc[4][JN];
 #pragma unroll
-    for (int i = 0; i < 2; i++)
+    for (int i = 0; i < 4; i++)
 #pragma unroll
-        for (int j = 0; j < 2; j++) acc[i][j] = make_float2(0.f, 0.f);
-    for (int kb = k0; kb < k1; kb += 32) {
-        for (int e = threadIdx.x; e < 32 * 32; e += 256) {
-            const int kk = e >> 5, c = e & 31;
-            const int x = kb + kk;
-            const bool ok = x < k1;
-            sD[kk][c] = (ok && m0 + c < M) ? D[static_cast<long>(x) * ldd + m0 + c] : make_float2(0.f, 0.f);
-            float2 av = make_float2(0.f, 0.f);
-            if (ok && n0 + c < Nn) {
-                if (AMODE == A_ACTS) av = A[static_cast<long>(x) * lda + n0 + c];
-                else if (AMODE == A_SPINS) {
-                    const int i = n0 + c;
-                    av.x = ((xsp[static_cast<long>(x) * xld + (i >> 6)] >> (i & 63)) & 1ull) ? 1.f : -1.f;
-                } else av.x = 1.f;
+        for (int j = 0; j < JN; j++) acc[i][j] = make_float2(0.f, 0.f);
+    // 8-byte asynchronous copies (rows are 8-byte aligned); outside the matrix zeros are written
+    auto copy = [](float2* dst, const float2* src, bool live) {
+        const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(live ? 8 : 0) : "memory");
+    };
+    auto stage = [&](int s, int kb) {
+        for (int e = tid; e < kAdjStage * kAdjTm; e += 128) {
+            const int kk = e / kAdjTm, c = e % kAdjTm, x = kb + kk;
+            const bool live = x < sp.k1 && m0 + c < M;
+            copy(&sD[s][kk][c], live ? D + static_cast<long>(x) * ldd + m0 + c : D, live);
+        }
+        for (int e = tid; e < kAdjStage * TN; e += 128) {
+            const int kk = e / TN, c = e % TN, x = kb + kk, n = n0 + c;
+            const bool row = x < sp.k1;
+            if constexpr (SPINS) {
+                float v = 0.0f;
+                if (row && n < Nn) v = ((xsp[static_cast<long>(x) * xld + (n >> 6)] >> (n & 63)) & 1ull) ? 1.0f : -1.0f;
+                else if (row && n == Nn) v = 1.0f;
+                sA[s][kk][c] = v;
+            } else {
+                const bool live = row && n < Nn;
+                if (n == Nn) sA[s][kk][c] = make_float2(1.0f, 0.0f);   // past the split D is zero
+                else copy(&sA[s][kk][c], live ? A + static_cast<long>(x) * lda + n : A, live);
             }
-            sA[kk][c] = av;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    stage(0, sp.k0);
+    for (int kb = sp.k0, s = 0; kb < sp.k1; kb += kAdjStage, s ^= 1) {
+        if (kb + kAdjStage < sp.k1) {
+            stage(s ^ 1, kb + kAdjStage);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
         }
         __syncthreads();
-#pragma unroll 8
-        for (int kk = 0; kk < 32; kk++) {
-            const float2 d0 = sD[kk][ty], d1 = sD[kk][ty + 16];
-            const float2 a0 = sA[kk][tx], a1 = sA[kk][tx + 16];
-            acc[0][0] = cadd(acc[0][0], cmul(d0, a0));
-            acc[0][1] = cadd(acc[0][1], cmul(d0, a1));
-            acc[1][0] = cadd(acc[1][0], cmul(d1, a0));
-            acc[1][1] = cadd(acc[1][1], cmul(d1, a1));
+#pragma unroll 4
+        for (int kk = 0; kk < kAdjStage; kk++) {
+            float2 d[4];
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const float4 v = *reinterpret_cast<const float4*>(&sD[s][kk][4 * ty + 2 * i]);
+                d[2 * i] = make_float2(v.x, v.y);
+                d[2 * i + 1] = make_float2(v.z, v.w);
+            }
+            if constexpr (SPINS) {
+                // columns 4 tx .. 4 tx + 3 and these + 64
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const float4 g4 = *reinterpret_cast<const float4*>(&sA[s][kk][4 * tx + 64 * h]);
+                    const float g[4] = {g4.x, g4.y, g4.z, g4.w};
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {   // g = +-1: cmul's products are exact
+                            acc[i][4 * h + j].x = fmaf(g[j], d[i].x, acc[i][4 * h + j].x);
+                            acc[i][4 * h + j].y = fmaf(g[j], d[i].y, acc[i][4 * h + j].y);
+                        }
+                }
+            } else {
+                // columns 2 tx, 2 tx + 1 and these + 32: neighbouring lanes read neighbouring 16 bytes
+                float2 a[4];
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const float4 v = *reinterpret_cast<const float4*>(&sA[s][kk][2 * tx + 32 * h]);
+                    a[2 * h] = make_float2(v.x, v.y);
+                    a[2 * h + 1] = make_float2(v.z, v.w);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++) acc[i][j] = cadd(acc[i][j], cmul(d[i], a[j]));
+            }
         }
         __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < 2; i++)
+    for (int i = 0; i < 4; i++)
 #pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const int m = m0 + ty + 16 * i, n = n0 + tx + 16 * j;
-            if (m < M && n < Nn)
-                partial[(static_cast<long>(blockIdx.z) * M + m) * Nn + n] =
-                    make_double2(acc[i][j].x, acc[i][j].y);
+        for (int j = 0; j < JN; j++) {
+            const int m = m0 + 4 * ty + i, n = n0 + (SPINS ? 4 * tx + 64 * (j >> 2) + (j & 3) : 2 * tx + 32 * (j >> 1) + (j & 1));
+            if (m < M && n <= Nn) partial[(static_cast<long>(blockIdx.z) * M + m) * (Nn + 1) + n] = acc[i][j];
         }
 }
 
-// G[m][n] += sum over splits (in order) of partial[z][m][n]
-__global__ void adj_split_sum_kernel(int M, int Nn, int splits, const double2* __restrict__ partial, double2* G) {
-    const long t = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (t >= static_cast<long>(M) * Nn) return;
-    double2 a = make_double2(0.0, 0.0);
-    for (int z = 0; z < splits; z++) {
-        const double2 v = partial[static_cast<long>(z) * M * Nn + t];
-        a.x += v.x;
-        a.y += v.y;
+// the final weights' sums: partial[z][j] = sum over split z of alpha[x] A[x * lda + j], in order
+// by one warp from rows that the block stages (the serial sum read from memory took 800 us for
+// 8192 samples of the 100-200-100-50 net)
+__global__ void __launch_bounds__(256) adj_final_kernel(int K, int rows, int last, const float2* __restrict__ alpha,
+                                                        const float2* __restrict__ A, int lda,
+                                                        float2* __restrict__ partial) {
+    constexpr int kRows = 64;
+    __shared__ float2 tile[2][kRows][32];
+    __shared__ float2 al[2][kRows];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = blockIdx.x * 32 + lane;
+    const AdjSplit sp = adj_split(K, rows, blockIdx.y);
+    float2 a = make_float2(0.f, 0.f);
+    float2 v[kRows / 8], w = make_float2(0.f, 0.f);
+    auto load = [&](int x0) {
+#pragma unroll
+        for (int q = 0; q < kRows / 8; q++) {
+            const int x = x0 + warp + 8 * q;
+            v[q] = x < sp.k1 && j < last ? A[static_cast<long>(x) * lda + j] : make_float2(0.f, 0.f);
+        }
+        if (threadIdx.x < kRows && x0 + static_cast<int>(threadIdx.x) < sp.k1) w = alpha[x0 + threadIdx.x];
+    };
+    load(sp.k0);
+    for (int x0 = sp.k0, s = 0; x0 < sp.k1; x0 += kRows, s ^= 1) {
+#pragma unroll
+        for (int q = 0; q < kRows / 8; q++) tile[s][warp + 8 * q][lane] = v[q];
+        if (threadIdx.x < kRows) al[s][threadIdx.x] = w;
+        __syncthreads();
+        if (x0 + kRows < sp.k1) load(x0 + kRows);
+        if (warp == 0)
+            for (int q = 0; q < min(kRows, sp.k1 - x0); q++) a = cadd(a, cmul(al[s][q], tile[s][q][lane]));
     }
-    G[t].x += a.x;
-    G[t].y += a.y;
+    if (warp == 0 && j < last) partial[static_cast<long>(blockIdx.y) * last + j] = a;
+}
+
+// G[m][n] (n < Nn) and Gb[m] (column Nn) += sum over splits of partial[z][m][n], in FP64: eight
+// slices of the splits, then the slices in order.  `cols` = Nn + 1, or Nn with no bias column.
+__global__ void __launch_bounds__(256) adj_split_sum_kernel(int M, int Nn, int cols, int splits,
+                                                            const float2* __restrict__ partial, double2* G,
+                                                            double2* Gb) {
+    __shared__ double2 red[8][32];
+    const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
+    const long total = static_cast<long>(M) * cols, e = blockIdx.x * 32L + lane;
+    double2 a = make_double2(0.0, 0.0);
+    if (e < total) {
+        const int per = (splits + 7) / 8, z1 = min(splits, (slice + 1) * per);
+#pragma unroll 8
+        for (int z = slice * per; z < z1; z++) {
+            const float2 v = partial[z * total + e];
+            a.x += v.x;
+            a.y += v.y;
+        }
+    }
+    red[slice][lane] = a;
+    __syncthreads();
+    if (slice != 0 || e >= total) return;
+    for (int q = 1; q < 8; q++) a = cadd(a, red[q][lane]);
+    const int m = static_cast<int>(e / cols), n = static_cast<int>(e - static_cast<long>(m) * cols);
+    double2* out = n < Nn ? G + static_cast<long>(m) * Nn + n : Gb + m;
+    *out = cadd(*out, a);
 }
 
 int threads_for(const DeepNetDev& n) {
@@ -1755,7 +1873,11 @@ int deep_adjoint_chunk(const rbmg_psi* psi, const rbmg_operator* op, const Chunk
     static thread_local DevBuf acts, dlts, alpha, xsp, dltsO, alphaO, partial;
     const size_t per_sample = static_cast<size_t>(xs) * (2 * sizeof(float2) * net.units + sizeof(float2) + 8 * nw) +
                               sizeof(float2) * (net.units + 1);
-    const int chunk = std::max(1, static_cast<int>(std::min<size_t>(c.count, (size_t(768) << 20) / per_sample)));
+    // parts of the FP32 sums (AdjSplit), and as many of them per launch as fit 4 GB of the
+    // stored activations and errors
+    const int part = std::max(1, static_cast<int>(std::min<size_t>(c.count, (size_t(768) << 20) / per_sample)));
+    const int chunk = static_cast<int>(std::min<size_t>(
+        c.count, static_cast<size_t>(part) * std::max<size_t>(1, (size_t(4) << 30) / (per_sample * part))));
     RBMG_CK(acts.ensure(sizeof(float2) * static_cast<size_t>(chunk) * xs * net.units));
     RBMG_CK(dlts.ensure(sizeof(float2) * static_cast<size_t>(chunk) * xs * net.units));
     RBMG_CK(alpha.ensure(sizeof(float2) * static_cast<size_t>(chunk) * xs));
@@ -1774,7 +1896,6 @@ int deep_adjoint_chunk(const rbmg_psi* psi, const rbmg_operator* op, const Chunk
     if (nbatch == 2) RBMG_CK(set_smem(deep_adjoint_pairs_kernel<1>, smb));
     if (nbatch == 4) RBMG_CK(set_smem(deep_adjoint_pairs_kernel<2>, smb));
     if (nbatch == 8) RBMG_CK(set_smem(deep_adjoint_pairs_kernel<4>, smb));
-    constexpr int kMaxSplits = 64;
     for (int base = 0; base < c.count; base += chunk) {
         const int cnt = std::min(chunk, c.count - base);
         const uint64_t* sp = c.spins ? c.spins + static_cast<size_t>(base) * nw : nullptr;
@@ -1800,52 +1921,43 @@ int deep_adjoint_chunk(const rbmg_psi* psi, const rbmg_operator* op, const Chunk
                 acts.as<float2>(), dlts.as<float2>(), alpha.as<float2>(), xsp.as<uint64_t>(), xs, dltsO.as<float2>(),
                 alphaO.as<float2>());
         RBMG_CK(cudaGetLastError());
-        // reduce over K configurations whose rows are `stride` configurations apart
-        auto reduce = [&](int K, int amode, int M, int Nn, const float2* D, int ldd, const float2* A, int lda, int xld,
-                          double2* out) -> int {
-            const int splits = std::min(kMaxSplits, std::max(1, K / 256));
-            const int per = (K + splits - 1) / splits;
-            RBMG_CK(partial.ensure(sizeof(double2) * static_cast<size_t>(splits) * M * Nn));
-            const dim3 grid((M + 31) / 32, (Nn + 31) / 32, splits);
-            if (amode == A_ACTS)
-                adj_cgemm_kernel<A_ACTS><<<grid, 256, 0, st>>>(K, M, Nn, D, ldd, A, lda, xsp.as<uint64_t>(), xld, per,
-                                                                partial.as<double2>());
-            else if (amode == A_SPINS)
-                adj_cgemm_kernel<A_SPINS><<<grid, 256, 0, st>>>(K, M, Nn, D, ldd, A, lda, xsp.as<uint64_t>(), xld, per,
-                                                                 partial.as<double2>());
-            else
-                adj_cgemm_kernel<A_ONES><<<grid, 256, 0, st>>>(K, M, Nn, D, ldd, A, lda, xsp.as<uint64_t>(), xld, per,
-                                                                partial.as<double2>());
-            RBMG_CK(cudaGetLastError());
-            const long tot = static_cast<long>(M) * Nn;
-            adj_split_sum_kernel<<<static_cast<unsigned>((tot + 255) / 256), 256, 0, st>>>(M, Nn, splits,
-                                                                                         partial.as<double2>(), out);
-            RBMG_CK(cudaGetLastError());
-            return RBMG_OK;
+        auto sum = [&](int M, int Nn, int cols, int splits, double2* out, double2* bias) -> cudaError_t {
+            const long total = static_cast<long>(M) * cols;
+            adj_split_sum_kernel<<<static_cast<unsigned>((total + 31) / 32), 256, 0, st>>>(M, Nn, cols, splits,
+                                                                                         partial.as<float2>(), out, bias);
+            return cudaGetLastError();
         };
         // pass 0: all configurations with alpha-weighted deltas -> G; pass 1 (score): the
         // samples themselves with weight w_s -> GO
         for (int pass = 0; pass < (score ? 2 : 1); pass++) {
-            const int K = pass == 0 ? cnt * xs : cnt;
+            const int K = pass == 0 ? cnt * xs : cnt, rows = pass == 0 ? part * xs : part;
+            const int splits = adj_grid_splits(K, rows);
             const int row = pass == 0 ? net.units : xs * net.units;     // activation row stride
             const float2* dl = pass == 0 ? dlts.as<float2>() : dltsO.as<float2>();
             double2* out = pass == 0 ? G : GO;
             for (int l = 0; l < net.L; l++) {
-                const int size = net.size[l];
-                const int in = l == 0 ? net.N : net.size[l - 1];
-                const float2* D = dl + net.begin_angle[l];
-                int r = l == 0 ? reduce(K, A_SPINS, size, in, D, net.units, nullptr, 0, pass == 0 ? nw : xs * nw,
-                                        out + goff[2 * l])
-                               : reduce(K, A_ACTS, size, in, D, net.units, acts.as<float2>() + net.begin_angle[l - 1],
-                                        row, 0, out + goff[2 * l]);
-                if (r != RBMG_OK) return r;
-                r = reduce(K, A_ONES, size, 1, D, net.units, nullptr, 0, 0, out + goff[2 * l + 1]);
-                if (r != RBMG_OK) return r;
+                const int size = net.size[l], in = l == 0 ? net.N : net.size[l - 1];
+                RBMG_CK(partial.ensure(sizeof(float2) * static_cast<size_t>(splits) * size * (in + 1)));
+                const int tn = l == 0 ? 128 : 64;
+                const dim3 grid((size + kAdjTm - 1) / kAdjTm, (in + tn) / tn, splits);
+                if (l == 0)
+                    adj_cgemm_kernel<true><<<grid, 128, 0, st>>>(K, rows, size, in, dl, net.units, nullptr, 0,
+                                                                  xsp.as<uint64_t>(), pass == 0 ? nw : xs * nw,
+                                                                  partial.as<float2>());
+                else
+                    adj_cgemm_kernel<false><<<grid, 128, 0, st>>>(
+                        K, rows, size, in, dl + net.begin_angle[l], net.units, acts.as<float2>() + net.begin_angle[l - 1], row,
+                        nullptr, 0, partial.as<float2>());
+                RBMG_CK(cudaGetLastError());
+                RBMG_CK(sum(size, in, in + 1, splits, out + goff[2 * l], out + goff[2 * l + 1]));
             }
             const int last = net.size[net.L - 1];
-            const int r = reduce(K, A_ACTS, 1, last, pass == 0 ? alpha.as<float2>() : alphaO.as<float2>(), 1,
-                                 acts.as<float2>() + net.begin_angle[net.L - 1], row, 0, out + goff[2 * net.L]);
-            if (r != RBMG_OK) return r;
+            RBMG_CK(partial.ensure(sizeof(float2) * static_cast<size_t>(splits) * last));
+            adj_final_kernel<<<dim3((last + 31) / 32, splits), 256, 0, st>>>(
+                K, rows, last, pass == 0 ? alpha.as<float2>() : alphaO.as<float2>(),
+                acts.as<float2>() + net.begin_angle[net.L - 1], row, partial.as<float2>());
+            RBMG_CK(cudaGetLastError());
+            RBMG_CK(sum(1, last, last, splits, out + goff[2 * net.L], nullptr));
         }
     }
     return RBMG_OK;
