@@ -247,63 +247,7 @@ __device__ __forceinline__ bool rbm_mh_step2(const RbmDev& P, Spins<NW>& s, pair
                 ti[kk] = fma2(two_s[q], pk2(w.z, w.w), ti[kk]);
             }
             // lc_re2 of the new angles, formed by the same operations: kept from the proposal
-            // where the registers allow (the larger layers take rbm_mc_smem_kernel's buffers)
-            re[kk] = K <= 8 ? fnew[kk] : lc_re2(tr[kk], ti[kk]);
-        }
-    }
-    return accept;
-}
-
-// The single-flip proposal of rbm_mh_step2 with the walker's angles and Re f in this
-// warp's shared-memory slice st [4][KP][32] pairs (theta re, theta im, Re f in two buffers)
-// instead of registers: the same operations in the same order, so the same chain bit for
-// bit.  It frees ~3 KP registers per lane, which for the large hidden layers lets more warps
-// stay resident to hide the dependent chain of each proposal.  Buffer cur holds the walker's
-// Re f.  KEEP: the proposal writes its Re f(theta') into the other buffer, and an accepted
-// move takes that buffer as is (the values that recomputing from the new angles gives, bit
-// for bit) and only advances the angles; otherwise an accepted move recomputes Re f in
-// place.  Keeping costs KP stores per proposal and a quarter more shared memory (less L1 for
-// the W rows), and saves KP activations per acceptance: measured on N = 100, M = 416 and
-// 16384 walkers, 10 sweeps take 12.60 ms kept against 13.26 ms recomputed at an acceptance
-// of 0.235 (sigma 0.05 weights), but 12.44 against 11.79 ms at 0.026 (sigma 0.1).  The
-// sampler keeps; a per-warp switch on the running acceptance measured worse in both cases.
-template <int K, int KP, bool KEEP, int NW>
-__device__ __forceinline__ bool rbm_flip_step_s(const RbmDev& P, Spins<NW>& s, pair_t* st, int& cur, WarpRng& rng,
-                                                int lane, uint64_t nmagic) {
-    const int site = static_cast<int>(fastmod(rng.next(), nmagic, static_cast<uint32_t>(P.N)));
-    const pair_t two_s = splat2(s.up(site) ? -2.0f : 2.0f);   // 2 x the new spin
-    const float4* row = P.Wq + static_cast<long>(site) * KP * 32 + lane;
-    pair_t* re = st + (2 + cur) * KP * 32 + lane;
-    pair_t* re_new = st + (3 - cur) * KP * 32 + lane;
-    float4 w[KP];
-#pragma unroll
-    for (int kk = 0; kk < KP; kk++) w[kk] = __ldg(row + 32 * kk);
-    float part = 0.0f;
-#pragma unroll
-    for (int kk = 0; kk < KP; kk++) {
-        const pair_t nr = fma2(two_s, pk2(w[kk].x, w[kk].y), st[kk * 32 + lane]);
-        const pair_t ni = fma2(two_s, pk2(w[kk].z, w[kk].w), st[(KP + kk) * 32 + lane]);
-        const pair_t f = lc_re2(nr, ni);
-        if (KEEP) re_new[kk * 32] = f;
-        float d0, d1;
-        up2(sub2(f, re[kk * 32]), d0, d1);
-        part = __fadd_rn(part, d0);
-        if (2 * kk + 1 < K) part = __fadd_rn(part, d1);
-    }
-    const float delta = warp_sum_xor(part);
-    bool accept = delta > 0.0f;
-    if (!accept) accept = rng.uniform() <= expf_det(__fmul_rn(2.0f, delta));
-    if (accept) {
-        s.flip(site);
-        if (KEEP) cur ^= 1;
-#pragma unroll
-        for (int kk = 0; kk < KP; kk++) {
-            const float4 ww = __ldg(row + 32 * kk);
-            const pair_t tr = fma2(two_s, pk2(ww.x, ww.y), st[kk * 32 + lane]);
-            const pair_t ti = fma2(two_s, pk2(ww.z, ww.w), st[(KP + kk) * 32 + lane]);
-            st[kk * 32 + lane] = tr;
-            st[(KP + kk) * 32 + lane] = ti;
-            if (!KEEP) re[kk * 32] = lc_re2(tr, ti);
+            re[kk] = fnew[kk];
         }
     }
     return accept;
@@ -512,7 +456,7 @@ __device__ __forceinline__ double2 warp_log_psi(const float2 (&f)[K]) {
 // the sampler's register footprint to the walker state.
 // ---------------------------------------------------------------------------
 template <int K, int NW>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, K > 13 ? 3 : 4) rbm_mc_kernel(RbmDev P, McLaunch L) {
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, 4) rbm_mc_kernel(RbmDev P, McLaunch L) {
     const int lane = threadIdx.x & 31;
     const int w = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     if (w >= L.B) return;
@@ -560,66 +504,6 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, K > 13 ? 3 : 4) rbm_mc_ke
     }
 }
 
-// The sampler for large hidden layers (K >= 13) without the S_z constraint: the walker
-// state in shared memory (rbm_flip_step_s), 6 blocks of 4 warps per SM instead of 4 (3).
-// Chains, samples and counters are those of rbm_mc_kernel.
-template <int K, int NW>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, 6) rbm_mc_smem_kernel(RbmDev P, McLaunch L) {
-    const int lane = threadIdx.x & 31;
-    const int w = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-    if (w >= L.B) return;
-    constexpr int KP = (K + 1) / 2;
-    extern __shared__ pair_t s_state[];
-    pair_t* st = s_state + (threadIdx.x >> 5) * 4 * KP * 32;
-    int cur = 0;
-    WarpRng rng;
-    rng.init(L.seed, L.walker_base + static_cast<uint32_t>(w), L.rng_index[w], lane);
-    const uint64_t nmagic = fastmod_magic(static_cast<uint32_t>(P.N));
-    Spins<NW> s;
-    if (L.init) {
-#pragma unroll
-        for (int k = 0; k < NW; k++) s.w[k] = 0;
-        draw_spins(rng, P.N, s);
-    } else {
-#pragma unroll
-        for (int k = 0; k < NW; k++) s.w[k] = L.spins[static_cast<long>(w) * NW + k];
-    }
-    unsigned long long acc = 0, props = 0;
-    const int total_sweeps = L.n_therm + L.n_samples * L.sweeps_per_sample;
-    int sample = 0;
-    for (int sw = 0; sw < total_sweeps; sw++) {
-        {
-            pair_t tr[KP], ti[KP];
-            rbm_refresh2(P, s, tr, ti, lane);
-            cur = 0;
-#pragma unroll
-            for (int kk = 0; kk < KP; kk++) {
-                st[kk * 32 + lane] = tr[kk];
-                st[(KP + kk) * 32 + lane] = ti[kk];
-                st[(2 * KP + kk) * 32 + lane] = lc_re2(tr[kk], ti[kk]);
-            }
-        }
-        for (int p = 0; p < P.N; p++) acc += rbm_flip_step_s<K, KP, true>(P, s, st, cur, rng, lane, nmagic);
-        props += P.N;
-        const int done = sw + 1 - L.n_therm;
-        if (done > 0 && done % L.sweeps_per_sample == 0) {
-            const long row = static_cast<long>(L.sample_base + sample) * L.B + w;
-            if (L.sample_spins && lane == 0) {
-#pragma unroll
-                for (int k = 0; k < NW; k++) L.sample_spins[row * NW + k] = s.w[k];
-            }
-            sample++;
-        }
-    }
-    if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < NW; k++) L.spins[static_cast<long>(w) * NW + k] = s.w[k];
-        L.rng_index[w] = rng.index;
-        L.accepts[w] += acc;
-        L.proposals[w] += props;
-    }
-}
-
 // ---------------------------------------------------------------------------
 // The sampler with several walkers per warp: G lanes share a walker (rbm_group), each with
 // PP = 16 K / G pairs of hidden units.  What a proposal does once per walker -- the random words,
@@ -634,9 +518,13 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, 6) rbm_mc_smem_kernel(Rbm
 // 38 / 24, 124 / 76; N = 64, M = 128: 33 / 32, 97 / 72, 344 / 233.  Blocks of one, two or four
 // warps and keeping the proposed angles measured alike; G = 8 at K = 2 and 4 (G = 4 at K = 1)
 // was slower up to 4096 walkers (K = 4: 33 / 57 at 16, 97 / 75) and gained 6 % at 16384.
+// Large layers have the registers of three (K = 13) and two (K = 18) blocks an SM; against one
+// walker a warp with its state in shared memory, K = 13 (N = 100, M = 400): 155 / 149 at 16, 388 /
+// 365 at 4096, 1253 / 1120 at 16384; K = 18 (N = 140, M = 576): 330 / 253, 832 / 667, 2421 / 2281.
+// With four blocks and spills K = 13 took 250 and 1239; state in shared memory here, the same.
 // ---------------------------------------------------------------------------
 template <int K, int G, int NW, bool SZ>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, 4) rbm_mc_group_kernel(RbmDev P, McLaunch L) {
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, K >= 18 ? 2 : (K >= 13 ? 3 : 4)) rbm_mc_group_kernel(RbmDev P, McLaunch L) {
     constexpr int H = 16 / G, PP = K * H, PW = 32 / G;   // PW walkers per warp
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, g = lane % G;
     const int w0 = (blockIdx.x * kWarpsPerBlock + wib) * PW;
@@ -1166,37 +1054,10 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) rbm_eloc_t_kernel(RbmDev 
 // ---------------------------------------------------------------------------
 // launchers for this K (instantiated by rbm_k<K>.cu)
 // ---------------------------------------------------------------------------
-// Several walkers per warp: always up to K = 4; at K = 8 (N = 90, M = 250) from 2048 walkers on
-// (66 / 78 us a sweep at 16, 79 / 81 at 1024, 119 / 105 at 2048, 730 / 595 at 16384, one walker
-// a warp / grouped); not above (K = 13, N = 100, M = 400: 158 / 250 at 256, 1251 / 1239 at 16384
-// with the state in shared memory, K = 18: 2425 / 2766 at 16384)
-constexpr bool rbm_grouped(int K, int walkers) { return K <= 4 || (K == 8 && walkers >= 2048); }
-
-// one walker per warp (K > 4)
-template <int K>
-cudaError_t rbm_mc_wide_launch_k(const RbmDev& P, const McLaunch& L, dim3 grid, dim3 block, cudaStream_t st) {
-    const int nw = (P.N + 63) / 64;
-    if (K >= 13 && !L.total_z) {
-        constexpr int KP = (K + 1) / 2;
-        const size_t sm = sizeof(pair_t) * 4 * KP * 32 * kWarpsPerBlock;
-        switch (nw) {
-            case 1: rbm_mc_smem_kernel<K, 1><<<grid, block, sm, st>>>(P, L); break;
-            case 2: rbm_mc_smem_kernel<K, 2><<<grid, block, sm, st>>>(P, L); break;
-            case 3: rbm_mc_smem_kernel<K, 3><<<grid, block, sm, st>>>(P, L); break;
-            case 4: rbm_mc_smem_kernel<K, 4><<<grid, block, sm, st>>>(P, L); break;
-            default: return cudaErrorInvalidValue;
-        }
-        return cudaGetLastError();
-    }
-    switch (nw) {
-        case 1: rbm_mc_kernel<K, 1><<<grid, block, 0, st>>>(P, L); break;
-        case 2: rbm_mc_kernel<K, 2><<<grid, block, 0, st>>>(P, L); break;
-        case 3: rbm_mc_kernel<K, 3><<<grid, block, 0, st>>>(P, L); break;
-        case 4: rbm_mc_kernel<K, 4><<<grid, block, 0, st>>>(P, L); break;
-        default: return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
-}
+// Several walkers per warp, except at K = 8 with few walkers, where a lane's sixteen units in
+// sequence take longer than the shared work saves (N = 90, M = 250, one walker a warp / grouped:
+// 66 / 78 us a sweep at 16 walkers, 79 / 81 at 1024, 119 / 105 at 2048, 730 / 595 at 16384)
+constexpr bool rbm_grouped(int K, int walkers) { return K != 8 || walkers >= 2048; }
 
 template <int K>
 cudaError_t rbm_mc_launch_k(const RbmDev& P, const OpDev* op, const McLaunch& L, cudaStream_t st) {
@@ -1214,21 +1075,28 @@ cudaError_t rbm_mc_launch_k(const RbmDev& P, const OpDev* op, const McLaunch& L,
         }
         return cudaGetLastError();
     }
-    if constexpr (K <= 8) {
-        if (rbm_grouped(K, L.B)) {
-            constexpr int G = rbm_group(K), per_block = kWarpsPerBlock * 32 / G;
-            const dim3 blocks((L.B + per_block - 1) / per_block);
-            if (L.total_z && nw != 1) return cudaErrorInvalidValue;
-            if (L.total_z) rbm_mc_group_kernel<K, G, 1, true><<<blocks, block, 0, st>>>(P, L);
-            else if (nw == 1) rbm_mc_group_kernel<K, G, 1, false><<<blocks, block, 0, st>>>(P, L);
-            else if (nw == 2) rbm_mc_group_kernel<K, G, 2, false><<<blocks, block, 0, st>>>(P, L);
-            else if (nw == 3) rbm_mc_group_kernel<K, G, 3, false><<<blocks, block, 0, st>>>(P, L);
-            else if (nw == 4) rbm_mc_group_kernel<K, G, 4, false><<<blocks, block, 0, st>>>(P, L);
-            else return cudaErrorInvalidValue;
-            return cudaGetLastError();
-        }
+    if (rbm_grouped(K, L.B)) {
+        constexpr int G = rbm_group(K), per_block = kWarpsPerBlock * 32 / G;
+        const dim3 blocks((L.B + per_block - 1) / per_block);
+        if (L.total_z && nw != 1) return cudaErrorInvalidValue;
+        if (L.total_z) rbm_mc_group_kernel<K, G, 1, true><<<blocks, block, 0, st>>>(P, L);
+        else if (nw == 1) rbm_mc_group_kernel<K, G, 1, false><<<blocks, block, 0, st>>>(P, L);
+        else if (nw == 2) rbm_mc_group_kernel<K, G, 2, false><<<blocks, block, 0, st>>>(P, L);
+        else if (nw == 3) rbm_mc_group_kernel<K, G, 3, false><<<blocks, block, 0, st>>>(P, L);
+        else if (nw == 4) rbm_mc_group_kernel<K, G, 4, false><<<blocks, block, 0, st>>>(P, L);
+        else return cudaErrorInvalidValue;
+        return cudaGetLastError();
     }
-    if constexpr (K > 4) return rbm_mc_wide_launch_k<K>(P, L, grid, block, st);
+    if constexpr (K == 8) {   // one walker per warp
+        switch (nw) {
+            case 1: rbm_mc_kernel<K, 1><<<grid, block, 0, st>>>(P, L); break;
+            case 2: rbm_mc_kernel<K, 2><<<grid, block, 0, st>>>(P, L); break;
+            case 3: rbm_mc_kernel<K, 3><<<grid, block, 0, st>>>(P, L); break;
+            case 4: rbm_mc_kernel<K, 4><<<grid, block, 0, st>>>(P, L); break;
+            default: return cudaErrorInvalidValue;
+        }
+        return cudaGetLastError();
+    }
     return cudaErrorInvalidValue;
 }
 
