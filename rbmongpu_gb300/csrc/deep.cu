@@ -17,6 +17,7 @@
 
 #include "device_math.cuh"
 #include "host.h"
+#include "math64.cuh"
 #include "reduce.h"
 
 namespace rbmg {
@@ -48,7 +49,8 @@ template <typename V> __device__ __forceinline__ V creal(double x);
 template <> __device__ __forceinline__ float2 creal<float2>(double x) { return make_float2(float(x), 0.f); }
 template <> __device__ __forceinline__ double2 creal<double2>(double x) { return make_double2(x, 0.0); }
 
-__device__ __forceinline__ double2 lc64(double2 z) {
+// the activation in the reference's order of operations (math64.cuh has the faster form)
+__device__ __forceinline__ double2 lc64_plain(double2 z) {
     const double s = z.x > 0.0 ? 1.0 : -1.0;
     double2 t = make_double2(s * 3.746646023906276 + z.x, z.y);
     t = cmul(z, t); t.x += 7.771429504240965;
@@ -66,7 +68,7 @@ template <bool REAL> __device__ __forceinline__ float2 act(float2 a) {
     return REAL ? make_float2(a.x > 0.f ? a.x : 0.f, 0.f) : lc_c(a.x, a.y);
 }
 template <bool REAL> __device__ __forceinline__ double2 act(double2 a) {
-    return REAL ? make_double2(a.x > 0.0 ? a.x : 0.0, 0.0) : lc64(a);
+    return REAL ? make_double2(a.x > 0.0 ? a.x : 0.0, 0.0) : lc64_plain(a);
 }
 // derivative: my_tanh for complex nets, 1 for the real nets (psi_functions.hpp:127-136)
 template <bool REAL> __device__ __forceinline__ float2 dact(float2 a) {
@@ -410,6 +412,7 @@ __global__ void deep_eloc_kernel(DeepNetDev n0, DeepNetDev n1, int pair, DeepNet
             continue;
         }
         const V lq = state_log_psi<V>(n0, n1, pair, sp, w, shifted);
+        if (threadIdx.x >= 32) continue;   // thread 0 writes the sum: the FP64 exponentials of one warp
         const double dr = static_cast<double>(lq.x) - static_cast<double>(lp.x);
         const double di = static_cast<double>(lq.y) - static_cast<double>(lp.y);
         const double m = exp(dr);
@@ -443,49 +446,311 @@ __global__ void deep_ok_kernel(DeepNetDev net, int count, const uint64_t* spins,
     backward<double2, REAL>(net, w.s, w, lp, [&](int k, double2 v) { row[k] = v; });
 }
 
-// per sample (FP64): E_loc, O_k(s) row, and the centred E_k row
+// FP64 local energy of a complex net (no translation sums) and, with GRAD, per sample the O_k
+// row and the centred E_k row
 //   Ek[s] = (E_diag - E0) O(s) + sum_{off-diagonal n} e_n O(s'_n)
-// (Operator.hpp:145-179 with the shift of the gradient estimator)
-__global__ void deep_grad_kernel(DeepNetDev net, OpDev op, int count, const uint64_t* spins, uint64_t enum_base,
-                                 int enumerate, double2 e_shift, double2* eloc, double2* Orows, double2* Ekrows,
-                                 long ld) {
+// (Operator.hpp:145-179 with the shift of the gradient estimator); with prime, also
+// log psi'(s) - log psi(s).  One block per sample.
+//
+// Bound by the FP64 pipe, whose instructions take 16 cycles of the SM whatever the number of
+// active lanes, so the work is counted and packed: `nb` neighbours at a time, their units side
+// by side in the threads; a neighbour's layer 0 is the sample's moved by the flipped spins; an
+// activation and its derivative come from one D(u) (math64.cuh); exp, cos and sin run one
+// neighbour a lane (in every thread of a block before); the reverse pass carries e_n delta and
+// a parameter's entries are summed over the neighbours of a batch before its one read and write
+// of the row (one per neighbour before, and ten FP64 operations per entry instead of four).
+// 512 samples of the 20-40-20-10 net, 20 strings: gradient pass 2066 -> 489 us, energies 750 ->
+// 171 us.
+constexpr int kThreads64 = 128;
+
+size_t deep_local64_smem(const DeepNetDev& n, int nb, bool grad) {
+    return sizeof(double2) * ((grad ? 2 : 1) * static_cast<size_t>(nb) * n.units + n.size[0] + 2 * nb) +
+           sizeof(uint64_t) * (1 + nb) * kMaxWords;
+}
+
+template <bool GRAD>
+__global__ void __launch_bounds__(kThreads64) deep_local64_kernel(DeepNetDev net, OpDev op, int count,
+                                                                  const uint64_t* spins, uint64_t enum_base,
+                                                                  int enumerate, int nbatch, DeepNetDev prime,
+                                                                  double2* dlp, double2 e_shift, double2* eloc,
+                                                                  double2* Orows, double2* Ekrows, long ld) {
     extern __shared__ __align__(16) unsigned char smem[];
-    Work<double2> w = carve<double2>(smem, net, true);
-    uint64_t* sp = w.s + kMaxWords;
+    const int units = net.units, size0 = net.size[0], L = net.L;
+    double2* A = reinterpret_cast<double2*>(smem);           // [nb][units] activations
+    double2* H = A + nbatch * units;                         // GRAD: [nb][units] derivatives, then e_n delta
+    double2* z0s = GRAD ? H + nbatch * units : H;            // [size0] the sample's layer 0
+    double2* lq = z0s + size0;                               // [nb] log psi
+    double2* en = lq + nbatch;                               // [nb] terms e_n
+    uint64_t* s = reinterpret_cast<uint64_t*>(en + nbatch);  // [kMaxWords] the sample
+    uint64_t* sp = s + kMaxWords;                            // [nb][kMaxWords] the neighbours
     const long t = blockIdx.x;
     if (t >= count) return;
-    load_config(spins, enum_base, enumerate, t, net.N, w.s);
-    double2* orow = Orows + t * ld;
-    double2* erow = Ekrows + t * ld;
-    const double2 lp = forward_once<double2, false, true>(net, w.s, w);
-    backward<double2, false>(net, w.s, w, lp, [&](int k, double2 v) { orow[k] = v; });
-    double dr_ = 0.0, di_ = 0.0;
-    for (int n = 0; n < op.S; n++) {
-        if (op.nflip[n] != 0) continue;
-        const double2 cf = apply_string(op, n, w.s, sp);
-        dr_ += cf.x;
-        di_ += cf.y;
-    }
-    double er = dr_, ei = di_;
-    {
-        const double2 c = make_double2(dr_ - e_shift.x, di_ - e_shift.y);
-        const int P = net.P - 2 * net.N;
-        for (int k = threadIdx.x; k < P; k += blockDim.x) erow[k] = cmul(c, orow[k]);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    load_config(spins, enum_base, enumerate, t, net.N, s);
+    for (int u = tid; u < size0; u += kThreads64) {
+        double2 a = net.b64[0][u];
+        for (int c = 0; c < net.conn[0]; c++) {
+            const double2 w = net.w64[0][c * size0 + u];
+            const double sg = bit_up(s, net.cidx[0][c * size0 + u]) ? 1.0 : -1.0;
+            a.x = fma(sg, w.x, a.x);
+            a.y = fma(sg, w.y, a.y);
+        }
+        z0s[u] = a;
     }
     __syncthreads();
-    for (int n = 0; n < op.S; n++) {
-        if (op.nflip[n] == 0) continue;
-        const double2 cf = apply_string(op, n, w.s, sp);
-        const double2 lq = forward_once<double2, false, true>(net, sp, w);
-        const double dr = lq.x - lp.x, di = lq.y - lp.y;
-        const double m = exp(dr);
-        const double xr = m * cos(di), xi = m * sin(di);
-        const double2 e = make_double2(cf.x * xr - cf.y * xi, cf.x * xi + cf.y * xr);
-        er += e.x;
-        ei += e.y;
-        backward<double2, false>(net, sp, w, lq, [&](int k, double2 v) { erow[k] = cadd(erow[k], cmul(e, v)); });
+    // activations (and derivatives) of nb configurations whose layer 0 is z0of(k, u); log psi to lq
+    auto forward = [&](auto z0of, int nb) {
+        const DeepNetDev& n = net;
+        auto unit = [&](int k, int at, double2 z) {
+            const Lc64 f = lc64(z);
+            A[k * units + at] = f.value();
+            if (GRAD) H[k * units + at] = f.tanh();
+        };
+        for (int e = tid; e < nb * n.size[0]; e += kThreads64) {
+            const int k = e / n.size[0], u = e - k * n.size[0];
+            unit(k, u, z0of(k, u));
+        }
+        __syncthreads();
+        for (int l = 1; l < L; l++) {
+            const int size = n.size[l], conn = n.conn[l], at = n.begin_angle[l], below = n.begin_angle[l - 1];
+            const int* ci = n.cidx[l];
+            const double2* w = n.w64[l];
+            for (int e = tid; e < nb * size; e += kThreads64) {
+                const int k = e / size, u = e - k * size;
+                const double2* in = A + k * units + below;
+                double2 a = n.b64[l][u], b = make_double2(0.0, 0.0);
+                for (int c = 0; c < conn; c++) {
+                    const double2 wv = w[c * size + u], x = in[ci[c * size + u]];
+                    a.x = fma(wv.x, x.x, a.x);
+                    b.x = fma(-wv.y, x.y, b.x);
+                    a.y = fma(wv.x, x.y, a.y);
+                    b.y = fma(wv.y, x.x, b.y);
+                }
+                unit(k, at + u, cadd(a, b));
+            }
+            __syncthreads();
+        }
+        const int last = n.size[L - 1];
+        for (int k = warp; k < nb; k += kThreads64 / 32) {
+            double2 v = make_double2(0.0, 0.0);
+            for (int u = lane; u < last; u += 32) v = cadd(v, cmul(A[k * units + n.begin_angle[L - 1] + u], n.fw64[u]));
+#pragma unroll
+            for (int off = 16; off >= 1; off >>= 1) {
+                v.x += __shfl_xor_sync(0xffffffffu, v.x, off);
+                v.y += __shfl_xor_sync(0xffffffffu, v.y, off);
+            }
+            if (lane == 0) lq[k] = v;
+        }
+        __syncthreads();
+    };
+    // H: en[k] delta_l of nb configurations
+    auto backward = [&](int nb) {
+        for (int l = L - 1; l >= 0; l--) {
+            const int size = net.size[l], at = net.begin_angle[l];
+            for (int e = tid; e < nb * size; e += kThreads64) {
+                const int k = e / size, u = e - k * size;
+                double2 a = make_double2(0.0, 0.0);
+                if (l == L - 1) {
+                    a = cmul(en[k], net.fw64[u]);
+                } else {
+                    const int above = net.size[l + 1];
+                    const double2* d = H + k * units + net.begin_angle[l + 1];
+                    const double2* w = net.w64[l + 1];
+                    for (int q = net.rptr[l][u]; q < net.rptr[l][u + 1]; q++) {
+                        const int i = net.rq[l][q];
+                        const double2 wv = w[i], x = d[i % above];
+                        a.x = fma(wv.x, x.x, fma(-wv.y, x.y, a.x));
+                        a.y = fma(wv.x, x.y, fma(wv.y, x.x, a.y));
+                    }
+                }
+                H[k * units + at + u] = cmul(a, H[k * units + at + u]);
+            }
+            __syncthreads();
+        }
+    };
+    // parameter k (counted from the first O_k entry): emit(k, sum over the nb configurations)
+    auto parameters = [&](int nb, const uint64_t* cfg, auto emit) {
+        for (int l = 0; l < L; l++) {
+            const int size = net.size[l], total = size + net.conn[l] * size, at = net.begin_angle[l];
+            for (int e = tid; e < total; e += kThreads64) {
+                double2 v = make_double2(0.0, 0.0);
+                if (e < size) {
+                    for (int k = 0; k < nb; k++) v = cadd(v, H[k * units + at + e]);
+                } else {
+                    const int u = (e - size) % size, src = net.cidx[l][e - size];
+                    for (int k = 0; k < nb; k++) {
+                        const double2 d = H[k * units + at + u];
+                        if (l == 0) {
+                            const double sg = bit_up(cfg + k * kMaxWords, src) ? 1.0 : -1.0;
+                            v.x = fma(sg, d.x, v.x);
+                            v.y = fma(sg, d.y, v.y);
+                        } else {
+                            const double2 a = A[k * units + net.begin_angle[l - 1] + src];
+                            v.x = fma(d.x, a.x, fma(-d.y, a.y, v.x));
+                            v.y = fma(d.x, a.y, fma(d.y, a.x, v.y));
+                        }
+                    }
+                }
+                emit(net.begin_params[l] + e, v);
+            }
+        }
+        // final weights: log psi * activation of the last layer (PsiDeep.hpp:285-292)
+        const int last = net.size[L - 1];
+        for (int u = tid; u < last; u += kThreads64) {
+            double2 v = make_double2(0.0, 0.0);
+            for (int k = 0; k < nb; k++)
+                v = cadd(v, cmul(cmul(en[k], lq[k]), A[k * units + net.begin_angle[L - 1] + u]));
+            emit(net.P - 2 * net.N - last + u, v);
+        }
+    };
+    auto factor = [&](int n) {
+        int parity = 0;
+        for (int k = 0; k < kMaxWords; k++) parity += __popcll(op.zmask[n * kMaxWords + k] & ~s[k]);
+        const double2 c = op.coef[n];
+        const int yp = op.ypow[n] & 3;
+        const double2 r = yp == 0 ? c : (yp == 1 ? make_double2(c.y, -c.x)
+                                                 : (yp == 2 ? make_double2(-c.x, -c.y) : make_double2(-c.y, c.x)));
+        return (parity & 1) ? make_double2(-r.x, -r.y) : r;
+    };
+    auto warp_sum = [&](double2 v) {
+#pragma unroll
+        for (int off = 16; off >= 1; off >>= 1) {
+            v.x += __shfl_xor_sync(0xffffffffu, v.x, off);
+            v.y += __shfl_xor_sync(0xffffffffu, v.y, off);
+        }
+        return v;
+    };
+    forward([&](int, int u) { return z0s[u]; }, 1);
+    const double2 lp = lq[0];
+    double2* orow = Orows + t * ld;
+    double2* erow = Ekrows + t * ld;
+    // the diagonal strings (every warp: the E_k row needs their sum)
+    double2 diag = make_double2(0.0, 0.0);
+    for (int n = lane; n < op.S; n += 32)
+        if (op.nflip[n] == 0) diag = cadd(diag, factor(n));
+    diag = warp_sum(diag);
+    if (GRAD) {
+        if (tid == 0) en[0] = make_double2(1.0, 0.0);
+        __syncthreads();
+        backward(1);
+        const double2 c = make_double2(diag.x - e_shift.x, diag.y - e_shift.y);
+        parameters(1, s, [&](int k, double2 v) {
+            orow[k] = v;
+            erow[k] = cmul(c, v);
+        });
+        __syncthreads();
     }
-    if (threadIdx.x == 0) eloc[t] = make_double2(er, ei);
+    double2 E = make_double2(0.0, 0.0);   // warp 0: the neighbours' terms, a lane's own
+    for (int q = 0; q < op.num_offdiag; q += nbatch) {
+        const int nb = min(nbatch, op.num_offdiag - q);
+        for (int i = tid; i < nb * kMaxWords; i += kThreads64) {
+            const int k = i / kMaxWords, word = i - k * kMaxWords, n = op.offdiag[q + k];
+            uint64_t v = s[word];
+            for (int f = 0; f < op.nflip[n]; f++) {
+                const int site = op.flip_sites[op.flip_off[n] + f];
+                if ((site >> 6) == word) v ^= 1ull << (site & 63);
+            }
+            sp[i] = v;
+        }
+        forward([&](int k, int u) {
+            double2 z = z0s[u];
+            const int n = op.offdiag[q + k];
+            for (int f = 0; f < op.nflip[n]; f++) {
+                const int site = op.flip_sites[op.flip_off[n] + f];
+                const double ts = bit_up(s, site) ? -2.0 : 2.0;
+                for (int d = 0; d < net.w0n; d++) {
+                    const double2 w = net.w064[(static_cast<long>(d) * net.N + site) * size0 + u];
+                    z.x = fma(ts, w.x, z.x);
+                    z.y = fma(ts, w.y, z.y);
+                }
+            }
+            return z;
+        }, nb);
+        if (warp == 0 && lane < nb) {
+            const double2 cf = factor(op.offdiag[q + lane]);
+            const double m = exp(lq[lane].x - lp.x);
+            double sn, cs;
+            sincos(lq[lane].y - lp.y, &sn, &cs);
+            const double2 e = cmul(cf, make_double2(m * cs, m * sn));
+            en[lane] = e;
+            E = cadd(E, e);
+        }
+        __syncthreads();
+        if (GRAD) {
+            backward(nb);
+            parameters(nb, sp, [&](int k, double2 v) { erow[k] = cadd(erow[k], v); });
+            __syncthreads();
+        }
+    }
+    if (warp == 0) {
+        E = warp_sum(E);
+        if (lane == 0 && eloc) eloc[t] = cadd(diag, E);
+    }
+    if (dlp) {
+        // log psi'(s) - log psi(s) by forward_once's operations in its order: the distance is a
+        // difference of nearly equal sums, down to the last bits of these two
+        auto plain = [&](const DeepNetDev& n) {
+            for (int l = 0; l < L; l++) {
+                const int size = n.size[l], conn = n.conn[l];
+                for (int u = tid; u < size; u += kThreads64) {
+                    double2 a = make_double2(0.0, 0.0);
+                    for (int c = 0; c < conn; c++) {
+                        const int i = n.cidx[l][c * size + u];
+                        const double2 x = l == 0 ? make_double2(bit_up(s, i) ? 1.0 : -1.0, 0.0)
+                                                 : A[n.begin_angle[l - 1] + i];
+                        a = cadd(a, cmul(n.w64[l][c * size + u], x));
+                    }
+                    A[n.begin_angle[l] + u] = lc64_plain(cadd(a, n.b64[l][u]));
+                }
+                __syncthreads();
+            }
+            const int last = n.size[L - 1];
+            double2 r = make_double2(0.0, 0.0);
+            for (int q = 0; q < last; q += 32)
+                r = cadd(r, warp_sum(q + lane < last ? cmul(A[n.begin_angle[L - 1] + q + lane], n.fw64[q + lane])
+                                                     : make_double2(0.0, 0.0)));
+            __syncthreads();
+            return r;
+        };
+        const double2 l0 = plain(net), l1 = plain(prime);
+        if (tid == 0) dlp[t] = make_double2(l1.x - l0.x, l1.y - l0.y);
+    }
+}
+
+// sums over the samples of the O_k and E_k rows (FP64), one pass over both:
+//   0: c1 O, 1: c2 conj(O), 2: c1 Ek, 3 (c3): c3 Ek;  partial [split][4][P]
+__global__ void __launch_bounds__(128) row_sums_kernel(int count, int P, const double2* __restrict__ c1,
+                                                       const double2* __restrict__ c2, const double2* __restrict__ c3,
+                                                       const double2* __restrict__ O, const double2* __restrict__ Ek,
+                                                       long ld, double2* __restrict__ partial, int per_split) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const long s0 = static_cast<long>(blockIdx.y) * per_split;
+    const long s1 = min(static_cast<long>(count), s0 + per_split);
+    if (k >= P) return;
+    double2 a[4] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0), make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+#pragma unroll 2
+    for (long s = s0; s < s1; s++) {
+        const double2 o = O[s * ld + k], e = Ek[s * ld + k], u = c1[s], v = c2[s];
+        a[0] = cadd(a[0], cmul(u, o));
+        a[1] = cadd(a[1], cmul(v, make_double2(o.x, -o.y)));
+        a[2] = cadd(a[2], cmul(u, e));
+        if (c3) a[3] = cadd(a[3], cmul(c3[s], e));
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) partial[(static_cast<long>(blockIdx.y) * 4 + q) * P + k] = a[q];
+}
+
+struct RowSums {
+    double2* out[4];
+};
+__global__ void __launch_bounds__(128) row_sums_finish_kernel(int P, int splits, const double2* __restrict__ partial,
+                                                              RowSums sums) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y;
+    if (k >= P || !sums.out[q]) return;
+    double2 a = make_double2(0.0, 0.0);
+#pragma unroll 8
+    for (int z = 0; z < splits; z++) a = cadd(a, partial[(static_cast<long>(z) * 4 + q) * P + k]);
+    sums.out[q][k] = cadd(sums.out[q][k], a);
 }
 
 // out[k] += sum_s c[s] f(A[s][k]) over count samples, f = conj if conj_a (FP64)
@@ -1536,9 +1801,13 @@ static cudaError_t upload(DeepHost* h, const std::vector<T>& v, const T** out) {
     return e;
 }
 
-// dst[at[e]] = src[e]
-__global__ void scatter_entries_kernel(int n, const float2* src, const int* at, float2* dst) {
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) dst[at[e]] = src[e];
+// dst[at[e]] = src[e], in both precisions
+__global__ void scatter_entries_kernel(int n, const float2* src, const double2* src64, const int* at, float2* dst,
+                                       double2* dst64) {
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+        dst[at[e]] = src[e];
+        dst64[at[e]] = src64[e];
+    }
 }
 
 // dst[c][r] = src[r][c]
@@ -1552,7 +1821,8 @@ int deep_derive(const rbmg_psi* psi) {
     if (psi->kind == 2) return RBMG_OK;
     const DeepNetDev& d = psi->deep_dev[0];
     const int n0 = d.conn[0] * d.size[0];
-    scatter_entries_kernel<<<(n0 + 255) / 256, 256, 0, stream()>>>(n0, d.w[0], d.w0at, const_cast<float2*>(d.w0));
+    scatter_entries_kernel<<<(n0 + 255) / 256, 256, 0, stream()>>>(n0, d.w[0], d.w64[0], d.w0at, const_cast<float2*>(d.w0),
+                                                                       const_cast<double2*>(d.w064));
     RBMG_CK(cudaGetLastError());
     for (int l = 1; l < d.L; l++) {
         if (!d.wt[l]) continue;
@@ -1659,12 +1929,15 @@ int deep_upload(rbmg_psi* psi) {
                 at[e] = static_cast<int>(static_cast<size_t>(plane) * psi->N * L0.size + cell);
             }
             RBMG_CK(upload(h.get(), at, &d.w0at));
-            auto w0 = std::make_unique<DevBuf>();
-            const size_t bytes = sizeof(float2) * d.w0n * psi->N * L0.size;
-            RBMG_CK(w0->ensure(bytes));
-            RBMG_CK(cudaMemset(w0->p, 0, bytes));
-            d.w0 = w0->as<float2>();
-            h->bufs.push_back(std::move(w0));
+            for (const size_t bytes : {sizeof(float2), sizeof(double2)}) {
+                auto w0 = std::make_unique<DevBuf>();
+                const size_t n = bytes * d.w0n * psi->N * L0.size;
+                RBMG_CK(w0->ensure(n));
+                RBMG_CK(cudaMemset(w0->p, 0, n));
+                (bytes == sizeof(float2) ? reinterpret_cast<const void*&>(d.w0)
+                                         : reinterpret_cast<const void*&>(d.w064)) = w0->p;
+                h->bufs.push_back(std::move(w0));
+            }
             for (int l = 1; l < L; l++) {
                 const auto& Ly = psi->layers[l];
                 bool dense = Ly.conn == psi->layers[l - 1].size;
@@ -1720,31 +1993,47 @@ int deep_log_psi(const rbmg_psi* psi, int count, const uint64_t* d_spins, uint64
     return RBMG_OK;
 }
 
-int deep_eloc_chunk(const rbmg_psi* psi, const rbmg_operator* op, const Chunk& c, double2* d_eloc, cudaStream_t st) {
-    if (c.count <= 0) return RBMG_OK;
-    const DeepNetDev n0 = net_of(psi, 0), n1 = net_of(psi, 1);
-    const size_t sm = smem_for(n0, sizeof(double2), false) + 2 * sizeof(uint64_t) * kMaxWords;
-    RBMG_CK(set_smem(deep_eloc_kernel<double2, false>, sm));
-    deep_eloc_kernel<double2, false><<<c.count, threads_for(n0), sm, st>>>(n0, n1, psi->kind == 2, n0, n1, op->dev(),
-                                                                           c.count, c.spins, c.enum_base, c.enumerate,
-                                                                           d_eloc, nullptr);
-    RBMG_CK(cudaGetLastError());
-    return RBMG_OK;
+// neighbours per batch of deep_local64_kernel: as many as leave room for three blocks an SM, at
+// most 16, at least one
+static int local64_batch(const DeepNetDev& n, bool grad) {
+    int nb = 16;
+    while (nb > 1 && deep_local64_smem(n, nb, grad) > 72 * 1024) nb /= 2;
+    return nb;
 }
 
 int deep_hsd64_chunk(const rbmg_psi* psi, const rbmg_psi* pp, const rbmg_operator* op, const Chunk& c,
                      double2* d_eloc, double2* d_dlp, cudaStream_t st) {
     if (c.count <= 0) return RBMG_OK;
-    if (pp->width != psi->width || pp->layers.size() != psi->layers.size())
+    if (pp && (pp->width != psi->width || pp->layers.size() != psi->layers.size()))
         return fail(RBMG_EUNSUPPORTED, "hsd: psi and psi_prime need the same layer shapes");
-    const DeepNetDev n0 = net_of(psi, 0), n1 = net_of(psi, 1), q0 = net_of(pp, 0), q1 = net_of(pp, 1);
-    const size_t sm = smem_for(n0, sizeof(double2), false) + 2 * sizeof(uint64_t) * kMaxWords;
-    RBMG_CK(set_smem(deep_eloc_kernel<double2, true>, sm));
-    deep_eloc_kernel<double2, true><<<c.count, threads_for(n0), sm, st>>>(n0, n1, psi->kind == 2, q0, q1, op->dev(),
-                                                                         c.count, c.spins, c.enum_base, c.enumerate,
-                                                                         d_eloc, d_dlp);
+    const rbmg_psi* p = pp ? pp : psi;
+    const DeepNetDev n0 = net_of(psi, 0), n1 = net_of(psi, 1), q0 = net_of(p, 0), q1 = net_of(p, 1);
+    bool alike = psi->kind == 1 && !n0.ti && !q0.ti;   // psi' is evaluated in psi's buffers
+    for (int l = 0; l < n0.L; l++) alike = alike && n0.size[l] == q0.size[l];
+    if (alike) {
+        const int nb = local64_batch(n0, false);
+        const size_t sm = deep_local64_smem(n0, nb, false);
+        RBMG_CK(set_smem(deep_local64_kernel<false>, sm));
+        deep_local64_kernel<false><<<c.count, kThreads64, sm, st>>>(n0, op->dev(), c.count, c.spins, c.enum_base,
+                                                                    c.enumerate, nb, q0, d_dlp, make_double2(0.0, 0.0),
+                                                                    d_eloc, nullptr, nullptr, 0);
+    } else {
+        const size_t sm = smem_for(n0, sizeof(double2), false) + 2 * sizeof(uint64_t) * kMaxWords;
+        auto run = [&](auto kernel) -> cudaError_t {
+            const cudaError_t e = set_smem(kernel, sm);
+            if (e != cudaSuccess) return e;
+            kernel<<<c.count, threads_for(n0), sm, st>>>(n0, n1, psi->kind == 2, q0, q1, op->dev(), c.count, c.spins,
+                                                         c.enum_base, c.enumerate, d_eloc, d_dlp);
+            return cudaSuccess;
+        };
+        RBMG_CK(pp ? run(deep_eloc_kernel<double2, true>) : run(deep_eloc_kernel<double2, false>));
+    }
     RBMG_CK(cudaGetLastError());
     return RBMG_OK;
+}
+
+int deep_eloc_chunk(const rbmg_psi* psi, const rbmg_operator* op, const Chunk& c, double2* d_eloc, cudaStream_t st) {
+    return deep_hsd64_chunk(psi, nullptr, op, c, d_eloc, nullptr, st);
 }
 
 static DevBuf& rows_buf(int which) {
@@ -1836,28 +2125,33 @@ int deep_gradient_chunk(const rbmg_psi* psi, const rbmg_operator* op, const Chun
     DevBuf& erows = rows_buf(1);
     RBMG_CK(orows.ensure(sizeof(double2) * static_cast<size_t>(std::min(chunk, c.count)) * P));
     RBMG_CK(erows.ensure(sizeof(double2) * static_cast<size_t>(std::min(chunk, c.count)) * P));
-    const size_t sm = smem_for(net, sizeof(double2), true) + sizeof(uint64_t) * kMaxWords;
-    RBMG_CK(set_smem(deep_grad_kernel, sm));
+    const int nb = local64_batch(net, true);
+    const size_t sm = deep_local64_smem(net, nb, true);
+    RBMG_CK(set_smem(deep_local64_kernel<true>, sm));
+    DevBuf& part = rows_buf(2);
     RBMG_CK(launch_coef(c.count, c.weights, nullptr, 1.0, coef1, st));
     for (int base = 0; base < c.count; base += chunk) {
         const int cnt = std::min(chunk, c.count - base);
         const uint64_t* sp = c.spins ? c.spins + static_cast<size_t>(base) * ((net.N + 63) / 64) : nullptr;
-        deep_grad_kernel<<<cnt, threads_for(net), sm, st>>>(net, op->dev(), cnt, sp, c.enum_base + base, c.enumerate,
-                                                            e_shift, d_eloc + base, orows.as<double2>(),
-                                                            erows.as<double2>(), P);
+        deep_local64_kernel<true><<<cnt, kThreads64, sm, st>>>(net, op->dev(), cnt, sp, c.enum_base + base, c.enumerate,
+                                                               nb, net, nullptr, e_shift, d_eloc + base,
+                                                               orows.as<double2>(), erows.as<double2>(), P);
         RBMG_CK(cudaGetLastError());
-        RBMG_CK(launch_coef(cnt, c.weights ? c.weights + base : nullptr, d_eloc + base, 1.0, coef2 + base, st,
-                            e_shift));
-        int r = col_reduce(cnt, P, coef1 + base, orows.as<double2>(), P, 0, acc_O, st);
-        if (r == RBMG_OK) r = col_reduce(cnt, P, coef2 + base, orows.as<double2>(), P, 1, acc_EO, st);
-        if (r == RBMG_OK) r = col_reduce(cnt, P, coef1 + base, erows.as<double2>(), P, 0, acc_Ek, st);
-        if (r == RBMG_OK && acc_B) {
-            // sum w conj(E - E0) (E_k - E0 O_k): the fluctuation gradient's covariance term
-            RBMG_CK(launch_coef_conj(cnt, c.weights ? c.weights + base : nullptr, d_eloc + base, e_shift, coef3 + base,
-                                     st));
-            r = col_reduce(cnt, P, coef3 + base, erows.as<double2>(), P, 0, acc_B, st);
-        }
-        if (r != RBMG_OK) return r;
+        const double* wb = c.weights ? c.weights + base : nullptr;
+        RBMG_CK(launch_coef(cnt, wb, d_eloc + base, 1.0, coef2 + base, st, e_shift));
+        // sum w conj(E - E0) (E_k - E0 O_k): the fluctuation gradient's covariance term
+        if (acc_B) RBMG_CK(launch_coef_conj(cnt, wb, d_eloc + base, e_shift, coef3 + base, st));
+        // enough splits of the samples to fill the GPU, of eight samples at least
+        const int cols = (P + 127) / 128;
+        const int per = std::max(8, (cnt + std::max(1, 608 / cols) - 1) / std::max(1, 608 / cols));
+        const int splits = (cnt + per - 1) / per;
+        RBMG_CK(part.ensure(sizeof(double2) * 4 * static_cast<size_t>(splits) * P));
+        row_sums_kernel<<<dim3(cols, splits), 128, 0, st>>>(cnt, P, coef1 + base, coef2 + base,
+                                                            acc_B ? coef3 + base : nullptr, orows.as<double2>(),
+                                                            erows.as<double2>(), P, part.as<double2>(), per);
+        row_sums_finish_kernel<<<dim3(cols, 4), 128, 0, st>>>(P, splits, part.as<double2>(),
+                                                              RowSums{{acc_O, acc_EO, acc_Ek, acc_B}});
+        RBMG_CK(cudaGetLastError());
     }
     return RBMG_OK;
 }

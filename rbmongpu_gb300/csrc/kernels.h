@@ -129,6 +129,7 @@ struct DeepNetDev {
     // entry e of w[0] at w0at[e]; per dense layer l >= 1 (connection c is unit c of the layer
     // below) its weights transposed, wt[l] [size[l]][size[l - 1]], null otherwise
     const float2* w0;
+    const double2* w064;
     const int* w0at;
     int w0n;
     const float2* wt[3];

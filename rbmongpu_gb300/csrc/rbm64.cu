@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include "kernels.h"
+#include "math64.cuh"
 #include "rbm64.h"
 
 namespace rbmg {
@@ -17,56 +18,6 @@ namespace {
 
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
     return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-
-// The rational log-cosh (include/quantum_state/psi_functions.hpp:49-57) in FP64, kept open as
-// f + C = A u + n / D(u): u = sign(Re z) z, n / D = (nr + i ni) inv.  FP64 instructions issue
-// at 1/64 of the FP32 rate and are all that these kernels wait for, so they are counted: the
-// quartic with real coefficients runs on u's trace 2p and norm |u|^2 (11 operations against
-// 13 of the complex Horner scheme), the sign is folded in by integer operations, and one
-// reciprocal serves both parts: the hardware's estimate (at least 19 bits) and one cubic step
-// r (1 + e + e^2), e = 1 - den r, which leaves e^3 < 2^-57.  32 FP64 operations with the
-// difference and its sum, against 61 with two divisions.
-constexpr double kLcC = 0.598139;
-constexpr double kLcA = 0.9003320053750442;
-
-struct Lc64 {
-    double p, q, nr, ni, inv;
-    __device__ __forceinline__ double2 open() const { return make_double2(fma(kLcA, p, nr * inv), fma(kLcA, q, ni * inv)); }
-    // d += (f + C) - g
-    __device__ __forceinline__ void add_difference(double2 g, double2& d) const {
-        d.x += fma(kLcA, p, fma(nr, inv, -g.x));
-        d.y += fma(kLcA, q, fma(ni, inv, -g.y));
-    }
-};
-
-__device__ __forceinline__ double rcp64(double den) {
-    // |D|^2 overflows for |z| > 1e38 only; the clamp keeps 0 rather than NaN there, as a
-    // division does
-    const int hi = min(__double2hiint(den), 0x7FD00000);
-    den = __hiloint2double(hi, __double2loint(den));
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(den));
-    const double e = fma(-den, r, 1.0);
-    return fma(r, fma(e, e, e), r);
-}
-
-__device__ __forceinline__ Lc64 lc64(double2 z) {
-    // sign = z.x > 0 ? 1 : -1 (positive doubles are positive integers; zero counts as -1)
-    const long long flip = __double_as_longlong(z.x) > 0 ? 0ll : static_cast<long long>(0x8000000000000000ull);
-    Lc64 f;
-    f.p = __longlong_as_double(__double_as_longlong(z.x) ^ flip);
-    f.q = __longlong_as_double(__double_as_longlong(z.y) ^ flip);
-    const double r = f.p + f.p, n = fma(f.q, f.q, f.p * f.p);
-    const double b3 = r + 3.746646023906276;
-    const double b2 = fma(r, b3, 7.771429504240965 - n);
-    const double b1 = fma(r, b2, fma(-n, b3, 10.2180213465));
-    const double dr = fma(f.p, b1, fma(-n, b2, 9.19376335670885)), di = f.q * b1;
-    const double ur = fma(-2.16564366435, f.p, 5.49914721954), ui = -2.16564366435 * f.q;
-    f.nr = fma(ur, dr, ui * di);
-    f.ni = fma(ui, dr, -(ur * di));
-    f.inv = rcp64(fma(dr, dr, di * di));
-    return f;
 }
 
 __device__ __forceinline__ double2 warp_sum64(double2 v) {
