@@ -5,9 +5,7 @@
 #include <cmath>
 #include <functional>
 #include <memory>
-#include <thread>
 #include <vector>
-#include <unistd.h>
 
 #include <cuda_profiler_api.h>
 
@@ -850,6 +848,7 @@ extern "C" int rbmg_psi_log_psi(const rbmg_psi* psi, int count, const uint64_t* 
     RBMG_CK(cudaMemcpyAsync(W.sample_spins.p, spins, sizeof(uint64_t) * nw * count, cudaMemcpyHostToDevice, stream()));
     const int r = psi_log_psi_dev(psi, count, W.sample_spins.as<uint64_t>(), 0, 0, W.logpsi_p.as<double2>());
     if (r != RBMG_OK) return r;
+    prefault(out, sizeof(double2) * count);
     RBMG_CK(cudaMemcpyAsync(out, W.logpsi_p.p, sizeof(double2) * count, cudaMemcpyDeviceToHost, stream()));
     RBMG_CK(cudaStreamSynchronize(stream()));
     return RBMG_OK;
@@ -1537,6 +1536,7 @@ extern "C" int rbmg_local_energies(const rbmg_psi* psi, const rbmg_operator* op,
     const double2* e = nullptr;
     const int r = chunk_eloc(psi, op, c, &e);
     if (r != RBMG_OK) return r;
+    prefault(out, sizeof(double2) * count);
     RBMG_CK(cudaMemcpyAsync(out, e, sizeof(double2) * count, cudaMemcpyDeviceToHost, stream()));
     RBMG_CK(cudaStreamSynchronize(stream()));
     return RBMG_OK;
@@ -2132,6 +2132,7 @@ extern "C" int rbmg_ensemble_samples(rbmg_ensemble* ens, const rbmg_psi* psi, co
     r = run_stream(ens, psi, op, eloc != nullptr, size_t(1) << 22, &res, [&](const Chunk& c) -> int {
         if (spins) {
             if (c.spins) {
+                prefault(spins + offset * nw, sizeof(uint64_t) * nw * c.count);
                 RBMG_CK(cudaMemcpyAsync(spins + offset * nw, c.spins, sizeof(uint64_t) * nw * c.count,
                                         cudaMemcpyDeviceToHost, stream()));
             } else {
@@ -2145,6 +2146,7 @@ extern "C" int rbmg_ensemble_samples(rbmg_ensemble* ens, const rbmg_psi* psi, co
             RBMG_CK(W.logpsi_p.ensure(sizeof(double2) * c.count));
             const int rr = psi_log_psi_dev(psi, c.count, c.spins, c.enum_base, c.enumerate, W.logpsi_p.as<double2>());
             if (rr != RBMG_OK) return rr;
+            prefault(log_psi + 2 * offset, sizeof(double2) * c.count);
             RBMG_CK(cudaMemcpyAsync(log_psi + 2 * offset, W.logpsi_p.p, sizeof(double2) * c.count,
                                     cudaMemcpyDeviceToHost, stream()));
         }
@@ -2152,6 +2154,7 @@ extern "C" int rbmg_ensemble_samples(rbmg_ensemble* ens, const rbmg_psi* psi, co
             const double2* e = nullptr;
             const int rr = chunk_eloc(psi, op, c, &e);
             if (rr != RBMG_OK) return rr;
+            prefault(eloc + 2 * offset, sizeof(double2) * c.count);
             RBMG_CK(cudaMemcpyAsync(eloc + 2 * offset, e, sizeof(double2) * c.count, cudaMemcpyDeviceToHost, stream()));
         }
         RBMG_CK(cudaStreamSynchronize(stream()));
@@ -2216,35 +2219,6 @@ int deep_ok_rows(const rbmg_psi* psi, int count, const uint64_t* d_spins, uint64
                  double2* rows, long ld, cudaStream_t st);
 }  // namespace rbmg
 
-// Writes one word of every page of a large host output from several threads while the GPU
-// works, so that the device-to-host copy of the result does not take the first-touch page
-// faults of a freshly allocated array one by one (joined before the copy).
-class Prefault {
-  public:
-    Prefault(void* p, size_t bytes) {
-        const size_t page = static_cast<size_t>(std::max(4096L, sysconf(_SC_PAGESIZE)));
-        if (bytes < (size_t(64) << 20)) return;
-        const int n = static_cast<int>(std::min(16u, std::max(1u, std::thread::hardware_concurrency())));
-        const size_t pages = (bytes + page - 1) / page, per = (pages + n - 1) / n;
-        char* base = static_cast<char*>(p);
-        for (int t = 0; t < n; t++) {
-            const size_t p0 = t * per, p1 = std::min(pages, p0 + per);
-            if (p0 >= p1) break;
-            threads_.emplace_back([=]() {
-                for (size_t q = p0; q < p1; q++) *reinterpret_cast<volatile char*>(base + q * page) = 0;
-            });
-        }
-    }
-    void join() {
-        for (auto& t : threads_) t.join();
-        threads_.clear();
-    }
-    ~Prefault() { join(); }
-
-  private:
-    std::vector<std::thread> threads_;
-};
-
 // get_S_matrix (source/network_functions/S_matrix.cu:10-53, instantiated for Psi with
 // ExactSummation only): S[k][k'] = sum_s O_k(s) conj(O_k'(s)) / num_steps over every
 // configuration of the ensemble, without the ensemble's weight (the reference ignores the
@@ -2259,7 +2233,7 @@ extern "C" int rbmg_s_matrix(const rbmg_psi* psi, rbmg_ensemble* ens, int flags,
     const bool use_tc = (flags & RBMG_S_SIMT) == 0;
     Workspace& W = ws();
     const size_t sbytes = sizeof(double2) * static_cast<size_t>(L) * L;
-    Prefault prefault(out, sizeof(double2) * static_cast<size_t>(P) * P);
+    Prefault pages(out, sizeof(double2) * static_cast<size_t>(P) * P);
     RBMG_CK(W.smat.ensure(sbytes));
     RBMG_CK(W.smean.ensure(sizeof(double2) * L));
     RBMG_CK(cudaMemsetAsync(W.smat.p, 0, sbytes, stream()));
@@ -2389,7 +2363,7 @@ extern "C" int rbmg_s_matrix(const rbmg_psi* psi, rbmg_ensemble* ens, int flags,
                                   sizeof(double2) * 2 * N, L, stream()));
     RBMG_CK(launch_sm_finish(L, W.smat.as<double2>(), W.smean.as<double2>(), 1.0 / z, centered ? 1 : 0,
                              W.sout.as<double2>(), P, 2 * N, stream()));
-    prefault.join();
+    pages.join();
     RBMG_CK(cudaMemcpyAsync(out, W.sout.p, obytes, cudaMemcpyDeviceToHost, stream()));
     int tc_err = 0;
     if (use_tc) RBMG_CK(cudaMemcpyAsync(&tc_err, W.serror.p, sizeof(int), cudaMemcpyDeviceToHost, stream()));

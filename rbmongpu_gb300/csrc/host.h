@@ -1,12 +1,17 @@
 // Host-side objects behind the C ABI handles, shared by capi.cu and deep.cu.
 #pragma once
 
+#include <unistd.h>
+
+#include <algorithm>
 #include <complex>
 #include <cstdint>
 #include <cstring>
+#include <exception>
 #include <functional>
 #include <memory>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include <cuda_bf16.h>
@@ -53,6 +58,55 @@ struct DevBuf {
     template <typename T>
     T* as() const { return static_cast<T*>(p); }
 };
+
+// Makes the pages of a host output present before the GPU writes them: the copy to pageable
+// memory is a direct write of the GPU, which takes the first-touch fault of every page of a
+// freshly allocated array one by one (measured: 300 KB into fresh pages 226 us, into touched
+// ones 18 us and 25 us for the touches; 16 MB 13.5 ms against 0.10 and 0.73).  One byte of
+// every page is written, so only for memory that the copy then overwrites.  Large outputs are
+// touched by a thread per 4 MB (16 at most) from the construction on, while the GPU works;
+// join() ends them, or touches a smaller output itself, and comes before the copy.
+class Prefault {
+  public:
+    Prefault(void* p, size_t bytes) : p_(static_cast<char*>(p)), bytes_(bytes) {
+        const size_t n = std::min<size_t>({16, std::max(1u, std::thread::hardware_concurrency()), bytes >> 22});
+        if (n < 2) return;
+        const size_t per = ((bytes + n - 1) / n + 65535) / 65536 * 65536;
+        try {
+            threads_.reserve(n);
+            for (; started_ < bytes; started_ += per) {
+                char* a = p_ + started_;
+                const size_t len = std::min(per, bytes - started_);
+                threads_.emplace_back([=]() { touch(a, len); });
+            }
+        } catch (const std::exception&) {   // no more threads: join() touches the rest
+        }
+    }
+    Prefault(const Prefault&) = delete;
+    Prefault& operator=(const Prefault&) = delete;
+    void join() {
+        if (started_ < bytes_ && bytes_ >= kSmall) touch(p_ + started_, bytes_ - started_);
+        started_ = bytes_;
+        for (auto& t : threads_) t.join();
+        threads_.clear();
+    }
+    ~Prefault() {
+        for (auto& t : threads_) t.join();
+    }
+
+  private:
+    // below, the array comes from pages the process already holds (19 us either way at 64 KB)
+    static constexpr size_t kSmall = size_t(96) << 10;
+    static void touch(char* a, size_t bytes) {
+        static const size_t page = static_cast<size_t>(std::max(4096L, sysconf(_SC_PAGESIZE)));
+        for (size_t q = 0; q < bytes; q += page) *reinterpret_cast<volatile char*>(a + q) = 0;
+        *reinterpret_cast<volatile char*>(a + bytes - 1) = 0;   // the last page of an unaligned array
+    }
+    char* p_;
+    size_t bytes_, started_ = 0;
+    std::vector<std::thread> threads_;
+};
+inline void prefault(void* p, size_t bytes) { Prefault(p, bytes).join(); }
 
 cudaStream_t stream();
 
