@@ -5,12 +5,11 @@
 // queue (one atomic counter): first the walker tasks of every instance, longest first
 // (sweeps of single-flip Metropolis, then at the final configuration the local energy,
 // tanh(theta), the angles, U_j = sum_n e_n tanh(theta''_nj) over every string and the
-// terms e_n of the off-diagonal strings), then the reduction tasks,
-// each a tile of rows by a chunk of walkers of one instance's sums, which start once that
+// terms e_n of the off-diagonal strings), then the reduction tasks, each a tile of rows by a chunk of walkers of one instance's sums, which start once that
 // instance's walkers are all done (a per-instance counter; the wait is bounded by a
 // wall-clock limit after which the kernel raises an error flag and returns).  Each tile
 // writes its chunk's partial sums; a second kernel of the graph adds the chunks in a fixed
-// order, so every replay gives the same sums bit for bit.  The walker tasks are compiled
+// order and forms the gradient, so every replay gives the same bits.  The walker tasks are compiled
 // for each hidden-unit count per lane (1, 2, 4, 8, 13, 18: M <= 576) as separate functions
 // of the one kernel.  The launch (counter resets + both kernels) is captured once in a
 // CUDA graph and replayed; the warps per block, the reduction tile height and a register
@@ -22,6 +21,11 @@
 // W_ij, s_i (U_j - 2 V_ij) with V_ij = sum of e_n tanh(theta''_nj) over the strings n
 // flipping site i, recomputed in the tiles from the stored angles (storing these terms
 // per walker and string would move O(N^2 M) bytes per walker through HBM).
+// Both the measurement and the tiles are bound by FP32 arithmetic and the latency of the
+// L2 loads beside it at 8 to 16 warps per SM (the walker tasks' registers), so they take two
+// strings, or two rows, per packed operation, which leaves half of the issue slots, and the
+// tiles fetch a walker ahead: 64 instances of 16 to 144 spins, 30.7 -> 26.2 ms a replay.
+//
 // The sums run centred on the instance's mean energy E (the same value in every tile):
 //   gO = sum conj(O),  gE = sum (E_w - E) conj(O),  gK = sum conj(E_k) - conj(E) conj(O),
 //   gradient = (gE + gK) / W + (conj(E) - E) gO / W.
@@ -60,7 +64,7 @@ struct SInst {
     uint64_t* rng_index;  // [walkers]
     int chunks;           // walker chunks of kReduceWalkers
     float2* part;         // [chunks][3][N + 1][Mpad] a chunk's gO, gE, gK (row N: the biases)
-    double2* g;           // [3][N + 1][Mpad] the sums over all chunks
+    double2* grad;        // [2 N + M + N M] the gradient, the reference's layout (alpha, beta: 0)
     double2* emean;       // [1] the mean local energy the sums are centred on
     unsigned int* done;   // walkers finished in this replay
 };
@@ -222,94 +226,147 @@ __device__ __noinline__ void walker_task(const SLaunch& L, const SInst& Ig, int 
         }
     }
     // measurement at the final configuration: the local energy, tanh(theta), and for the
-    // E_k term the angles, U_j = sum_n e_n tanh(theta''_nj) and the e_n.  Three
-    // shared-memory slices [kSK][32] of this warp hold f(theta), the current string's
-    // tanh(theta'') and U, keeping the register footprint of the sweeps; f and tanh of an
-    // angle come from one evaluation with the approximate reciprocal (lc_tanh_approx; the
-    // local-energy differences, as rbm_eloc_t_kernel takes them)
+    // E_k term the angles, U_j = sum_n e_n tanh(theta''_nj) and the e_n.  Two consecutive
+    // off-diagonal strings at a time, in the halves of the packed operations: their four lane
+    // sums fold into one butterfly and their terms' exponentials run in the two halves of the
+    // warp (12 shuffles and one exponential for 40 and two).  f and tanh of an angle come from
+    // one evaluation with the approximate reciprocal (the local-energy differences, as
+    // rbm_eloc_t_kernel takes them).  f(theta), U and, between the two uses, tanh(theta'') are in
+    // registers up to K = 8; above, f, U and the real parts of tanh in this warp's shared-memory
+    // slices [3][kSK][32].
+    constexpr bool REGS = K <= 8;
     float tr[K], ti[K];
     s_refresh(I, s, tr, ti, lane);
     extern __shared__ float2 s_f[];
     float2* myf = s_f + (threadIdx.x >> 5) * 3 * kSK * 32 + lane;
     float2* myt = myf + kSK * 32;
     float2* myu = myt + kSK * 32;
+    float2 freg[REGS ? K : 1], ureg[REGS ? K : 1];
     const long row_w = static_cast<long>(w) * I.Mpad + lane;
 #pragma unroll
     for (int k = 0; k < K; k++) {
         float2 f, t;
         lc_tanh_approx(tr[k], ti[k], f, t);
-        myf[32 * k] = f;
+        if (REGS) {
+            freg[REGS ? k : 0] = f;
+            ureg[REGS ? k : 0] = make_float2(0.0f, 0.0f);
+        } else {
+            myf[32 * k] = f;
+            myu[32 * k] = make_float2(0.0f, 0.0f);
+        }
         I.T[row_w + 32 * k] = t;
         I.theta[row_w + 32 * k] = make_float2(tr[k], ti[k]);
-        myu[32 * k] = make_float2(0.0f, 0.0f);
     }
     float2 dsum = make_float2(0.0f, 0.0f);   // the diagonal strings' summed coefficient
     KahanC e;
-    for (int n = 0; n < I.op.S; n++) {
-        const float2 cf = string_factor(I.op, n, s);
-        const int nf = I.op.nflip[n];
-        if (nf == 0) {
+    for (int n = 0; n < I.op.S;) {
+        if (I.op.nflip[n] == 0) {
+            const float2 cf = string_factor(I.op, n, s);
             e.add(cf.x, cf.y);
             dsum.x += cf.x;
             dsum.y += cf.y;
+            n++;
             continue;
         }
-        const int off = I.op.flip_off[n];
-        float2 part = make_float2(0.0f, 0.0f);
-        if (nf == 1) {
-            const int site = I.op.flip_sites[off];
-            const float two_s = s.up(site) ? -2.0f : 2.0f;
-            const float2* row = I.W + static_cast<long>(site) * I.Mpad + lane;
-            float2 wv[K];
-#pragma unroll
-            for (int k = 0; k < K; k++) wv[k] = __ldg(row + 32 * k);
+        // strings n and, if it is off-diagonal, n + 1 (else n twice, used once)
+        const bool two = n + 1 < I.op.S && I.op.nflip[n + 1] != 0;
+        const int n1 = two ? n + 1 : n;
+        pair_t pr = splat2(0.0f), pi = pr;
+        pair_t hr[REGS ? K : 1], hi[K];
+        auto unit = [&](int k, pair_t x, pair_t y) {
+            Pair2 g, h;
+            lc_tanh2_approx(x, y, g, h);
+            const float2 f0 = REGS ? freg[REGS ? k : 0] : myf[32 * k];
+            pr = add2(pr, sub2(g.re, splat2(f0.x)));
+            pi = add2(pi, sub2(g.im, splat2(f0.y)));
+            if (REGS) hr[REGS ? k : 0] = h.re;
+            else up2(h.re, myt[32 * k].x, myt[32 * k].y);
+            hi[k] = h.im;
+        };
+        if (I.op.nflip[n] == 1 && I.op.nflip[n1] == 1) {
+            const int s0 = I.op.flip_sites[I.op.flip_off[n]], s1 = I.op.flip_sites[I.op.flip_off[n1]];
+            const pair_t ts = pk2(s.up(s0) ? -2.0f : 2.0f, s.up(s1) ? -2.0f : 2.0f);
+            const float2* r0 = I.W + static_cast<long>(s0) * I.Mpad + lane;
+            const float2* r1 = I.W + static_cast<long>(s1) * I.Mpad + lane;
 #pragma unroll
             for (int k = 0; k < K; k++) {
-                float2 g, h;
-                lc_tanh_approx(fmaf(two_s, wv[k].x, tr[k]), fmaf(two_s, wv[k].y, ti[k]), g, h);
-                const float2 f0 = myf[32 * k];
-                part.x += g.x - f0.x;
-                part.y += g.y - f0.y;
-                myt[32 * k] = h;
+                const float2 wa = __ldg(r0 + 32 * k), wb = __ldg(r1 + 32 * k);
+                unit(k, fma2(ts, pk2(wa.x, wb.x), splat2(tr[k])), fma2(ts, pk2(wa.y, wb.y), splat2(ti[k])));
             }
         } else {
 #pragma unroll
             for (int k = 0; k < K; k++) {
-                float nr = tr[k], ni = ti[k];
-                for (int q = 0; q < nf; q++) {
-                    const int site = I.op.flip_sites[off + q];
-                    const float two_s = s.up(site) ? -2.0f : 2.0f;
-                    const float2 wv = __ldg(I.W + static_cast<long>(site) * I.Mpad + lane + 32 * k);
-                    nr = fmaf(two_s, wv.x, nr);
-                    ni = fmaf(two_s, wv.y, ni);
+                float x[2], y[2];
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int m = h == 0 ? n : n1;
+                    float nr = tr[k], ni = ti[k];
+                    for (int q = 0; q < I.op.nflip[m]; q++) {
+                        const int site = I.op.flip_sites[I.op.flip_off[m] + q];
+                        const float two_s = s.up(site) ? -2.0f : 2.0f;
+                        const float2 wv = __ldg(I.W + static_cast<long>(site) * I.Mpad + lane + 32 * k);
+                        nr = fmaf(two_s, wv.x, nr);
+                        ni = fmaf(two_s, wv.y, ni);
+                    }
+                    x[h] = nr;
+                    y[h] = ni;
                 }
-                float2 g, h;
-                lc_tanh_approx(nr, ni, g, h);
-                const float2 f0 = myf[32 * k];
-                part.x += g.x - f0.x;
-                part.y += g.y - f0.y;
-                myt[32 * k] = h;
+                unit(k, pk2(x[0], x[1]), pk2(y[0], y[1]));
             }
         }
-        const float2 t = string_term(cf, warp_sum_xor2(part));
-        e.add(t.x, t.y);
-        if (lane == 0) I.en[static_cast<long>(w) * I.op.num_offdiag + I.op.offdiag_slot[n]] = t;
+        // lanes 8 v .. 8 v + 7 end with the sum of value v of (Re 0, Im 0, Re 1, Im 1), added in
+        // warp_sum_xor2's order
+        float v[4];
+        up2(pr, v[0], v[2]);
+        up2(pi, v[1], v[3]);
+#pragma unroll
+        for (int half = 2, off = 16; half >= 1; half >>= 1, off >>= 1) {
+            const bool up = (lane & off) != 0;
+#pragma unroll
+            for (int q = 0; q < half; q++) {
+                const float send = up ? v[q] : v[q + half], keep = up ? v[q + half] : v[q];
+                v[q] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+            }
+        }
+#pragma unroll
+        for (int off = 4; off >= 1; off >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
+        // the lower half of the warp forms string n's term, the upper string n1's
+        const int half0 = lane & 16, mine = half0 ? n1 : n;
+        const float dx = __shfl_sync(0xffffffffu, v[0], half0), dy = __shfl_sync(0xffffffffu, v[0], half0 + 8);
+        const float2 t = string_term(string_factor(I.op, mine, s), make_float2(dx, dy));
+        if ((lane & 15) == 0 && (two || lane == 0))
+            I.en[static_cast<long>(w) * I.op.num_offdiag + I.op.offdiag_slot[mine]] = t;
+        const float2 t0 = make_float2(__shfl_sync(0xffffffffu, t.x, 0), __shfl_sync(0xffffffffu, t.y, 0));
+        const float2 t1 = make_float2(__shfl_sync(0xffffffffu, t.x, 16), __shfl_sync(0xffffffffu, t.y, 16));
+        e.add(t0.x, t0.y);
+        if (two) e.add(t1.x, t1.y);
+        const pair_t tx = pk2(t0.x, t1.x), ty = pk2(t0.y, t1.y);
 #pragma unroll
         for (int k = 0; k < K; k++) {
-            const float2 h = myt[32 * k];
-            const float2 x = make_float2(t.x * h.x - t.y * h.y, t.x * h.y + t.y * h.x);
-            float2 u = myu[32 * k];
-            u.x += x.x;
-            u.y += x.y;
-            myu[32 * k] = u;
+            const pair_t a = REGS ? hr[REGS ? k : 0] : pk2(myt[32 * k].x, myt[32 * k].y), b = hi[k];
+            const pair_t xr = fma2(tx, a, mul2(splat2(-1.0f), mul2(ty, b)));
+            const pair_t xi = fma2(ty, a, mul2(tx, b));
+            float x0, x1, y0, y1;
+            up2(xr, x0, x1);
+            up2(xi, y0, y1);
+            float2 u = REGS ? ureg[REGS ? k : 0] : myu[32 * k];
+            u.x += x0;
+            u.y += y0;
+            if (two) {
+                u.x += x1;
+                u.y += y1;
+            }
+            if (REGS) ureg[REGS ? k : 0] = u;
+            else myu[32 * k] = u;
         }
+        n = n1 + 1;
     }
 #pragma unroll
     for (int k = 0; k < K; k++) {
         const float2 h = I.T[row_w + 32 * k];
-        float2 u = myu[32 * k];
-        u.x += dsum.x * h.x - dsum.y * h.y;
-        u.y += dsum.x * h.y + dsum.y * h.x;
+        float2 u = REGS ? ureg[REGS ? k : 0] : myu[32 * k];
+        u.x += __fmaf_rn(dsum.x, h.x, -__fmul_rn(dsum.y, h.y));
+        u.y += __fmaf_rn(dsum.x, h.y, __fmul_rn(dsum.y, h.x));
         I.U[row_w + 32 * k] = u;
     }
     if (lane == 0) {
@@ -383,24 +440,29 @@ __device__ __noinline__ void reduce_task(const SLaunch& L, const SInst& Ig, int 
             if (I.op.nflip[n] == 1) fslot[r] = slot;
         }
     }
-    // the e_n of a block of 32 walkers, [R][32], in this warp's shared-memory slice
+    // rows r0 + 2 q and r0 + 2 q + 1 in the halves of the packed operations.  A block of 32
+    // walkers' e_n (Re, Re', Im, Im') and spins (+-1, +-1') of each row pair, [R / 2][32], are in
+    // this warp's shared-memory slice
     extern __shared__ float2 s_f[];
-    float2* sen = s_f + (threadIdx.x >> 5) * 3 * kSK * 32;
+    float4* sen = reinterpret_cast<float4*>(s_f + (threadIdx.x >> 5) * 3 * kSK * 32);
+    float2* ssg = reinterpret_cast<float2*>(sen + R / 2 * 32);
     const long estride = I.op.num_offdiag;
     const uint64_t* spins = reinterpret_cast<const uint64_t*>(I.spins);
     for (int kc = 0; kc < I.K; kc++) {
-        float2 aO[R], aE[R], aK[R];
+        pair_t aOx[R / 2], aOy[R / 2], aEx[R / 2], aEy[R / 2], aKx[R / 2], aKy[R / 2];
 #pragma unroll
-        for (int r = 0; r < R; r++) {
-            aO[r] = make_float2(0.0f, 0.0f);
-            aE[r] = make_float2(0.0f, 0.0f);
-            aK[r] = make_float2(0.0f, 0.0f);
-        }
+        for (int q = 0; q < R / 2; q++) aOx[q] = aOy[q] = aEx[q] = aEy[q] = aKx[q] = aKy[q] = splat2(0.0f);
         const int j = lane + 32 * kc;
-        float2 wr[R];   // W[i][j] of each row's site (the single-flip case)
+        pair_t wx[R / 2], wy[R / 2];   // -2 W[i][j] of each row pair's sites (the single-flip case)
 #pragma unroll
-        for (int r = 0; r < R; r++)
-            wr[r] = (r0 + r < I.N) ? __ldg(I.W + static_cast<long>(r0 + r) * I.Mpad + j) : make_float2(0.0f, 0.0f);
+        for (int q = 0; q < R / 2; q++) {
+            float2 a = make_float2(0.0f, 0.0f), b = a;
+            const float2* wp = I.W + static_cast<long>(r0 + 2 * q) * I.Mpad + j;
+            if (r0 + 2 * q < I.N) a = __ldg(wp);
+            if (r0 + 2 * q + 1 < I.N) b = __ldg(wp + I.Mpad);
+            wx[q] = pk2(-2.0f * a.x, -2.0f * b.x);
+            wy[q] = pk2(-2.0f * a.y, -2.0f * b.y);
+        }
         for (int wb = w0; wb < w1; wb += 32) {
             // a block of 32 walkers: lane b fetches walker wb + b's centred energy, the spins
             // of the tile's rows (bit r: row r0 + r up) and the e_n of the rows' single-flip
@@ -408,7 +470,6 @@ __device__ __noinline__ void reduce_task(const SLaunch& L, const SInst& Ig, int 
             // (__ldcg): the walkers' results were written by other SMs
             const int nb = min(32, w1 - wb);
             float sdx = 0.0f, sdy = 0.0f;
-            unsigned int sbits = 0u;
             __syncwarp();   // the previous block's reads of the slice are done
             if (lane < nb) {
                 const int ws = wb + lane;
@@ -420,29 +481,41 @@ __device__ __noinline__ void reduce_task(const SLaunch& L, const SInst& Ig, int 
                 const uint64_t lo = __ldcg(spins + static_cast<long>(ws) * I.nw + q0);
                 const uint64_t hi = q1 != q0 ? __ldcg(spins + static_cast<long>(ws) * I.nw + q1) : lo;
 #pragma unroll
-                for (int r = 0; r < R; r++) {
-                    const int i = r0 + r;
-                    if (i < I.N) {
+                for (int q = 0; q < R / 2; q++) {
+                    float sg[2] = {1.0f, 1.0f};   // the bias row's factor
+                    float2 en[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const int i = r0 + 2 * q + h;
+                        if (i >= I.N) continue;
                         const uint64_t wd = (i >> 6) == q0 ? lo : hi;
-                        sbits |= static_cast<unsigned int>((wd >> (i & 63)) & 1ull) << r;
-                        if (fslot[r] >= 0) sen[r * 32 + lane] = __ldcg(I.en + ws * estride + fslot[r]);
+                        sg[h] = (wd >> (i & 63)) & 1ull ? 1.0f : -1.0f;
+                        if (fslot[2 * q + h] >= 0) en[h] = __ldcg(I.en + ws * estride + fslot[2 * q + h]);
                     }
+                    sen[q * 32 + lane] = make_float4(en[0].x, en[1].x, en[0].y, en[1].y);
+                    ssg[q * 32 + lane] = make_float2(sg[0], sg[1]);
                 }
             }
             __syncwarp();
+            // the next walker's column is fetched while this one's rows are formed
+            long o = static_cast<long>(wb) * I.Mpad + j;
+            float2 tn = __ldcg(I.T + o), un = __ldcg(I.U + o), thn = __ldcg(I.theta + o);
             for (int bw = 0; bw < nb; bw++) {
                 const int w = wb + bw;
-                const long o = static_cast<long>(w) * I.Mpad + j;
-                const float2 t = __ldcg(I.T + o);
-                const float2 u = __ldcg(I.U + o);
-                const float2 th = __ldcg(I.theta + o);
+                const float2 t = tn, u = un, th = thn;
+                if (bw + 1 < nb) {
+                    o += I.Mpad;
+                    tn = __ldcg(I.T + o);
+                    un = __ldcg(I.U + o);
+                    thn = __ldcg(I.theta + o);
+                }
                 const float dx = __shfl_sync(0xffffffffu, sdx, bw);
                 const float dy = __shfl_sync(0xffffffffu, sdy, bw);
-                const unsigned int bits = __shfl_sync(0xffffffffu, sbits, bw);
                 // conj(t), (E - <E>) conj(t), and U - <E> t (E_k of the biases, centred)
                 const float cx = t.x, cy = -t.y;
-                const float ex = dx * cx - dy * cy, ey = dx * cy + dy * cx;
-                const float kx = u.x - (Er * t.x - Ei * t.y), ky = u.y - (Er * t.y + Ei * t.x);
+                const float ex = __fmaf_rn(dx, cx, -__fmul_rn(dy, cy)), ey = __fmaf_rn(dy, cx, __fmul_rn(dx, cy));
+                const float kx = __fsub_rn(u.x, __fmaf_rn(Er, t.x, -__fmul_rn(Ei, t.y)));
+                const float ky = __fsub_rn(u.y, __fmaf_rn(Er, t.y, __fmul_rn(Ei, t.x)));
                 uint64_t sw[kSW];
 #pragma unroll
                 for (int q = 0; q < kSW; q++)
@@ -455,26 +528,32 @@ __device__ __noinline__ void reduce_task(const SLaunch& L, const SInst& Ig, int 
                     return ((wd >> (site & 63)) & 1ull) != 0ull;
                 };
 #pragma unroll
-                for (int r = 0; r < R; r++) {
-                    const int i = r0 + r;
-                    if (i > I.N) continue;
-                    float sg = 1.0f;
-                    float vx = 0.0f, vy = 0.0f;
-                    if (i < I.N) {
-                        sg = (bits >> r) & 1u ? 1.0f : -1.0f;
-                        // V_ij = sum over the strings n flipping site i of e_n tanh(theta''_nj),
-                        // the angles theta'' formed as the walker task formed them
-                        if (fslot[r] >= 0) {
-                            const float two_s = sg > 0.0f ? -2.0f : 2.0f;
-                            float2 g, h;
-                            lc_tanh_approx(fmaf(two_s, wr[r].x, th.x), fmaf(two_s, wr[r].y, th.y), g, h);
-                            const float2 en = sen[r * 32 + bw];
-                            vx = en.x * h.x - en.y * h.y;
-                            vy = en.x * h.y + en.y * h.x;
-                        } else if (GENERAL) {
+                for (int q = 0; q < R / 2; q++) {
+                    if (r0 + 2 * q > I.N) continue;
+                    const float2 sgf = ssg[q * 32 + bw];
+                    const pair_t sg = pk2(sgf.x, sgf.y);
+                    // V_ij = sum over the strings n flipping site i of e_n tanh(theta''_nj),
+                    // the angles theta'' formed as the walker task formed them
+                    pair_t vx = splat2(0.0f), vy = vx;
+                    if (!GENERAL || fslot[2 * q] >= 0 || fslot[2 * q + 1] >= 0) {
+                        const Pair2 h = tanh2_approx(fma2(sg, wx[q], splat2(th.x)), fma2(sg, wy[q], splat2(th.y)));
+                        const float4 en = sen[q * 32 + bw];
+                        const pair_t enx = pk2(en.x, en.y), eny = pk2(en.z, en.w);
+                        vx = fma2(enx, h.re, mul2(splat2(-1.0f), mul2(eny, h.im)));
+                        vy = fma2(enx, h.im, mul2(eny, h.re));
+                    }
+                    if (GENERAL) {
+                        float v0[2], v1[2];
+                        up2(vx, v0[0], v0[1]);
+                        up2(vy, v1[0], v1[1]);
+#pragma unroll
+                        for (int hf = 0; hf < 2; hf++) {
+                            const int r = 2 * q + hf;
+                            if (fslot[r] >= 0 || r0 + r >= I.N) continue;
+                            float vrx = 0.0f, vry = 0.0f;
                             const float2* enw = I.en + w * estride;
-                            for (int q = sb[r]; q < se[r]; q++) {
-                                const int slot = I.site_slots[q];
+                            for (int p = sb[r]; p < se[r]; p++) {
+                                const int slot = I.site_slots[p];
                                 const int n = I.op.offdiag[slot];
                                 const int nf = I.op.nflip[n], fo = I.op.flip_off[n];
                                 float nr = th.x, ni = th.y;
@@ -488,47 +567,69 @@ __device__ __noinline__ void reduce_task(const SLaunch& L, const SInst& Ig, int 
                                 float2 g, h;
                                 lc_tanh_approx(nr, ni, g, h);
                                 const float2 en = __ldcg(enw + slot);
-                                vx += en.x * h.x - en.y * h.y;
-                                vy += en.x * h.y + en.y * h.x;
+                                vrx += en.x * h.x - en.y * h.y;
+                                vry += en.x * h.y + en.y * h.x;
                             }
+                            v0[hf] = vrx;
+                            v1[hf] = vry;
                         }
+                        vx = pk2(v0[0], v0[1]);
+                        vy = pk2(v1[0], v1[1]);
                     }
-                    aO[r].x += sg * cx;
-                    aO[r].y += sg * cy;
-                    aE[r].x += sg * ex;
-                    aE[r].y += sg * ey;
-                    // conj(s_i (U - 2 V) - <E> O) = sg conj(U - <E> t - 2 V)
-                    aK[r].x += sg * (kx - 2.0f * vx);
-                    aK[r].y -= sg * (ky - 2.0f * vy);
+                    aOx[q] = fma2(sg, splat2(cx), aOx[q]);   // sg = +-1: the products are exact
+                    aOy[q] = fma2(sg, splat2(cy), aOy[q]);
+                    aEx[q] = fma2(sg, splat2(ex), aEx[q]);
+                    aEy[q] = fma2(sg, splat2(ey), aEy[q]);
+                    // conj(s_i (U - 2 V) - <E> O) = sg conj(U - <E> t - 2 V); aKy holds its negative
+                    aKx[q] = fma2(sg, fma2(splat2(-2.0f), vx, splat2(kx)), aKx[q]);
+                    aKy[q] = fma2(sg, fma2(splat2(-2.0f), vy, splat2(ky)), aKy[q]);
                 }
             }
         }
+        auto put = [&](pair_t x, pair_t y, float sy, float2* out, int q) {
+            float x0, x1, y0, y1;
+            up2(x, x0, x1);
+            up2(y, y0, y1);
+            const long e = static_cast<long>(r0 + 2 * q) * I.Mpad + j;
+            if (r0 + 2 * q <= I.N) out[e] = make_float2(x0, sy * y0);
+            if (r0 + 2 * q + 1 <= I.N) out[e + I.Mpad] = make_float2(x1, sy * y1);
+        };
 #pragma unroll
-        for (int r = 0; r < R; r++) {
-            const int i = r0 + r;
-            if (i <= I.N) {
-                const long e = static_cast<long>(i) * I.Mpad + j;
-                part[e] = aO[r];
-                part[plane + e] = aE[r];
-                part[2 * plane + e] = aK[r];
-            }
+        for (int q = 0; q < R / 2; q++) {
+            put(aOx[q], aOy[q], 1.0f, part, q);
+            put(aEx[q], aEy[q], 1.0f, part + plane, q);
+            put(aKx[q], aKy[q], -1.0f, part + 2 * plane, q);
         }
     }
 }
 
-// the sums over the walker chunks, in chunk order (FP64): blockIdx.y is the instance
+// the sums over the walker chunks, in chunk order, and from them the gradient in the
+// reference's parameter layout (FP64): blockIdx.y is the instance, e a row and column of its
+// sums.  Formed here, a result is one copy of 16 bytes per parameter; three sums per padded
+// entry and the combination on the host took 8.6 ms for 64 instances of up to 144 spins, 30 ms
+// of kernel.
 __global__ void serve_finish_kernel(const SInst* inst) {
     const SInst& I = inst[blockIdx.y];
-    const long n = 3L * (I.N + 1) * I.Mpad;
-    for (long e = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; e < n;
+    const long plane = static_cast<long>(I.N + 1) * I.Mpad, n = 3 * plane;
+    const double inv = 1.0 / I.walkers;
+    const double shift = -2.0 * I.emean->y;   // conj(E) - E = i shift
+    for (long e = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; e < plane;
          e += static_cast<long>(gridDim.x) * blockDim.x) {
-        double sx = 0.0, sy = 0.0;
+        const int row = static_cast<int>(e / I.Mpad), j = static_cast<int>(e - static_cast<long>(row) * I.Mpad);
+        if (j >= I.M) continue;
+        double ox = 0.0, oy = 0.0, ex = 0.0, ey = 0.0, kx = 0.0, ky = 0.0;
         for (int c = 0; c < I.chunks; c++) {
-            const float2 v = I.part[c * n + e];
-            sx += v.x;
-            sy += v.y;
+            const float2 o = I.part[c * n + e], v = I.part[c * n + plane + e], k = I.part[c * n + 2 * plane + e];
+            ox += o.x;
+            oy += o.y;
+            ex += v.x;
+            ey += v.y;
+            kx += k.x;
+            ky += k.y;
         }
-        I.g[e] = make_double2(sx, sy);
+        // the biases (row N) come before the weights
+        const long at = 2L * I.N + j + (row == I.N ? 0L : I.M + static_cast<long>(row) * I.M);
+        I.grad[at] = make_double2((ex + kx - shift * oy) * inv, (ey + ky + shift * ox) * inv);
     }
 }
 
@@ -574,8 +675,11 @@ struct rbmg_batch {
     std::vector<SInst> host_inst;
     std::vector<std::vector<char>> single_flip;   // [instance][site]: the single-flip tile serves the site
     std::vector<uint32_t> walkers;
-    DevBuf d_inst, d_tasks, d_next, d_done, d_error, d_accepts;
-    int max_elems = 0;          // largest instance's 3 (N + 1) Mpad (the finish kernel's grid)
+    DevBuf d_inst, d_tasks, d_next, d_done, d_accepts;
+    DevBuf d_status;            // [n] mean energies, then the error flag: one copy per replay
+    std::vector<double2> status;   // the last replay's
+    int* d_error() const { return reinterpret_cast<int*>(d_status.as<double2>() + n); }
+    int max_elems = 0;          // largest instance's (N + 1) Mpad (the finish kernel's grid)
     std::vector<std::unique_ptr<DevBuf>> bufs;
     int ntasks_walk = 0, ntasks = 0;
     int rows = 16;              // reduction tile height
@@ -662,7 +766,7 @@ cudaError_t launch_serve(rbmg_batch* b, cudaStream_t st) {
     L.therm = b->therm;
     L.sweeps = b->sweeps;
     L.first = b->first ? 1 : 0;
-    L.error = b->d_error.as<int>();
+    L.error = b->d_error();
     L.accepts = b->d_accepts.as<unsigned long long>();
     L.wait_ns = b->wait_ns;
     L.wait_extra = b->wait_extra;
@@ -723,15 +827,23 @@ int batch_capture(rbmg_batch* b) {
     return RBMG_OK;
 }
 
+// waits for the replays and takes the mean energies and the error flag
+cudaError_t batch_status(rbmg_batch* b, int* err) {
+    cudaError_t e = cudaMemcpyAsync(b->status.data(), b->d_status.p, sizeof(double2) * (b->n + 1), cudaMemcpyDeviceToHost,
+                                    stream());
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream());
+    std::memcpy(err, &b->status[b->n], sizeof(int));
+    return e;
+}
+
 int batch_replay(rbmg_batch* b) {
     int r = batch_capture(b);
     if (r != RBMG_OK) return r;
     RBMG_CK(cudaGraphLaunch(b->exec, stream()));
     int err = 0;
-    RBMG_CK(cudaMemcpyAsync(&err, b->d_error.p, sizeof(int), cudaMemcpyDeviceToHost, stream()));
-    RBMG_CK(cudaStreamSynchronize(stream()));
+    RBMG_CK(batch_status(b, &err));
     if (err) {
-        RBMG_CK(cudaMemset(b->d_error.p, 0, sizeof(int)));
+        RBMG_CK(cudaMemset(b->d_error(), 0, sizeof(int)));
         return fail(RBMG_ETIMEOUT, "batch: a reduction task timed out waiting for its walkers");
     }
     b->first = false;
@@ -745,6 +857,9 @@ extern "C" int rbmg_batch_create(int n, const rbmg_psi* const* psis, const rbmg_
     if (n <= 0 || !psis || !ops || !walkers || !seeds || !out) return fail(RBMG_EINVAL, "batch: bad arguments");
     auto b = std::make_unique<rbmg_batch>();
     b->n = n;
+    b->status.resize(n + 1);
+    RBMG_CK(b->d_status.ensure(sizeof(double2) * (n + 1)));
+    RBMG_CK(cudaMemset(b->d_status.p, 0, sizeof(double2) * (n + 1)));
     for (int i = 0; i < n; i++) {
         const rbmg_psi* p = psis[i];
         const rbmg_operator* o = ops[i];
@@ -794,10 +909,11 @@ extern "C" int rbmg_batch_create(int n, const rbmg_psi* const* psis, const rbmg_
         I.spins = static_cast<uint64_t*>(alloc(sizeof(uint64_t) * B * nw));
         I.rng_index = static_cast<uint64_t*>(alloc(sizeof(uint64_t) * B));
         I.chunks = static_cast<int>((B + kReduceWalkers - 1) / kReduceWalkers);
-        const size_t elems = 3 * static_cast<size_t>(p->N + 1) * p->Mpad;
-        I.part = static_cast<float2*>(alloc(sizeof(float2) * I.chunks * elems));
-        I.g = static_cast<double2*>(alloc(sizeof(double2) * elems));
-        I.emean = static_cast<double2*>(alloc(sizeof(double2)));
+        const size_t elems = static_cast<size_t>(p->N + 1) * p->Mpad;
+        const size_t params = 2 * static_cast<size_t>(p->N) + p->M + static_cast<size_t>(p->N) * p->M;
+        I.part = static_cast<float2*>(alloc(sizeof(float2) * 3 * I.chunks * elems));
+        I.grad = static_cast<double2*>(alloc(sizeof(double2) * params));
+        I.emean = b->d_status.as<double2>() + i;
         // the batch's own copy of the site lists (the operator's are rebuilt when it is used
         // with another N), and per site whether the single-flip tile serves it: exactly one
         // off-diagonal string flips the site and flips it alone (reduce_task's test)
@@ -821,10 +937,10 @@ extern "C" int rbmg_batch_create(int n, const rbmg_psi* const* psis, const rbmg_
             b->single_flip.push_back(std::move(single));
         }
         b->max_elems = std::max(b->max_elems, static_cast<int>(elems));
-        if (!I.eloc || !I.T || !I.U || !I.theta || !I.en || !I.spins || !I.rng_index || !I.part || !I.g ||
-            !I.emean)
+        if (!I.eloc || !I.T || !I.U || !I.theta || !I.en || !I.spins || !I.rng_index || !I.part || !I.grad)
             return fail(RBMG_ENOMEM, "batch: device allocation failed");
         RBMG_CK(cudaMemset(I.rng_index, 0, sizeof(uint64_t) * B));
+        RBMG_CK(cudaMemset(I.grad, 0, sizeof(double2) * 2 * p->N));   // alpha and beta
         b->psis.push_back(p);
         b->ops.push_back(o);
         b->walkers.push_back(walkers[i]);
@@ -835,9 +951,7 @@ extern "C" int rbmg_batch_create(int n, const rbmg_psi* const* psis, const rbmg_
     RBMG_CK(b->d_inst.ensure(sizeof(SInst) * n));
     RBMG_CK(cudaMemcpy(b->d_inst.p, b->host_inst.data(), sizeof(SInst) * n, cudaMemcpyHostToDevice));
     RBMG_CK(b->d_next.ensure(sizeof(unsigned int)));
-    RBMG_CK(b->d_error.ensure(sizeof(int)));
     RBMG_CK(b->d_accepts.ensure(sizeof(unsigned long long)));
-    RBMG_CK(cudaMemset(b->d_error.p, 0, sizeof(int)));
     const int r = batch_tasks(b.get());
     if (r != RBMG_OK) return r;
     *out = b.release();
@@ -930,7 +1044,7 @@ extern "C" int rbmg_batch_autotune(rbmg_batch* b, int sweeps, int reps, double* 
             cudaEventDestroy(e0);
             cudaEventDestroy(e1);
             int err = 0;
-            RBMG_CK(cudaMemcpy(&err, b->d_error.p, sizeof(int), cudaMemcpyDeviceToHost));
+            RBMG_CK(batch_status(b, &err));
             if (err) return fail(RBMG_ETIMEOUT, "batch autotune: a reduction task timed out");
             const double per = ms / reps;
             if (ms_out) ms_out[c] = per;
@@ -953,29 +1067,16 @@ extern "C" int rbmg_batch_autotune(rbmg_batch* b, int sweeps, int reps, double* 
 extern "C" int rbmg_batch_result(const rbmg_batch* b, int i, double* energy, double* grad, double* eloc) {
     if (!b || i < 0 || i >= b->n || !energy) return fail(RBMG_EINVAL, "batch result: bad arguments");
     const SInst& I = b->host_inst[i];
-    double2 em;
-    RBMG_CK(cudaMemcpy(&em, I.emean, sizeof(double2), cudaMemcpyDeviceToHost));
-    const cplx E(em.x, em.y);
-    energy[0] = E.real();
-    energy[1] = E.imag();
-    if (eloc) RBMG_CK(cudaMemcpy(eloc, I.eloc, sizeof(double2) * I.walkers, cudaMemcpyDeviceToHost));
+    energy[0] = b->status[i].x;
+    energy[1] = b->status[i].y;
+    if (eloc) {
+        prefault(eloc, sizeof(double2) * I.walkers);
+        RBMG_CK(cudaMemcpy(eloc, I.eloc, sizeof(double2) * I.walkers, cudaMemcpyDeviceToHost));
+    }
     if (grad) {
-        const size_t plane = static_cast<size_t>(I.N + 1) * I.Mpad;
-        std::vector<double2> g(3 * plane);
-        RBMG_CK(cudaMemcpy(g.data(), I.g, sizeof(double2) * 3 * plane, cudaMemcpyDeviceToHost));
-        cplx* out = reinterpret_cast<cplx*>(grad);
-        const int N = I.N, M = I.M;
-        const double inv = 1.0 / I.walkers;
-        const cplx shift = std::conj(E) - E;
-        for (int k = 0; k < 2 * N; k++) out[k] = 0.0;
-        auto val = [&](int row, int j) {
-            const size_t e = static_cast<size_t>(row) * I.Mpad + j;
-            const cplx gO(g[e].x, g[e].y), gE(g[plane + e].x, g[plane + e].y), gK(g[2 * plane + e].x, g[2 * plane + e].y);
-            return (gE + gK) * inv + shift * gO * inv;
-        };
-        for (int j = 0; j < M; j++) out[2 * N + j] = val(N, j);
-        for (int r = 0; r < N; r++)
-            for (int j = 0; j < M; j++) out[2 * N + M + static_cast<size_t>(r) * M + j] = val(r, j);
+        const size_t params = 2 * static_cast<size_t>(I.N) + I.M + static_cast<size_t>(I.N) * I.M;
+        prefault(grad, sizeof(double2) * params);
+        RBMG_CK(cudaMemcpy(grad, I.grad, sizeof(double2) * params, cudaMemcpyDeviceToHost));
     }
     return RBMG_OK;
 }
