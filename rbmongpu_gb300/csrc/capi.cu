@@ -52,8 +52,11 @@ int deep_log_psi(const rbmg_psi* psi, int count, const uint64_t* d_spins, uint64
 // Grow-only scratch buffers shared by all calls on this thread's device.
 struct Workspace {
     DevBuf sample_spins, eloc, logpsi, logpsi_p, T, U, X, theta, en, vpart, Tp, weights, coef1, coef2, coef3, omega, pr, nn;
-    DevBuf partial, block_scratch, sums, acc_O, acc_EO, acc_Ek, acc_wO, acc_pO, block_max, zsum;
+    DevBuf partial, block_scratch, sums, acc_O, acc_EO, acc_Ek, acc_wO, acc_pO;
     DevBuf smat, smean, spart, okrows, sshift, splanes, serror, sout;
+    DevBuf stat;      // (m, sum), (log Z, -) of exact summation's weights, then the first chunk's mean energy
+    DevBuf gout;      // a gradient on its way to the host
+    HostBuf status;   // GradOut::status
     DevBuf acc_B, eabs2, lsums, rw, rwc, acc_C2, acc_C3;
     DevBuf tab64, tab64_p;   // spin-group sums of psi's and psi''s FP64 weights
     DevBuf fqa_qa, fqa_r, fqa_flip, fqa_lpf, fqa_lp, fqa_out;   // free-quantum-axis terms of the HSD
@@ -62,6 +65,13 @@ struct Workspace {
 static Workspace& ws() {
     static thread_local Workspace w;
     return w;
+}
+
+// the sums' scratch, its counter zero from the start
+static cudaError_t sum_scratch(Workspace& W) {
+    if (W.block_scratch.p) return cudaSuccess;
+    const cudaError_t e = W.block_scratch.ensure(sizeof(double2) * kSumScratch);
+    return e != cudaSuccess ? e : cudaMemsetAsync(W.block_scratch.p, 0, sizeof(double2) * kSumScratch, stream());
 }
 
 
@@ -665,6 +675,10 @@ struct Chunk {
 };
 
 struct StreamResult {
+    // set by a caller that takes the results on the device: exact summation then leaves its
+    // factor in Workspace::stat, and a Monte-Carlo pass leaves its counts on their way, for
+    // stream_done after the caller's own wait
+    bool defer = false;
     double norm_factor = 1.0;   // reference weight scale: sum_s prefactor^2 |psi|^2 (exact) or 1/num_samples (MC)
     double log_norm = 0.0;      // log of sum_s prefactor^2 |psi|^2 (exact)
 };
@@ -697,11 +711,12 @@ static int psi_log_psi_dev(const rbmg_psi* psi, int count, const uint64_t* d_spi
 }
 
 constexpr int kExactChunk = 1 << 16;
+constexpr const char* kNonFiniteLogPsi = "ExactSummation: non-finite log psi";
 
 // MonteCarloLoop::foreach (include/spin_ensembles/MonteCarloLoop.hpp:294-339): every call
 // re-draws the start configurations and thermalises; the chains' Philox streams continue.
 static int mc_stream(rbmg_ensemble* e, const rbmg_psi* psi, const rbmg_operator* op, bool want_eloc,
-                     size_t max_chunk_samples, const std::function<int(const Chunk&)>& fn) {
+                     size_t max_chunk_samples, bool defer, const std::function<int(const Chunk&)>& fn) {
     if (psi->kind != 0) return fail(RBMG_EUNSUPPORTED, "MonteCarloLoop: PsiDeep / PsiPair chains are sampled by deep.cu");
     if (e->fast_sweep_tries && e->total_z)
         return fail(RBMG_EUNSUPPORTED, "fast sweep with total_z symmetry (the reference pairs a mask with an unset site)");
@@ -756,12 +771,10 @@ static int mc_stream(rbmg_ensemble* e, const rbmg_psi* psi, const rbmg_operator*
         const int r = fn(c);
         if (r != RBMG_OK) return r;
     }
-    std::vector<unsigned long long> a(B), p(B);
-    RBMG_CK(cudaMemcpyAsync(a.data(), e->accepts.p, sizeof(unsigned long long) * B, cudaMemcpyDeviceToHost, stream()));
-    RBMG_CK(cudaMemcpyAsync(p.data(), e->proposals.p, sizeof(unsigned long long) * B, cudaMemcpyDeviceToHost, stream()));
+    RBMG_CK(e->counts_copy());
+    if (defer) return RBMG_OK;
     RBMG_CK(cudaStreamSynchronize(stream()));
-    e->last_accepts.assign(a.begin(), a.end());
-    e->last_proposals.assign(p.begin(), p.end());
+    e->counts_take();
     return RBMG_OK;
 }
 
@@ -784,35 +797,11 @@ static int exact_stream(rbmg_ensemble* e, const rbmg_psi* psi, StreamResult* res
                                       W.logpsi.as<double2>() + base);
         if (r != RBMG_OK) return r;
     }
-    // FP64 log-sum-exp of 2 Re log psi
-    RBMG_CK(W.block_max.ensure(sizeof(double) * kSumBlocks));
-    int blocks = 0;
-    RBMG_CK(launch_max_re2(static_cast<int>(total), W.logpsi.as<double2>(), W.block_max.as<double>(), &blocks, stream()));
-    std::vector<double> bm(blocks);
-    RBMG_CK(cudaMemcpyAsync(bm.data(), W.block_max.p, sizeof(double) * blocks, cudaMemcpyDeviceToHost, stream()));
-    RBMG_CK(cudaStreamSynchronize(stream()));
-    const double mx = *std::max_element(bm.begin(), bm.end());
-    if (!std::isfinite(mx)) return fail(RBMG_ENAN, "ExactSummation: non-finite log psi");
-    RBMG_CK(launch_exp_weights(static_cast<int>(total), W.logpsi.as<double2>(), mx, W.weights.as<double>(), stream()));
-    RBMG_CK(W.block_scratch.ensure(sizeof(double2) * kSumBlocks * kMaxSeries));
-    RBMG_CK(W.zsum.ensure(sizeof(double2) * kMaxSeries));
-    RBMG_CK(cudaMemsetAsync(W.zsum.p, 0, sizeof(double2) * kMaxSeries, stream()));
-    // sum of the weights (its own accumulator: the caller's sums are already armed)
-    RBMG_CK(W.coef1.ensure(sizeof(double2) * total));
-    RBMG_CK(launch_coef(static_cast<int>(total), W.weights.as<double>(), nullptr, 1.0, W.coef1.as<double2>(), stream()));
-    SeriesSet set{};
-    set.n = 1;
-    set.v[0] = W.coef1.as<double2>();
-    RBMG_CK(launch_weighted_sums(static_cast<int>(total), nullptr, set, W.block_scratch.as<double2>(),
-                                 W.zsum.as<double2>(), stream()));
-    double2 z;
-    RBMG_CK(cudaMemcpyAsync(&z, W.zsum.p, sizeof(double2), cudaMemcpyDeviceToHost, stream()));
-    RBMG_CK(cudaStreamSynchronize(stream()));
-    const double logZ = mx + std::log(z.x);
-    // normalised weights w_s = |psi_s|^2 / Z
-    RBMG_CK(launch_exp_weights(static_cast<int>(total), W.logpsi.as<double2>(), logZ, W.weights.as<double>(), stream()));
-    res->log_norm = 2.0 * std::log(psi->prefactor) + logZ;
-    res->norm_factor = std::exp(res->log_norm);
+    // normalised weights w_s = |psi_s|^2 / Z, Z from the FP64 log-sum-exp of 2 Re log psi
+    RBMG_CK(sum_scratch(W));
+    RBMG_CK(W.stat.ensure(sizeof(double2) * 3));
+    RBMG_CK(launch_exact_weights(static_cast<int>(total), W.logpsi.as<double2>(), W.weights.as<double>(),
+                                 W.block_scratch.as<double2>(), W.stat.as<double2>(), stream()));
     for (uint64_t base = 0; base < total; base += kExactChunk) {
         Chunk c;
         c.count = static_cast<int>(std::min<uint64_t>(kExactChunk, total - base));
@@ -823,6 +812,13 @@ static int exact_stream(rbmg_ensemble* e, const rbmg_psi* psi, StreamResult* res
         const int r = fn(c);
         if (r != RBMG_OK) return r;
     }
+    if (res->defer) return RBMG_OK;
+    double2 stat[2];
+    RBMG_CK(cudaMemcpyAsync(stat, W.stat.p, sizeof(stat), cudaMemcpyDeviceToHost, stream()));
+    RBMG_CK(cudaStreamSynchronize(stream()));
+    if (!std::isfinite(stat[0].x)) return fail(RBMG_ENAN, kNonFiniteLogPsi);
+    res->log_norm = 2.0 * std::log(psi->prefactor) + stat[1].x;
+    res->norm_factor = std::exp(res->log_norm);
     return RBMG_OK;
 }
 
@@ -888,7 +884,7 @@ int deep_gradient_chunk(const rbmg_psi* psi, const rbmg_operator* op, const Chun
                         double2* acc_B = nullptr, double2* coef3 = nullptr);
 int deep_eloc_chunk(const rbmg_psi* psi, const rbmg_operator* op, const Chunk& c, double2* d_eloc, cudaStream_t st);
 int deep_stream(rbmg_ensemble* e, const rbmg_psi* psi, const rbmg_operator* op, bool want_eloc,
-                size_t max_chunk_samples, const std::function<int(const Chunk&)>& fn);
+                size_t max_chunk_samples, bool defer, const std::function<int(const Chunk&)>& fn);
 
 // local energies of one chunk into W.eloc (unless the sampler already produced them)
 static int chunk_eloc(const rbmg_psi* psi, const rbmg_operator* op, const Chunk& c, const double2** out) {
@@ -916,38 +912,17 @@ static int chunk_eloc(const rbmg_psi* psi, const rbmg_operator* op, const Chunk&
     return RBMG_OK;
 }
 
-// weighted mean of a per-sample complex series over one chunk (sum w v / sum w)
+// weighted mean of a per-sample complex series over one chunk (sum w v / sum w), left in
+// Workspace::stat; out (may be null) takes it to the host
 static int chunk_mean(const Chunk& c, const double2* v, cplx* out) {
     Workspace& W = ws();
-    RBMG_CK(W.coef3.ensure(sizeof(double2) * c.count));
-    RBMG_CK(launch_coef(c.count, c.weights, nullptr, 1.0, W.coef3.as<double2>(), stream()));
-    RBMG_CK(W.zsum.ensure(sizeof(double2) * kMaxSeries));
-    RBMG_CK(W.block_scratch.ensure(sizeof(double2) * kSumBlocks * kMaxSeries));
-    RBMG_CK(cudaMemsetAsync(W.zsum.p, 0, sizeof(double2) * kMaxSeries, stream()));
-    SeriesSet set{};
-    set.n = 2;
-    set.v[0] = v;
-    set.v[1] = W.coef3.as<double2>();   // the weights themselves, summed with unit weight below
-    RBMG_CK(launch_weighted_sums(c.count, c.weights, set, W.block_scratch.as<double2>(), W.zsum.as<double2>(),
-                                 stream()));
-    double2 m[2];
-    RBMG_CK(cudaMemcpyAsync(m, W.zsum.p, sizeof(m), cudaMemcpyDeviceToHost, stream()));
+    RBMG_CK(sum_scratch(W));
+    RBMG_CK(W.stat.ensure(sizeof(double2) * 3));
+    double2* mean = W.stat.as<double2>() + 2;
+    RBMG_CK(launch_weighted_mean(c.count, c.weights, v, W.block_scratch.as<double2>(), mean, stream()));
+    if (!out) return RBMG_OK;
+    RBMG_CK(cudaMemcpyAsync(out, mean, sizeof(double2), cudaMemcpyDeviceToHost, stream()));
     RBMG_CK(cudaStreamSynchronize(stream()));
-    // m[1] = sum w * w when weighted; the weight total needs the plain sum: recompute it
-    double wtot = static_cast<double>(c.count);
-    if (c.weights) {
-        SeriesSet s1{};
-        s1.n = 1;
-        s1.v[0] = W.coef3.as<double2>();
-        RBMG_CK(cudaMemsetAsync(W.zsum.p, 0, sizeof(double2) * kMaxSeries, stream()));
-        RBMG_CK(launch_weighted_sums(c.count, nullptr, s1, W.block_scratch.as<double2>(), W.zsum.as<double2>(),
-                                     stream()));
-        double2 t;
-        RBMG_CK(cudaMemcpyAsync(&t, W.zsum.p, sizeof(t), cudaMemcpyDeviceToHost, stream()));
-        RBMG_CK(cudaStreamSynchronize(stream()));
-        wtot = t.x;
-    }
-    *out = wtot > 0.0 ? cplx(m[0].x, m[0].y) / wtot : cplx(0.0, 0.0);
     return RBMG_OK;
 }
 
@@ -973,15 +948,15 @@ static int run_stream(rbmg_ensemble* ens, const rbmg_psi* psi, const rbmg_operat
     if (ens->kind == 1) return exact_stream(ens, psi, res, fn);
     if (ens->kind == 2) return fixed_stream(ens, psi, max_chunk, res, fn);
     res->norm_factor = 1.0 / static_cast<double>(ens->num_samples);
-    if (psi->kind != 0) return deep_stream(ens, psi, op, sampler_eloc, max_chunk, fn);
-    return mc_stream(ens, psi, op, sampler_eloc, max_chunk, fn);
+    if (psi->kind != 0) return deep_stream(ens, psi, op, sampler_eloc, max_chunk, res->defer, fn);
+    return mc_stream(ens, psi, op, sampler_eloc, max_chunk, res->defer, fn);
 }
 
 // <E> and <|E|^2> with reference weights
 static int energy_sums(const rbmg_psi* psi, const rbmg_operator* op, rbmg_ensemble* ens, Sums* out) {
     Workspace& W = ws();
     RBMG_CK(W.sums.ensure(sizeof(double2) * kMaxSeries));
-    RBMG_CK(W.block_scratch.ensure(sizeof(double2) * kSumBlocks * kMaxSeries));
+    RBMG_CK(sum_scratch(W));
     RBMG_CK(cudaMemsetAsync(W.sums.p, 0, sizeof(double2) * kMaxSeries, stream()));
     StreamResult res;
     int r = run_stream(ens, psi, op, true, size_t(1) << 22, &res, [&](const Chunk& c) -> int {
@@ -1043,7 +1018,7 @@ static int zero_sums(DevBuf& b, int n) {
 // sums[0] += sum_s w[s] v[s]
 static int add_sum(const Chunk& c, const double* w, const double2* v, double2* sum) {
     Workspace& W = ws();
-    RBMG_CK(W.block_scratch.ensure(sizeof(double2) * kSumBlocks * kMaxSeries));
+    RBMG_CK(sum_scratch(W));
     SeriesSet set{};
     set.n = 1;
     set.v[0] = v;
@@ -1200,39 +1175,42 @@ extern "C" int rbmg_ev_fluctuation(const rbmg_psi* psi, const rbmg_operator* op,
 }
 
 // The gradient's sums, left on the device: acc_O = sum w O, acc_EO = sum w (E - E0) O*,
-// acc_Ek = sum w (E_k - E0 O) over the O_k entries k >= 2N, sums[0] = sum w E; E0 (the
-// first chunk's mean local energy) and the ensemble's normalisation factor come back.
+// acc_Ek = sum w (E_k - E0 O) over the O_k entries k >= 2N, sums[0] = sum w E, and E0 (the
+// first chunk's mean local energy) and the factor of exact summation in Workspace::stat.
 // fluct: also B = sum w conj(E - E0) (E_k - E0 O_k) into acc_B and sum w |E|^2 into sums[1]
-// (the further sums of ExpectationValue::fluctuation_gradient).  adjoint (complex RBM): also
-// C2 = sum w (E - E0) O_k into acc_C2 and C3 = sum w (Re E - Re E0) conj(O_k) into acc_C3
-// (the derivative of <E_loc>, rbmg_ev_eloc_gradient).
-static int ev_gradient_sums(const rbmg_psi* psi, const rbmg_operator* op, rbmg_ensemble* ens, cplx* E0_out,
-                            double* norm_out, bool fluct = false, bool adjoint = false) {
+// (the further sums of ExpectationValue::fluctuation_gradient).  adjoint (complex RBM): in
+// place of acc_EO, C2 = sum w (E - E0) O_k into acc_C2 and C3 = sum w (Re E - Re E0) conj(O_k)
+// into acc_C3 (the derivative of <E_loc>, rbmg_ev_eloc_gradient).
+static int ev_gradient_sums(const rbmg_psi* psi, const rbmg_operator* op, rbmg_ensemble* ens, StreamResult* res,
+                            bool fluct = false, bool adjoint = false) {
     int r = check_pair(psi, op, ens);
     if (r != RBMG_OK) return r;
     const int N = psi->N, P = psi->num_params();
     const int nw = nwords_of(N);
     Workspace& W = ws();
     const size_t ok_len = static_cast<size_t>(P - 2 * N);   // O_k entries the accumulators hold
-    RBMG_CK(W.acc_O.ensure(sizeof(double2) * ok_len));
-    RBMG_CK(W.acc_EO.ensure(sizeof(double2) * ok_len));
-    RBMG_CK(W.acc_Ek.ensure(sizeof(double2) * ok_len));
-    RBMG_CK(cudaMemsetAsync(W.acc_O.p, 0, sizeof(double2) * ok_len, stream()));
-    RBMG_CK(cudaMemsetAsync(W.acc_EO.p, 0, sizeof(double2) * ok_len, stream()));
-    RBMG_CK(cudaMemsetAsync(W.acc_Ek.p, 0, sizeof(double2) * ok_len, stream()));
-    if (fluct) {
-        RBMG_CK(W.acc_B.ensure(sizeof(double2) * ok_len));
-        RBMG_CK(cudaMemsetAsync(W.acc_B.p, 0, sizeof(double2) * ok_len, stream()));
-    }
+    // the accumulators of this pass; the RBM's first chunk stores into them, the others add
+    DevBuf* acc[5] = {&W.acc_O, &W.acc_Ek, nullptr, nullptr, nullptr};
+    int naccs = 2;
+    if (!adjoint) acc[naccs++] = &W.acc_EO;
+    if (fluct) acc[naccs++] = &W.acc_B;
     if (adjoint) {
         if (psi->kind != 0) return fail(RBMG_EUNSUPPORTED, "adjoint sums: complex RBM only");
-        RBMG_CK(W.acc_C2.ensure(sizeof(double2) * ok_len));
-        RBMG_CK(W.acc_C3.ensure(sizeof(double2) * ok_len));
-        RBMG_CK(cudaMemsetAsync(W.acc_C2.p, 0, sizeof(double2) * ok_len, stream()));
-        RBMG_CK(cudaMemsetAsync(W.acc_C3.p, 0, sizeof(double2) * ok_len, stream()));
+        acc[naccs++] = &W.acc_C2;
+        acc[naccs++] = &W.acc_C3;
     }
+    auto zero_accs = [&]() -> int {
+        for (int q = 0; q < naccs; q++) RBMG_CK(cudaMemsetAsync(acc[q]->p, 0, sizeof(double2) * ok_len, stream()));
+        return RBMG_OK;
+    };
+    for (int q = 0; q < naccs; q++) RBMG_CK(acc[q]->ensure(sizeof(double2) * ok_len));
+    if (psi->kind != 0) {
+        r = zero_accs();
+        if (r != RBMG_OK) return r;
+    }
+    RBMG_CK(W.stat.ensure(sizeof(double2) * 3));
     RBMG_CK(W.sums.ensure(sizeof(double2) * kMaxSeries));
-    RBMG_CK(W.block_scratch.ensure(sizeof(double2) * kSumBlocks * kMaxSeries));
+    RBMG_CK(sum_scratch(W));
     RBMG_CK(cudaMemsetAsync(W.sums.p, 0, sizeof(double2) * kMaxSeries, stream()));
     constexpr int kSplits = 64;
     size_t per_sample = 0;
@@ -1240,16 +1218,17 @@ static int ev_gradient_sums(const rbmg_psi* psi, const rbmg_operator* op, rbmg_e
         r = op_site_lists(const_cast<rbmg_operator*>(op), N);
         if (r != RBMG_OK) return r;
         per_sample = sizeof(float2) * psi->Mpad * (2 + op->num_offdiag) + 64;
-        RBMG_CK(W.partial.ensure(sizeof(double2) * kMaxOuter * kSplits * (1 + N) * psi->M));
+        // of the sums over T, and of those over U
+        RBMG_CK(W.partial.ensure(sizeof(double2) * ((adjoint ? 3 : 2) + (fluct ? 2 : 1)) * kSplits * (1 + N) * psi->M));
     }
     const size_t max_chunk = psi->kind == 0 ? std::max<size_t>(256, (size_t(512) << 20) / per_sample) : 4096;
     // The sums are centred on E0, the mean local energy of the first chunk:
     // EO' = sum w (E - E0) O*, Ek' = sum w (E_k - E0 O), so that FP32 partial sums keep
     // the small covariance the gradient is made of (see the formula below).
     cplx E0(0.0, 0.0);
-    bool have_shift = false;
-    StreamResult res;
-    r = run_stream(ens, psi, op, false, max_chunk, &res, [&](const Chunk& c) -> int {
+    bool have_shift = false, first = true;
+    double2* e0_dev = W.stat.as<double2>() + 2;
+    r = run_stream(ens, psi, op, false, max_chunk, res, [&](const Chunk& c) -> int {
         RBMG_CK(W.eloc.ensure(sizeof(double2) * c.count));
         if (psi->kind != 0) {
             if (!have_shift) {
@@ -1275,7 +1254,7 @@ static int ev_gradient_sums(const rbmg_psi* psi, const rbmg_operator* op, rbmg_e
                 const double2* e0 = nullptr;
                 const int rr0 = chunk_eloc(psi, op, c, &e0);
                 if (rr0 != RBMG_OK) return rr0;
-                const int rr1 = chunk_mean(c, e0, &E0);
+                const int rr1 = chunk_mean(c, e0, nullptr);
                 if (rr1 != RBMG_OK) return rr1;
                 have_shift = true;
             }
@@ -1303,13 +1282,15 @@ static int ev_gradient_sums(const rbmg_psi* psi, const rbmg_operator* op, rbmg_e
             L.T = W.T.as<float2>();
             L.U = W.U.as<float2>();
             L.X = W.X.as<float2>();
-            L.e_shift = make_double2(E0.real(), E0.imag());
+            L.e_shift = e0_dev;
             RBMG_CK(launch_rbm_estimate(psi->rbm_dev(), &od, nullptr, L, stream()));
             RBMG_CK(W.coef1.ensure(sizeof(double2) * c.count));
             RBMG_CK(W.coef2.ensure(sizeof(double2) * c.count));
-            RBMG_CK(launch_coef(c.count, c.weights, nullptr, 1.0, W.coef1.as<double2>(), stream()));
-            RBMG_CK(launch_coef(c.count, c.weights, W.eloc.as<double2>(), 1.0, W.coef2.as<double2>(), stream(),
-                                make_double2(E0.real(), E0.imag())));
+            if (adjoint || fluct) RBMG_CK(W.coef3.ensure(sizeof(double2) * c.count));
+            RBMG_CK(launch_grad_coefs(c.count, c.weights, W.eloc.as<double2>(), e0_dev, W.coef1.as<double2>(),
+                                      W.coef2.as<double2>(), adjoint || fluct ? W.coef3.as<double2>() : nullptr,
+                                      fluct ? 1 : 0, stream()));
+            SplitSum jobs[2] = {};   // the sums over T, and over U (with the V sums of a transverse field)
             if (single) {
                 RBMG_CK(W.vpart.ensure(grad_vectors_bytes(c.count, N, psi->M, kSplits)));
                 GradVectors G{};
@@ -1327,34 +1308,30 @@ static int ev_gradient_sums(const rbmg_psi* psi, const rbmg_operator* op, rbmg_e
                 G.T = L.T;
                 G.en = L.en;
                 G.U = W.U.as<float2>();
-                G.e_shift = make_float2(static_cast<float>(E0.real()), static_cast<float>(E0.imag()));
+                G.e_shift = e0_dev;
                 G.site_ptr = op->d_site_ptr.as<int>();
-                RBMG_CK(launch_grad_vectors(G, od, W.acc_Ek.as<double2>(), W.vpart.as<double2>(), kSplits, stream()));
+                RBMG_CK(launch_grad_vectors(G, od, W.vpart.as<double2>(), kSplits, stream(), &jobs[1]));
             }
             double2* part = W.partial.as<double2>();
             // the sums over T, together: O, and (E - E0) O* or, for the adjoint, C2 and C3
             OuterSet sums_t{}, sums_u{};
             sums_t.add(W.coef1.as<double2>(), 0, W.acc_O.as<double2>());
             if (adjoint) {
-                RBMG_CK(W.coef3.ensure(sizeof(double2) * c.count));
-                RBMG_CK(launch_coef_real(c.count, c.weights, W.eloc.as<double2>(), E0.real(), W.coef3.as<double2>(),
-                                         stream()));
                 sums_t.add(W.coef2.as<double2>(), 0, W.acc_C2.as<double2>());
                 sums_t.add(W.coef3.as<double2>(), 1, W.acc_C3.as<double2>());
             } else {
                 sums_t.add(W.coef2.as<double2>(), 1, W.acc_EO.as<double2>());
             }
             RBMG_CK(launch_outer_reduce(c.count, N, nw, psi->M, c.spins, c.enum_base, c.enumerate, sums_t,
-                                        W.T.as<float2>(), psi->Mpad, part, kSplits, stream()));
+                                        W.T.as<float2>(), psi->Mpad, part, kSplits, stream(), &jobs[0]));
             sums_u.add(W.coef1.as<double2>(), 0, W.acc_Ek.as<double2>());
-            if (fluct) {
-                RBMG_CK(W.coef3.ensure(sizeof(double2) * c.count));
-                RBMG_CK(launch_coef_conj(c.count, c.weights, W.eloc.as<double2>(), make_double2(E0.real(), E0.imag()),
-                                         W.coef3.as<double2>(), stream()));
-                sums_u.add(W.coef3.as<double2>(), 0, W.acc_B.as<double2>());
-            }
+            if (fluct) sums_u.add(W.coef3.as<double2>(), 0, W.acc_B.as<double2>());
             RBMG_CK(launch_outer_reduce(c.count, N, nw, psi->M, c.spins, c.enum_base, c.enumerate, sums_u,
-                                        W.U.as<float2>(), psi->Mpad, part, kSplits, stream()));
+                                        W.U.as<float2>(), psi->Mpad,
+                                        part + static_cast<size_t>(sums_t.n) * kSplits * (1 + N) * psi->M, kSplits,
+                                        stream(), &jobs[1]));
+            RBMG_CK(launch_split_sums(jobs, 2, !first, stream()));
+            first = false;
             if (!single)
                 RBMG_CK(launch_vterm_reduce(c.count, N, nw, psi->M, psi->Mpad, c.spins, c.enum_base, c.enumerate,
                                             c.weights, W.X.as<float2>(), op->num_offdiag, op->d_site_ptr.as<int>(),
@@ -1380,42 +1357,56 @@ static int ev_gradient_sums(const rbmg_psi* psi, const rbmg_operator* op, rbmg_e
         return RBMG_OK;
     });
     if (r != RBMG_OK) return r;
-    *E0_out = E0;
-    *norm_out = res.norm_factor;
+    if (!have_shift) {   // an ensemble without samples
+        RBMG_CK(cudaMemsetAsync(e0_dev, 0, sizeof(double2), stream()));
+        return zero_accs();
+    }
+    return RBMG_OK;
+}
+
+// the gradient (GradOut::mode) of ev_gradient_sums's sums into d_grad [P] or, if that is null,
+// to the host's grad, and the energy: one wait for the whole pass
+static int ev_gradient_take(const rbmg_psi* psi, rbmg_ensemble* ens, const StreamResult& res, int mode,
+                            double2* d_grad, double* grad, double* value) {
+    const int N = psi->N;
+    Workspace& W = ws();
+    const size_t P = static_cast<size_t>(psi->num_params());
+    RBMG_CK(W.status.ensure(sizeof(double) * 4));
+    if (!d_grad) RBMG_CK(W.gout.ensure(sizeof(double2) * P));
+    GradOut G{};
+    G.mode = mode;
+    G.O = W.acc_O.as<double2>();
+    G.A = mode == 0 ? W.acc_EO.as<double2>() : W.acc_Ek.as<double2>();
+    G.B = mode == 0 ? W.acc_Ek.as<double2>() : W.acc_C2.as<double2>();
+    G.C = mode == 2 ? W.acc_C3.as<double2>() : nullptr;
+    G.sums = W.sums.as<double2>();
+    G.e0 = W.stat.as<double2>() + 2;
+    G.stat = ens->kind == 1 ? W.stat.as<double2>() : nullptr;
+    G.norm = ens->kind == 1 ? 2.0 * std::log(psi->prefactor) : res.norm_factor;
+    G.first = 2 * N;
+    G.count = static_cast<long>(P) - 2 * N;
+    G.grad = d_grad ? d_grad : W.gout.as<double2>();
+    G.status = W.status.as<double>();
+    RBMG_CK(launch_grad_out(G, stream()));
+    if (!d_grad) {
+        prefault(grad, sizeof(double2) * P);
+        RBMG_CK(cudaMemcpyAsync(grad, G.grad, sizeof(double2) * P, cudaMemcpyDeviceToHost, stream()));
+    }
+    RBMG_CK(cudaStreamSynchronize(stream()));
+    if (ens->kind == 0) ens->counts_take();
+    if (ens->kind == 1 && !std::isfinite(G.status[3])) return fail(RBMG_ENAN, kNonFiniteLogPsi);
+    value[0] = G.status[0];
+    value[1] = G.status[1];
     return RBMG_OK;
 }
 
 extern "C" int rbmg_ev_gradient(const rbmg_psi* psi, const rbmg_operator* op, rbmg_ensemble* ens, double* grad,
                                 double* value) {
     if (!op || !grad || !value) return fail(RBMG_EINVAL, "gradient: null");
-    cplx E0;
-    double f = 0.0;
-    int r = ev_gradient_sums(psi, op, ens, &E0, &f);
-    if (r != RBMG_OK) return r;
-    const int N = psi->N;
-    const size_t ok_len = static_cast<size_t>(psi->num_params() - 2 * N);
-    Workspace& W = ws();
-    std::vector<double2> O(ok_len), EO(ok_len), Ek(ok_len);
-    double2 Es;
-    RBMG_CK(cudaMemcpyAsync(O.data(), W.acc_O.p, sizeof(double2) * ok_len, cudaMemcpyDeviceToHost, stream()));
-    RBMG_CK(cudaMemcpyAsync(EO.data(), W.acc_EO.p, sizeof(double2) * ok_len, cudaMemcpyDeviceToHost, stream()));
-    RBMG_CK(cudaMemcpyAsync(Ek.data(), W.acc_Ek.p, sizeof(double2) * ok_len, cudaMemcpyDeviceToHost, stream()));
-    RBMG_CK(cudaMemcpyAsync(&Es, W.sums.p, sizeof(double2), cudaMemcpyDeviceToHost, stream()));
-    RBMG_CK(cudaStreamSynchronize(stream()));
-    // ExpectationValue.cu:243-253: grad = <E O*> + conj<E_k> - 2 <E> <O*>.  With the centred
-    // sums <E O*> = EO' + E0 conj<O> and <E_k> = Ek' + E0 <O>, so
-    // grad = EO' + conj(Ek') + (E0 + conj(E0) - 2 <E>) conj<O>.
-    const cplx E = cplx(Es.x, Es.y) * f;
-    const cplx shift_sum = E0 + std::conj(E0) - 2.0 * E;
-    cplx* g = reinterpret_cast<cplx*>(grad);
-    for (int k = 0; k < 2 * N; k++) g[k] = 0.0;
-    for (size_t k = 0; k < ok_len; k++) {
-        const cplx o = cplx(O[k].x, O[k].y) * f, eo = cplx(EO[k].x, EO[k].y) * f, ek = cplx(Ek[k].x, Ek[k].y) * f;
-        g[2 * N + k] = eo + std::conj(ek) + shift_sum * std::conj(o);
-    }
-    value[0] = E.real();
-    value[1] = E.imag();
-    return RBMG_OK;
+    StreamResult res;
+    res.defer = true;
+    const int r = ev_gradient_sums(psi, op, ens, &res);
+    return r != RBMG_OK ? r : ev_gradient_take(psi, ens, res, 0, nullptr, grad, value);
 }
 
 // ExpectationValue::fluctuation_gradient (ExpectationValue.cu:258-348): the gradient of
@@ -1428,21 +1419,23 @@ extern "C" int rbmg_ev_gradient(const rbmg_psi* psi, const rbmg_operator* op, rb
 extern "C" int rbmg_ev_fluctuation_gradient(const rbmg_psi* psi, const rbmg_operator* op, rbmg_ensemble* ens,
                                             double* grad, double* sigma) {
     if (!op || !grad) return fail(RBMG_EINVAL, "fluctuation_gradient: null");
-    cplx E0;
-    double f = 0.0;
-    int r = ev_gradient_sums(psi, op, ens, &E0, &f, true);
+    StreamResult res;
+    int r = ev_gradient_sums(psi, op, ens, &res, true);
     if (r != RBMG_OK) return r;
+    const double f = res.norm_factor;
     const int N = psi->N;
     const size_t ok_len = static_cast<size_t>(psi->num_params() - 2 * N);
     Workspace& W = ws();
     std::vector<double2> O(ok_len), EO(ok_len), Ek(ok_len), B(ok_len);
-    double2 Es[2];
+    double2 Es[2], e0;
     RBMG_CK(cudaMemcpyAsync(O.data(), W.acc_O.p, sizeof(double2) * ok_len, cudaMemcpyDeviceToHost, stream()));
     RBMG_CK(cudaMemcpyAsync(EO.data(), W.acc_EO.p, sizeof(double2) * ok_len, cudaMemcpyDeviceToHost, stream()));
     RBMG_CK(cudaMemcpyAsync(Ek.data(), W.acc_Ek.p, sizeof(double2) * ok_len, cudaMemcpyDeviceToHost, stream()));
     RBMG_CK(cudaMemcpyAsync(B.data(), W.acc_B.p, sizeof(double2) * ok_len, cudaMemcpyDeviceToHost, stream()));
     RBMG_CK(cudaMemcpyAsync(Es, W.sums.p, sizeof(Es), cudaMemcpyDeviceToHost, stream()));
+    RBMG_CK(cudaMemcpyAsync(&e0, W.stat.as<double2>() + 2, sizeof(e0), cudaMemcpyDeviceToHost, stream()));
     RBMG_CK(cudaStreamSynchronize(stream()));
+    const cplx E0(e0.x, e0.y);
     const cplx E = cplx(Es[0].x, Es[0].y) * f;
     const double E2 = Es[1].x * f;
     const double var = std::max(0.0, E2 - std::norm(E));
@@ -1463,26 +1456,14 @@ extern "C" int rbmg_ev_fluctuation_gradient(const rbmg_psi* psi, const rbmg_oper
 }
 
 // The same gradient left on the device: d_grad [P] complex128 (entries below 2N zero),
-// formed by launch_grad_final from the sums above; the energy comes back to the host.
+// formed by launch_grad_out from the sums above; the energy comes back to the host.
 int rbmg::ev_gradient_device(const rbmg_psi* psi, const rbmg_operator* op, rbmg_ensemble* ens, double2* d_grad,
                        double* value) {
     if (!op || !d_grad || !value) return fail(RBMG_EINVAL, "gradient: null");
-    cplx E0;
-    double f = 0.0;
-    int r = ev_gradient_sums(psi, op, ens, &E0, &f);
-    if (r != RBMG_OK) return r;
-    Workspace& W = ws();
-    const int N = psi->N;
-    const long ok_len = psi->num_params() - 2 * N;
-    RBMG_CK(launch_grad_final(W.acc_O.as<double2>(), W.acc_EO.as<double2>(), W.acc_Ek.as<double2>(),
-                              W.sums.as<double2>(), f, make_double2(E0.real(), E0.imag()), 2 * N, ok_len, d_grad,
-                              stream()));
-    double2 Es;
-    RBMG_CK(cudaMemcpyAsync(&Es, W.sums.p, sizeof(double2), cudaMemcpyDeviceToHost, stream()));
-    RBMG_CK(cudaStreamSynchronize(stream()));
-    value[0] = Es.x * f;
-    value[1] = Es.y * f;
-    return RBMG_OK;
+    StreamResult res;
+    res.defer = true;
+    const int r = ev_gradient_sums(psi, op, ens, &res);
+    return r != RBMG_OK ? r : ev_gradient_take(psi, ens, res, 0, d_grad, nullptr, value);
 }
 
 // Extension: the hidden angles theta = b + s W of given configurations (spins
@@ -1564,37 +1545,10 @@ int deep_adjoint_chunk(const rbmg_psi* psi, const rbmg_operator* op, const Chunk
 // 2 <(Re E - <Re E>) O_k*> = 2 (C3 - (<Re E> - Re E0) <O_k>*).
 static int rbm_eloc_gradient(const rbmg_psi* psi, const rbmg_operator* op, rbmg_ensemble* ens, int score,
                              double* grad, double* value) {
-    cplx E0;
-    double f = 0.0;
-    int r = ev_gradient_sums(psi, op, ens, &E0, &f, false, true);
-    if (r != RBMG_OK) return r;
-    const int N = psi->N;
-    const size_t ok_len = static_cast<size_t>(psi->num_params() - 2 * N);
-    Workspace& W = ws();
-    std::vector<double2> O(ok_len), C1(ok_len), C2(ok_len), C3(ok_len);
-    double2 Es;
-    RBMG_CK(cudaMemcpyAsync(O.data(), W.acc_O.p, sizeof(double2) * ok_len, cudaMemcpyDeviceToHost, stream()));
-    RBMG_CK(cudaMemcpyAsync(C1.data(), W.acc_Ek.p, sizeof(double2) * ok_len, cudaMemcpyDeviceToHost, stream()));
-    RBMG_CK(cudaMemcpyAsync(C2.data(), W.acc_C2.p, sizeof(double2) * ok_len, cudaMemcpyDeviceToHost, stream()));
-    RBMG_CK(cudaMemcpyAsync(C3.data(), W.acc_C3.p, sizeof(double2) * ok_len, cudaMemcpyDeviceToHost, stream()));
-    RBMG_CK(cudaMemcpyAsync(&Es, W.sums.p, sizeof(double2), cudaMemcpyDeviceToHost, stream()));
-    RBMG_CK(cudaStreamSynchronize(stream()));
-    const cplx E = cplx(Es.x, Es.y) * f;
-    const double dre = E.real() - E0.real();
-    cplx* g = reinterpret_cast<cplx*>(grad);
-    for (int k = 0; k < 2 * N; k++) g[k] = 0.0;
-    for (size_t k = 0; k < ok_len; k++) {
-        const cplx c1 = cplx(C1[k].x, C1[k].y) * f, c2 = cplx(C2[k].x, C2[k].y) * f;
-        cplx v = std::conj(c1 - c2);
-        if (score) {
-            const cplx o = cplx(O[k].x, O[k].y) * f, c3 = cplx(C3[k].x, C3[k].y) * f;
-            v += 2.0 * (c3 - dre * std::conj(o));
-        }
-        g[2 * N + k] = v;
-    }
-    value[0] = E.real();
-    value[1] = E.imag();
-    return RBMG_OK;
+    StreamResult res;
+    res.defer = true;
+    const int r = ev_gradient_sums(psi, op, ens, &res, false, true);
+    return r != RBMG_OK ? r : ev_gradient_take(psi, ens, res, score ? 2 : 1, nullptr, grad, value);
 }
 
 extern "C" int rbmg_ev_eloc_gradient(const rbmg_psi* psi, const rbmg_operator* op, rbmg_ensemble* ens, int score,
@@ -1625,7 +1579,7 @@ extern "C" int rbmg_ev_eloc_gradient(const rbmg_psi* psi, const rbmg_operator* o
     RBMG_CK(cudaMemsetAsync(W.acc_O.p, 0, sizeof(double2) * tot, stream()));
     RBMG_CK(cudaMemsetAsync(W.acc_EO.p, 0, sizeof(double2) * tot, stream()));
     RBMG_CK(W.sums.ensure(sizeof(double2) * kMaxSeries));
-    RBMG_CK(W.block_scratch.ensure(sizeof(double2) * kSumBlocks * kMaxSeries));
+    RBMG_CK(sum_scratch(W));
     RBMG_CK(cudaMemsetAsync(W.sums.p, 0, sizeof(double2) * kMaxSeries, stream()));
     StreamResult res;
     r = run_stream(ens, psi, op, false, 4096, &res, [&](const Chunk& c) -> int {
@@ -1760,7 +1714,7 @@ extern "C" int rbmg_hsd_gradient(const rbmg_psi* psi, const rbmg_psi* pp, const 
         RBMG_CK(W.coef3.ensure(sizeof(double) * total));      // weights of all samples
         RBMG_CK(W.Tp.ensure(sizeof(uint64_t) * nw * total));   // spins of all samples
         RBMG_CK(W.sums.ensure(sizeof(double2) * kMaxSeries));
-        RBMG_CK(W.block_scratch.ensure(sizeof(double2) * kSumBlocks * kMaxSeries));
+        RBMG_CK(sum_scratch(W));
         RBMG_CK(cudaMemsetAsync(W.sums.p, 0, sizeof(double2) * kMaxSeries, stream()));
         uint64_t* all_spins = W.Tp.as<uint64_t>();
         double* all_w = W.coef3.as<double>();
@@ -1918,7 +1872,7 @@ extern "C" int rbmg_kl_gradient(const rbmg_psi* psi, const rbmg_psi* pp, rbmg_en
     RBMG_CK(W.coef3.ensure(sizeof(double) * total));       // weights of every sample
     RBMG_CK(W.Tp.ensure(sizeof(uint64_t) * nw * total));  // spins of every sample
     RBMG_CK(W.sums.ensure(sizeof(double2) * kMaxSeries));
-    RBMG_CK(W.block_scratch.ensure(sizeof(double2) * kSumBlocks * kMaxSeries));
+    RBMG_CK(sum_scratch(W));
     RBMG_CK(cudaMemsetAsync(W.sums.p, 0, sizeof(double2) * kMaxSeries, stream()));
     double2* D = W.omega.as<double2>();
     uint64_t* all_spins = W.Tp.as<uint64_t>();
@@ -2058,7 +2012,7 @@ extern "C" int rbmg_hsd_distance_2nd_order(const rbmg_psi* psi, const rbmg_psi* 
     }
     Workspace& W = ws();
     RBMG_CK(W.sums.ensure(sizeof(double2) * kMaxSeries));
-    RBMG_CK(W.block_scratch.ensure(sizeof(double2) * kSumBlocks * kMaxSeries));
+    RBMG_CK(sum_scratch(W));
     RBMG_CK(cudaMemsetAsync(W.sums.p, 0, sizeof(double2) * kMaxSeries, stream()));
     const OpDev od = op->dev(), od2 = op2->dev();
     StreamResult res;

@@ -2259,7 +2259,7 @@ int deep_adjoint_chunk(const rbmg_psi* psi, const rbmg_operator* op, const Chunk
 
 // MonteCarloLoop::foreach for PsiDeep / PsiPair (MonteCarloLoop.hpp:294-339)
 int deep_stream(rbmg_ensemble* e, const rbmg_psi* psi, const rbmg_operator* op, bool want_eloc,
-                size_t max_chunk_samples, const std::function<int(const Chunk&)>& fn) {
+                size_t max_chunk_samples, bool defer, const std::function<int(const Chunk&)>& fn) {
     (void)op;
     (void)want_eloc;
     if (e->total_z) return fail(RBMG_EUNSUPPORTED, "PsiDeep chains: S_z symmetry is not provided");
@@ -2319,12 +2319,10 @@ int deep_stream(rbmg_ensemble* e, const rbmg_psi* psi, const rbmg_operator* op, 
         const int r = fn(c);
         if (r != RBMG_OK) return r;
     }
-    std::vector<unsigned long long> a(B), p(B);
-    RBMG_CK(cudaMemcpyAsync(a.data(), e->accepts.p, sizeof(unsigned long long) * B, cudaMemcpyDeviceToHost, stream()));
-    RBMG_CK(cudaMemcpyAsync(p.data(), e->proposals.p, sizeof(unsigned long long) * B, cudaMemcpyDeviceToHost, stream()));
+    RBMG_CK(e->counts_copy());
+    if (defer) return RBMG_OK;
     RBMG_CK(cudaStreamSynchronize(stream()));
-    e->last_accepts.assign(a.begin(), a.end());
-    e->last_proposals.assign(p.begin(), p.end());
+    e->counts_take();
     return RBMG_OK;
 }
 

@@ -59,6 +59,31 @@ struct DevBuf {
     T* as() const { return static_cast<T*>(p); }
 };
 
+// grow-only pinned host buffer, addressable by the device
+struct HostBuf {
+    void* p = nullptr;
+    size_t bytes = 0;
+    HostBuf() = default;
+    HostBuf(const HostBuf&) = delete;
+    HostBuf& operator=(const HostBuf&) = delete;
+    ~HostBuf() { release(); }
+    void release() {
+        if (p) cudaFreeHost(p);
+        p = nullptr;
+        bytes = 0;
+    }
+    cudaError_t ensure(size_t n) {
+        if (n <= bytes) return cudaSuccess;
+        release();
+        cudaError_t e = cudaMallocHost(&p, n);
+        if (e != cudaSuccess) { p = nullptr; return e; }
+        bytes = n;
+        return cudaSuccess;
+    }
+    template <typename T>
+    T* as() const { return static_cast<T*>(p); }
+};
+
 // Makes the pages of a host output present before the GPU writes them: the copy to pageable
 // memory is a direct write of the GPU, which takes the first-touch fault of every page of a
 // freshly allocated array one by one (measured: 300 KB into fresh pages 226 us, into touched
@@ -188,8 +213,6 @@ cudaError_t launch_sub(int count, const double2* a, const double2* b, double2* o
 // density.cu: out [2^na] += w_s |eloc_s|^2 at the bin of the first na spins
 cudaError_t launch_diag_density(int count, int enumerate, uint64_t enum_base, const uint64_t* spins, int nw,
                                 const double* w, const double2* eloc, int na, double* out, cudaStream_t st);
-cudaError_t launch_grad_final(const double2* O, const double2* EO, const double2* Ek, const double2* sums,
-                              double norm, double2 E0, int first, long count, double2* grad, cudaStream_t st);
 }  // namespace rbmg
 
 struct rbmg_operator {
@@ -239,6 +262,7 @@ struct rbmg_ensemble {
     rbmg::DevBuf spins, rng_index, accepts, proposals;
     int spins_words = 0;
     std::vector<uint64_t> last_accepts, last_proposals;
+    rbmg::HostBuf counts;   // the accept and proposal counts of a pass, on their way to the two above
     // ExactSummation
     uint32_t num_spins = 0;
     int exact_total_z = 0;
@@ -247,6 +271,21 @@ struct rbmg_ensemble {
     uint64_t fixed_count = 0;               // fixed sample set: number of configurations
 
     uint64_t num_steps() const;
+
+    // a Monte-Carlo pass's counts: the copies enqueued; taken once the stream has been waited for
+    cudaError_t counts_copy() {
+        const size_t n = sizeof(unsigned long long) * num_chains;
+        cudaError_t e = counts.ensure(2 * n);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(counts.p, accepts.p, n, cudaMemcpyDeviceToHost, rbmg::stream());
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(counts.as<char>() + n, proposals.p, n, cudaMemcpyDeviceToHost, rbmg::stream());
+        return e;
+    }
+    void counts_take() {
+        const unsigned long long* c = counts.as<unsigned long long>();
+        last_accepts.assign(c, c + num_chains);
+        last_proposals.assign(c + num_chains, c + 2 * static_cast<size_t>(num_chains));
+    }
 };
 
 // walkers that persist on the device between calls (capi.cu); the learned-proposal

@@ -98,7 +98,7 @@ struct EstLaunch {
     float2* X;                  // [count][num_offdiag][Mpad]
     double2* logpsi_prime;      // [count]
     float2* Tp;                 // [count][Mpad'] tanh of psi' angles
-    double2 e_shift;            // U is stored as U - e_shift * T (centred E_k sums)
+    const double2* e_shift;     // U is stored as U - *e_shift T (centred E_k sums; EST_GRADVEC)
     // EST_GRADVEC of a single-flip operator: the angles and the off-diagonal strings' terms in
     // place of U and X, which launch_grad_vectors forms (null: the general form above)
     float2* theta;              // [count][Mpad]

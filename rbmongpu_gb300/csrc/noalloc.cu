@@ -31,8 +31,8 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 constexpr size_t kOffLogPsi = 0;                                            // double2 [states]
 constexpr size_t kOffWeights = kOffLogPsi + kNoAllocStates * sizeof(double2);   // double  [states]
 constexpr size_t kOffEloc = kOffWeights + kNoAllocStates * sizeof(double);      // double2 [states]
-constexpr size_t kOffBlocks = kOffEloc + kNoAllocStates * sizeof(double2);      // double2 [kSumBlocks * kMaxSeries]
-constexpr size_t kOffBlockMax = kOffBlocks + kSumBlocks * kMaxSeries * sizeof(double2);   // double [kSumBlocks]
+constexpr size_t kOffBlocks = kOffEloc + kNoAllocStates * sizeof(double2);      // double2 [kSumScratch], the counter zero
+constexpr size_t kOffBlockMax = kOffBlocks + kSumScratch * sizeof(double2);   // double [kSumBlocks]
 constexpr size_t kOffSums = kOffBlockMax + kSumBlocks * sizeof(double);         // double2 [kMaxSeries]
 static_assert(kOffSums + kMaxSeries * sizeof(double2) <= kNoAllocBytes, "no-alloc scratch too small");
 

@@ -114,26 +114,6 @@ __global__ void lookahead_kernel(long n, const double* p, const double* v, doubl
     if (i < n) out[i] = __dsub_rn(p[i], __dmul_rn(gamma, v[i]));
 }
 
-// ExpectationValue.cu:243-253: grad = <E O*> + conj<E_k> - 2 <E> <O*>, from the centred
-// sums EO' = sum w (E - E0) O*, Ek' = sum w (E_k - E0 O):
-// grad = EO' + conj(Ek') + (E0 + conj(E0) - 2 <E>) conj<O>   (all sums times norm)
-__global__ void grad_final_kernel(const double2* O, const double2* EO, const double2* Ek, const double2* sums,
-                                  double norm, double2 E0, int first, long count, double2* grad) {
-    const long k = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (k < first) grad[k] = make_double2(0.0, 0.0);
-    if (k >= count) return;
-    const double Er = __dmul_rn(sums[0].x, norm), Ei = __dmul_rn(sums[0].y, norm);
-    const double sr = __dsub_rn(__dadd_rn(E0.x, E0.x), __dmul_rn(2.0, Er));
-    const double si = __dsub_rn(__dsub_rn(E0.y, E0.y), __dmul_rn(2.0, Ei));
-    const double orr = __dmul_rn(O[k].x, norm), oi = __dmul_rn(O[k].y, norm);
-    const double eor = __dmul_rn(EO[k].x, norm), eoi = __dmul_rn(EO[k].y, norm);
-    const double ekr = __dmul_rn(Ek[k].x, norm), eki = __dmul_rn(Ek[k].y, norm);
-    // shift * conj(o) = (sr + i si)(orr - i oi)
-    const double tr = __dadd_rn(__dmul_rn(sr, orr), __dmul_rn(si, oi));
-    const double ti = __dsub_rn(__dmul_rn(si, orr), __dmul_rn(sr, oi));
-    grad[first + k] = make_double2(__dadd_rn(__dadd_rn(eor, ekr), tr), __dadd_rn(__dsub_rn(eoi, eki), ti));
-}
-
 // RBM parameters the kernels read: b [Mpad], W [N][Mpad] complex64 (zero padding untouched)
 __global__ void rbm_scatter_kernel(const double2* packed, int N, int M, int Mpad, float2* b, float2* W) {
     const long q = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -197,13 +177,6 @@ void pack_host(const rbmg_psi* psi, std::vector<cplx>& out) {
 }
 
 }  // namespace
-
-cudaError_t launch_grad_final(const double2* O, const double2* EO, const double2* Ek, const double2* sums,
-                              double norm, double2 E0, int first, long count, double2* grad, cudaStream_t st) {
-    const long n = std::max<long>(count, first);
-    grad_final_kernel<<<blocks_of(n, 256), 256, 0, st>>>(O, EO, Ek, sums, norm, E0, first, count, grad);
-    return cudaGetLastError();
-}
 
 int psi_sync_host(const rbmg_psi* cpsi) {
     if (!cpsi->host_stale) return RBMG_OK;

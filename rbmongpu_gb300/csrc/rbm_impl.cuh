@@ -773,7 +773,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) rbm_est_kernel(RbmDev P, 
             for (int k = 0; k < K; k++) L.T[t * P.Mpad + lane + 32 * k] = T[k];
             const double2 e = rbm_local_energy<true>(P, op, s, tr, ti, f, T, U,
                                                      L.X + t * op.num_offdiag * P.Mpad, lane);
-            const float shx = static_cast<float>(L.e_shift.x), shy = static_cast<float>(L.e_shift.y);
+            const float shx = static_cast<float>(L.e_shift->x), shy = static_cast<float>(L.e_shift->y);
 #pragma unroll
             for (int k = 0; k < K; k++) {
                 U[k].x -= shx * T[k].x - shy * T[k].y;

@@ -113,37 +113,50 @@ __global__ void __launch_bounds__(32 * kOmMaxTy) outer_reduce_kernel(
         }
 }
 
-// set.out[q][e] += scale * sum_z partial[z][q][e]: a block takes 32 entries, eight slices of
-// the splits, each in z order with its loads in flight together, then the slices in order
-// (one thread an entry walked the 64 splits of 8320 sums in 12.5 us; now 25000 take 10)
-__global__ void __launch_bounds__(256) finish_splits_kernel(long elems, int splits, int nc,
-                                                            const double2* __restrict__ partial, OuterSet set,
-                                                            double scale) {
-    __shared__ double2 red[8][32];
+// SplitSum, blockIdx.y the job: a block takes 32 entries, eight slices of the splits, each in z
+// order with its loads in flight together, then the slices in order (one thread an entry walked
+// the 64 splits of 8320 sums in 12.5 us; now 25000 take 10).  The sums of one pass go together:
+// three launches of 4 us each were a sixth of the GPU's work for 4096 states of 12 spins.
+struct SplitSums {
+    SplitSum job[2];
+};
+__global__ void __launch_bounds__(256) finish_splits_kernel(SplitSums jobs, int add) {
+    __shared__ double2 red[2][8][32];
+    const SplitSum& J = jobs.job[blockIdx.y];
     const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
-    const long total = elems * nc;
+    const long total = J.elems * J.nc;
+    auto slice_sum = [&](const double2* partial, int splits, long stride, long e) {
+        double2 a = make_double2(0.0, 0.0);
+        const int per = (splits + 7) / 8, z1 = min(splits, (slice + 1) * per);
+#pragma unroll 8
+        for (int z = slice * per; z < z1; z++) {
+            const double2 p = partial[z * stride + e];
+            a.x += p.x;
+            a.y += p.y;
+        }
+        return a;
+    };
     for (long e0 = blockIdx.x * 32L; e0 < total; e0 += gridDim.x * 32L) {
         const long e = e0 + lane;
-        double2 a = make_double2(0.0, 0.0);
-        if (e < total) {
-            const int per = (splits + 7) / 8, z1 = min(splits, (slice + 1) * per);
-#pragma unroll 8
-            for (int z = slice * per; z < z1; z++) {
-                const double2 p = partial[z * total + e];
-                a.x += p.x;
-                a.y += p.y;
-            }
-        }
-        red[slice][lane] = a;
+        const bool pre = J.pre && e < J.elems;
+        if (e < total) red[0][slice][lane] = slice_sum(J.partial, J.splits, total, e);
+        if (pre) red[1][slice][lane] = slice_sum(J.pre, J.pre_splits, J.elems, e);
         __syncthreads();
         if (slice == 0 && e < total) {
-            for (int q = 1; q < 8; q++) {
-                a.x += red[q][lane].x;
-                a.y += red[q][lane].y;
-            }
-            double2* out = set.out[e / elems] + e % elems;
-            out->x += scale * a.x;
-            out->y += scale * a.y;
+            double2* out = J.out[e / J.elems] + e % J.elems;
+            double2 o = add ? *out : make_double2(0.0, 0.0);
+            auto slices = [&](int k, double scale) {
+                double2 a = red[k][0][lane];
+                for (int q = 1; q < 8; q++) {
+                    a.x += red[k][q][lane].x;
+                    a.y += red[k][q][lane].y;
+                }
+                o.x += scale * a.x;
+                o.y += scale * a.y;
+            };
+            if (pre) slices(1, -2.0);
+            slices(0, J.scale);
+            *out = o;
         }
         __syncthreads();
     }
@@ -377,7 +390,7 @@ __global__ void __launch_bounds__(32 * kGvWarps) grad_vectors_kernel(GradVectors
         }
         n0 += nb;
     }
-    const float shx = g.e_shift.x, shy = g.e_shift.y;
+    const float shx = static_cast<float>(g.e_shift->x), shy = static_cast<float>(g.e_shift->y);
     for (int k = 0; k < cnt; k++) {
         const float2 t = load(g.T, k);
         float x[2], y[2];
@@ -391,43 +404,147 @@ __global__ void __launch_bounds__(32 * kGvWarps) grad_vectors_kernel(GradVectors
 }
 
 // ---- weighted sums of complex series -------------------------------------
-__global__ void wsum_blocks_kernel(int count, const double* __restrict__ w, SeriesSet set,
-                                   double2* __restrict__ block_out) {
-    __shared__ double2 red[kMaxSeries][256 / 32];
+// The block's sums of n series go to block_out; the block that arrives last adds up all blocks'
+// in a fixed order (warp q series q: lane l blocks l, l + 32, ..., then a butterfly) into total,
+// and returns true.  A second launch of one thread per series walked 512 blocks in 26 us.
+constexpr int kSumThreads = 256;
+static_assert(kSumThreads / 32 >= kMaxSeries, "a warp per series");
+__device__ bool block_totals(double2 (&acc)[kMaxSeries], int n, double2* block_out, double2 (&total)[kMaxSeries]) {
+    __shared__ double2 red[kMaxSeries][kSumThreads / 32];
+    __shared__ bool last;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    double2 acc[kMaxSeries];
-    for (int q = 0; q < kMaxSeries; q++) acc[q] = make_double2(0.0, 0.0);
-    for (long s = blockIdx.x * 256L + tid; s < count; s += static_cast<long>(gridDim.x) * 256) {
-        const double ws = w ? w[s] : 1.0;
-        for (int q = 0; q < set.n; q++) {
-            const double2 v = set.v[q][s];
-            acc[q].x += ws * v.x;
-            acc[q].y += ws * v.y;
-        }
-    }
-    for (int q = 0; q < set.n; q++) {
-        double x = acc[q].x, y = acc[q].y;
+    auto warp_sum = [](double2 v) {
         for (int off = 16; off >= 1; off >>= 1) {
-            x += __shfl_down_sync(0xffffffffu, x, off);
-            y += __shfl_down_sync(0xffffffffu, y, off);
+            v.x += __shfl_down_sync(0xffffffffu, v.x, off);
+            v.y += __shfl_down_sync(0xffffffffu, v.y, off);
         }
-        if (lane == 0) red[q][warp] = make_double2(x, y);
+        return v;
+    };
+#pragma unroll
+    for (int q = 0; q < kMaxSeries; q++)
+        if (q < n) {
+            const double2 t = warp_sum(acc[q]);
+            if (lane == 0) red[q][warp] = t;
+        }
+    __syncthreads();
+    if (tid < n) {
+        double2 t = make_double2(0.0, 0.0);
+        for (int q = 0; q < kSumThreads / 32; q++) { t.x += red[tid][q].x; t.y += red[tid][q].y; }
+        block_out[blockIdx.x * kMaxSeries + tid] = t;
+        __threadfence();
     }
     __syncthreads();
-    if (tid < set.n) {
+    if (tid == 0) {
+        unsigned int* ticket = reinterpret_cast<unsigned int*>(block_out + kSumBlocks * kMaxSeries);
+        last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;   // back to zero after the last block
+    }
+    __syncthreads();
+    if (!last) return false;
+    __threadfence();
+    if (warp < n) {
         double2 t = make_double2(0.0, 0.0);
-        for (int q = 0; q < 256 / 32; q++) { t.x += red[tid][q].x; t.y += red[tid][q].y; }
-        block_out[blockIdx.x * kMaxSeries + tid] = t;
+        for (int b = lane; b < gridDim.x; b += 32) {
+            const double2 v = __ldcg(block_out + b * kMaxSeries + warp);
+            t.x += v.x;
+            t.y += v.y;
+        }
+        t = warp_sum(t);
+        if (lane == 0) red[warp][0] = t;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kMaxSeries; q++) total[q] = q < n ? red[q][0] : make_double2(0.0, 0.0);
+    return true;
+}
+
+// MEAN: the mean of set.v[0] (sums of w v and w); otherwise sums[q] += the sums of w v_q
+template <bool MEAN>
+__global__ void __launch_bounds__(kSumThreads) wsum_kernel(int count, const double* __restrict__ w, SeriesSet set,
+                                                           double2* block_out, double2* sums) {
+    double2 acc[kMaxSeries], total[kMaxSeries];
+#pragma unroll
+    for (int q = 0; q < kMaxSeries; q++) acc[q] = make_double2(0.0, 0.0);
+    for (long s = blockIdx.x * long(kSumThreads) + threadIdx.x; s < count; s += static_cast<long>(gridDim.x) * kSumThreads) {
+        const double ws = w ? w[s] : 1.0;
+#pragma unroll
+        for (int q = 0; q < kMaxSeries; q++)
+            if (q < (MEAN ? 1 : set.n)) {
+                const double2 v = set.v[q][s];
+                acc[q].x += ws * v.x;
+                acc[q].y += ws * v.y;
+            }
+        if (MEAN) acc[1].x += ws;
+    }
+    if (!block_totals(acc, MEAN ? 2 : set.n, block_out, total)) return;
+    if (MEAN) {
+        const double wt = total[1].x;
+        if (threadIdx.x == 0)
+            sums[0] = wt > 0.0 ? make_double2(total[0].x / wt, total[0].y / wt) : make_double2(0.0, 0.0);
+    } else {
+#pragma unroll
+        for (int q = 0; q < kMaxSeries; q++)
+            if (threadIdx.x == q && q < set.n) {
+                sums[q].x += total[q].x;
+                sums[q].y += total[q].y;
+            }
     }
 }
 
-__global__ void wsum_finish_kernel(int blocks, int n, const double2* __restrict__ block_out, double2* sums) {
-    const int q = threadIdx.x;
-    if (q >= n) return;
-    double2 t = make_double2(0.0, 0.0);
-    for (int b = 0; b < blocks; b++) { t.x += block_out[b * kMaxSeries + q].x; t.y += block_out[b * kMaxSeries + q].y; }
-    sums[q].x += t.x;
-    sums[q].y += t.y;
+// ---- weights of exact summation: the largest 2 Re log psi, the sum over exp(2 Re log psi - m),
+// the weights; on the device from end to end (a maximum and a sum taken through the host put two
+// waits of 25 us each before the first weight)
+__global__ void __launch_bounds__(kSumThreads) exact_max_kernel(int count, const double2* __restrict__ lp,
+                                                                double2* block_out, double2* stat) {
+    __shared__ double red[kSumThreads];
+    __shared__ bool last;
+    auto block_max = [&](double m) {
+        red[threadIdx.x] = m;
+        __syncthreads();
+        for (int h = kSumThreads / 2; h >= 1; h >>= 1) {
+            if (threadIdx.x < h) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + h]);
+            __syncthreads();
+        }
+        return red[0];
+    };
+    double m = -INFINITY;
+    for (long s = blockIdx.x * long(kSumThreads) + threadIdx.x; s < count; s += static_cast<long>(gridDim.x) * kSumThreads)
+        m = fmax(m, 2.0 * lp[s].x);
+    m = block_max(m);
+    if (threadIdx.x == 0) {
+        block_out[blockIdx.x].x = m;
+        __threadfence();
+        unsigned int* ticket = reinterpret_cast<unsigned int*>(block_out + kSumBlocks * kMaxSeries);
+        last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    m = -INFINITY;
+    for (int b = threadIdx.x; b < gridDim.x; b += kSumThreads) m = fmax(m, __ldcg(&block_out[b].x));
+    m = block_max(m);
+    if (threadIdx.x == 0) stat[0].x = m;
+}
+
+__global__ void __launch_bounds__(kSumThreads) exact_norm_kernel(int count, const double2* __restrict__ lp,
+                                                                 double2* block_out, double2* stat) {
+    double2 acc[kMaxSeries], total[kMaxSeries];
+#pragma unroll
+    for (int q = 0; q < kMaxSeries; q++) acc[q] = make_double2(0.0, 0.0);
+    const double m = stat[0].x;
+    for (long s = blockIdx.x * long(kSumThreads) + threadIdx.x; s < count; s += static_cast<long>(gridDim.x) * kSumThreads)
+        acc[0].x += exp(2.0 * lp[s].x - m);
+    if (!block_totals(acc, 1, block_out, total)) return;
+    if (threadIdx.x == 0) {
+        stat[0].y = total[0].x;
+        stat[1].x = m + log(total[0].x);
+    }
+}
+
+__global__ void exact_weights_kernel(int count, const double2* __restrict__ lp, const double2* __restrict__ stat,
+                                     double* w) {
+    const double log_z = stat[1].x;
+    for (long s = blockIdx.x * 256L + threadIdx.x; s < count; s += static_cast<long>(gridDim.x) * 256)
+        w[s] = exp(2.0 * lp[s].x - log_z);
 }
 
 // ---- elementwise per-sample coefficients ---------------------------------
@@ -467,11 +584,59 @@ __global__ void coef_conj_kernel(int count, const double* __restrict__ w, const 
     }
 }
 
-// c[s] = (w[s] (Re v[s] - shift), 0)
-__global__ void coef_real_kernel(int count, const double* __restrict__ w, const double2* __restrict__ v, double shift,
-                                 double2* c) {
-    for (long s = blockIdx.x * 256L + threadIdx.x; s < count; s += static_cast<long>(gridDim.x) * 256)
-        c[s] = make_double2((w ? w[s] : 1.0) * (v[s].x - shift), 0.0);
+// launch_grad_coefs: one pass over the samples (two or three launches before)
+__global__ void grad_coefs_kernel(int count, const double* __restrict__ w, const double2* __restrict__ v,
+                                  const double2* __restrict__ shift, double2* c1, double2* c2, double2* c3,
+                                  int conj3) {
+    const double2 sh = *shift;
+    for (long s = blockIdx.x * 256L + threadIdx.x; s < count; s += static_cast<long>(gridDim.x) * 256) {
+        const double ws = w ? w[s] : 1.0;
+        const double x = ws * (v[s].x - sh.x), y = ws * (v[s].y - sh.y);
+        c1[s] = make_double2(ws, 0.0);
+        c2[s] = make_double2(x, y);
+        if (c3) c3[s] = make_double2(x, conj3 ? -y : 0.0);
+    }
+}
+
+// launch_grad_out.  Estimator (ExpectationValue.cu:243-253): grad = <E O*> + conj<E_k> - 2 <E> <O*>,
+// from the centred sums EO' = sum w (E - E0) O*, Ek' = sum w (E_k - E0 O):
+//   grad = EO' + conj(Ek') + (E0 + conj(E0) - 2 <E>) conj<O>   (all sums times the factor).
+// Derivative of <E_loc>: conj(C1 - C2) and, with the sampling term, + 2 (C3 - (<Re E> - Re E0) <O>*).
+// Formed here, the result is one copy; four or five copies and the host's loop were 60 to 100 us
+// of a call.
+__global__ void grad_out_kernel(GradOut g) {
+    const long k = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (k < g.first) g.grad[k] = make_double2(0.0, 0.0);
+    const double f = g.stat ? exp(g.norm + g.stat[1].x) : g.norm;
+    const double2 E0 = *g.e0;
+    const double Er = __dmul_rn(g.sums[0].x, f), Ei = __dmul_rn(g.sums[0].y, f);
+    if (k == 0) {
+        g.status[0] = Er;
+        g.status[1] = Ei;
+        g.status[2] = f;
+        g.status[3] = g.stat ? g.stat[0].x : 0.0;
+    }
+    if (k >= g.count) return;
+    auto scaled = [&](const double2* p) { return make_double2(__dmul_rn(p[k].x, f), __dmul_rn(p[k].y, f)); };
+    const double2 o = scaled(g.O), a = scaled(g.A), b = scaled(g.B);
+    double2 v;
+    if (g.mode == 0) {
+        const double sr = __dsub_rn(__dadd_rn(E0.x, E0.x), __dmul_rn(2.0, Er));
+        const double si = __dsub_rn(__dsub_rn(E0.y, E0.y), __dmul_rn(2.0, Ei));
+        // shift * conj(o) = (sr + i si)(o.x - i o.y)
+        const double tr = __dadd_rn(__dmul_rn(sr, o.x), __dmul_rn(si, o.y));
+        const double ti = __dsub_rn(__dmul_rn(si, o.x), __dmul_rn(sr, o.y));
+        v = make_double2(__dadd_rn(__dadd_rn(a.x, b.x), tr), __dadd_rn(__dsub_rn(a.y, b.y), ti));
+    } else {
+        v = make_double2(__dsub_rn(a.x, b.x), -__dsub_rn(a.y, b.y));
+        if (g.mode == 2) {
+            const double2 c = scaled(g.C);
+            const double dre = __dsub_rn(Er, E0.x);
+            v.x = __dadd_rn(v.x, __dmul_rn(2.0, __dsub_rn(c.x, __dmul_rn(dre, o.x))));
+            v.y = __dadd_rn(v.y, __dmul_rn(2.0, __dadd_rn(c.y, __dmul_rn(dre, o.y))));
+        }
+    }
+    g.grad[g.first + k] = v;
 }
 
 // rw[s] = w[s] exp(2 (Re lp[s] - Re lpp[s])) (ExpectationValue.cu:391-395), rwc[s] = (rw[s], 0)
@@ -526,16 +691,22 @@ inline int grid_for(long count) { return static_cast<int>(min(1024L, max(1L, (co
 
 }  // namespace
 
-static cudaError_t finish_splits(long elems, int splits, int nc, const double2* partial, const OuterSet& set,
-                                 double scale, cudaStream_t st) {
-    const int blocks = static_cast<int>(min(4096L, (elems * nc + 31) / 32));
-    finish_splits_kernel<<<blocks, 256, 0, st>>>(elems, splits, nc, partial, set, scale);
+cudaError_t launch_split_sums(const SplitSum* jobs, int n, bool add, cudaStream_t st) {
+    if (n < 1 || n > 2) return cudaErrorInvalidValue;
+    SplitSums set{};
+    long most = 0;
+    for (int q = 0; q < n; q++) {
+        set.job[q] = jobs[q];
+        most = max(most, jobs[q].elems * jobs[q].nc);
+    }
+    const dim3 grid(static_cast<int>(min(4096L, (most + 31) / 32)), n);
+    finish_splits_kernel<<<grid, 256, 0, st>>>(set, add ? 1 : 0);
     return cudaGetLastError();
 }
 
 cudaError_t launch_outer_reduce(int count, int N, int nw, int M, const uint64_t* spins, uint64_t enum_base,
                                 int enumerate, const OuterSet& set, const float2* A, int lda, double2* partial,
-                                int max_splits, cudaStream_t st) {
+                                int max_splits, cudaStream_t st, SplitSum* job) {
     if (count <= 0) return cudaSuccess;
     const int per_split = max(kChunk, ((count + max_splits - 1) / max_splits + kChunk - 1) / kChunk * kChunk);
     const int splits = (count + per_split - 1) / per_split;
@@ -551,7 +722,15 @@ cudaError_t launch_outer_reduce(int count, int N, int nw, int M, const uint64_t*
     else return cudaErrorInvalidValue;
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    return finish_splits(static_cast<long>(1 + N) * M, splits, set.n, partial, set, 1.0, st);
+    SplitSum own{};
+    if (!job) job = &own;
+    job->elems = static_cast<long>(1 + N) * M;
+    job->splits = splits;
+    job->nc = set.n;
+    job->partial = partial;
+    for (int q = 0; q < set.n; q++) job->out[q] = set.out[q];
+    job->scale = 1.0;
+    return job == &own ? launch_split_sums(job, 1, true, st) : cudaSuccess;
 }
 
 cudaError_t launch_vterm_reduce(int count, int N, int nw, int M, int Mpad, const uint64_t* spins, uint64_t enum_base,
@@ -564,9 +743,14 @@ cudaError_t launch_vterm_reduce(int count, int N, int nw, int M, int Mpad, const
     const dim3 grid((M + 31) / 32, N, splits);
     vterm_kernel<<<grid, 256, 0, st>>>(count, N, nw, M, Mpad, spins, enum_base, enumerate, w, cw, X, num_offdiag,
                                        site_ptr, site_slots, partial, per_split);
-    OuterSet set{};
-    set.out[0] = out;
-    return finish_splits(static_cast<long>(1 + N) * M, splits, 1, partial, set, -2.0, st);
+    SplitSum job{};
+    job.elems = static_cast<long>(1 + N) * M;
+    job.splits = splits;
+    job.nc = 1;
+    job.partial = partial;
+    job.out[0] = out;
+    job.scale = -2.0;
+    return launch_split_sums(&job, 1, true, st);
 }
 
 // vterm_kernel's split of the samples, and chunks of 32 samples a warp
@@ -584,8 +768,8 @@ size_t grad_vectors_bytes(int count, int N, int M, int max_splits) {
     return sizeof(double2) * static_cast<size_t>(splits) * chunks * (1 + N) * M;
 }
 
-cudaError_t launch_grad_vectors(const GradVectors& g, const OpDev& op, double2* out, double2* partial, int max_splits,
-                                cudaStream_t st) {
+cudaError_t launch_grad_vectors(const GradVectors& g, const OpDev& op, double2* partial, int max_splits,
+                                cudaStream_t st, SplitSum* job) {
     if (g.count <= 0) return cudaSuccess;
     int per_split, splits, chunks, cap;
     grad_vectors_shape(g.count, max_splits, &per_split, &splits, &chunks, &cap);
@@ -599,17 +783,47 @@ cudaError_t launch_grad_vectors(const GradVectors& g, const OpDev& op, double2* 
     }
     const dim3 grid(g.Mpad / 32, splits * chunks);
     kernel<<<grid, 32 * kGvWarps, sm, st>>>(g, op, per_split, chunks, cap, partial);
-    OuterSet set{};
-    set.out[0] = out;
-    return finish_splits(static_cast<long>(1 + g.N) * g.M, splits * chunks, 1, partial, set, -2.0, st);
+    job->pre = partial;
+    job->pre_splits = splits * chunks;
+    return cudaGetLastError();
 }
 
 cudaError_t launch_weighted_sums(int count, const double* w, const SeriesSet& set, double2* block_scratch,
                                  double2* sums, cudaStream_t st) {
     if (count <= 0) return cudaSuccess;
     const int blocks = min(kSumBlocks, max(1, (count + 255) / 256));
-    wsum_blocks_kernel<<<blocks, 256, 0, st>>>(count, w, set, block_scratch);
-    wsum_finish_kernel<<<1, 32, 0, st>>>(blocks, set.n, block_scratch, sums);
+    wsum_kernel<false><<<blocks, kSumThreads, 0, st>>>(count, w, set, block_scratch, sums);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_weighted_mean(int count, const double* w, const double2* v, double2* block_scratch, double2* mean,
+                                 cudaStream_t st) {
+    if (count <= 0) return cudaErrorInvalidValue;
+    SeriesSet set{};
+    set.n = 1;
+    set.v[0] = v;
+    wsum_kernel<true><<<min(kSumBlocks, (count + 255) / 256), kSumThreads, 0, st>>>(count, w, set, block_scratch, mean);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_exact_weights(int count, const double2* lp, double* w, double2* block_scratch, double2* stat,
+                                 cudaStream_t st) {
+    const int blocks = min(kSumBlocks, max(1, (count + 255) / 256));
+    exact_max_kernel<<<blocks, kSumThreads, 0, st>>>(count, lp, block_scratch, stat);
+    exact_norm_kernel<<<blocks, kSumThreads, 0, st>>>(count, lp, block_scratch, stat);
+    exact_weights_kernel<<<grid_for(count), 256, 0, st>>>(count, lp, stat, w);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_grad_coefs(int count, const double* w, const double2* v, const double2* shift, double2* c1,
+                              double2* c2, double2* c3, int conj3, cudaStream_t st) {
+    grad_coefs_kernel<<<grid_for(count), 256, 0, st>>>(count, w, v, shift, c1, c2, c3, conj3);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_grad_out(const GradOut& g, cudaStream_t st) {
+    const long n = max(1L, max(g.count, static_cast<long>(g.first)));
+    grad_out_kernel<<<static_cast<int>((n + 255) / 256), 256, 0, st>>>(g);
     return cudaGetLastError();
 }
 
@@ -634,12 +848,6 @@ cudaError_t launch_coef(int count, const double* w, const double2* v, double sca
 cudaError_t launch_coef_conj(int count, const double* w, const double2* v, double2 shift, double2* c,
                              cudaStream_t st) {
     coef_conj_kernel<<<grid_for(count), 256, 0, st>>>(count, w, v, shift, c);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_coef_real(int count, const double* w, const double2* v, double shift, double2* c,
-                             cudaStream_t st) {
-    coef_real_kernel<<<grid_for(count), 256, 0, st>>>(count, w, v, shift, c);
     return cudaGetLastError();
 }
 
