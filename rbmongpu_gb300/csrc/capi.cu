@@ -1071,7 +1071,7 @@ extern "C" int rbmg_ev_difference(const rbmg_psi* psi, const rbmg_psi* psi_prime
         return fail(RBMG_EINVAL, "difference: bad arguments");
     if (psi->kind != 0 || psi_prime->kind != 0)
         return fail(RBMG_EUNSUPPORTED, "difference: instantiated for Psi only (ExpectationValue.cu:529, 575)");
-    if (psi_prime->N != psi->N || psi_prime->Mpad != psi->Mpad)
+    if (psi_prime->N != psi->N || !rbm_pairable(psi_prime->M, psi->M))
         return fail(RBMG_EUNSUPPORTED, "difference: psi_prime must have psi's N and padded M");
     if (num_ops == 0) return RBMG_OK;
     for (int q = 0; q < num_ops; q++) {

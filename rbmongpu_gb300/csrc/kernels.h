@@ -140,6 +140,7 @@ cudaError_t launch_rbm_mc(const RbmDev& psi, const OpDev* op, const McLaunch& L,
 cudaError_t launch_rbm_estimate(const RbmDev& psi, const OpDev* op, const RbmDev* psi_prime, const EstLaunch& L,
                                 cudaStream_t st);
 
+bool rbm_pairable(int Ma, int Mb);
 int rbm_lanes_k(int M);   // instantiated hidden units per lane for M, -1 if too large
 
 }  // namespace rbmg

@@ -977,8 +977,12 @@ cudaError_t launch_learned(int which, const RbmDev& P, const LearnedLaunch& L, c
     switch (P.Mpad / 32) {
         case 1: return launch_learned_k<1>(which, nw, P, L, st);
         case 2: return launch_learned_k<2>(which, nw, P, L, st);
+        case 3: return launch_learned_k<3>(which, nw, P, L, st);
         case 4: return launch_learned_k<4>(which, nw, P, L, st);
+        case 5: return launch_learned_k<5>(which, nw, P, L, st);
+        case 6: return launch_learned_k<6>(which, nw, P, L, st);
         case 8: return launch_learned_k<8>(which, nw, P, L, st);
+        case 10: return launch_learned_k<10>(which, nw, P, L, st);
         case 13: return launch_learned_k<13>(which, nw, P, L, st);
         case 18: return launch_learned_k<18>(which, nw, P, L, st);
         default: return cudaErrorInvalidValue;
@@ -1006,8 +1010,12 @@ cudaError_t launch_lb_target(const RbmDev& P, int n, const uint64_t* spins, cons
     switch (P.Mpad / 32) {
         case 1: return launch_lb_k<1>(nw, P, n, spins, theta, re, logits, O, dl, st);
         case 2: return launch_lb_k<2>(nw, P, n, spins, theta, re, logits, O, dl, st);
+        case 3: return launch_lb_k<3>(nw, P, n, spins, theta, re, logits, O, dl, st);
         case 4: return launch_lb_k<4>(nw, P, n, spins, theta, re, logits, O, dl, st);
+        case 5: return launch_lb_k<5>(nw, P, n, spins, theta, re, logits, O, dl, st);
+        case 6: return launch_lb_k<6>(nw, P, n, spins, theta, re, logits, O, dl, st);
         case 8: return launch_lb_k<8>(nw, P, n, spins, theta, re, logits, O, dl, st);
+        case 10: return launch_lb_k<10>(nw, P, n, spins, theta, re, logits, O, dl, st);
         case 13: return launch_lb_k<13>(nw, P, n, spins, theta, re, logits, O, dl, st);
         case 18: return launch_lb_k<18>(nw, P, n, spins, theta, re, logits, O, dl, st);
         default: return cudaErrorInvalidValue;

@@ -8,7 +8,13 @@ cudaError_t rbm_mc_launch_k(const RbmDev&, const OpDev*, const McLaunch&, cudaSt
 template <int K>
 cudaError_t rbm_est_launch_k(const RbmDev&, const OpDev*, const RbmDev*, const EstLaunch&, cudaStream_t);
 
-static const int kInstantiated[] = {1, 2, 4, 8, 13, 18};
+// Every pass evaluates all 32 K units, the padding too, so the counts are at most a third (above
+// 32 units) over what M needs.  With 1, 2, 4, 8, 13 and 18 alone M = 75 ran 128 units and M = 150
+// ran 256.  Microseconds a sweep of 1024 and
+// 16384 walkers with those and now: N = 30, M = 75: 15 / 14 and 109 / 93; N = 40, M = 150: 34 / 24 and
+// 260 / 176; N = 64, M = 180: 54 / 45 and 411 / 324; N = 80, M = 300: 118 / 93 and 893 / 671; the
+// energies of 10007 configurations at N = 75, M = 150: 0.64 / 0.50 ms with their log psi.
+static const int kInstantiated[] = {1, 2, 3, 4, 5, 6, 8, 10, 13, 18};
 
 int rbm_lanes_k(int M) {
     const int need = (M + 31) / 32;
@@ -17,12 +23,26 @@ int rbm_lanes_k(int M) {
     return -1;
 }
 
+// two networks of one pass have their units in the same of these ranges
+bool rbm_pairable(int Ma, int Mb) {
+    auto range = [](int M) {
+        int r = 0;
+        for (int top : {32, 64, 128, 256, 416, 576}) r += M > top;
+        return r;
+    };
+    return range(Ma) == range(Mb);
+}
+
 cudaError_t launch_rbm_mc(const RbmDev& P, const OpDev* op, const McLaunch& L, cudaStream_t st) {
     switch (P.Mpad / 32) {
         case 1: return rbm_mc_launch_k<1>(P, op, L, st);
         case 2: return rbm_mc_launch_k<2>(P, op, L, st);
+        case 3: return rbm_mc_launch_k<3>(P, op, L, st);
         case 4: return rbm_mc_launch_k<4>(P, op, L, st);
+        case 5: return rbm_mc_launch_k<5>(P, op, L, st);
+        case 6: return rbm_mc_launch_k<6>(P, op, L, st);
         case 8: return rbm_mc_launch_k<8>(P, op, L, st);
+        case 10: return rbm_mc_launch_k<10>(P, op, L, st);
         case 13: return rbm_mc_launch_k<13>(P, op, L, st);
         case 18: return rbm_mc_launch_k<18>(P, op, L, st);
         default: return cudaErrorInvalidValue;
@@ -88,12 +108,23 @@ cudaError_t launch_rbm_pairs(int N, int Mpad, const float2* W, const float2* b, 
 
 cudaError_t launch_rbm_estimate(const RbmDev& P, const OpDev* op, const RbmDev* PP, const EstLaunch& L,
                                 cudaStream_t st) {
-    if (PP && PP->Mpad != P.Mpad) return cudaErrorInvalidValue;
+    if (PP && PP->Mpad != P.Mpad) {   // a launch per network: the kernel has one number of units
+        if (!rbm_pairable(P.M, PP->M)) return cudaErrorInvalidValue;
+        EstLaunch own = L, prime = L;
+        own.flags &= ~EST_PRIME;
+        prime.flags &= EST_PRIME | EST_ENUMERATE;
+        const cudaError_t e = launch_rbm_estimate(P, op, nullptr, own, st);
+        return e != cudaSuccess ? e : launch_rbm_estimate(*PP, nullptr, PP, prime, st);
+    }
     switch (P.Mpad / 32) {
         case 1: return rbm_est_launch_k<1>(P, op, PP, L, st);
         case 2: return rbm_est_launch_k<2>(P, op, PP, L, st);
+        case 3: return rbm_est_launch_k<3>(P, op, PP, L, st);
         case 4: return rbm_est_launch_k<4>(P, op, PP, L, st);
+        case 5: return rbm_est_launch_k<5>(P, op, PP, L, st);
+        case 6: return rbm_est_launch_k<6>(P, op, PP, L, st);
         case 8: return rbm_est_launch_k<8>(P, op, PP, L, st);
+        case 10: return rbm_est_launch_k<10>(P, op, PP, L, st);
         case 13: return rbm_est_launch_k<13>(P, op, PP, L, st);
         case 18: return rbm_est_launch_k<18>(P, op, PP, L, st);
         default: return cudaErrorInvalidValue;

@@ -10,7 +10,7 @@
 // wall-clock limit after which the kernel raises an error flag and returns).  Each tile
 // writes its chunk's partial sums; a second kernel of the graph adds the chunks in a fixed
 // order and forms the gradient, so every replay gives the same bits.  The walker tasks are compiled
-// for each hidden-unit count per lane (1, 2, 4, 8, 13, 18: M <= 576) as separate functions
+// for each hidden-unit count per lane (rbm_lanes_k: M <= 576) as separate functions
 // of the one kernel.  The launch (counter resets + both kernels) is captured once in a
 // CUDA graph and replayed; the warps per block, the reduction tile height and a register
 // cap come from an autotuner that times the candidates on the batch itself.
@@ -649,8 +649,12 @@ __global__ void __maxnreg__(REGS) serve_kernel(SLaunch L) {
             switch (I.K) {   // the hidden-unit counts per lane of rbm_lanes_k
                 case 1: walker_task<1>(L, I, task.index, lane); break;
                 case 2: walker_task<2>(L, I, task.index, lane); break;
+                case 3: walker_task<3>(L, I, task.index, lane); break;
                 case 4: walker_task<4>(L, I, task.index, lane); break;
+                case 5: walker_task<5>(L, I, task.index, lane); break;
+                case 6: walker_task<6>(L, I, task.index, lane); break;
                 case 8: walker_task<8>(L, I, task.index, lane); break;
+                case 10: walker_task<10>(L, I, task.index, lane); break;
                 case 13: walker_task<13>(L, I, task.index, lane); break;
                 default: walker_task<18>(L, I, task.index, lane); break;
             }
@@ -866,11 +870,7 @@ extern "C" int rbmg_batch_create(int n, const rbmg_psi* const* psis, const rbmg_
         if (!p || !o || walkers[i] == 0) return fail(RBMG_EINVAL, "batch: null instance or no walkers");
         if (p->kind != 0) return fail(RBMG_EUNSUPPORTED, "batch: complex RBM (Psi) instances only");
         if (p->Mpad / 32 > kSK) return fail(RBMG_EUNSUPPORTED, "batch: M <= 576");
-        {
-            const int K = p->Mpad / 32;
-            if (K != 1 && K != 2 && K != 4 && K != 8 && K != 13 && K != 18)
-                return fail(RBMG_EINVAL, "batch: unexpected hidden-unit padding");
-        }
+        if (p->Mpad != 32 * rbm_lanes_k(p->M)) return fail(RBMG_EINVAL, "batch: unexpected hidden-unit padding");
         if (p->N > 64 * kSW) return fail(RBMG_EUNSUPPORTED, "batch: N <= 192");
         if (o->max_site >= p->N) return fail(RBMG_EINVAL, "batch: operator acts on a site >= N");
         for (int q = 0; q < i; q++)
