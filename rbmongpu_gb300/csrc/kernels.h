@@ -34,7 +34,7 @@ struct RbmDev {
 };
 
 // lanes that share a walker in the grouped sampler
-constexpr int rbm_group(int K) { return K == 1 ? 8 : 16; }
+constexpr int rbm_group(int K) { return K == 1 ? 8 : (K < 18 ? 16 : 32); }   // 32: no groups
 
 // build Wq, bq, Wg, bg from W [N][Mpad], b [Mpad] (K = Mpad / 32 hidden units per lane), and Wt4
 cudaError_t launch_rbm_pairs(int N, int Mpad, const float2* W, const float2* b, float4* Wq, float4* bq,

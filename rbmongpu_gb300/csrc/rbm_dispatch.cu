@@ -97,7 +97,8 @@ cudaError_t launch_rbm_pairs(int N, int Mpad, const float2* W, const float2* b, 
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const long q = static_cast<long>(N + 1) * (Mpad / 2);
-    rbm_group_pairs_kernel<<<static_cast<int>((q + 255) / 256), 256, 0, st>>>(N, Mpad, rbm_group(Mpad / 32), W, b, Wg,
+    if (rbm_group(Mpad / 32) < 32)
+        rbm_group_pairs_kernel<<<static_cast<int>((q + 255) / 256), 256, 0, st>>>(N, Mpad, rbm_group(Mpad / 32), W, b, Wg,
                                                                               bg);
     e = cudaGetLastError();
     if (e != cudaSuccess || !Wt) return e;

@@ -6,6 +6,7 @@
 // per k) from global memory through L1/L2.  This file is included by the rbm_k*.cu
 // translation units, each instantiating one K.
 #pragma once
+#include <type_traits>
 
 #include "device_math.cuh"
 #include "kernels.h"
@@ -170,87 +171,6 @@ __device__ __forceinline__ void rbm_refresh2(const RbmDev& P, const Spins<NW>& s
             ti[kk] = fma2(sg, pk2(w.z, w.w), ti[kk]);
         }
     }
-}
-
-template <int K, int KP, int NW, class Rng>
-__device__ __forceinline__ bool rbm_mh_step2(const RbmDev& P, Spins<NW>& s, pair_t (&tr)[KP], pair_t (&ti)[KP],
-                                             pair_t (&re)[KP], Rng& rng, int lane, int total_z, uint64_t nmagic) {
-    const uint32_t N = static_cast<uint32_t>(P.N);
-    int sites[2];
-    int ns = 1;
-    sites[0] = static_cast<int>(fastmod(rng.next(), nmagic, N));
-    if (total_z) {
-        const bool first_new = !s.up(sites[0]);
-        int sec = sites[0];
-        for (int guard = 0; guard < (1 << 20); guard++) {
-            const int c = static_cast<int>(fastmod(rng.next(), nmagic, N));
-            const bool v = c == sites[0] ? first_new : s.up(c);
-            if (v == first_new) { sec = c; break; }
-        }
-        sites[1] = sec;
-        ns = 2;
-    }
-    Spins<NW> s2 = s;
-    pair_t two_s[2];
-    const float4* rows[2];
-#pragma unroll
-    for (int q = 0; q < 2; q++) {
-        if (q >= ns) break;
-        const int site = q == 0 ? sites[0] : sites[1];
-        s2.flip(site);
-        two_s[q] = splat2(s2.up(site) ? 2.0f : -2.0f);
-        rows[q] = P.Wq + static_cast<long>(site) * KP * 32 + lane;
-    }
-    float part = 0.0f;
-    pair_t fnew[KP];   // Re f of the proposed angles
-    if (ns == 1) {
-        // single flip: the KP loads of the paired W row are issued together
-        float4 w[KP];
-#pragma unroll
-        for (int kk = 0; kk < KP; kk++) w[kk] = __ldg(rows[0] + 32 * kk);
-#pragma unroll
-        for (int kk = 0; kk < KP; kk++) {
-            const pair_t nr = fma2(two_s[0], pk2(w[kk].x, w[kk].y), tr[kk]);
-            const pair_t ni = fma2(two_s[0], pk2(w[kk].z, w[kk].w), ti[kk]);
-            fnew[kk] = lc_re2(nr, ni);
-            float d0, d1;
-            up2(sub2(fnew[kk], re[kk]), d0, d1);
-            part = __fadd_rn(part, d0);
-            if (2 * kk + 1 < K) part = __fadd_rn(part, d1);
-        }
-    } else {
-#pragma unroll
-        for (int kk = 0; kk < KP; kk++) {
-            pair_t nr = tr[kk], ni = ti[kk];
-            for (int q = 0; q < ns; q++) {
-                const float4 w = __ldg(rows[q] + 32 * kk);
-                nr = fma2(two_s[q], pk2(w.x, w.y), nr);
-                ni = fma2(two_s[q], pk2(w.z, w.w), ni);
-            }
-            fnew[kk] = lc_re2(nr, ni);
-            float d0, d1;
-            up2(sub2(fnew[kk], re[kk]), d0, d1);
-            part = __fadd_rn(part, d0);
-            if (2 * kk + 1 < K) part = __fadd_rn(part, d1);
-        }
-    }
-    const float delta = warp_sum_xor(part);
-    bool accept = delta > 0.0f;
-    if (!accept) accept = rng.uniform() <= expf_det(__fmul_rn(2.0f, delta));
-    if (accept) {
-        s = s2;
-#pragma unroll
-        for (int kk = 0; kk < KP; kk++) {
-            for (int q = 0; q < ns; q++) {
-                const float4 w = __ldg(rows[q] + 32 * kk);
-                tr[kk] = fma2(two_s[q], pk2(w.x, w.y), tr[kk]);
-                ti[kk] = fma2(two_s[q], pk2(w.z, w.w), ti[kk]);
-            }
-            // lc_re2 of the new angles, formed by the same operations: kept from the proposal
-            re[kk] = fnew[kk];
-        }
-    }
-    return accept;
 }
 
 // One update of the fast sweep (MonteCarloLoop.hpp:162-171): the proposal flips the spins
@@ -449,83 +369,41 @@ __device__ __forceinline__ double2 warp_log_psi(const float2 (&f)[K]) {
 }
 
 // ---------------------------------------------------------------------------
-// Metropolis sampler: one warp per walker for a whole launch
-// (include/spin_ensembles/MonteCarloLoop.hpp:55-138).  The angles are recomputed
-// from the spins at the start of every sweep.  Measurements (local energies, log psi)
-// are a separate pass (rbm_est_kernel) over the recorded configurations, which keeps
-// the sampler's register footprint to the walker state.
-// ---------------------------------------------------------------------------
-template <int K, int NW>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, 4) rbm_mc_kernel(RbmDev P, McLaunch L) {
-    const int lane = threadIdx.x & 31;
-    const int w = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-    if (w >= L.B) return;
-    WarpRng rng;
-    rng.init(L.seed, L.walker_base + static_cast<uint32_t>(w), L.rng_index[w], lane);
-    const uint64_t nmagic = fastmod_magic(static_cast<uint32_t>(P.N));
-    Spins<NW> s;
-    if (L.init) {
-#pragma unroll
-        for (int k = 0; k < NW; k++) s.w[k] = 0;
-        if (L.total_z) s.w[0] = draw_n_over_k(rng, P.N, static_cast<unsigned>((L.sector + P.N) / 2));
-        else draw_spins(rng, P.N, s);
-    } else {
-#pragma unroll
-        for (int k = 0; k < NW; k++) s.w[k] = L.spins[static_cast<long>(w) * NW + k];
-    }
-    constexpr int KP = (K + 1) / 2;
-    pair_t tr[KP], ti[KP], re[KP];
-    unsigned long long acc = 0, props = 0;
-    const int total_sweeps = L.n_therm + L.n_samples * L.sweeps_per_sample;
-    int sample = 0;
-    for (int sw = 0; sw < total_sweeps; sw++) {
-        rbm_refresh2(P, s, tr, ti, lane);
-#pragma unroll
-        for (int kk = 0; kk < KP; kk++) re[kk] = lc_re2(tr[kk], ti[kk]);
-        for (int p = 0; p < P.N; p++)
-            acc += rbm_mh_step2<K>(P, s, tr, ti, re, rng, lane, L.total_z, nmagic);
-        props += P.N;
-        const int done = sw + 1 - L.n_therm;
-        if (done > 0 && done % L.sweeps_per_sample == 0) {
-            const long row = static_cast<long>(L.sample_base + sample) * L.B + w;
-            if (L.sample_spins && lane == 0) {
-#pragma unroll
-                for (int k = 0; k < NW; k++) L.sample_spins[row * NW + k] = s.w[k];
-            }
-            sample++;
-        }
-    }
-    if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < NW; k++) L.spins[static_cast<long>(w) * NW + k] = s.w[k];
-        L.rng_index[w] = rng.index;
-        L.accepts[w] += acc;
-        L.proposals[w] += props;
-    }
-}
-
-// ---------------------------------------------------------------------------
-// The sampler with several walkers per warp: G lanes share a walker (rbm_group), each with
-// PP = 16 K / G pairs of hidden units.  What a proposal does once per walker -- the random words,
-// the site, the last steps of the lane sum, the exponential, the test -- was 65 % of the warp's
-// instructions at K = 4 (273 a proposal, 96 of them activations) and now serves 32 / G walkers.
-// Lane g holds what lanes g, g + G, g + 2 G, ... of the one-walker kernel hold: their partial
-// sums stay apart until they meet in the order of its butterfly (offsets 16, 8, ... down to G
-// within the lane, the rest by shuffles), so angles, sums and decisions are the same bit for bit.
-// Bound by the FP32 pipe (16384 walkers: its floor is half of the time) and, with few walkers,
-// by one proposal's latency.  Microseconds a sweep with one walker a warp and grouped: N = 24,
-// M = 24: 12 / 10 at 16 walkers, 29 / 13 at 4096, 92 / 32 at 16384; N = 32, M = 64: 16 / 13,
-// 38 / 24, 124 / 76; N = 64, M = 128: 33 / 32, 97 / 72, 344 / 233.  Blocks of one, two or four
-// warps and keeping the proposed angles measured alike; G = 8 at K = 2 and 4 (G = 4 at K = 1)
-// was slower up to 4096 walkers (K = 4: 33 / 57 at 16, 97 / 75) and gained 6 % at 16384.
-// Large layers have the registers of three (K = 13) and two (K = 18) blocks an SM; against one
-// walker a warp with its state in shared memory, K = 13 (N = 100, M = 400): 155 / 149 at 16, 388 /
-// 365 at 4096, 1253 / 1120 at 16384; K = 18 (N = 140, M = 576): 330 / 253, 832 / 667, 2421 / 2281.
-// With four blocks and spills K = 13 took 250 and 1239; state in shared memory here, the same.
+// Metropolis sampler (include/spin_ensembles/MonteCarloLoop.hpp:55-138).  The angles are
+// recomputed from the spins at the start of every sweep.  Measurements (local energies, log psi)
+// are a separate pass over the recorded configurations, which keeps the registers to the
+// walkers' state.
+//
+// G lanes share a walker, each with PP pairs of hidden units.  G = 32, one walker per warp, where
+// walkers are few: a proposal is a chain of dependent steps, and half the units a lane make it
+// shorter.  G = 16 (8 at K = 1), two to four walkers per warp, where they fill the chip: what a
+// proposal does once per walker -- the random words, the site, the last steps of the lane sum, the
+// exponential, the test -- was 65 % of the warp's instructions at K = 4 (273 a proposal, 96 of them
+// activations) and serves 32 / G walkers.  Lane g of a group holds what lanes g, g + G, g + 2 G, ...
+// of a whole warp hold: their partial sums stay apart until they meet in the order of its
+// butterfly (offsets 16, 8, ... down to G within the lane, the rest by shuffles), so angles, sums
+// and decisions are the same bit for bit.
+// Bound by the FP32 pipe with many walkers (16384: its floor is half of the time) and by one
+// proposal's latency with few; the next site is found while a proposal is evaluated, both ways
+// the test's number may or may not be used.  Microseconds a sweep at 512 / 4096 / 16384 walkers,
+// G = 32 and 16: K = 3 (N = 30): 10, 36, 130 and 13, 29, 94; K = 4 (N = 64): 21, 75, 273 and 31, 73,
+// 236; K = 8 (N = 90): 41, 172, 630 and 74, 183, 597; K = 13 (N = 100): 74, 306, 1119 and 146, 355,
+// 1096; K = 18 (N = 140): 139, 551, 1996 and 252, 652, 2250.  Before, with G = 16 throughout (32 at K = 8):
+// 14, 29, 93; 32, 72, 233; 66, 183, 595; 149, 365, 1120; 253, 667, 2281.
+// Blocks of one, two or four warps and keeping the proposed angles measured alike; G = 8 at K = 2
+// and 4 was slower up to 4096 walkers.  Five blocks an SM where the registers allow it gained 3 %
+// at 16384 walkers and lost 8 % at 512.
+//
+// total_z: the partner of a flip is the first of a stream of draws whose spin fits; the group's
+// lanes test G of them at once (one at a time took two to four rounds of dependent steps: N = 36,
+// M = 75, 2048 walkers 44 -> 29 us a sweep with its energies, and 90 -> 32 in a nearly full sector).
 // ---------------------------------------------------------------------------
 template <int K, int G, int NW, bool SZ>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, K >= 18 ? 2 : (K >= 13 ? 3 : 4)) rbm_mc_group_kernel(RbmDev P, McLaunch L) {
-    constexpr int H = 16 / G, PP = K * H, PW = 32 / G;   // PW walkers per warp
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, K >= 13 ? 3 : 4) rbm_mc_group_kernel(RbmDev P, McLaunch L) {
+    constexpr bool WARP = G == 32;   // one walker: a lane's units pair up as in Wq
+    constexpr int H = WARP ? 1 : 16 / G, PP = WARP ? (K + 1) / 2 : K * H, PW = 32 / G;   // PW walkers per warp
+    const float4* __restrict__ Wp = WARP ? P.Wq : P.Wg;
+    const float4* __restrict__ bp = WARP ? P.bq : P.bg;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, g = lane % G;
     const int w0 = (blockIdx.x * kWarpsPerBlock + wib) * PW;
     if (w0 >= L.B) return;
@@ -552,6 +430,10 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, K >= 18 ? 2 : (K >= 13 ? 
         __syncwarp();
         rng.init(L.seed, L.walker_base + static_cast<uint32_t>(w), start, words_sm[wib] + (lane - g), g);
     }
+    // the next proposal's site, should the words up to it be used: found while the last one is
+    // evaluated, off the chain of dependent steps that one walker's proposals are
+    rng.ensure(3, g);
+    int next = static_cast<int>(fastmod(rng.peek(), nmagic, static_cast<uint32_t>(P.N)));
     pair_t tr[PP], ti[PP], re[PP];
     unsigned long long acc = 0, props = 0;
     const int total_sweeps = L.n_therm + L.n_samples * L.sweeps_per_sample;
@@ -560,11 +442,11 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, K >= 18 ? 2 : (K >= 13 ? 
         // angles from the spins
 #pragma unroll
         for (int p = 0; p < PP; p++) {
-            const float4 b = __ldg(P.bg + p * G + g);
+            const float4 b = __ldg(bp + p * G + g);
             tr[p] = pk2(b.x, b.y);
             ti[p] = pk2(b.z, b.w);
         }
-        const float4* row = P.Wg + g;
+        const float4* row = Wp + g;
         for (int i = 0; i < P.N; i++, row += PP * G) {
             const pair_t sg = splat2(s.up(i) ? 1.0f : -1.0f);
 #pragma unroll
@@ -577,37 +459,44 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, K >= 18 ? 2 : (K >= 13 ? 
 #pragma unroll
         for (int p = 0; p < PP; p++) re[p] = lc_re2(tr[p], ti[p]);
         for (int prop = 0; prop < P.N; prop++) {
-            rng.ensure(2, g);
-            const int site = static_cast<int>(fastmod(rng.peek(), nmagic, static_cast<uint32_t>(P.N)));
+            // words: the site, the partner's candidates, the test's number and the next site
+            rng.ensure(SZ ? G + 3 : 3, g);
+            const int site = next;
             rng.pos++;
             Spins<NW> s2 = s;
             s2.flip(site);
             const bool first_new = s2.up(site);
             const pair_t t0 = splat2(first_new ? 2.0f : -2.0f);
-            const float4* row0 = P.Wg + static_cast<long>(site) * PP * G + g;
+            const float4* row0 = Wp + static_cast<long>(site) * PP * G + g;
             pair_t t1 = t0;
             const float4* row1 = row0;
             if (SZ) {
-                // the partner: drawn until its spin equals the first site's new one
+                // the partner: drawn until its spin equals the first site's new one; the group's
+                // lanes test G draws at once and the first that fits is taken
                 int sec = site;
                 bool found = false;
-                for (int guard = 0; guard < (1 << 20) && __any_sync(0xffffffffu, !found); guard++) {
-                    rng.ensure(1, g);
+                for (int guard = 0; guard < (1 << 20) / G; guard++) {
+                    const int c = static_cast<int>(fastmod(rng.words[rng.pos + g], nmagic, static_cast<uint32_t>(P.N)));
+                    const bool fits = (c == site ? first_new : s.up(c)) == first_new;
+                    const unsigned int fit = (__ballot_sync(0xffffffffu, fits) >> (lane - g)) & (0xffffffffu >> (32 - G));
+                    const int taken = __ffs(static_cast<int>(fit)) - 1;
+                    const int c2 = __shfl_sync(0xffffffffu, c, (lane - g) + max(taken, 0));
                     if (!found) {
-                        const int c = static_cast<int>(fastmod(rng.peek(), nmagic, static_cast<uint32_t>(P.N)));
-                        rng.pos++;
-                        if ((c == site ? first_new : s.up(c)) == first_new) {
-                            sec = c;
-                            found = true;
-                        }
+                        if (fit) sec = c2;
+                        rng.pos += fit ? taken + 1 : G;
+                        found = fit != 0;
                     }
+                    if (!__any_sync(0xffffffffu, !found)) break;
+                    rng.ensure(G + 2, g);
                 }
                 s2.flip(sec);
                 t1 = splat2(s2.up(sec) ? 2.0f : -2.0f);
-                row1 = P.Wg + static_cast<long>(sec) * PP * G + g;
-                rng.ensure(1, g);
+                row1 = Wp + static_cast<long>(sec) * PP * G + g;
             }
+            const int next0 = static_cast<int>(fastmod(rng.peek(), nmagic, static_cast<uint32_t>(P.N)));
+            const int next1 = static_cast<int>(fastmod(rng.words[rng.pos + 1], nmagic, static_cast<uint32_t>(P.N)));
             pair_t part[H], fnew[PP];
+            float delta = 0.0f;
 #pragma unroll
             for (int h = 0; h < H; h++) part[h] = splat2(0.0f);
 #pragma unroll
@@ -620,20 +509,31 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, K >= 18 ? 2 : (K >= 13 ? 
                     ni = fma2(t1, pk2(u.z, u.w), ni);
                 }
                 fnew[p] = lc_re2(nr, ni);
-                part[p % H] = add2(part[p % H], sub2(fnew[p], re[p]));
+                const pair_t d = sub2(fnew[p], re[p]);
+                if (WARP) {
+                    float d0, d1;
+                    up2(d, d0, d1);
+                    delta = __fadd_rn(delta, d0);
+                    if (2 * p + 1 < K) delta = __fadd_rn(delta, d1);
+                } else {
+                    part[p % H] = add2(part[p % H], d);
+                }
             }
             // the butterfly of the one-walker kernel: lanes l and l ^ off, off = 16, 8, 4, 2, 1
+            if (!WARP) {
 #pragma unroll
-            for (int half = H / 2; half >= 1; half >>= 1)
+                for (int half = H / 2; half >= 1; half >>= 1)
 #pragma unroll
-                for (int h = 0; h < half; h++) part[h] = add2(part[h], part[h + half]);
-            float d0, d1;
-            up2(part[0], d0, d1);
-            float delta = __fadd_rn(d0, d1);
+                    for (int h = 0; h < half; h++) part[h] = add2(part[h], part[h + half]);
+                float d0, d1;
+                up2(part[0], d0, d1);
+                delta = __fadd_rn(d0, d1);
+            }
 #pragma unroll
             for (int off = G / 2; off >= 1; off >>= 1)
                 delta = __fadd_rn(delta, __shfl_xor_sync(0xffffffffu, delta, off));
             bool accept = delta > 0.0f;
+            next = accept ? next0 : next1;
             if (!accept) {
                 const float u = __fmul_rn(static_cast<float>((rng.peek() >> 8) + 1u), 5.9604644775390625e-8f);
                 rng.pos++;
@@ -1054,10 +954,16 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) rbm_eloc_t_kernel(RbmDev 
 // ---------------------------------------------------------------------------
 // launchers for this K (instantiated by rbm_k<K>.cu)
 // ---------------------------------------------------------------------------
-// Several walkers per warp, except at K = 8 with few walkers, where a lane's sixteen units in
-// sequence take longer than the shared work saves (N = 90, M = 250, one walker a warp / grouped:
-// 66 / 78 us a sweep at 16 walkers, 79 / 81 at 1024, 119 / 105 at 2048, 730 / 595 at 16384)
-constexpr bool rbm_grouped(int K, int walkers) { return K != 8 || walkers >= 2048; }
+// One walker per warp or a group of lanes each (rbm_mc_group_kernel's figures).  At an odd K the
+// whole warp leaves half a pair of units empty, which tells most at K = 3; from K = 8 on the
+// groups' longer chains still cost more at 4096 walkers, where both forms fill the chip's last
+// wave alike, but not between 1536 and 3584, where only the groups' first wave has room; K = 18 has
+// no groups (1996 against 2250 us at 16384 walkers).
+constexpr bool rbm_grouped(int K, int walkers) {
+    if (rbm_group(K) == 32) return false;
+    if (walkers <= (K == 3 ? 608 : (K == 1 ? 1216 : 1536))) return false;
+    return !(K >= 8 && walkers >= 3584 && walkers <= 6144);
+}
 
 template <int K>
 cudaError_t rbm_mc_launch_k(const RbmDev& P, const OpDev* op, const McLaunch& L, cudaStream_t st) {
@@ -1075,8 +981,8 @@ cudaError_t rbm_mc_launch_k(const RbmDev& P, const OpDev* op, const McLaunch& L,
         }
         return cudaGetLastError();
     }
-    if (rbm_grouped(K, L.B)) {
-        constexpr int G = rbm_group(K), per_block = kWarpsPerBlock * 32 / G;
+    auto sampler = [&](auto group) {
+        constexpr int G = decltype(group)::value, per_block = kWarpsPerBlock * 32 / G;
         const dim3 blocks((L.B + per_block - 1) / per_block);
         if (L.total_z && nw != 1) return cudaErrorInvalidValue;
         if (L.total_z) rbm_mc_group_kernel<K, G, 1, true><<<blocks, block, 0, st>>>(P, L);
@@ -1086,18 +992,9 @@ cudaError_t rbm_mc_launch_k(const RbmDev& P, const OpDev* op, const McLaunch& L,
         else if (nw == 4) rbm_mc_group_kernel<K, G, 4, false><<<blocks, block, 0, st>>>(P, L);
         else return cudaErrorInvalidValue;
         return cudaGetLastError();
-    }
-    if constexpr (K == 8) {   // one walker per warp
-        switch (nw) {
-            case 1: rbm_mc_kernel<K, 1><<<grid, block, 0, st>>>(P, L); break;
-            case 2: rbm_mc_kernel<K, 2><<<grid, block, 0, st>>>(P, L); break;
-            case 3: rbm_mc_kernel<K, 3><<<grid, block, 0, st>>>(P, L); break;
-            case 4: rbm_mc_kernel<K, 4><<<grid, block, 0, st>>>(P, L); break;
-            default: return cudaErrorInvalidValue;
-        }
-        return cudaGetLastError();
-    }
-    return cudaErrorInvalidValue;
+    };
+    if (rbm_grouped(K, L.B)) return sampler(std::integral_constant<int, rbm_group(K)>());
+    return sampler(std::integral_constant<int, 32>());
 }
 
 template <int K>

@@ -121,7 +121,7 @@ __device__ __forceinline__ void s_refresh(const SInst& I, const Spins<NW>& s, fl
     }
 }
 
-// the sweeps on packed pairs (rbm_refresh2 / rbm_mh_step2 of the single-network sampler,
+// the sweeps on packed pairs (rbm_mc_group_kernel of a single network with 32 lanes a walker, the
 // same arithmetic and draw order)
 template <int KP, int NW>
 __device__ __forceinline__ void s_refresh2(const SInst& I, const Spins<NW>& s, pair_t (&tr)[KP], pair_t (&ti)[KP],
