@@ -824,9 +824,15 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) rbm_grad_terms_kernel(Rbm
 // string's quarters; one warp reduction per configuration joins the strings.  No
 // per-string reduction sits on the critical path, and each lane's loop over units is
 // independent work.
+// Bound by shared-memory reads of theta and f and the latency of W's loads beside the FP32 pipe
+// (62 to 70 %); a lane takes two items per round, which halve those reads, and four units in flight
+// at large K, where W exceeds the L1.  16384 energies, one item a round / now: N = 64, M = 128 238 /
+// 209 us; N = 75, M = 150 366 / 324; N = 100, M = 400 1061 / 1002; N = 140, M = 576 2057 / 1867; 512
+// of them 37 / 25, 76 / 37, 154 / 80, 264 / 127.  Two configurations a warp, sharing the loads of W
+// instead, took 225, 336, 1129 and 2330, and half as long again at 512.
 // ---------------------------------------------------------------------------
 template <int K, int NW>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock) rbm_eloc_t_kernel(RbmDev P, OpDev op, EstLaunch L) {
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, K >= 18 ? 4 : (K >= 13 ? 5 : 7)) rbm_eloc_t_kernel(RbmDev P, OpDev op, EstLaunch L) {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const long t = static_cast<long>(blockIdx.x) * kWarpsPerBlock + wib;
     if (t >= L.count) return;
@@ -887,59 +893,110 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) rbm_eloc_t_kernel(RbmDev 
     }
     const int items = 4 * op.num_offdiag;
     const int N = P.N;
-    for (int it0 = 0; it0 < items; it0 += 32) {
-        const int it = it0 + lane;
-        const bool live = it < items;
-        const int n = live ? op.offdiag[it >> 2] : 0;
-        const int q = it & 3;
+    // rounds of 64 items, a lane's two 32 apart: they share the loads of theta and f
+    for (int it0 = 0; it0 < items; it0 += 64) {
+        const int q = lane & 3;
+        const bool two = it0 + 32 < items;   // for the whole warp
+        bool live[2];
+        int n[2], nf[2], off[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int it = it0 + 32 * h + lane;
+            live[h] = it < items;
+            n[h] = op.offdiag[live[h] ? it >> 2 : 0];
+            nf[h] = op.nflip[n[h]];
+            off[h] = op.flip_off[n[h]];
+        }
         // sums of the real and imaginary differences on pairs (units j, j + 4)
-        pair_t sr = splat2(0.0f), si = sr;
-        if (live) {
-            const int nf = op.nflip[n];
-            const int off = op.flip_off[n];
-            // pairs p = q, q + 4, ...: units (j, j + 4), j = q, q + 8, ...
-            if (nf == 1) {
-                const int site = op.flip_sites[off];
-                const pair_t two_s = splat2(s.up(site) ? -2.0f : 2.0f);
-                const float4* wcol = P.Wt4 + site;
+        pair_t sr[2], si[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) sr[h] = si[h] = splat2(0.0f);
+        auto unit = [&](int h, float4 f, pair_t xr, pair_t xi) {
+            const Pair2 g = lc_c2_approx(xr, xi);
+            sr[h] = add2(sr[h], sub2(g.re, pk2(f.x, f.y)));
+            si[h] = add2(si[h], sub2(g.im, pk2(f.z, f.w)));
+        };
+        // pairs p = q, q + 4, ...: units (j, j + 4), j = q, q + 8, ...
+        if (two && __all_sync(0xffffffffu, nf[0] == 1 && nf[1] == 1)) {
+            const int s0 = op.flip_sites[off[0]], s1 = op.flip_sites[off[1]];
+            const pair_t t0 = splat2(s.up(s0) ? -2.0f : 2.0f), t1 = splat2(s.up(s1) ? -2.0f : 2.0f);
+            const float4* w0 = P.Wt4 + s0;
+            const float4* w1 = P.Wt4 + s1;
+#pragma unroll (K >= 13 ? 4 : 2)
+            for (int p = q; p < MP / 2; p += 4) {
+                const float4 wa = __ldg(w0 + static_cast<long>(p) * N), wb = __ldg(w1 + static_cast<long>(p) * N);
+                const float4 a = tA[p], f = tB[p];
+                unit(0, f, fma2(t0, pk2(wa.x, wa.y), pk2(a.x, a.y)), fma2(t0, pk2(wa.z, wa.w), pk2(a.z, a.w)));
+                unit(1, f, fma2(t1, pk2(wb.x, wb.y), pk2(a.x, a.y)), fma2(t1, pk2(wb.z, wb.w), pk2(a.z, a.w)));
+            }
+        } else {
+            for (int h = 0; h < (two ? 2 : 1); h++) {
+                const int nfh = h ? nf[1] : nf[0], offh = h ? off[1] : off[0];
+                pair_t r = splat2(0.0f), i = r;
+                if (nfh == 1) {
+                    const int site = op.flip_sites[offh];
+                    const pair_t two_s = splat2(s.up(site) ? -2.0f : 2.0f);
+                    const float4* wcol = P.Wt4 + site;
 #pragma unroll 2
-                for (int p = q; p < MP / 2; p += 4) {
-                    const float4 w = __ldg(wcol + static_cast<long>(p) * N);
-                    const float4 a = tA[p], f = tB[p];
-                    const Pair2 g = lc_c2_approx(fma2(two_s, pk2(w.x, w.y), pk2(a.x, a.y)),
-                                                 fma2(two_s, pk2(w.z, w.w), pk2(a.z, a.w)));
-                    sr = add2(sr, sub2(g.re, pk2(f.x, f.y)));
-                    si = add2(si, sub2(g.im, pk2(f.z, f.w)));
-                }
-            } else {
-                for (int p = q; p < MP / 2; p += 4) {
-                    const float4 a = tA[p], f = tB[p];
-                    pair_t xr = pk2(a.x, a.y), xi = pk2(a.z, a.w);
-                    for (int u = 0; u < nf; u++) {
-                        const int site = op.flip_sites[off + u];
-                        const pair_t two_s = splat2(s.up(site) ? -2.0f : 2.0f);
-                        const float4 w = __ldg(P.Wt4 + static_cast<long>(p) * N + site);
-                        xr = fma2(two_s, pk2(w.x, w.y), xr);
-                        xi = fma2(two_s, pk2(w.z, w.w), xi);
+                    for (int p = q; p < MP / 2; p += 4) {
+                        const float4 w = __ldg(wcol + static_cast<long>(p) * N);
+                        const float4 a = tA[p], f = tB[p];
+                        const Pair2 g = lc_c2_approx(fma2(two_s, pk2(w.x, w.y), pk2(a.x, a.y)),
+                                                     fma2(two_s, pk2(w.z, w.w), pk2(a.z, a.w)));
+                        r = add2(r, sub2(g.re, pk2(f.x, f.y)));
+                        i = add2(i, sub2(g.im, pk2(f.z, f.w)));
                     }
-                    const Pair2 g = lc_c2_approx(xr, xi);
-                    sr = add2(sr, sub2(g.re, pk2(f.x, f.y)));
-                    si = add2(si, sub2(g.im, pk2(f.z, f.w)));
+                } else {
+                    for (int p = q; p < MP / 2; p += 4) {
+                        const float4 a = tA[p], f = tB[p];
+                        pair_t xr = pk2(a.x, a.y), xi = pk2(a.z, a.w);
+                        for (int u = 0; u < nfh; u++) {
+                            const int site = op.flip_sites[offh + u];
+                            const pair_t two_s = splat2(s.up(site) ? -2.0f : 2.0f);
+                            const float4 w = __ldg(P.Wt4 + static_cast<long>(p) * N + site);
+                            xr = fma2(two_s, pk2(w.x, w.y), xr);
+                            xi = fma2(two_s, pk2(w.z, w.w), xi);
+                        }
+                        const Pair2 g = lc_c2_approx(xr, xi);
+                        r = add2(r, sub2(g.re, pk2(f.x, f.y)));
+                        i = add2(i, sub2(g.im, pk2(f.z, f.w)));
+                    }
+                }
+                if (h) {
+                    sr[1] = r;
+                    si[1] = i;
+                } else {
+                    sr[0] = r;
+                    si[0] = i;
                 }
             }
         }
-        float r0, r1, i0, i1;
-        up2(sr, r0, r1);
-        up2(si, i0, i1);
-        float dx = r0 + r1, dy = i0 + i1;
-        // the four quarters of a string are lanes 4m .. 4m + 3
-        dx += __shfl_xor_sync(0xffffffffu, dx, 1);
-        dy += __shfl_xor_sync(0xffffffffu, dy, 1);
-        dx += __shfl_xor_sync(0xffffffffu, dx, 2);
-        dy += __shfl_xor_sync(0xffffffffu, dy, 2);
-        if (live && q == 0) {
-            const float2 e = string_term(string_factor(op, n, s), make_float2(dx, dy));
-            acc.add(e.x, e.y);
+        // the four quarters of a string are lanes 4m .. 4m + 3, of which lane 4m + h forms the
+        // term of item h
+        float2 d = make_float2(0.0f, 0.0f);
+        int mine = n[0];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            if (h && !two) break;
+            float r0, r1, i0, i1;
+            up2(sr[h], r0, r1);
+            up2(si[h], i0, i1);
+            float dx = r0 + r1, dy = i0 + i1;
+            dx += __shfl_xor_sync(0xffffffffu, dx, 1);
+            dy += __shfl_xor_sync(0xffffffffu, dy, 1);
+            dx += __shfl_xor_sync(0xffffffffu, dx, 2);
+            dy += __shfl_xor_sync(0xffffffffu, dy, 2);
+            if (h == 0 || q == 1) {
+                d = make_float2(dx, dy);
+                mine = n[h];
+            }
+        }
+        float2 e = make_float2(0.0f, 0.0f);
+        if (q < 2) e = string_term(string_factor(op, mine, s), d);
+        const float ex = __shfl_down_sync(0xffffffffu, e.x, 1), ey = __shfl_down_sync(0xffffffffu, e.y, 1);
+        if (q == 0) {
+            if (live[0]) acc.add(e.x, e.y);
+            if (live[1]) acc.add(ex, ey);
         }
     }
     double2 v = acc.value();
