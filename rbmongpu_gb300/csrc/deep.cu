@@ -936,7 +936,7 @@ __device__ __forceinline__ void cmac(CPair& a, float2 w, CPair b) {
     a.im = add2(a.im, fma2(wx, b.im, mul2(wy, b.re)));
 }
 __device__ __forceinline__ CPair cmul(CPair a, CPair b) {
-    const pair_t nay = mul2(splat2(-1.0f), a.im);
+    const pair_t nay = neg2(a.im);
     return CPair{fma2(a.re, b.re, mul2(nay, b.im)), fma2(a.re, b.im, mul2(a.im, b.re))};
 }
 __device__ __forceinline__ CPair act_pair(CPair z) {

@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(32 * kGvWarps) grad_vectors_kernel(GradVectors
                     if (q >= pairs) break;
                     const float2 a0 = load(g.T, 2 * q), a1 = load(g.T, 2 * q + 1);
                     const pair_t tx = pk2(a0.x, a1.x), ty = pk2(a0.y, a1.y);
-                    const pair_t nty = mul2(splat2(-1.0f), ty);
+                    const pair_t nty = neg2(ty);
                     pair_t ur = us[(2 * q) * 32], ui = us[(2 * q + 1) * 32];
                     for (int u = 0; u < nb; u++) {
                         const float4 e = stA[u * pairs + q];
@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(32 * kGvWarps) grad_vectors_kernel(GradVectors
                         const pair_t ts = pk2(b.x, b.y);
                         const Pair2 h = tanh2_approx(fma2(ts, wx, tr[v]), fma2(ts, wy, ti[v]));
                         const pair_t ex = pk2(e.x, e.y), ey = pk2(e.z, e.w);
-                        const pair_t vx = fma2(ex, h.re, mul2(splat2(-1.0f), mul2(ey, h.im)));
+                        const pair_t vx = fma2(ex, h.re, neg2(mul2(ey, h.im)));
                         const pair_t vy = ONE ? fma2(ex, h.im, mul2(ey, h.re)) : fma2(ey, h.re, mul2(ex, h.im));
                         ur[v] = add2(ur[v], vx);
                         ui[v] = add2(ui[v], vy);

@@ -344,7 +344,7 @@ __device__ __noinline__ void walker_task(const SLaunch& L, const SInst& Ig, int 
 #pragma unroll
         for (int k = 0; k < K; k++) {
             const pair_t a = REGS ? hr[REGS ? k : 0] : pk2(myt[32 * k].x, myt[32 * k].y), b = hi[k];
-            const pair_t xr = fma2(tx, a, mul2(splat2(-1.0f), mul2(ty, b)));
+            const pair_t xr = fma2(tx, a, neg2(mul2(ty, b)));
             const pair_t xi = fma2(ty, a, mul2(tx, b));
             float x0, x1, y0, y1;
             up2(xr, x0, x1);
@@ -539,7 +539,7 @@ __device__ __noinline__ void reduce_task(const SLaunch& L, const SInst& Ig, int 
                         const Pair2 h = tanh2_approx(fma2(sg, wx[q], splat2(th.x)), fma2(sg, wy[q], splat2(th.y)));
                         const float4 en = sen[q * 32 + bw];
                         const pair_t enx = pk2(en.x, en.y), eny = pk2(en.z, en.w);
-                        vx = fma2(enx, h.re, mul2(splat2(-1.0f), mul2(eny, h.im)));
+                        vx = fma2(enx, h.re, neg2(mul2(eny, h.im)));
                         vy = fma2(enx, h.im, mul2(eny, h.re));
                     }
                     if (GENERAL) {
