@@ -5,15 +5,16 @@
 // queue (one atomic counter): first the walker tasks of every instance, longest first
 // (sweeps of single-flip Metropolis, then at the final configuration the local energy,
 // tanh(theta), the angles, U_j = sum_n e_n tanh(theta''_nj) over every string and the
-// terms e_n of the off-diagonal strings), then the reduction tasks, each a tile of rows by a chunk of walkers of one instance's sums, which start once that
-// instance's walkers are all done (a per-instance counter; the wait is bounded by a
-// wall-clock limit after which the kernel raises an error flag and returns).  Each tile
-// writes its chunk's partial sums; a second kernel of the graph adds the chunks in a fixed
-// order and forms the gradient, so every replay gives the same bits.  The walker tasks are compiled
-// for each hidden-unit count per lane (rbm_lanes_k: M <= 576) as separate functions
-// of the one kernel.  The launch (counter resets + both kernels) is captured once in a
-// CUDA graph and replayed; the warps per block, the reduction tile height and a register
-// cap come from an autotuner that times the candidates on the batch itself.
+// terms e_n of the off-diagonal strings), then the reduction tasks, each a tile of rows by
+// a chunk of walkers of one instance's sums, which start once that instance's walkers are
+// all done (a per-instance counter; the wait is bounded by a wall-clock limit after which
+// the kernel raises an error flag and returns).  Each tile writes its chunk's partial sums;
+// a second kernel of the graph adds the chunks in a fixed order and forms the gradient, so
+// every replay gives the same bits.  The walker tasks are compiled for each hidden-unit
+// count per lane (rbm_lanes_k: M <= 576) as separate functions of the one kernel.  The
+// launch (counter resets + both kernels) is captured once in a CUDA graph and replayed; the
+// warps per block, the reduction tile height and a register cap come from an autotuner that
+// times the candidates on the batch itself.
 //
 // Per instance and replay the result is <E_loc> over its walkers and the reference's O_k
 // gradient <E O*> + conj<E_k> - 2 <E> <O*> (source/network_functions/ExpectationValue.cu:
@@ -21,10 +22,14 @@
 // W_ij, s_i (U_j - 2 V_ij) with V_ij = sum of e_n tanh(theta''_nj) over the strings n
 // flipping site i, recomputed in the tiles from the stored angles (storing these terms
 // per walker and string would move O(N^2 M) bytes per walker through HBM).
-// Both the measurement and the tiles are bound by FP32 arithmetic and the latency of the
-// L2 loads beside it at 8 to 16 warps per SM (the walker tasks' registers), so they take two
-// strings, or two rows, per packed operation, which leaves half of the issue slots, and the
-// tiles fetch a walker ahead: 64 instances of 16 to 144 spins, 30.7 -> 26.2 ms a replay.
+//
+// All parts are bound by FP32 arithmetic and, at the 8 to 16 warps per SM that the walker
+// tasks' registers leave, by latency: of a proposal's dependent steps (the next site is found
+// ahead, the random words wait in shared memory) and of the L2 loads beside the arithmetic
+// (the measurement and the tiles take two strings, or two rows, per packed operation, and the
+// tiles fetch a walker ahead).  64 instances of 16 to 144 spins, a replay: 30.7 ms at first,
+// 26.2 with packed measurement and tiles, 24.0 with hidden-unit counts between 2 and 13 and
+// signs off the FP32 pipe, 22.2 with the shorter proposals.
 //
 // The sums run centred on the instance's mean energy E (the same value in every tile):
 //   gO = sum conj(O),  gE = sum (E_w - E) conj(O),  gK = sum conj(E_k) - conj(E) conj(O),
@@ -146,8 +151,15 @@ __device__ __forceinline__ void s_refresh2(const SInst& I, const Spins<NW>& s, p
 
 template <int K, int KP, int NW>
 __device__ __forceinline__ bool s_mh_step2(const SInst& I, Spins<NW>& s, pair_t (&tr)[KP], pair_t (&ti)[KP],
-                                           pair_t (&re)[KP], WarpRng& rng, int lane, uint64_t nmagic) {
-    const int site = static_cast<int>(fastmod(rng.next(), nmagic, static_cast<uint32_t>(I.N)));
+                                           pair_t (&re)[KP], GroupRng<32>& rng, int& next, int lane,
+                                           uint64_t nmagic) {
+    // words: the site, the test's number and the next site, found ahead for both ways the test's
+    // number may or may not be used
+    rng.ensure(3, lane);
+    const int site = next;
+    rng.pos++;
+    const int next0 = static_cast<int>(fastmod(rng.peek(), nmagic, static_cast<uint32_t>(I.N)));
+    const int next1 = static_cast<int>(fastmod(rng.words[rng.pos + 1], nmagic, static_cast<uint32_t>(I.N)));
     Spins<NW> s2 = s;
     s2.flip(site);
     const pair_t two_s = splat2(s2.up(site) ? 2.0f : -2.0f);
@@ -169,7 +181,12 @@ __device__ __forceinline__ bool s_mh_step2(const SInst& I, Spins<NW>& s, pair_t 
     }
     const float delta = warp_sum_xor(part);
     bool accept = delta > 0.0f;
-    if (!accept) accept = rng.uniform() <= expf_det(__fmul_rn(2.0f, delta));
+    next = accept ? next0 : next1;
+    if (!accept) {
+        const float u = __fmul_rn(static_cast<float>((rng.peek() >> 8) + 1u), 5.9604644775390625e-8f);
+        rng.pos++;
+        accept = u <= expf_det(__fmul_rn(2.0f, delta));
+    }
     if (accept) {
         s = s2;
 #pragma unroll
@@ -190,8 +207,11 @@ template <int K>
 __device__ __noinline__ void walker_task(const SLaunch& L, const SInst& Ig, int w, int lane) {
     constexpr int NW = kSW;
     const SInst I = Ig;   // the descriptor in registers / local memory, not re-read from global
-    WarpRng rng;
-    rng.init(I.seed, static_cast<uint32_t>(w), I.rng_index[w], lane);
+    // the random words sit in this warp's slice of shared memory, which the measurement uses later
+    extern __shared__ float2 s_f[];
+    GroupRng<32> rng;
+    rng.init(I.seed, static_cast<uint32_t>(w), I.rng_index[w],
+             reinterpret_cast<uint4*>(s_f + (threadIdx.x >> 5) * 3 * kSK * 32), lane);
     const uint64_t nmagic = fastmod_magic(static_cast<uint32_t>(I.N));
     Spins<NW> s;
 #pragma unroll
@@ -201,8 +221,9 @@ __device__ __noinline__ void walker_task(const SLaunch& L, const SInst& Ig, int 
 #pragma unroll
         for (int k = 0; k < NW; k++)
             if (k < I.nw) {
-                const uint64_t lo = rng.next();
-                const uint64_t hi = rng.next();
+                rng.ensure(2, lane);
+                const uint64_t lo = rng.peek(), hi = rng.words[rng.pos + 1];
+                rng.pos += 2;
                 s.w[k] = lo | (hi << 32);
             }
 #pragma unroll
@@ -218,11 +239,13 @@ __device__ __noinline__ void walker_task(const SLaunch& L, const SInst& Ig, int 
         constexpr int KP = (K + 1) / 2;
         pair_t tp[KP], tq[KP], rp[KP];
         const int total = (L.first ? L.therm : 0) + L.sweeps;
+        rng.ensure(3, lane);
+        int next = static_cast<int>(fastmod(rng.peek(), nmagic, static_cast<uint32_t>(I.N)));
         for (int sw = 0; sw < total; sw++) {
             s_refresh2(I, s, tp, tq, lane);
 #pragma unroll
             for (int kk = 0; kk < KP; kk++) rp[kk] = lc_re2(tp[kk], tq[kk]);
-            for (int p = 0; p < I.N; p++) acc += s_mh_step2<K>(I, s, tp, tq, rp, rng, lane, nmagic);
+            for (int p = 0; p < I.N; p++) acc += s_mh_step2<K>(I, s, tp, tq, rp, rng, next, lane, nmagic);
         }
     }
     // measurement at the final configuration: the local energy, tanh(theta), and for the
@@ -237,7 +260,7 @@ __device__ __noinline__ void walker_task(const SLaunch& L, const SInst& Ig, int 
     constexpr bool REGS = K <= 8;
     float tr[K], ti[K];
     s_refresh(I, s, tr, ti, lane);
-    extern __shared__ float2 s_f[];
+    __syncwarp();   // the random words have been read
     float2* myf = s_f + (threadIdx.x >> 5) * 3 * kSK * 32 + lane;
     float2* myt = myf + kSK * 32;
     float2* myu = myt + kSK * 32;
@@ -373,7 +396,7 @@ __device__ __noinline__ void walker_task(const SLaunch& L, const SInst& Ig, int 
 #pragma unroll
         for (int k = 0; k < NW; k++)
             if (k < I.nw) I.spins[static_cast<long>(w) * I.nw + k] = s.w[k];
-        I.rng_index[w] = rng.index;
+        I.rng_index[w] = rng.index();
         I.eloc[w] = e.value();
         atomicAdd(L.accepts, acc);
     }
