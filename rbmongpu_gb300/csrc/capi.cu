@@ -667,6 +667,7 @@ namespace rbmg {
 // per-sample weights (null = equal weights) and, for MC, the sampler's log psi / E_loc.
 struct Chunk {
     int count = 0;
+    int group = 0;   // StreamResult::batch: the samples of a chunk of the plain size
     const uint64_t* spins = nullptr;
     int enumerate = 0;
     uint64_t enum_base = 0;
@@ -679,6 +680,11 @@ struct StreamResult {
     // factor in Workspace::stat, and a Monte-Carlo pass leaves its counts on their way, for
     // stream_done after the caller's own wait
     bool defer = false;
+    // chunks of several plain ones, up to so many samples, for a pass that sums within the plain
+    // chunks' 32-sample groups (0: plain chunks)
+    size_t batch = 0;
+    // plain chunks of n samples in one: only whole 32-sample groups join
+    int chunks_in_one(int n) const { return n % 32 ? 1 : std::max(1, static_cast<int>(batch / n)); }
     double norm_factor = 1.0;   // reference weight scale: sum_s prefactor^2 |psi|^2 (exact) or 1/num_samples (MC)
     double log_norm = 0.0;      // log of sum_s prefactor^2 |psi|^2 (exact)
 };
@@ -716,7 +722,7 @@ constexpr const char* kNonFiniteLogPsi = "ExactSummation: non-finite log psi";
 // MonteCarloLoop::foreach (include/spin_ensembles/MonteCarloLoop.hpp:294-339): every call
 // re-draws the start configurations and thermalises; the chains' Philox streams continue.
 static int mc_stream(rbmg_ensemble* e, const rbmg_psi* psi, const rbmg_operator* op, bool want_eloc,
-                     size_t max_chunk_samples, bool defer, const std::function<int(const Chunk&)>& fn) {
+                     size_t max_chunk_samples, const StreamResult& res, const std::function<int(const Chunk&)>& fn) {
     if (psi->kind != 0) return fail(RBMG_EUNSUPPORTED, "MonteCarloLoop: PsiDeep / PsiPair chains are sampled by deep.cu");
     if (e->fast_sweep_tries && e->total_z)
         return fail(RBMG_EUNSUPPORTED, "fast sweep with total_z symmetry (the reference pairs a mask with an unset site)");
@@ -729,7 +735,8 @@ static int mc_stream(rbmg_ensemble* e, const rbmg_psi* psi, const rbmg_operator*
     RBMG_CK(cudaMemsetAsync(e->accepts.p, 0, sizeof(unsigned long long) * B, stream()));
     RBMG_CK(cudaMemsetAsync(e->proposals.p, 0, sizeof(unsigned long long) * B, stream()));
     Workspace& W = ws();
-    const int rows_per_chunk = static_cast<int>(std::max<size_t>(1, std::min<size_t>(steps, max_chunk_samples / B)));
+    const int group_rows = static_cast<int>(std::max<size_t>(1, std::min<size_t>(steps, max_chunk_samples / B)));
+    const int rows_per_chunk = static_cast<int>(std::min<int64_t>(steps, int64_t(group_rows) * res.chunks_in_one(group_rows * B)));
     RBMG_CK(W.sample_spins.ensure(sizeof(uint64_t) * nw * B * rows_per_chunk));
     if (want_eloc) RBMG_CK(W.eloc.ensure(sizeof(double2) * B * rows_per_chunk));
     OpDev od;
@@ -758,6 +765,7 @@ static int mc_stream(rbmg_ensemble* e, const rbmg_psi* psi, const rbmg_operator*
         first = false;
         Chunk c;
         c.count = rows * B;
+        c.group = group_rows * B;
         c.spins = W.sample_spins.as<uint64_t>();
         if (want_eloc && op) {
             EstLaunch E{};
@@ -772,7 +780,7 @@ static int mc_stream(rbmg_ensemble* e, const rbmg_psi* psi, const rbmg_operator*
         if (r != RBMG_OK) return r;
     }
     RBMG_CK(e->counts_copy());
-    if (defer) return RBMG_OK;
+    if (res.defer) return RBMG_OK;
     RBMG_CK(cudaStreamSynchronize(stream()));
     e->counts_take();
     return RBMG_OK;
@@ -805,6 +813,7 @@ static int exact_stream(rbmg_ensemble* e, const rbmg_psi* psi, StreamResult* res
     for (uint64_t base = 0; base < total; base += kExactChunk) {
         Chunk c;
         c.count = static_cast<int>(std::min<uint64_t>(kExactChunk, total - base));
+        c.group = c.count;
         c.enumerate = enumerate;
         c.enum_base = base;
         c.spins = sp ? sp + base : nullptr;
@@ -932,9 +941,11 @@ static int fixed_stream(rbmg_ensemble* e, const rbmg_psi* psi, size_t max_chunk,
     if (static_cast<int>(e->num_spins) != psi->N) return fail(RBMG_EINVAL, "fixed samples: N does not match psi");
     const uint64_t total = e->num_steps();
     res->norm_factor = 1.0 / static_cast<double>(total);
-    const uint64_t per = std::max<uint64_t>(1, max_chunk);
+    const uint64_t group = std::min<uint64_t>(total, std::max<uint64_t>(1, max_chunk));
+    const uint64_t per = group * res->chunks_in_one(static_cast<int>(group));
     for (uint64_t base = 0; base < total; base += per) {
         Chunk c;
+        c.group = static_cast<int>(group);
         c.count = static_cast<int>(std::min<uint64_t>(per, total - base));
         c.spins = e->d_allowed.as<uint64_t>() + base * e->spins_words;
         const int r = fn(c);
@@ -949,7 +960,7 @@ static int run_stream(rbmg_ensemble* ens, const rbmg_psi* psi, const rbmg_operat
     if (ens->kind == 2) return fixed_stream(ens, psi, max_chunk, res, fn);
     res->norm_factor = 1.0 / static_cast<double>(ens->num_samples);
     if (psi->kind != 0) return deep_stream(ens, psi, op, sampler_eloc, max_chunk, res->defer, fn);
-    return mc_stream(ens, psi, op, sampler_eloc, max_chunk, res->defer, fn);
+    return mc_stream(ens, psi, op, sampler_eloc, max_chunk, *res, fn);
 }
 
 // <E> and <|E|^2> with reference weights
@@ -1212,14 +1223,29 @@ static int ev_gradient_sums(const rbmg_psi* psi, const rbmg_operator* op, rbmg_e
     RBMG_CK(W.sums.ensure(sizeof(double2) * kMaxSeries));
     RBMG_CK(sum_scratch(W));
     RBMG_CK(cudaMemsetAsync(W.sums.p, 0, sizeof(double2) * kMaxSeries, stream()));
-    constexpr int kSplits = 64;
+    constexpr int kSplits = 64, kBatchSplits = 152;   // of a plain chunk, and of several at a time
+    int dev = 0, sms = 0;
+    RBMG_CK(cudaGetDevice(&dev));
+    RBMG_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    // a transverse field (each string one site's own): the strings' terms e_n are formed
+    // first, then U and the V sums from the stored angles; otherwise e_n tanh(theta''_n)
+    // of every string and sample is stored.  The fluctuation gradient's second V sum has
+    // the stored form only
+    bool single = false;
     size_t per_sample = 0;
     if (psi->kind == 0) {
         r = op_site_lists(const_cast<rbmg_operator*>(op), N);
         if (r != RBMG_OK) return r;
-        per_sample = sizeof(float2) * psi->Mpad * (2 + op->num_offdiag) + 64;
+        single = op->single_flips && !fluct;
+        per_sample = sizeof(float2) * rbm_range_top(psi->M) * (2 + op->num_offdiag) + 64;
+        // a transverse field stores no string's terms per unit: its chunks of that size go several
+        // at a time, which keeps the chip's last wave full and launches once for all (81920 samples
+        // at N = 64, M = 128 in chunks of 4096, 20 times nine launches: 10.5 ms
+        // with the sweeps, now 8.4)
+        if (single)
+            res->batch = (size_t(512) << 20) / (sizeof(float2) * (3 * psi->Mpad + op->num_offdiag) + 64);
         // of the sums over T, and of those over U
-        RBMG_CK(W.partial.ensure(sizeof(double2) * ((adjoint ? 3 : 2) + (fluct ? 2 : 1)) * kSplits * (1 + N) * psi->M));
+        RBMG_CK(W.partial.ensure(sizeof(double2) * ((adjoint ? 3 : 2) + (fluct ? 2 : 1)) * kBatchSplits * (1 + N) * psi->M));
     }
     const size_t max_chunk = psi->kind == 0 ? std::max<size_t>(256, (size_t(512) << 20) / per_sample) : 4096;
     // The sums are centred on E0, the mean local energy of the first chunk:
@@ -1251,20 +1277,17 @@ static int ev_gradient_sums(const rbmg_psi* psi, const rbmg_operator* op, rbmg_e
         } else {
             const OpDev od = op->dev();
             if (!have_shift) {
+                Chunk c0 = c;
+                c0.count = std::min(c.count, c.group);
                 const double2* e0 = nullptr;
-                const int rr0 = chunk_eloc(psi, op, c, &e0);
+                const int rr0 = chunk_eloc(psi, op, c0, &e0);
                 if (rr0 != RBMG_OK) return rr0;
-                const int rr1 = chunk_mean(c, e0, nullptr);
+                const int rr1 = chunk_mean(c0, e0, nullptr);
                 if (rr1 != RBMG_OK) return rr1;
                 have_shift = true;
             }
             RBMG_CK(W.T.ensure(sizeof(float2) * c.count * psi->Mpad));
             RBMG_CK(W.U.ensure(sizeof(float2) * c.count * psi->Mpad));
-            // a transverse field (each string one site's own): the strings' terms e_n are formed
-            // first, then U and the V sums from the stored angles; otherwise e_n tanh(theta''_n)
-            // of every string and sample is stored.  The fluctuation gradient's second V sum has
-            // the stored form only
-            const bool single = op->single_flips && !fluct;
             EstLaunch L{};
             if (single) {
                 RBMG_CK(W.theta.ensure(sizeof(float2) * c.count * psi->Mpad));
@@ -1292,9 +1315,11 @@ static int ev_gradient_sums(const rbmg_psi* psi, const rbmg_operator* op, rbmg_e
                                       fluct ? 1 : 0, stream()));
             SplitSum jobs[2] = {};   // the sums over T, and over U (with the V sums of a transverse field)
             if (single) {
-                RBMG_CK(W.vpart.ensure(grad_vectors_bytes(c.count, N, psi->M, kSplits)));
+                RBMG_CK(W.vpart.ensure(grad_vectors_bytes(c.count, c.group, N, psi->M, psi->Mpad, kSplits, sms)));
                 GradVectors G{};
                 G.count = c.count;
+                G.group = c.group;
+                G.max_splits = kSplits;
                 G.N = N;
                 G.nw = nw;
                 G.M = psi->M;
@@ -1310,9 +1335,10 @@ static int ev_gradient_sums(const rbmg_psi* psi, const rbmg_operator* op, rbmg_e
                 G.U = W.U.as<float2>();
                 G.e_shift = e0_dev;
                 G.site_ptr = op->d_site_ptr.as<int>();
-                RBMG_CK(launch_grad_vectors(G, od, W.vpart.as<double2>(), kSplits, stream(), &jobs[1]));
+                RBMG_CK(launch_grad_vectors(G, od, W.vpart.as<double2>(), sms, stream(), &jobs[1]));
             }
             double2* part = W.partial.as<double2>();
+            const int splits = c.count > c.group ? kBatchSplits : kSplits;
             // the sums over T, together: O, and (E - E0) O* or, for the adjoint, C2 and C3
             OuterSet sums_t{}, sums_u{};
             sums_t.add(W.coef1.as<double2>(), 0, W.acc_O.as<double2>());
@@ -1323,12 +1349,12 @@ static int ev_gradient_sums(const rbmg_psi* psi, const rbmg_operator* op, rbmg_e
                 sums_t.add(W.coef2.as<double2>(), 1, W.acc_EO.as<double2>());
             }
             RBMG_CK(launch_outer_reduce(c.count, N, nw, psi->M, c.spins, c.enum_base, c.enumerate, sums_t,
-                                        W.T.as<float2>(), psi->Mpad, part, kSplits, stream(), &jobs[0]));
+                                        W.T.as<float2>(), psi->Mpad, part, splits, stream(), &jobs[0]));
             sums_u.add(W.coef1.as<double2>(), 0, W.acc_Ek.as<double2>());
             if (fluct) sums_u.add(W.coef3.as<double2>(), 0, W.acc_B.as<double2>());
             RBMG_CK(launch_outer_reduce(c.count, N, nw, psi->M, c.spins, c.enum_base, c.enumerate, sums_u,
                                         W.U.as<float2>(), psi->Mpad,
-                                        part + static_cast<size_t>(sums_t.n) * kSplits * (1 + N) * psi->M, kSplits,
+                                        part + static_cast<size_t>(sums_t.n) * splits * (1 + N) * psi->M, splits,
                                         stream(), &jobs[1]));
             RBMG_CK(launch_split_sums(jobs, 2, !first, stream()));
             first = false;
@@ -1796,7 +1822,7 @@ extern "C" int rbmg_hsd_gradient(const rbmg_psi* psi, const rbmg_psi* pp, const 
         const int enumerate = (enumerated && !ens->exact_total_z) ? 1 : 0;
         if (pp->kind == 0) {
             RBMG_CK(W.partial.ensure(sizeof(double2) * kSplits * (1 + N) * pp->M));
-            const int chunk = std::max(1024, static_cast<int>((size_t(256) << 20) / (sizeof(float2) * pp->Mpad)));
+            const int chunk = std::max(1024, static_cast<int>((size_t(256) << 20) / (sizeof(float2) * pp->Mpad)) / 32 * 32);
             RBMG_CK(W.T.ensure(sizeof(float2) * std::min(chunk, count) * pp->Mpad));
             RBMG_CK(W.logpsi.ensure(sizeof(double2) * std::min(chunk, count)));
             const RbmDev pd = pp->rbm_dev();
@@ -1930,7 +1956,7 @@ extern "C" int rbmg_kl_gradient(const rbmg_psi* psi, const rbmg_psi* pp, rbmg_en
     if (pp->kind == 0) {
         constexpr int kSplits = 64;
         RBMG_CK(W.partial.ensure(sizeof(double2) * kSplits * (1 + N) * pp->M));
-        const int chunk = std::max(1024, static_cast<int>((size_t(256) << 20) / (sizeof(float2) * pp->Mpad)));
+        const int chunk = std::max(1024, static_cast<int>((size_t(256) << 20) / (sizeof(float2) * pp->Mpad)) / 32 * 32);
         RBMG_CK(W.T.ensure(sizeof(float2) * std::min(chunk, count) * pp->Mpad));
         RBMG_CK(W.logpsi_p.ensure(sizeof(double2) * std::min(chunk, count)));
         const RbmDev pd = pp->rbm_dev();

@@ -140,6 +140,9 @@ cudaError_t launch_rbm_mc(const RbmDev& psi, const OpDev* op, const McLaunch& L,
 cudaError_t launch_rbm_estimate(const RbmDev& psi, const OpDev* op, const RbmDev* psi_prime, const EstLaunch& L,
                                 cudaStream_t st);
 
+// the largest number of units of M's range: what sizes the chunks that samples are summed in, and
+// what two networks of one pass share
+int rbm_range_top(int M);
 bool rbm_pairable(int Ma, int Mb);
 int rbm_lanes_k(int M);   // instantiated hidden units per lane for M, -1 if too large
 

@@ -23,15 +23,12 @@ int rbm_lanes_k(int M) {
     return -1;
 }
 
-// two networks of one pass have their units in the same of these ranges
-bool rbm_pairable(int Ma, int Mb) {
-    auto range = [](int M) {
-        int r = 0;
-        for (int top : {32, 64, 128, 256, 416, 576}) r += M > top;
-        return r;
-    };
-    return range(Ma) == range(Mb);
+int rbm_range_top(int M) {
+    for (int top : {32, 64, 128, 256, 416})
+        if (M <= top) return top;
+    return 576;
 }
+bool rbm_pairable(int Ma, int Mb) { return rbm_range_top(Ma) == rbm_range_top(Mb); }
 
 cudaError_t launch_rbm_mc(const RbmDev& P, const OpDev* op, const McLaunch& L, cudaStream_t st) {
     switch (P.Mpad / 32) {

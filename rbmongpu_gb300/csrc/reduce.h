@@ -61,6 +61,8 @@ cudaError_t launch_vterm_reduce(int count, int N, int nw, int M, int Mpad, const
 // [count][num_offdiag] and the angles `theta` [count][Mpad]; partial: grad_vectors_bytes
 struct GradVectors {
     int count, N, nw, M, Mpad;
+    int group;            // the samples come in groups of so many, the FP32 sums formed within each
+    int max_splits;       // over at most so many splits of a group
     const uint64_t* spins;
     uint64_t enum_base;
     int enumerate;
@@ -73,10 +75,10 @@ struct GradVectors {
     const double2* e_shift;   // U is stored as U - e_shift T
     const int* site_ptr;  // [N + 1]
 };
-size_t grad_vectors_bytes(int count, int N, int M, int max_splits);
+size_t grad_vectors_bytes(int count, int group, int N, int M, int Mpad, int max_splits, int sms);
 // the V sums' partials are left in job's pre
-cudaError_t launch_grad_vectors(const GradVectors& g, const OpDev& op, double2* partial, int max_splits,
-                                cudaStream_t st, SplitSum* job);
+cudaError_t launch_grad_vectors(const GradVectors& g, const OpDev& op, double2* partial, int sms, cudaStream_t st,
+                                SplitSum* job);
 // sums[q] += sum_s w[s] v_q[s]; block_scratch: kSumScratch double2
 cudaError_t launch_weighted_sums(int count, const double* w, const SeriesSet& set, double2* block_scratch,
                                  double2* sums, cudaStream_t st);

@@ -4,6 +4,8 @@
 // most 32 samples, accumulated in FP64, then per-block partials combined by a
 // second kernel in block order.  No floating-point atomics, so results are
 // bit-reproducible run to run.
+#include <algorithm>
+
 #include "device_math.cuh"
 #include "kernels.h"
 #include "reduce.h"
@@ -220,20 +222,35 @@ __global__ void vterm_kernel(int count, int N, int nw, int M, int Mpad, const ui
 // tanh(theta'') is evaluated again here instead of being stored by the pass that forms the e_n:
 // per sample and string that is a second activation of every unit against 16 bytes written and
 // read (268 MB a 4096-sample chunk at N = 64, M = 128).
-// Warp q of the block takes samples z per_split + q + 8 k of split z (k < 32 of chunk c), its
-// lanes 32 hidden units: vterm_kernel's FP32 groups, summed in its order.  The strings go by
-// eight in the operator's order, so that every U_j is the same ordered sum; a block's terms and
+// A unit of work is chunk c of split z of a group: warp q takes samples z per_split + q + 8 k
+// (k < 32 of the chunk), its lanes 32 hidden units: vterm_kernel's FP32 sums, one by one in its
+// order, added up in FP64 over the block's warps and units.  The strings go by eight in the
+// operator's order, so that every U_j is the same ordered sum; a block's terms and
 // signs are staged in shared memory, two samples side by side for the packed operations.  A
 // thread holds eight V sums; its samples' U are in shared memory between blocks of strings.
-// Bound by the FP32 pipe (57 lane operations per sample, string and unit; 42 % busy) and the
-// latency of the staging: 178 us a chunk, against 354 us of vterm_kernel on stored terms.
-constexpr int kGvStrings = 8, kGvTile = 8, kGvWarps = 8;
+// Bound by the FP32 pipe (57 lane operations per sample, string and unit; half of its cycles) and
+// the latency of its reads of shared memory: four samples in flight and three blocks an SM walking
+// the units, 2.57 ms for 81920 samples at N = 64, M = 128; eight samples and two blocks 2.85, and
+// with a launch and 256 blocks per 4096 samples, which left a sixth of the SMs' places empty, 3.6;
+// vterm_kernel on stored terms 7.1.
+constexpr int kGvStrings = 8, kGvTile = 4, kGvWarps = 8;
+
+// vterm_kernel's split of a group's samples, and chunks of 32 samples a warp
+__host__ __device__ inline void grad_vectors_shape(int count, int max_splits, int* per_split, int* splits, int* chunks,
+                                                   int* cap) {
+    const int even = (count + max_splits - 1) / max_splits;
+    *per_split = even > 64 ? even : 64;
+    *splits = (count + *per_split - 1) / *per_split;
+    const int per_warp = (*per_split + 7) / 8, two = (per_warp + 1) / 2 * 2;
+    *chunks = (per_warp + 31) / 32;
+    *cap = two < 32 ? two : 32;
+}
 
 // ONE: a lane of the general pass holds one hidden unit (Mpad = 32); its compiled form joins the
 // other product of Im(e tanh) into an FMA than with more units, and so does this one.
 template <bool ONE>
-__global__ void __launch_bounds__(32 * kGvWarps) grad_vectors_kernel(GradVectors g, OpDev op, int per_split,
-                                                                     int chunks, int cap, double2* partial) {
+__global__ void __launch_bounds__(32 * kGvWarps, 3) grad_vectors_kernel(GradVectors g, OpDev op, int per_group,
+                                                                     int units, int cap, double2* partial) {
     extern __shared__ __align__(16) unsigned char gv_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int pairs = cap / 2;
@@ -243,12 +260,19 @@ __global__ void __launch_bounds__(32 * kGvWarps) grad_vectors_kernel(GradVectors
     float2* red = reinterpret_cast<float2*>(reinterpret_cast<float4*>(gv_smem) + kGvWarps * 2 * kGvStrings * pairs);
     pair_t* us = reinterpret_cast<pair_t*>(red + kGvStrings * kGvWarps * 32) + warp * 2 * pairs * 32 + lane;
     const int j = blockIdx.x * 32 + lane;
-    const int z = blockIdx.y / chunks, c = blockIdx.y - z * chunks;
-    const int s_end = min(g.count, (z + 1) * per_split);
-    const int s0 = z * per_split + warp + 8 * 32 * c;
+    const int nw = g.nw;
+    double2* out = partial + static_cast<long>(blockIdx.y) * (1 + g.N) * g.M;
+    for (int i = warp; i <= g.N; i += kGvWarps)   // the rows no string writes
+        if (j < g.M && (i == 0 || g.site_ptr[i - 1] == g.site_ptr[i])) out[static_cast<long>(i) * g.M + j] = make_double2(0.0, 0.0);
+    for (int unit = blockIdx.y; unit < units; unit += gridDim.y) {
+    const int group0 = unit / per_group * g.group, in_group = min(g.group, g.count - group0);
+    int per_split, splits, chunks, cap_g;
+    grad_vectors_shape(in_group, g.max_splits, &per_split, &splits, &chunks, &cap_g);
+    const int z = unit % per_group / chunks, c = unit % per_group - z * chunks;
+    const int s_end = group0 + min(in_group, (z + 1) * per_split);
+    const int s0 = group0 + z * per_split + warp + 8 * 32 * c;
     const int cnt = s0 < s_end ? min(32, (s_end - s0 + 7) / 8) : 0;   // sample k of the warp: s0 + 8 k
     for (int q = 0; q < pairs; q++) us[(2 * q) * 32] = us[(2 * q + 1) * 32] = splat2(0.0f);
-    const int nw = g.nw;
     auto word = [&](int s, int k) -> uint64_t {
         if (!g.enumerate) return k < nw ? g.spins[static_cast<long>(s) * nw + k] : 0ull;
         if (k != 0) return 0ull;
@@ -258,9 +282,6 @@ __global__ void __launch_bounds__(32 * kGvWarps) grad_vectors_kernel(GradVectors
     auto load = [&](const float2* a, int k) {
         return k < cnt ? a[static_cast<long>(s0 + 8 * k) * g.Mpad + j] : make_float2(0.0f, 0.0f);
     };
-    double2* out = partial + static_cast<long>(blockIdx.y) * (1 + g.N) * g.M;
-    for (int i = warp; i <= g.N; i += kGvWarps)   // the rows no string writes
-        if (j < g.M && (i == 0 || g.site_ptr[i - 1] == g.site_ptr[i])) out[static_cast<long>(i) * g.M + j] = make_double2(0.0, 0.0);
     for (int n0 = 0; n0 < op.S;) {
         // up to eight consecutive strings of one kind
         const bool diag = op.nflip[n0] == 0;
@@ -385,7 +406,12 @@ __global__ void __launch_bounds__(32 * kGvWarps) grad_vectors_kernel(GradVectors
                     t.y += v.y;
                 }
                 const int site = op.flip_sites[op.flip_off[n0 + warp]];
-                out[static_cast<long>(1 + site) * g.M + j] = t;
+                double2* o = out + static_cast<long>(1 + site) * g.M + j;
+                if (unit != blockIdx.y) {   // the block's earlier units
+                    t.x += o->x;
+                    t.y += o->y;
+                }
+                *o = t;
             }
         }
         n0 += nb;
@@ -400,6 +426,7 @@ __global__ void __launch_bounds__(32 * kGvWarps) grad_vectors_kernel(GradVectors
         u.x -= __fmaf_rn(shx, t.x, -__fmul_rn(shy, t.y));
         u.y -= __fmaf_rn(shx, t.y, __fmul_rn(shy, t.x));
         g.U[static_cast<long>(s0 + 8 * k) * g.Mpad + j] = u;
+    }
     }
 }
 
@@ -753,38 +780,37 @@ cudaError_t launch_vterm_reduce(int count, int N, int nw, int M, int Mpad, const
     return launch_split_sums(&job, 1, true, st);
 }
 
-// vterm_kernel's split of the samples, and chunks of 32 samples a warp
-static void grad_vectors_shape(int count, int max_splits, int* per_split, int* splits, int* chunks, int* cap) {
-    *per_split = max(64, (count + max_splits - 1) / max_splits);
-    *splits = (count + *per_split - 1) / *per_split;
-    const int per_warp = (*per_split + 7) / 8;
-    *chunks = (per_warp + 31) / 32;
-    *cap = min(32, (per_warp + 1) / 2 * 2);
-}
-
-size_t grad_vectors_bytes(int count, int N, int M, int max_splits) {
+// the blocks of a column of 32 hidden units walk its units of work, three blocks an SM in all
+struct GradVectorsShape {
+    int per_group, units, rows, cap;   // units of a full group, of all groups; blocks a column of units
+};
+static GradVectorsShape grad_vectors_grid(int count, int group, int Mpad, int max_splits, int sms) {
     int per_split, splits, chunks, cap;
-    grad_vectors_shape(count, max_splits, &per_split, &splits, &chunks, &cap);
-    return sizeof(double2) * static_cast<size_t>(splits) * chunks * (1 + N) * M;
+    grad_vectors_shape(std::min(count, group), max_splits, &per_split, &splits, &chunks, &cap);
+    const int per_group = splits * chunks, units = (count + group - 1) / group * per_group;
+    return {per_group, units, std::min(units, std::max(1, 3 * sms / (Mpad / 32))), cap};
 }
 
-cudaError_t launch_grad_vectors(const GradVectors& g, const OpDev& op, double2* partial, int max_splits,
-                                cudaStream_t st, SplitSum* job) {
+size_t grad_vectors_bytes(int count, int group, int N, int M, int Mpad, int max_splits, int sms) {
+    return sizeof(double2) * static_cast<size_t>(grad_vectors_grid(count, group, Mpad, max_splits, sms).rows) * (1 + N) * M;
+}
+
+cudaError_t launch_grad_vectors(const GradVectors& g, const OpDev& op, double2* partial, int sms, cudaStream_t st,
+                                SplitSum* job) {
     if (g.count <= 0) return cudaSuccess;
-    int per_split, splits, chunks, cap;
-    grad_vectors_shape(g.count, max_splits, &per_split, &splits, &chunks, &cap);
-    const size_t sm = sizeof(float4) * kGvWarps * kGvStrings * cap + sizeof(float2) * kGvStrings * kGvWarps * 32 +
-                      sizeof(pair_t) * kGvWarps * 32 * cap;
+    const GradVectorsShape S = grad_vectors_grid(g.count, g.group, g.Mpad, g.max_splits, sms);
+    const size_t sm = sizeof(float4) * kGvWarps * kGvStrings * S.cap + sizeof(float2) * kGvStrings * kGvWarps * 32 +
+                      sizeof(pair_t) * kGvWarps * 32 * S.cap;
     const auto kernel = g.Mpad == 32 ? grad_vectors_kernel<true> : grad_vectors_kernel<false>;
     if (sm > 48 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                    static_cast<int>(sm));
         if (e != cudaSuccess) return e;
     }
-    const dim3 grid(g.Mpad / 32, splits * chunks);
-    kernel<<<grid, 32 * kGvWarps, sm, st>>>(g, op, per_split, chunks, cap, partial);
+    const dim3 grid(g.Mpad / 32, S.rows);
+    kernel<<<grid, 32 * kGvWarps, sm, st>>>(g, op, S.per_group, S.units, S.cap, partial);
     job->pre = partial;
-    job->pre_splits = splits * chunks;
+    job->pre_splits = S.rows;
     return cudaGetLastError();
 }
 
