@@ -803,19 +803,24 @@ __device__ __forceinline__ float log_add(float a, float b) {
 // cross-entropy -sum p* log q with respect to the seed and length logits (q factorises
 // into the seed and length softmaxes, whose optimum is the marginals of p*).
 //
-// One block of four warps per walker, a pair of neighbouring seeds per warp at a time, both in
-// the halves of each packed operation, lanes over the hidden units; the 16 lane sums of a pair
+// One block of four warps per walker, a pair of neighbouring seeds per warp at a time, lanes over
+// the hidden units, two of a lane's in the halves of each packed operation: the seeds' moves end on
+// the same site one after the other, so that a row of W is loaded once for both and comes in as
+// the pairs the operations take (seeds in the halves instead took two loads of half the width and
+// four moves a unit).  The 16 lane sums of a pair
 // of seeds fold into one butterfly (16 shuffles for 80), and the log-sums over lengths and seeds
 // run at the end, a seed or a length a thread, in the order of one warp's loop (which spent a
-// tenth of its instructions on them in every lane).  Bound by the FP32 pipe: 72 of its cycles per
-// unit of a pair: N = 100, M = 400, 4096 walkers take 2.23 ms, 3.33 ms with a warp per walker.
+// tenth of its instructions on them in every lane).  Bound by the FP32 pipe: 64 of its cycles per
+// pair of units, seed and length.  A training step of 4096 walkers, of which this is most, with
+// seeds in the halves and now: N = 64, M = 128 633 / 598 us, N = 60, M = 240 1035 / 916, N = 100,
+// M = 400 2341 / 2318, M = 520 3188 / 3014; there 3.33 ms for this alone with a warp per walker.
 template <int K, int NW>
 __global__ void __launch_bounds__(32 * kWarpsPerBlock, 4) lb_target_kernel(RbmDev P, const uint64_t* spins,
                                                                           const float4* theta, const float2* re_all,
                                                                           const float* logits, int O, float* dl) {
     constexpr int KP = (K + 1) / 2;
-    __shared__ float2 th_sm[32 * K];                      // the angles
-    __shared__ float re_sm[32 * K];                       // Re f of them
+    __shared__ float4 th_sm[32 * KP];                     // the angles of a lane's unit pairs, as in Wq
+    __shared__ float2 re_sm[32 * KP];                     // Re f of them
     __shared__ float d_sm[64 * NW * kLengths];            // Re Delta [i][l - 1]
     __shared__ float ml_sm[kLengths];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -824,48 +829,48 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, 4) lb_target_kernel(RbmDe
 #pragma unroll
     for (int k = 0; k < NW; k++) s.w[k] = spins[static_cast<long>(w) * NW + k];
     for (int e = tid; e < KP * 32; e += 32 * kWarpsPerBlock) {
-        const float4 t = theta[static_cast<long>(w) * KP * 32 + e];
-        const float2 f = re_all[static_cast<long>(w) * KP * 32 + e];
-        const int j = (e >> 5) * 64 + (e & 31);   // units j, j + 32
-        th_sm[j] = make_float2(t.x, t.z);
-        re_sm[j] = f.x;
-        if (j + 32 < 32 * K) {
-            th_sm[j + 32] = make_float2(t.y, t.w);
-            re_sm[j + 32] = f.y;
-        }
+        th_sm[e] = theta[static_cast<long>(w) * KP * 32 + e];
+        re_sm[e] = re_all[static_cast<long>(w) * KP * 32 + e];
     }
     __syncthreads();
     for (int i0 = 2 * warp; i0 < N; i0 += 2 * kWarpsPerBlock) {
-        const int i1 = min(i0 + 1, N - 1);
-        pair_t nr[K], ni[K], part[kLengths];
+        const int seeds = i0 + 1 < N ? 2 : 1;
+        pair_t nr[2][KP], ni[2][KP];
+        float v[16];   // value 8 seed + length - 1
 #pragma unroll
-        for (int k = 0; k < K; k++) {
-            const float2 t = th_sm[lane + 32 * k];
-            nr[k] = splat2(t.x);
-            ni[k] = splat2(t.y);
+        for (int kk = 0; kk < KP; kk++) {
+            const float4 t = th_sm[kk * 32 + lane];
+            nr[0][kk] = nr[1][kk] = pk2(t.x, t.y);
+            ni[0][kk] = ni[1][kk] = pk2(t.z, t.w);
         }
+        // site i0 + r is the last of seed i0's move of length r + 1 and of seed i0 + 1's of length r
 #pragma unroll
-        for (int q = 0; q < kLengths; q++) {
-            int c0 = i0 + q, c1 = i1 + q;
-            if (c0 >= N) c0 -= N;
-            if (c1 >= N) c1 -= N;
-            const pair_t ts = pk2(s.up(c0) ? -2.0f : 2.0f, s.up(c1) ? -2.0f : 2.0f);
-            const float2* r0 = P.W + static_cast<long>(c0) * P.Mpad + lane;
-            const float2* r1 = P.W + static_cast<long>(c1) * P.Mpad + lane;
-            part[q] = splat2(0.0f);
+        for (int r = 0; r <= kLengths; r++) {
+            int c = i0 + r;
+            if (c >= N) c -= N;
+            const pair_t ts = splat2(s.up(c) ? -2.0f : 2.0f);
+            const float4* row = P.Wq + static_cast<long>(c) * KP * 32 + lane;
+            float part[2] = {0.0f, 0.0f};
 #pragma unroll
-            for (int k = 0; k < K; k++) {
-                const float2 wa = __ldg(r0 + 32 * k), wb = __ldg(r1 + 32 * k);
-                nr[k] = fma2(ts, pk2(wa.x, wb.x), nr[k]);
-                ni[k] = fma2(ts, pk2(wa.y, wb.y), ni[k]);
-                part[q] = add2(part[q], sub2(lc_re2(nr[k], ni[k]), splat2(re_sm[lane + 32 * k])));
+            for (int kk = 0; kk < KP; kk++) {
+                const float4 wv = __ldg(row + 32 * kk);
+                const float2 re = re_sm[kk * 32 + lane];
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    if (h == 0 ? r == kLengths : r == 0) continue;
+                    nr[h][kk] = fma2(ts, pk2(wv.x, wv.y), nr[h][kk]);
+                    ni[h][kk] = fma2(ts, pk2(wv.z, wv.w), ni[h][kk]);
+                    float d0, d1;
+                    up2(sub2(lc_re2(nr[h][kk], ni[h][kk]), pk2(re.x, re.y)), d0, d1);
+                    part[h] = __fadd_rn(part[h], d0);
+                    if (2 * kk + 1 < K) part[h] = __fadd_rn(part[h], d1);
+                }
             }
+            if (r < kLengths) v[r < kLengths ? r : 0] = part[0];
+            if (r > 0) v[r > 0 ? 8 + r - 1 : 8] = part[1];
         }
         // the folding butterfly of the 16 sums: lanes 2 v, 2 v + 1 end with value v = 8 seed + q,
         // added in warp_sum_xor's order
-        float v[16];
-#pragma unroll
-        for (int q = 0; q < kLengths; q++) up2(part[q], v[q], v[8 + q]);
 #pragma unroll
         for (int half = 8, off = 16; half >= 1; half >>= 1, off >>= 1) {
             const bool up = (lane & off) != 0;
@@ -877,7 +882,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, 4) lb_target_kernel(RbmDe
         }
         const float d = __fadd_rn(v[0], __shfl_xor_sync(0xffffffffu, v[0], 1));
         const int i = (lane & 16) ? i0 + 1 : i0;
-        if (!(lane & 1) && i < N) d_sm[i * kLengths + ((lane >> 1) & 7)] = d;
+        if (!(lane & 1) && i < i0 + seeds) d_sm[i * kLengths + ((lane >> 1) & 7)] = d;
     }
     __syncthreads();
     // log-sums over the seeds (a length per thread), then over the lengths (a seed per thread)
