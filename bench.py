@@ -64,7 +64,8 @@ METRIC = "effective samples/s (ESS of E_loc) at N=100: learned-proposal MCMC (pl
 UNIT = "samples/s"
 L2_FLUSH_BYTES = 256 << 20
 # DRAM bytes of one sampler launch: dram__bytes_read.sum + dram__bytes_write.sum of an ncu
-# capture of rbm_mc_smem_kernel<13,2> on these 16384 walkers
+# capture of the one-walker-per-warp sampler on these 16384 walkers (rbm_mc_group_kernel<13,16,2>
+# moves the same spins, stream positions and counts)
 SAMPLER_DRAM_BYTES = 1.059e6
 # DRAM bytes of one learned_accept_kernel<13,2> launch of 16384 walkers (ncu, sigma 0.05, mean
 # of three launches: 100.3 MB read, 4.1 MB written -- accepted angles stay in L2 within a launch)
@@ -863,7 +864,7 @@ def run_deep(args):
         "roofline": {"bound": "fp32", "achieved": flops / sec / 1e12, "peak": v, "unit": "TFLOP/s",
                      "frac": flops / sec / 1e12 / v if v else None, "traffic": None,
                      "peak_source": "measured in this run: the larger of the library's scalar and packed-pair FP32 FMA probes",
-                     "kernel": "deep_mc_multi_kernel + deep_adjoint_multi_kernel + adj_cgemm_kernel (the whole step)",
+                     "kernel": "deep_mc_pairs_kernel + deep_adjoint_pairs_kernel + adj_cgemm_kernel (the whole step)",
                      "flops_per_step": flops},
         "cpu_baseline": cpu,
         "clocks": clk,
@@ -922,7 +923,7 @@ def run_plain(args):
                      "frac": flops / sec / 1e12 / peak, "traffic": SAMPLER_DRAM_BYTES,
                      "peak_source": "measured in this run: the larger of the library's scalar and packed-pair FP32 "
                                     "FMA probes",
-                     "kernel": "rbm_mc_smem_kernel<13,2>", "flops_per_launch": flops},
+                     "kernel": "rbm_mc_group_kernel<13,16,2>", "flops_per_launch": flops},
         "clocks": clk,
     }
     print(json.dumps(line))
@@ -1213,7 +1214,7 @@ def main():
                                    "traffic": SAMPLER_DRAM_BYTES,
                                    "peak_source": "measured in this run: the larger of the library's scalar and "
                                                   "packed-pair FP32 FMA probes",
-                                   "kernel": "rbm_mc_smem_kernel<13,2> (plain sampler, 10 sweeps per launch, sigma 0.05)",
+                                   "kernel": "rbm_mc_group_kernel<13,16,2> (plain sampler, 10 sweeps per launch, sigma 0.05)",
                                    "flops_per_launch": fl, "ms_per_launch": avg_launch * 1e3},
         "glass_sigma0.1": r.get("glass"),
         "cpu_baseline": cpu,

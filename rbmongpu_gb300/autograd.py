@@ -11,8 +11,9 @@ set of configurations, and the backward pass returns the stored gradient.  Other
 forward pass samples (or enumerates) and evaluates the local energies only, with no
 gradient work.  (Evaluating the energy in the forward pass and the gradient in the backward
 pass on the kept samples gives the same numbers, but for a PsiDeep on Monte Carlo samples
-costs the estimator's FP64 local-energy pass on top of the adjoint: 716 ms against 161 ms
-per step of the 100-200-100-50 net over 8192 walkers.)  PyTorch is used only for this
+costs the estimator's FP64 local-energy pass on top of the adjoint, which alone is 69 ms
+per step of the 100-200-100-50 net over 8192 walkers; 716 ms against 161 ms when both were
+slower.)  PyTorch is used only for this
 wrapper: the value and the gradient both come from the CUDA library.
 
     params = torch.tensor(psi.params, requires_grad=True)
