@@ -52,7 +52,7 @@ int deep_log_psi(const rbmg_psi* psi, int count, const uint64_t* d_spins, uint64
 // Grow-only scratch buffers shared by all calls on this thread's device.
 struct Workspace {
     DevBuf sample_spins, eloc, logpsi, logpsi_p, T, U, X, theta, en, vpart, Tp, weights, coef1, coef2, coef3, omega, pr, nn;
-    DevBuf partial, block_scratch, sums, acc_O, acc_EO, acc_Ek, acc_wO, acc_pO;
+    DevBuf partial, block_scratch, sums, acc_O, acc_EO, acc_Ek, acc_wO;
     DevBuf smat, smean, spart, okrows, sshift, splanes, serror, sout;
     DevBuf stat;      // (m, sum), (log Z, -) of exact summation's weights, then the first chunk's mean energy
     DevBuf gout;      // a gradient on its way to the host

@@ -67,86 +67,8 @@ __device__ __forceinline__ uint64_t draw_n_over_k(Rng& rng, unsigned n, unsigned
     return result;
 }
 
-// One Metropolis proposal (include/spin_ensembles/MonteCarloLoop.hpp:153-256): flip
-// site `u32 % N` (and a partner with the same new spin under S_z symmetry), update the
-// angles of the trial state, accept if Delta > 0 or u <= exp(2 Delta), u drawn only
-// when Delta <= 0.
-template <int K, int NW, class Rng>
-__device__ __forceinline__ bool rbm_mh_step(const RbmDev& P, Spins<NW>& s, float (&tr)[K], float (&ti)[K],
-                                            float (&re)[K], Rng& rng, int lane, int total_z, uint64_t nmagic) {
-    const uint32_t N = static_cast<uint32_t>(P.N);
-    int sites[2];
-    int ns = 1;
-    sites[0] = static_cast<int>(fastmod(rng.next(), nmagic, N));
-    if (total_z) {
-        const bool first_new = !s.up(sites[0]);
-        int sec = sites[0];
-        for (int guard = 0; guard < (1 << 20); guard++) {
-            const int c = static_cast<int>(fastmod(rng.next(), nmagic, N));
-            const bool v = c == sites[0] ? first_new : s.up(c);
-            if (v == first_new) { sec = c; break; }
-        }
-        sites[1] = sec;
-        ns = 2;
-    }
-    // The trial angles are not kept: each is formed, evaluated and dropped, and on the
-    // (rare) accept they are formed again -- bit-identical -- to commit.  Only theta and
-    // Re f(theta) stay live, which keeps the register footprint low.
-    Spins<NW> s2 = s;
-    float two_s[2];
-    const float2* rows[2];
-#pragma unroll
-    for (int q = 0; q < 2; q++) {
-        if (q >= ns) break;
-        const int site = q == 0 ? sites[0] : sites[1];
-        s2.flip(site);
-        two_s[q] = s2.up(site) ? 2.0f : -2.0f;
-        rows[q] = P.W + static_cast<long>(site) * P.Mpad + lane;
-    }
-    float part = 0.0f;
-    if (ns == 1) {
-        // single flip: the K loads of the W row are issued together
-        float2 w[K];
-#pragma unroll
-        for (int k = 0; k < K; k++) w[k] = __ldg(rows[0] + 32 * k);
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-            const float nr = __fmaf_rn(two_s[0], w[k].x, tr[k]);
-            const float ni = __fmaf_rn(two_s[0], w[k].y, ti[k]);
-            part = __fadd_rn(part, __fsub_rn(lc_re(nr, ni), re[k]));
-        }
-    } else {
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-            float nr = tr[k], ni = ti[k];
-            for (int q = 0; q < ns; q++) {
-                const float2 w = __ldg(rows[q] + 32 * k);
-                nr = __fmaf_rn(two_s[q], w.x, nr);
-                ni = __fmaf_rn(two_s[q], w.y, ni);
-            }
-            part = __fadd_rn(part, __fsub_rn(lc_re(nr, ni), re[k]));
-        }
-    }
-    const float delta = warp_sum_xor(part);
-    bool accept = delta > 0.0f;
-    if (!accept) accept = rng.uniform() <= expf_det(__fmul_rn(2.0f, delta));
-    if (accept) {
-        s = s2;
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-            for (int q = 0; q < ns; q++) {
-                const float2 w = __ldg(rows[q] + 32 * k);
-                tr[k] = __fmaf_rn(two_s[q], w.x, tr[k]);
-                ti[k] = __fmaf_rn(two_s[q], w.y, ti[k]);
-            }
-            re[k] = lc_re(tr[k], ti[k]);
-        }
-    }
-    return accept;
-}
-
 // ---------------------------------------------------------------------------
-// The sampler's form of the above on packed pairs (device_math.cuh: pair_t, FP32x2):
+// A walker's state on packed pairs (device_math.cuh: pair_t, FP32x2):
 // pair kk of a lane holds hidden units k = 2 kk and 2 kk + 1; every half is computed with
 // the scalar form's operations in its order, so angles, Re f and the decision are the
 // scalar ones bit for bit.  KP = ceil(K / 2); for odd K the last pair's second unit is a
