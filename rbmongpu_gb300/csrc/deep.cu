@@ -2180,10 +2180,18 @@ int deep_adjoint_chunk(const rbmg_psi* psi, const rbmg_operator* op, const Chunk
     RBMG_CK(alphaO.ensure(sizeof(float2) * static_cast<size_t>(chunk)));
     const size_t sm = smem_for(net, sizeof(float2), true) + 2 * sizeof(float2) * net.size[0];
     RBMG_CK(set_smem(deep_adjoint_kernel, sm));
-    // neighbours per pass of the reverse kernel (RBMG_DEEP_ADJOINT_BATCH = 1, 2, 4 or 8;
-    // default 8), the same outputs
+    // neighbours per pass of the reverse kernel: eight, or as many as the widest nets leave room
+    // for in a block's shared memory (three layers of 720 units: four), or what
+    // RBMG_DEEP_ADJOINT_BATCH = 1, 2, 4 or 8 says; the same outputs
     int nbatch = 8;
-    if (const char* v = std::getenv("RBMG_DEEP_ADJOINT_BATCH")) nbatch = std::atoi(v);
+    if (const char* v = std::getenv("RBMG_DEEP_ADJOINT_BATCH")) {
+        nbatch = std::atoi(v);
+    } else {
+        int dev = 0, limit = 0;
+        RBMG_CK(cudaGetDevice(&dev));
+        RBMG_CK(cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+        while (nbatch > 2 && deep_adjoint_pairs_smem(net, nbatch / 2) > static_cast<size_t>(limit)) nbatch /= 2;
+    }
     if (nbatch != 1 && nbatch != 2 && nbatch != 4 && nbatch != 8)
         return fail(RBMG_EINVAL, "RBMG_DEEP_ADJOINT_BATCH: 1, 2, 4 or 8");
     const size_t smb = deep_adjoint_pairs_smem(net, nbatch / 2);
