@@ -286,11 +286,13 @@ RBMG_API int rbmg_stream(void** stream);
  * RBMG_EINVAL).  The first call on a device looks up the array's address with
  * cudaGetSymbolAddress (set-up done once per device, on the current device), so make that
  * first call before any stream capture.  Each call returns once the result is on the host.
- * Every call uses the same array and clears the sums it accumulates; calls that overlap on
+ * Every call uses the same array and clears what it accumulates; calls that overlap on
  * the GPU (other host threads, other streams) race.  After a cudaDeviceReset the cached
  * address is stale: do not call it on a device that was reset. */
 RBMG_API int rbmg_ev_value_exact_noalloc(const rbmg_psi* psi, const rbmg_operator* op, int num_spins,
                                          double* value /* [2] */);
+/* Fills that array with a byte.  No call depends on what the array holds when it starts. */
+RBMG_API int rbmg_noalloc_scratch_fill(int byte);
 
 /* ---------------------------------------------------------------- learned proposal
  * Extension (no reference counterpart): an MLP on the spins (BF16 operands, FP32

@@ -86,6 +86,7 @@ SIGNATURES = {
     "rbmg_probe_fp32_tflops": [C.c_int, _dp],
     "rbmg_probe_fp32x2_tflops": [C.c_int, _dp],
     "rbmg_ev_value_exact_noalloc": [_vp, _vp, C.c_int, _dp],
+    "rbmg_noalloc_scratch_fill": [C.c_int],
     "rbmg_proposal_create": [C.c_int, C.c_uint64, C.c_float, _vpp],
     "rbmg_proposal_destroy": [_vp],
     "rbmg_proposal_num_params": [_vp, C.POINTER(C.c_int64)],

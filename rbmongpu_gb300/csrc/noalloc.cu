@@ -31,10 +31,12 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 constexpr size_t kOffLogPsi = 0;                                            // double2 [states]
 constexpr size_t kOffWeights = kOffLogPsi + kNoAllocStates * sizeof(double2);   // double  [states]
 constexpr size_t kOffEloc = kOffWeights + kNoAllocStates * sizeof(double);      // double2 [states]
-constexpr size_t kOffBlocks = kOffEloc + kNoAllocStates * sizeof(double2);      // double2 [kSumScratch], the counter zero
-constexpr size_t kOffBlockMax = kOffBlocks + kSumScratch * sizeof(double2);   // double [kSumBlocks]
-constexpr size_t kOffSums = kOffBlockMax + kSumBlocks * sizeof(double);         // double2 [kMaxSeries]
-static_assert(kOffSums + kMaxSeries * sizeof(double2) <= kNoAllocBytes, "no-alloc scratch too small");
+constexpr size_t kOffBlocks = kOffEloc + kNoAllocStates * sizeof(double2);      // double2 [kSumScratch]: partial sums, counter
+constexpr size_t kOffSums = kOffBlocks + kSumScratch * sizeof(double2);         // double2 [kMaxSeries]
+constexpr size_t kOffBlockMax = kOffSums + kMaxSeries * sizeof(double2);        // double [kSumBlocks]
+static_assert(kOffBlockMax + kSumBlocks * sizeof(double) <= kNoAllocBytes, "no-alloc scratch too small");
+// what every call clears: the blocks' counter, the last entry of kSumScratch, and the sums behind it
+constexpr size_t kOffCleared = kOffSums - sizeof(double2), kCleared = (1 + kMaxSeries) * sizeof(double2);
 
 // FP64 log psi of basis state t, from the FP32 device parameters (one warp per state)
 __global__ void logpsi64_from32_kernel(RbmDev P, int count, double2* out) {
@@ -129,8 +131,10 @@ extern "C" int rbmg_ev_value_exact_noalloc(const rbmg_psi* psi, const rbmg_opera
     for (int b = 1; b < blocks_used; b++) mx = std::fmax(mx, hmax[b]);
     if (!std::isfinite(mx)) return fail(RBMG_ENAN, "no-alloc energy: non-finite log psi");
     RBMG_CK(launch_exp_weights(count, lp, mx, w, st));
-    // the sum is accumulated: it must start at zero on every call
-    RBMG_CK(cudaMemsetAsync(sums, 0, sizeof(double2) * kMaxSeries, st));
+    // the sum is accumulated and its blocks are counted: both start at zero on every call, since
+    // calls that overlapped (wrong themselves) may have left the counter anywhere, after which no
+    // block or the wrong one would add up the partial sums
+    RBMG_CK(cudaMemsetAsync(base + kOffCleared, 0, kCleared, st));
     // local energies (the same estimator kernel as rbmg_ev_value)
     EstLaunch L{};
     L.count = count;
@@ -151,5 +155,14 @@ extern "C" int rbmg_ev_value_exact_noalloc(const rbmg_psi* psi, const rbmg_opera
     value[0] = scale * h.x;
     value[1] = scale * h.y;
     if (!std::isfinite(value[0]) || !std::isfinite(value[1])) return fail(RBMG_ENAN, "no-alloc energy: non-finite");
+    return RBMG_OK;
+}
+
+extern "C" int rbmg_noalloc_scratch_fill(int byte) {
+    unsigned char* base = nullptr;
+    const int r = noalloc_scratch(&base);
+    if (r != RBMG_OK) return r;
+    RBMG_CK(cudaMemsetAsync(base, byte, kNoAllocBytes, stream()));
+    RBMG_CK(cudaStreamSynchronize(stream()));
     return RBMG_OK;
 }
