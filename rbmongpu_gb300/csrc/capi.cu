@@ -663,18 +663,6 @@ static int rbm64_for(const rbmg_psi* p, uint64_t count, DevBuf& tab, Rbm64* out)
 
 namespace rbmg {
 
-// One chunk of samples: spins on the device (or basis indices when enumerate),
-// per-sample weights (null = equal weights) and, for MC, the sampler's log psi / E_loc.
-struct Chunk {
-    int count = 0;
-    int group = 0;   // StreamResult::batch: the samples of a chunk of the plain size
-    const uint64_t* spins = nullptr;
-    int enumerate = 0;
-    uint64_t enum_base = 0;
-    const double* weights = nullptr;
-    const double2* eloc = nullptr;      // filled by the sampler when requested
-};
-
 struct StreamResult {
     // set by a caller that takes the results on the device: exact summation then leaves its
     // factor in Workspace::stat, and a Monte-Carlo pass leaves its counts on their way, for

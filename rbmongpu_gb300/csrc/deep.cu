@@ -22,15 +22,6 @@
 
 namespace rbmg {
 
-struct Chunk {
-    int count = 0;
-    const uint64_t* spins = nullptr;
-    int enumerate = 0;
-    uint64_t enum_base = 0;
-    const double* weights = nullptr;
-    const double2* eloc = nullptr;
-};
-
 namespace {
 
 // ---------------------------------------------------------------- complex helpers
@@ -2322,7 +2313,7 @@ int deep_stream(rbmg_ensemble* e, const rbmg_psi* psi, const rbmg_operator* op, 
         RBMG_CK(cudaGetLastError());
         first = false;
         Chunk c;
-        c.count = rows * B;
+        c.count = c.group = rows * B;
         c.spins = samples.as<uint64_t>();
         const int r = fn(c);
         if (r != RBMG_OK) return r;

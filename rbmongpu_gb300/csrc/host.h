@@ -195,6 +195,19 @@ namespace rbmg {
 int psi_sync_host(const rbmg_psi* psi);
 int psi_master_ensure(rbmg_psi* psi);
 int psi_scatter(rbmg_psi* psi, const double2* packed);
+
+// One chunk of samples: spins on the device (or basis indices when enumerate),
+// per-sample weights (null = equal weights) and, for MC, the sampler's log psi / E_loc.
+struct Chunk {
+    int count = 0;
+    int group = 0;   // the samples of a chunk of the plain size, of which this one may hold several
+    const uint64_t* spins = nullptr;
+    int enumerate = 0;
+    uint64_t enum_base = 0;
+    const double* weights = nullptr;
+    const double2* eloc = nullptr;      // filled by the sampler when requested
+};
+
 // deep.cu: the layouts of a deep net that are derived from its device weights
 int deep_derive(const rbmg_psi* psi);
 // capi.cu: the energy gradient formed on the device, d_grad [P]; energy to value[2]
