@@ -56,6 +56,7 @@ struct Workspace {
     DevBuf smat, smean, spart, okrows, sshift, splanes, serror, sout;
     DevBuf stat;      // (m, sum), (log Z, -) of exact summation's weights, then the first chunk's mean energy
     DevBuf gout;      // a gradient on its way to the host
+    HostBuf ghost;    // and, of exact summation, there
     HostBuf status;   // GradOut::status
     DevBuf acc_B, eabs2, lsums, rw, rwc, acc_C2, acc_C3;
     DevBuf tab64, tab64_p;   // spin-group sums of psi's and psi''s FP64 weights
@@ -668,6 +669,9 @@ struct StreamResult {
     // factor in Workspace::stat, and a Monte-Carlo pass leaves its counts on their way, for
     // stream_done after the caller's own wait
     bool defer = false;
+    // set by a caller whose chunks go to its own caller's memory: exact summation refuses a
+    // non-finite log psi before the first of them, not after the last
+    bool refuse_first = false;
     // chunks of several plain ones, up to so many samples, for a pass that sums within the plain
     // chunks' 32-sample groups (0: plain chunks)
     size_t batch = 0;
@@ -798,6 +802,19 @@ static int exact_stream(rbmg_ensemble* e, const rbmg_psi* psi, StreamResult* res
     RBMG_CK(W.stat.ensure(sizeof(double2) * 3));
     RBMG_CK(launch_exact_weights(static_cast<int>(total), W.logpsi.as<double2>(), W.weights.as<double>(),
                                  W.block_scratch.as<double2>(), W.stat.as<double2>(), stream()));
+    auto take_stat = [&]() -> int {
+        double2 stat[2];
+        RBMG_CK(cudaMemcpyAsync(stat, W.stat.p, sizeof(stat), cudaMemcpyDeviceToHost, stream()));
+        RBMG_CK(cudaStreamSynchronize(stream()));
+        if (!std::isfinite(stat[0].x)) return fail(RBMG_ENAN, kNonFiniteLogPsi);
+        res->log_norm = 2.0 * std::log(psi->prefactor) + stat[1].x;
+        res->norm_factor = std::exp(res->log_norm);
+        return RBMG_OK;
+    };
+    if (res->refuse_first) {
+        const int r = take_stat();
+        if (r != RBMG_OK) return r;
+    }
     for (uint64_t base = 0; base < total; base += kExactChunk) {
         Chunk c;
         c.count = static_cast<int>(std::min<uint64_t>(kExactChunk, total - base));
@@ -809,14 +826,7 @@ static int exact_stream(rbmg_ensemble* e, const rbmg_psi* psi, StreamResult* res
         const int r = fn(c);
         if (r != RBMG_OK) return r;
     }
-    if (res->defer) return RBMG_OK;
-    double2 stat[2];
-    RBMG_CK(cudaMemcpyAsync(stat, W.stat.p, sizeof(stat), cudaMemcpyDeviceToHost, stream()));
-    RBMG_CK(cudaStreamSynchronize(stream()));
-    if (!std::isfinite(stat[0].x)) return fail(RBMG_ENAN, kNonFiniteLogPsi);
-    res->log_norm = 2.0 * std::log(psi->prefactor) + stat[1].x;
-    res->norm_factor = std::exp(res->log_norm);
-    return RBMG_OK;
+    return res->defer || res->refuse_first ? RBMG_OK : take_stat();
 }
 
 }  // namespace rbmg
@@ -1402,13 +1412,20 @@ static int ev_gradient_take(const rbmg_psi* psi, rbmg_ensemble* ens, const Strea
     G.grad = d_grad ? d_grad : W.gout.as<double2>();
     G.status = W.status.as<double>();
     RBMG_CK(launch_grad_out(G, stream()));
-    if (!d_grad) {
+    // exact summation may yet be refused, which leaves the caller's memory as it is: its gradient
+    // goes by a buffer of the library's own
+    const bool stage = !d_grad && ens->kind == 1;
+    if (stage) {
+        RBMG_CK(W.ghost.ensure(sizeof(double2) * P));
+        RBMG_CK(cudaMemcpyAsync(W.ghost.p, G.grad, sizeof(double2) * P, cudaMemcpyDeviceToHost, stream()));
+    } else if (!d_grad) {
         prefault(grad, sizeof(double2) * P);
         RBMG_CK(cudaMemcpyAsync(grad, G.grad, sizeof(double2) * P, cudaMemcpyDeviceToHost, stream()));
     }
     RBMG_CK(cudaStreamSynchronize(stream()));
     if (ens->kind == 0) ens->counts_take();
     if (ens->kind == 1 && !std::isfinite(G.status[3])) return fail(RBMG_ENAN, kNonFiniteLogPsi);
+    if (stage) std::memcpy(grad, W.ghost.p, sizeof(double2) * P);
     value[0] = G.status[0];
     value[1] = G.status[1];
     return RBMG_OK;
@@ -2097,6 +2114,7 @@ extern "C" int rbmg_ensemble_samples(rbmg_ensemble* ens, const rbmg_psi* psi, co
     Workspace& W = ws();
     uint64_t offset = 0;
     StreamResult res;
+    res.refuse_first = true;
     r = run_stream(ens, psi, op, eloc != nullptr, size_t(1) << 22, &res, [&](const Chunk& c) -> int {
         if (spins) {
             if (c.spins) {
