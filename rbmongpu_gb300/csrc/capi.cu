@@ -5,6 +5,7 @@
 #include <cmath>
 #include <functional>
 #include <memory>
+#include <optional>
 #include <vector>
 
 #include <cuda_profiler_api.h>
@@ -2219,8 +2220,11 @@ extern "C" int rbmg_s_matrix(const rbmg_psi* psi, rbmg_ensemble* ens, int flags,
     const bool use_tc = (flags & RBMG_S_SIMT) == 0;
     Workspace& W = ws();
     const size_t sbytes = sizeof(double2) * static_cast<size_t>(L) * L;
-    Prefault pages(out, sizeof(double2) * static_cast<size_t>(P) * P);
+    const size_t obytes = sizeof(double2) * static_cast<size_t>(P) * P;
+    // started by the first chunk of samples: what can be refused has been by then
+    std::optional<Prefault> pages;
     RBMG_CK(W.smat.ensure(sbytes));
+    RBMG_CK(W.sout.ensure(obytes));
     RBMG_CK(W.smean.ensure(sizeof(double2) * L));
     RBMG_CK(cudaMemsetAsync(W.smat.p, 0, sbytes, stream()));
     RBMG_CK(cudaMemsetAsync(W.smean.p, 0, sizeof(double2) * L, stream()));
@@ -2229,6 +2233,7 @@ extern "C" int rbmg_s_matrix(const rbmg_psi* psi, rbmg_ensemble* ens, int flags,
     RBMG_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     uint64_t total = 0;
     StreamResult res;
+    res.refuse_first = true;
     // centred: every row is shifted by the first chunk's mean row (in FP64) before the FP32
     // products, so that the covariance is not the small difference of two large sums
     RBMG_CK(W.sshift.ensure(sizeof(double2) * L));
@@ -2261,7 +2266,9 @@ extern "C" int rbmg_s_matrix(const rbmg_psi* psi, rbmg_ensemble* ens, int flags,
             e = launch_sm_accumulate(a, W.smat.as<double2>(), sms, stream());
             nlaunch++;
         }
-        if (e != cudaSuccess || !centered) return e;
+        if (e != cudaSuccess) return e;
+        if (!pages) pages.emplace(out, obytes);
+        if (!centered) return e;
         nlaunch++;
         return launch_sm_mean(a, W.smean.as<double2>(), W.spart.as<double2>(), stream());
     };
@@ -2341,15 +2348,13 @@ extern "C" int rbmg_s_matrix(const rbmg_psi* psi, rbmg_ensemble* ens, int flags,
     // the exact-summation weights are normalised to sum 1; otherwise divide by the count
     const double z = (weighted && ens->kind == 1) ? 1.0 : static_cast<double>(total);
     // the P x P result on the device (zero rows and columns below 2N), then one contiguous copy
-    const size_t obytes = sizeof(double2) * static_cast<size_t>(P) * P;
-    RBMG_CK(W.sout.ensure(obytes));
     RBMG_CK(cudaMemsetAsync(W.sout.p, 0, sizeof(double2) * static_cast<size_t>(2 * N) * P, stream()));
     if (N > 0)
         RBMG_CK(cudaMemset2DAsync(W.sout.as<double2>() + static_cast<size_t>(2 * N) * P, sizeof(double2) * P, 0,
                                   sizeof(double2) * 2 * N, L, stream()));
     RBMG_CK(launch_sm_finish(L, W.smat.as<double2>(), W.smean.as<double2>(), 1.0 / z, centered ? 1 : 0,
                              W.sout.as<double2>(), P, 2 * N, stream()));
-    pages.join();
+    pages->join();
     RBMG_CK(cudaMemcpyAsync(out, W.sout.p, obytes, cudaMemcpyDeviceToHost, stream()));
     int tc_err = 0;
     if (use_tc) RBMG_CK(cudaMemcpyAsync(&tc_err, W.serror.p, sizeof(int), cudaMemcpyDeviceToHost, stream()));

@@ -38,3 +38,13 @@ def test_samples(call):
     assert lib.rbmg_ensemble_samples(ens._h, psi._h, op._h, spins.ctypes.data_as(C.POINTER(C.c_uint64)), doubles(lp),
                                      doubles(e)) == _lib.RBMG_ENAN
     assert (spins == 7).all() and (lp == 7.0).all() and (e == 7.0).all()
+
+
+def test_s_matrix():
+    """Of 8 MB and more, whose pages are made present while the GPU works."""
+    N, M = 8, 80
+    psi, lib = rg.Psi(np.zeros(N), np.zeros(N), 1e308 * np.ones(M), np.zeros((N, M))), _lib.lib()
+    out = np.full(2 * psi.num_params ** 2, 7.0)
+    assert out.nbytes >= 8 << 20
+    assert lib.rbmg_s_matrix(psi._h, rg.ExactSummation(N)._h, 0, doubles(out)) == _lib.RBMG_ENAN
+    assert (out == 7.0).all()
