@@ -1222,10 +1222,15 @@ static int ev_gradient_sums(const rbmg_psi* psi, const rbmg_operator* op, rbmg_e
     RBMG_CK(W.sums.ensure(sizeof(double2) * kMaxSeries));
     RBMG_CK(sum_scratch(W));
     RBMG_CK(cudaMemsetAsync(W.sums.p, 0, sizeof(double2) * kMaxSeries, stream()));
-    constexpr int kSplits = 64, kBatchSplits = 152;   // of a plain chunk, and of several at a time
     int dev = 0, sms = 0;
     RBMG_CK(cudaGetDevice(&dev));
     RBMG_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    // splits of the samples of a plain chunk, and of several at a time: four blocks an SM, where 64
+    // make fewer, and no more, since each is (1 + N) M sums of 16 bytes three or four times over
+    // (N = 256, M = 576: at most 450 or 600 MB of scratch).  152 splits whatever the net, 1.1 or
+    // 1.4 GB there: 8192 samples 10.98 ms, now 10.81; 16384 at N = 140, M = 576 11.40 / 11.35
+    constexpr int kSplits = 64;
+    const int batch_splits = std::max(kSplits, std::min(sms, 4 * sms / outer_tiles(N, std::max(1, psi->M))));
     // a transverse field (each string one site's own): the strings' terms e_n are formed
     // first, then U and the V sums from the stored angles; otherwise e_n tanh(theta''_n)
     // of every string and sample is stored.  The fluctuation gradient's second V sum has
@@ -1243,8 +1248,6 @@ static int ev_gradient_sums(const rbmg_psi* psi, const rbmg_operator* op, rbmg_e
         // with the sweeps, now 8.4)
         if (single)
             res->batch = (size_t(512) << 20) / (sizeof(float2) * (3 * psi->Mpad + op->num_offdiag) + 64);
-        // of the sums over T, and of those over U
-        RBMG_CK(W.partial.ensure(sizeof(double2) * ((adjoint ? 3 : 2) + (fluct ? 2 : 1)) * kBatchSplits * (1 + N) * psi->M));
     }
     const size_t max_chunk = psi->kind == 0 ? std::max<size_t>(256, (size_t(512) << 20) / per_sample) : 4096;
     // The sums are centred on E0, the mean local energy of the first chunk:
@@ -1336,8 +1339,7 @@ static int ev_gradient_sums(const rbmg_psi* psi, const rbmg_operator* op, rbmg_e
                 G.site_ptr = op->d_site_ptr.as<int>();
                 RBMG_CK(launch_grad_vectors(G, od, W.vpart.as<double2>(), sms, stream(), &jobs[1]));
             }
-            double2* part = W.partial.as<double2>();
-            const int splits = c.count > c.group ? kBatchSplits : kSplits;
+            const int most = c.count > c.group ? batch_splits : kSplits, splits = outer_splits(c.count, most);
             // the sums over T, together: O, and (E - E0) O* or, for the adjoint, C2 and C3
             OuterSet sums_t{}, sums_u{};
             sums_t.add(W.coef1.as<double2>(), 0, W.acc_O.as<double2>());
@@ -1347,14 +1349,18 @@ static int ev_gradient_sums(const rbmg_psi* psi, const rbmg_operator* op, rbmg_e
             } else {
                 sums_t.add(W.coef2.as<double2>(), 1, W.acc_EO.as<double2>());
             }
-            RBMG_CK(launch_outer_reduce(c.count, N, nw, psi->M, c.spins, c.enum_base, c.enumerate, sums_t,
-                                        W.T.as<float2>(), psi->Mpad, part, splits, stream(), &jobs[0]));
             sums_u.add(W.coef1.as<double2>(), 0, W.acc_Ek.as<double2>());
             if (fluct) sums_u.add(W.coef3.as<double2>(), 0, W.acc_B.as<double2>());
+            const size_t plane = static_cast<size_t>(1 + N) * psi->M;
+            // the V sums of stored terms follow in the same scratch
+            const size_t planes = std::max((sums_t.n + sums_u.n) * splits, single ? 0 : vterm_splits(c.count, kSplits));
+            RBMG_CK(W.partial.ensure(sizeof(double2) * plane * planes));
+            double2* part = W.partial.as<double2>();
+            RBMG_CK(launch_outer_reduce(c.count, N, nw, psi->M, c.spins, c.enum_base, c.enumerate, sums_t,
+                                        W.T.as<float2>(), psi->Mpad, part, most, stream(), &jobs[0]));
             RBMG_CK(launch_outer_reduce(c.count, N, nw, psi->M, c.spins, c.enum_base, c.enumerate, sums_u,
-                                        W.U.as<float2>(), psi->Mpad,
-                                        part + static_cast<size_t>(sums_t.n) * splits * (1 + N) * psi->M, splits,
-                                        stream(), &jobs[1]));
+                                        W.U.as<float2>(), psi->Mpad, part + sums_t.n * splits * plane, most, stream(),
+                                        &jobs[1]));
             RBMG_CK(launch_split_sums(jobs, 2, !first, stream()));
             first = false;
             if (!single)

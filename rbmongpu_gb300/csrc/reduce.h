@@ -21,7 +21,7 @@ struct SeriesSet {
 
 // up to kMaxOuter sums over the same rows A: out_q[r][j] += sum_s c_q[s] f_q(A[s][j]) g_r(s),
 // g_0 = 1, g_{1+i} = s_i; f_q = conj if conj_q.  partial: scratch of
-// n * max_splits * (1+N) * M double2.
+// n * outer_splits(count, max_splits) * (1+N) * M double2.
 constexpr int kMaxOuter = 3;
 struct OuterSet {
     int n;
@@ -45,6 +45,10 @@ struct SplitSum {
     const double2* pre;
     int pre_splits;
 };
+// the splits that the sums below make of so many samples, and the blocks of one split of an outer sum
+int outer_splits(int count, int max_splits);
+int vterm_splits(int count, int max_splits);
+int outer_tiles(int N, int M);
 // with job: the partials are left for launch_split_sums
 cudaError_t launch_outer_reduce(int count, int N, int nw, int M, const uint64_t* spins, uint64_t enum_base,
                                 int enumerate, const OuterSet& set, const float2* A, int lda, double2* partial,

@@ -731,12 +731,25 @@ cudaError_t launch_split_sums(const SplitSum* jobs, int n, bool add, cudaStream_
     return cudaGetLastError();
 }
 
+static int outer_per_split(int count, int max_splits) {
+    return max(kChunk, ((count + max_splits - 1) / max_splits + kChunk - 1) / kChunk * kChunk);
+}
+static int vterm_per_split(int count, int max_splits) { return max(64, (count + max_splits - 1) / max_splits); }
+int outer_splits(int count, int max_splits) {
+    const int per_split = outer_per_split(count, max_splits);
+    return (count + per_split - 1) / per_split;
+}
+int vterm_splits(int count, int max_splits) {
+    const int per_split = vterm_per_split(count, max_splits);
+    return (count + per_split - 1) / per_split;
+}
+int outer_tiles(int N, int M) { return (M + 31) / 32 * ((N + 1 + kOmRows * kOmMaxTy - 1) / (kOmRows * kOmMaxTy)); }
+
 cudaError_t launch_outer_reduce(int count, int N, int nw, int M, const uint64_t* spins, uint64_t enum_base,
                                 int enumerate, const OuterSet& set, const float2* A, int lda, double2* partial,
                                 int max_splits, cudaStream_t st, SplitSum* job) {
     if (count <= 0) return cudaSuccess;
-    const int per_split = max(kChunk, ((count + max_splits - 1) / max_splits + kChunk - 1) / kChunk * kChunk);
-    const int splits = (count + per_split - 1) / per_split;
+    const int per_split = outer_per_split(count, max_splits), splits = outer_splits(count, max_splits);
     const int tiles = (N + 1 + kOmRows * kOmMaxTy - 1) / (kOmRows * kOmMaxTy);
     const int ty = (N + 1 + kOmRows * tiles - 1) / (kOmRows * tiles);
     const dim3 grid((M + 31) / 32, tiles, splits), block(32, ty);
@@ -765,8 +778,7 @@ cudaError_t launch_vterm_reduce(int count, int N, int nw, int M, int Mpad, const
                                 const int* site_ptr, const int* site_slots, double2* out, double2* partial,
                                 int max_splits, cudaStream_t st, const double2* cw) {
     if (count <= 0 || num_offdiag == 0) return cudaSuccess;
-    const int per_split = max(64, (count + max_splits - 1) / max_splits);
-    const int splits = (count + per_split - 1) / per_split;
+    const int per_split = vterm_per_split(count, max_splits), splits = vterm_splits(count, max_splits);
     const dim3 grid((M + 31) / 32, N, splits);
     vterm_kernel<<<grid, 256, 0, st>>>(count, N, nw, M, Mpad, spins, enum_base, enumerate, w, cw, X, num_offdiag,
                                        site_ptr, site_slots, partial, per_split);
