@@ -942,17 +942,15 @@ __device__ __forceinline__ CPair dact_pair(CPair z) {
     return CPair{pk2(a.x, b.x), pk2(a.y, b.y)};
 }
 
-constexpr int kPairThreads = 128;   // threads of the kernels below
-
 // sums over the connections of `size` units for `pairs` pairs, NP of them per thread: weight
 // w[c * size + t] of connection c times the input in[.][c] (a dense layer: the input is shared
 // by the warp) or in[.][ci[c * size + t]]; emit(pair, t, sum)
-template <int NP, bool DENSE, typename Emit>
+template <int T, int NP, bool DENSE, typename Emit>
 __device__ __forceinline__ void layer_sums(int size, int conn, const float2* __restrict__ w,
                                            const int* __restrict__ ci, const float4* in, int in_size, int pairs,
                                            Emit emit) {
     const int groups = pairs / NP;
-    for (int item = threadIdx.x; item < size * groups; item += kPairThreads) {
+    for (int item = threadIdx.x; item < size * groups; item += T) {
         const int grp = item / size, t = item - grp * size;
         const float4* x = in + grp * NP * in_size;
         CPair a[NP];
@@ -970,19 +968,20 @@ __device__ __forceinline__ void layer_sums(int size, int conn, const float2* __r
     }
 }
 
-// pairs per thread: as many as leave work for most threads
-template <int PAIRS, bool DENSE, typename Emit>
+// pairs per thread of T: as many as leave work for half of the threads
+template <int T, int PAIRS, bool DENSE, typename Emit>
 __device__ __forceinline__ void layer_sums_split(int size, int conn, const float2* w, const int* ci, const float4* in,
                                                  int in_size, Emit emit) {
-    if (PAIRS >= 4 && size >= 64) layer_sums<(PAIRS >= 4 ? 4 : 1), DENSE>(size, conn, w, ci, in, in_size, PAIRS, emit);
-    else if (PAIRS >= 2 && size * PAIRS >= 128)
-        layer_sums<(PAIRS >= 2 ? 2 : 1), DENSE>(size, conn, w, ci, in, in_size, PAIRS, emit);
-    else layer_sums<1, DENSE>(size, conn, w, ci, in, in_size, PAIRS, emit);
+    if (PAIRS >= 4 && 2 * size >= T)
+        layer_sums<T, (PAIRS >= 4 ? 4 : 1), DENSE>(size, conn, w, ci, in, in_size, PAIRS, emit);
+    else if (PAIRS >= 2 && size * PAIRS >= T)
+        layer_sums<T, (PAIRS >= 2 ? 2 : 1), DENSE>(size, conn, w, ci, in, in_size, PAIRS, emit);
+    else layer_sums<T, 1, DENSE>(size, conn, w, ci, in, in_size, PAIRS, emit);
 }
 
 // layers 1 .. L - 1 from layer 0's activations in bufs[0]; layer l's activations go to
 // bufs[l & 1], emit(l, pair, t, angle, activation) sees them.  Ends with a barrier.
-template <int PAIRS, typename Emit>
+template <int T, int PAIRS, typename Emit>
 __device__ __forceinline__ void forward_pairs(const DeepNetDev& net, float4* const (&bufs)[2], Emit emit) {
     __syncthreads();
     for (int l = 1; l < net.L; l++) {
@@ -997,8 +996,8 @@ __device__ __forceinline__ void forward_pairs(const DeepNetDev& net, float4* con
             st_pair(out + p * size + t, y);
             emit(l, p, t, z, y);
         };
-        if (net.wt[l]) layer_sums_split<PAIRS, true>(size, conn, net.w[l], nullptr, in, below, done);
-        else layer_sums_split<PAIRS, false>(size, conn, net.w[l], net.cidx[l], in, below, done);
+        if (net.wt[l]) layer_sums_split<T, PAIRS, true>(size, conn, net.w[l], nullptr, in, below, done);
+        else layer_sums_split<T, PAIRS, false>(size, conn, net.w[l], net.cidx[l], in, below, done);
         __syncthreads();
     }
 }
@@ -1053,8 +1052,15 @@ size_t deep_mc_pairs_smem(const DeepNetDev& n, int pairs) {
 // rest ran after the others (100-200-100-50 net, four sweeps: 67.5 ms with a thread per unit,
 // 54.8 ms with six blocks, 35.8 ms; two units per thread 57, weights fetched ahead of their
 // use into registers 40 to 43).
-template <int PAIRS>
-__global__ void __launch_bounds__(kPairThreads, 7) deep_mc_pairs_kernel(DeepNetDev net, McLaunch L) {
+// With fewer blocks an SM, of wide layers or few walkers, a block has more threads (pair_threads);
+// 128 whatever the layers left an SM with four warps and was slower than the thread per unit.  One
+// sweep of thermalisation and one of sampling at N = 32, ms with a thread per unit / 128 threads / now:
+// 2048 walkers of 256-256 6.9 / 9.2 / 5.8, 400-400 14.4 / 25.4 / 12.0, 700-700-700 79.6 / 226 / 66.3; 256
+// walkers of them 4.8 / 7.4 / 2.7, 8.0 / 21.0 / 5.3, 31.3 / 105 / 24.8; 8192 walkers of 200-200 15.0 /
+// 17.1 / 13.4, 200-100-50 15.1 / 9.6 / 9.6 (256 threads: 10.7).
+constexpr int kPairsMcBlocks = 7;
+template <int PAIRS, int T>
+__global__ void __launch_bounds__(T, T == 128 ? kPairsMcBlocks : 1024 / T) deep_mc_pairs_kernel(DeepNetDev net, McLaunch L) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int WPC = 2 * PAIRS;
     const int size0 = net.size[0], N = net.N, nw = (N + 63) / 64;
@@ -1115,7 +1121,7 @@ __global__ void __launch_bounds__(kPairThreads, 7) deep_mc_pairs_kernel(DeepNetD
     for (int sw = 0; sw < total; sw++) {
         __syncthreads();
         // layer 0 and log psi of every state from its spins
-        for (int item = t; item < PAIRS * size0; item += kPairThreads) {
+        for (int item = t; item < PAIRS * size0; item += T) {
             const int p = item / size0, u = item - p * size0;
             const uint64_t *s0 = s + 2 * p * nw, *s1 = s0 + nw;
             CPair a{splat2(0.0f), splat2(0.0f)};
@@ -1133,13 +1139,13 @@ __global__ void __launch_bounds__(kPairThreads, 7) deep_mc_pairs_kernel(DeepNetD
             st_pair(zs + item, z);
             st_pair(bufs[0] + item, act_pair(z));
         }
-        forward_pairs<PAIRS>(net, bufs, none);
+        forward_pairs<T, PAIRS>(net, bufs, none);
         lpr = log_psi();
         if (own) moved[k_own] = make_int2(0, 0);
         propose();
         __syncthreads();
         for (int p = 0; p < N; p++) {
-            for (int item = t; item < PAIRS * size0; item += kPairThreads) {
+            for (int item = t; item < PAIRS * size0; item += T) {
                 const int q = item / size0, u = item - q * size0;
                 float4 z = zs[item];
                 float2 z0 = make_float2(z.x, z.z), z1 = make_float2(z.y, z.w);
@@ -1154,7 +1160,7 @@ __global__ void __launch_bounds__(kPairThreads, 7) deep_mc_pairs_kernel(DeepNetD
                 z1 = move_z0(net, p1.x, __int_as_float(p1.y), u, z1);
                 st_pair(bufs[0] + item, act_pair(CPair{pk2(z0.x, z1.x), pk2(z0.y, z1.y)}));
             }
-            forward_pairs<PAIRS>(net, bufs, none);
+            forward_pairs<T, PAIRS>(net, bufs, none);
             const float nl = log_psi();
             if (own) {
                 bool accept = false;
@@ -1179,7 +1185,7 @@ __global__ void __launch_bounds__(kPairThreads, 7) deep_mc_pairs_kernel(DeepNetD
         if (done > 0 && done % L.sweeps_per_sample == 0) {
             const long row0 = static_cast<long>(L.sample_base + sample) * L.B;
             if (L.sample_spins)
-                for (int i = t; i < WPC * nw; i += kPairThreads) {
+                for (int i = t; i < WPC * nw; i += T) {
                     const int k = i / nw, word = i % nw;
                     if (first + k < L.B) L.sample_spins[(row0 + first + k) * nw + word] = s[k * nw + word];
                 }
@@ -1187,7 +1193,7 @@ __global__ void __launch_bounds__(kPairThreads, 7) deep_mc_pairs_kernel(DeepNetD
         }
     }
     __syncthreads();
-    for (int i = t; i < WPC * nw; i += kPairThreads) {
+    for (int i = t; i < WPC * nw; i += T) {
         const int k = i / nw, word = i % nw;
         if (first + k < L.B) L.spins[static_cast<long>(first + k) * nw + word] = s[k * nw + word];
     }
@@ -1353,8 +1359,12 @@ size_t deep_adjoint_pairs_smem(const DeepNetDev& n, int pairs) {
 // held the FP64 pipe for 28000 cycles a neighbour on the 100-200-100-50 net, which was the
 // kernel's whole time.  Bound by the FP32 pipe and, at 128 threads, by the layers' barriers.
 // 8192 samples of that net: 70.3 -> 19.4 ms.
-template <int PAIRS>
-__global__ void __launch_bounds__(kPairThreads, 5) deep_adjoint_pairs_kernel(
+// More threads a block for wide layers or few samples, as the sampler (pair_threads): 2048 samples at
+// N = 32, ms with a thread per unit / 128 threads / now: 200-200 9.1 / 4.6 / 3.9, 400-400 36 / 22 / 12.2,
+// 700-700-700 314 / 217 / 73; 256 samples of 400-400-400 12.1 / 13.0 / 6.3.
+constexpr int kPairsAdjBlocks = 5;
+template <int PAIRS, int T>
+__global__ void __launch_bounds__(T, T == 128 ? kPairsAdjBlocks : 1024 / T) deep_adjoint_pairs_kernel(
     DeepNetDev net, OpDev op, int count, const uint64_t* spins, uint64_t enum_base, int enumerate,
     const double* weights, int score, double2* eloc, float2* acts, float2* dlts, float2* alpha, uint64_t* xspins,
     int xs, float2* dltsO, float2* alphaO) {
@@ -1373,7 +1383,7 @@ __global__ void __launch_bounds__(kPairThreads, 5) deep_adjoint_pairs_kernel(
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nw = (net.N + 63) / 64;
     load_config(spins, enum_base, enumerate, t, net.N, s);
-    for (int u = tid; u < size0; u += kPairThreads) {
+    for (int u = tid; u < size0; u += T) {
         float2 a = make_float2(0.0f, 0.0f);
         for (int c = 0; c < net.conn[0]; c++) {
             const float2 w = __ldg(net.w[0] + c * size0 + u);
@@ -1413,14 +1423,14 @@ __global__ void __launch_bounds__(kPairThreads, 5) deep_adjoint_pairs_kernel(
             if (2 * p < nb) row[0] = make_float2(a0, b0);
             if (2 * p + 1 < nb) row[units] = make_float2(a1, b1);
         };
-        for (int item = tid; item < P * size0; item += kPairThreads) {
+        for (int item = tid; item < P * size0; item += T) {
             const int p = item / size0, u = item - p * size0;
             const CPair z = z0of(p, u);
             const CPair y = act_pair(z);
             st_pair(bufs[0] + item, y);
             keep(0, p, u, z, y);
         }
-        forward_pairs<P>(net, bufs, keep);
+        forward_pairs<T, P>(net, bufs, keep);
     };
     // reverse pass: alpha_x delta_l(x) of configurations x0 .. x0 + nb - 1; with self also
     // w_s delta_l of the sample
@@ -1443,7 +1453,7 @@ __global__ void __launch_bounds__(kPairThreads, 5) deep_adjoint_pairs_kernel(
                 if (self && p == 0) dltsO[t * units + at] = make_float2(wsf * d0x, wsf * d0y);
             };
             if (l == net.L - 1) {
-                for (int item = tid; item < P * size; item += kPairThreads) {
+                for (int item = tid; item < P * size; item += T) {
                     const int p = item / size, u = item - p * size;
                     const float2 f = net.fw[u];
                     done(p, u, CPair{splat2(f.x), splat2(f.y)});
@@ -1452,10 +1462,10 @@ __global__ void __launch_bounds__(kPairThreads, 5) deep_adjoint_pairs_kernel(
                 const int above = net.size[l + 1];
                 const float4* nxt = bufs[(l + 1) & 1];
                 if (net.wt[l + 1]) {
-                    layer_sums_split<P, true>(size, above, net.wt[l + 1], nullptr, nxt, above, done);
+                    layer_sums_split<T, P, true>(size, above, net.wt[l + 1], nullptr, nxt, above, done);
                 } else {
                     const float2* wn = net.w[l + 1];
-                    for (int item = tid; item < P * size; item += kPairThreads) {
+                    for (int item = tid; item < P * size; item += T) {
                         const int p = item / size, u = item - p * size;
                         CPair a{splat2(0.0f), splat2(0.0f)};
                         for (int e = net.rptr[l][u]; e < net.rptr[l][u + 1]; e++) {
@@ -1532,7 +1542,7 @@ __global__ void __launch_bounds__(kPairThreads, 5) deep_adjoint_pairs_kernel(
                 eoi += __shfl_sync(0xffffffffu, e.y, k);
             }
         }
-        for (int i = tid; i < nb * nw; i += kPairThreads) {
+        for (int i = tid; i < nb * nw; i += T) {
             const int k = i / nw, word = i - k * nw, n = op.offdiag[q + k];
             uint64_t v = s[word];
             for (int f = 0; f < op.nflip[n]; f++) {
@@ -1766,6 +1776,42 @@ template <typename K>
 cudaError_t set_smem(K kernel, size_t bytes) {
     if (bytes <= 48 * 1024) return cudaSuccess;
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+}
+
+// units of the widest layer
+int widest(const DeepNetDev& n) {
+    int w = 0;
+    for (int l = 0; l < n.L; l++) w = std::max(w, n.size[l]);
+    return w;
+}
+
+// Threads a block of the pairs kernels, of r blocks an SM (as many as shared memory holds, or the
+// launch has): 128 where `many` of them fill the SM, otherwise enough that about 1024 threads are
+// resident, but not so many that most have no unit in any layer (512 walkers, N = 20, 128 / 256 /
+// 512 / 1024 threads: 40-20-10 650 / 574 / 594 / 634 us, 20-10 392 / 399 / 403 / 450); 256 threads only
+// where they take a layer's units in one round (4096 walkers of 320-320-320 43 ms, with 512 29).
+int pair_threads(size_t smem, int units, int blocks, int sms, int many) {
+    const int r = std::min(static_cast<int>((size_t(228) << 10) / (smem + 1024)), (blocks + sms - 1) / sms);
+    int threads = r >= many ? 128 : (r >= 3 && units <= 256 ? 256 : (r >= 2 ? 512 : 1024));
+    while (threads > 128 && threads > 8 * units) threads /= 2;
+    return threads;
+}
+
+// f(PAIRS, T) of the pairs kernels; one and two pairs take 512 threads where four take 256 or 1024
+template <typename F>
+cudaError_t pairs_launch(int pairs, int threads, F f) {
+    if (pairs == 4) {
+        const std::integral_constant<int, 4> four;
+        if (threads == 128) return f(four, std::integral_constant<int, 128>());
+        if (threads == 256) return f(four, std::integral_constant<int, 256>());
+        if (threads == 512) return f(four, std::integral_constant<int, 512>());
+        return f(four, std::integral_constant<int, 1024>());
+    }
+    auto few = [&](auto p) {
+        if (threads == 128) return f(p, std::integral_constant<int, 128>());
+        return f(p, std::integral_constant<int, 512>());
+    };
+    return pairs == 2 ? few(std::integral_constant<int, 2>()) : few(std::integral_constant<int, 1>());
 }
 
 }  // namespace
@@ -2174,46 +2220,46 @@ int deep_adjoint_chunk(const rbmg_psi* psi, const rbmg_operator* op, const Chunk
     // neighbours per pass of the reverse kernel: eight, or as many as the widest nets leave room
     // for in a block's shared memory (three layers of 720 units: four), or what
     // RBMG_DEEP_ADJOINT_BATCH = 1, 2, 4 or 8 says; the same outputs
-    int nbatch = 8;
+    int nbatch = 8, dev = 0, sms = 0;
+    RBMG_CK(cudaGetDevice(&dev));
+    RBMG_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     if (const char* v = std::getenv("RBMG_DEEP_ADJOINT_BATCH")) {
         nbatch = std::atoi(v);
     } else {
-        int dev = 0, limit = 0;
-        RBMG_CK(cudaGetDevice(&dev));
+        int limit = 0;
         RBMG_CK(cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
         while (nbatch > 2 && deep_adjoint_pairs_smem(net, nbatch / 2) > static_cast<size_t>(limit)) nbatch /= 2;
     }
     if (nbatch != 1 && nbatch != 2 && nbatch != 4 && nbatch != 8)
         return fail(RBMG_EINVAL, "RBMG_DEEP_ADJOINT_BATCH: 1, 2, 4 or 8");
     const size_t smb = deep_adjoint_pairs_smem(net, nbatch / 2);
-    if (nbatch == 2) RBMG_CK(set_smem(deep_adjoint_pairs_kernel<1>, smb));
-    if (nbatch == 4) RBMG_CK(set_smem(deep_adjoint_pairs_kernel<2>, smb));
-    if (nbatch == 8) RBMG_CK(set_smem(deep_adjoint_pairs_kernel<4>, smb));
+    // narrow nets keep 128 threads from three blocks an SM on (512 samples of 128-128, N = 20: 672 us,
+    // with 256 threads 700)
+    const int units = widest(net);
+    const int threads = pair_threads(smb, units, std::min(c.count, chunk), sms, units <= 128 ? 3 : kPairsAdjBlocks);
     for (int base = 0; base < c.count; base += chunk) {
         const int cnt = std::min(chunk, c.count - base);
         const uint64_t* sp = c.spins ? c.spins + static_cast<size_t>(base) * nw : nullptr;
         const double* wb = c.weights ? c.weights + base : nullptr;
-        if (nbatch == 8)
-            deep_adjoint_pairs_kernel<4><<<cnt, kPairThreads, smb, st>>>(
+        auto pairs_kernel = [&](auto pairs, auto t) -> cudaError_t {
+            const auto kernel = deep_adjoint_pairs_kernel<decltype(pairs)::value, decltype(t)::value>;
+            const cudaError_t e = set_smem(kernel, smb);
+            if (e != cudaSuccess) return e;
+            kernel<<<cnt, decltype(t)::value, smb, st>>>(
                 net, op->dev(), cnt, sp, c.enum_base + base, c.enumerate, wb, score, d_eloc + base,
                 acts.as<float2>(), dlts.as<float2>(), alpha.as<float2>(), xsp.as<uint64_t>(), xs, dltsO.as<float2>(),
                 alphaO.as<float2>());
-        else if (nbatch == 4)
-            deep_adjoint_pairs_kernel<2><<<cnt, kPairThreads, smb, st>>>(
-                net, op->dev(), cnt, sp, c.enum_base + base, c.enumerate, wb, score, d_eloc + base,
-                acts.as<float2>(), dlts.as<float2>(), alpha.as<float2>(), xsp.as<uint64_t>(), xs, dltsO.as<float2>(),
-                alphaO.as<float2>());
-        else if (nbatch == 2)
-            deep_adjoint_pairs_kernel<1><<<cnt, kPairThreads, smb, st>>>(
-                net, op->dev(), cnt, sp, c.enum_base + base, c.enumerate, wb, score, d_eloc + base,
-                acts.as<float2>(), dlts.as<float2>(), alpha.as<float2>(), xsp.as<uint64_t>(), xs, dltsO.as<float2>(),
-                alphaO.as<float2>());
-        else
+            return cudaGetLastError();
+        };
+        if (nbatch > 1) {
+            RBMG_CK(pairs_launch(nbatch / 2, threads, pairs_kernel));
+        } else {
             deep_adjoint_kernel<<<cnt, threads_for(net), sm, st>>>(
                 net, op->dev(), cnt, sp, c.enum_base + base, c.enumerate, wb, score, d_eloc + base,
                 acts.as<float2>(), dlts.as<float2>(), alpha.as<float2>(), xsp.as<uint64_t>(), xs, dltsO.as<float2>(),
                 alphaO.as<float2>());
-        RBMG_CK(cudaGetLastError());
+            RBMG_CK(cudaGetLastError());
+        }
         auto sum = [&](int M, int Nn, int cols, int splits, double2* out, double2* bias) -> cudaError_t {
             const long total = static_cast<long>(M) * cols;
             adj_split_sum_kernel<<<static_cast<unsigned>((total + 31) / 32), 256, 0, st>>>(M, Nn, cols, splits,
@@ -2282,10 +2328,11 @@ int deep_stream(rbmg_ensemble* e, const rbmg_psi* psi, const rbmg_operator* op, 
     if (wpc != 1 && wpc != 2 && wpc != 4 && wpc != 8) return fail(RBMG_EINVAL, "RBMG_DEEP_WALKERS_PER_BLOCK: 1, 2, 4 or 8");
     if (e->fast_sweep_tries != 0 || psi->kind == 2 || n0.ti) wpc = 1;
     const size_t smm = deep_mc_pairs_smem(n0, wpc / 2);
-    if (wpc == 2) RBMG_CK(set_smem(deep_mc_pairs_kernel<1>, smm));
-    if (wpc == 4) RBMG_CK(set_smem(deep_mc_pairs_kernel<2>, smm));
-    if (wpc == 8) RBMG_CK(set_smem(deep_mc_pairs_kernel<4>, smm));
     const int blocks = (B + wpc - 1) / wpc;
+    int dev = 0, sms = 0;
+    RBMG_CK(cudaGetDevice(&dev));
+    RBMG_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int threads = pair_threads(smm, widest(n0), blocks, sms, kPairsMcBlocks);
     bool first = true;
     for (int row0 = 0; row0 < steps; row0 += rows_per_chunk) {
         const int rows = std::min(rows_per_chunk, steps - row0);
@@ -2302,15 +2349,19 @@ int deep_stream(rbmg_ensemble* e, const rbmg_psi* psi, const rbmg_operator* op, 
         L.sample_spins = samples.as<uint64_t>();
         L.accepts = e->accepts.as<unsigned long long>();
         L.proposals = e->proposals.as<unsigned long long>();
-        if (wpc == 2)
-            deep_mc_pairs_kernel<1><<<blocks, kPairThreads, smm, stream()>>>(n0, L);
-        else if (wpc == 4)
-            deep_mc_pairs_kernel<2><<<blocks, kPairThreads, smm, stream()>>>(n0, L);
-        else if (wpc == 8)
-            deep_mc_pairs_kernel<4><<<blocks, kPairThreads, smm, stream()>>>(n0, L);
-        else
+        auto pairs_kernel = [&](auto pairs, auto t) -> cudaError_t {
+            const auto kernel = deep_mc_pairs_kernel<decltype(pairs)::value, decltype(t)::value>;
+            const cudaError_t e = set_smem(kernel, smm);
+            if (e != cudaSuccess) return e;
+            kernel<<<blocks, decltype(t)::value, smm, stream()>>>(n0, L);
+            return cudaGetLastError();
+        };
+        if (wpc > 1) {
+            RBMG_CK(pairs_launch(wpc / 2, threads, pairs_kernel));
+        } else {
             deep_mc_kernel<<<B, threads_for(n0), sm, stream()>>>(n0, n1, psi->kind == 2, L);
-        RBMG_CK(cudaGetLastError());
+            RBMG_CK(cudaGetLastError());
+        }
         first = false;
         Chunk c;
         c.count = c.group = rows * B;
