@@ -451,16 +451,17 @@ __global__ void deep_ok_kernel(DeepNetDev net, int count, const uint64_t* spins,
 // a parameter's entries are summed over the neighbours of a batch before its one read and write
 // of the row (one per neighbour before, and ten FP64 operations per entry instead of four).
 // 512 samples of the 20-40-20-10 net, 20 strings: gradient pass 2066 -> 489 us, energies 750 ->
-// 171 us.
-constexpr int kThreads64 = 128;
-
+// 171 us.  128 threads a block up to 128 units, 512 above, whose batches are small and which wait for
+// the rows and the weights: 256 samples, N = 32, ms of the gradient pass with one neighbour at a time /
+// 128 threads / 512: 200-100-50 22.8 / 10.7 / 8.6, 256-256 55.9 / 37.3 / 27.7, 400-400 139 / 166 / 72,
+// 512-512 320 / 568 / 205; energies and log psi' of 1024 samples of 72-30 3.21 / 0.99 / 1.09.
 size_t deep_local64_smem(const DeepNetDev& n, int nb, bool grad) {
     return sizeof(double2) * ((grad ? 2 : 1) * static_cast<size_t>(nb) * n.units + n.size[0] + 2 * nb) +
            sizeof(uint64_t) * (1 + nb) * kMaxWords;
 }
 
-template <bool GRAD>
-__global__ void __launch_bounds__(kThreads64) deep_local64_kernel(DeepNetDev net, OpDev op, int count,
+template <bool GRAD, int T>
+__global__ void __launch_bounds__(T, 1024 / T) deep_local64_kernel(DeepNetDev net, OpDev op, int count,
                                                                   const uint64_t* spins, uint64_t enum_base,
                                                                   int enumerate, int nbatch, DeepNetDev prime,
                                                                   double2* dlp, double2 e_shift, double2* eloc,
@@ -478,7 +479,7 @@ __global__ void __launch_bounds__(kThreads64) deep_local64_kernel(DeepNetDev net
     if (t >= count) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     load_config(spins, enum_base, enumerate, t, net.N, s);
-    for (int u = tid; u < size0; u += kThreads64) {
+    for (int u = tid; u < size0; u += T) {
         double2 a = net.b64[0][u];
         for (int c = 0; c < net.conn[0]; c++) {
             const double2 w = net.w64[0][c * size0 + u];
@@ -497,7 +498,7 @@ __global__ void __launch_bounds__(kThreads64) deep_local64_kernel(DeepNetDev net
             A[k * units + at] = f.value();
             if (GRAD) H[k * units + at] = f.tanh();
         };
-        for (int e = tid; e < nb * n.size[0]; e += kThreads64) {
+        for (int e = tid; e < nb * n.size[0]; e += T) {
             const int k = e / n.size[0], u = e - k * n.size[0];
             unit(k, u, z0of(k, u));
         }
@@ -506,7 +507,7 @@ __global__ void __launch_bounds__(kThreads64) deep_local64_kernel(DeepNetDev net
             const int size = n.size[l], conn = n.conn[l], at = n.begin_angle[l], below = n.begin_angle[l - 1];
             const int* ci = n.cidx[l];
             const double2* w = n.w64[l];
-            for (int e = tid; e < nb * size; e += kThreads64) {
+            for (int e = tid; e < nb * size; e += T) {
                 const int k = e / size, u = e - k * size;
                 const double2* in = A + k * units + below;
                 double2 a = n.b64[l][u], b = make_double2(0.0, 0.0);
@@ -522,7 +523,7 @@ __global__ void __launch_bounds__(kThreads64) deep_local64_kernel(DeepNetDev net
             __syncthreads();
         }
         const int last = n.size[L - 1];
-        for (int k = warp; k < nb; k += kThreads64 / 32) {
+        for (int k = warp; k < nb; k += T / 32) {
             double2 v = make_double2(0.0, 0.0);
             for (int u = lane; u < last; u += 32) v = cadd(v, cmul(A[k * units + n.begin_angle[L - 1] + u], n.fw64[u]));
 #pragma unroll
@@ -538,7 +539,7 @@ __global__ void __launch_bounds__(kThreads64) deep_local64_kernel(DeepNetDev net
     auto backward = [&](int nb) {
         for (int l = L - 1; l >= 0; l--) {
             const int size = net.size[l], at = net.begin_angle[l];
-            for (int e = tid; e < nb * size; e += kThreads64) {
+            for (int e = tid; e < nb * size; e += T) {
                 const int k = e / size, u = e - k * size;
                 double2 a = make_double2(0.0, 0.0);
                 if (l == L - 1) {
@@ -563,7 +564,7 @@ __global__ void __launch_bounds__(kThreads64) deep_local64_kernel(DeepNetDev net
     auto parameters = [&](int nb, const uint64_t* cfg, auto emit) {
         for (int l = 0; l < L; l++) {
             const int size = net.size[l], total = size + net.conn[l] * size, at = net.begin_angle[l];
-            for (int e = tid; e < total; e += kThreads64) {
+            for (int e = tid; e < total; e += T) {
                 double2 v = make_double2(0.0, 0.0);
                 if (e < size) {
                     for (int k = 0; k < nb; k++) v = cadd(v, H[k * units + at + e]);
@@ -587,7 +588,7 @@ __global__ void __launch_bounds__(kThreads64) deep_local64_kernel(DeepNetDev net
         }
         // final weights: log psi * activation of the last layer (PsiDeep.hpp:285-292)
         const int last = net.size[L - 1];
-        for (int u = tid; u < last; u += kThreads64) {
+        for (int u = tid; u < last; u += T) {
             double2 v = make_double2(0.0, 0.0);
             for (int k = 0; k < nb; k++)
                 v = cadd(v, cmul(cmul(en[k], lq[k]), A[k * units + net.begin_angle[L - 1] + u]));
@@ -634,7 +635,7 @@ __global__ void __launch_bounds__(kThreads64) deep_local64_kernel(DeepNetDev net
     double2 E = make_double2(0.0, 0.0);   // warp 0: the neighbours' terms, a lane's own
     for (int q = 0; q < op.num_offdiag; q += nbatch) {
         const int nb = min(nbatch, op.num_offdiag - q);
-        for (int i = tid; i < nb * kMaxWords; i += kThreads64) {
+        for (int i = tid; i < nb * kMaxWords; i += T) {
             const int k = i / kMaxWords, word = i - k * kMaxWords, n = op.offdiag[q + k];
             uint64_t v = s[word];
             for (int f = 0; f < op.nflip[n]; f++) {
@@ -683,7 +684,7 @@ __global__ void __launch_bounds__(kThreads64) deep_local64_kernel(DeepNetDev net
         auto plain = [&](const DeepNetDev& n) {
             for (int l = 0; l < L; l++) {
                 const int size = n.size[l], conn = n.conn[l];
-                for (int u = tid; u < size; u += kThreads64) {
+                for (int u = tid; u < size; u += T) {
                     double2 a = make_double2(0.0, 0.0);
                     for (int c = 0; c < conn; c++) {
                         const int i = n.cidx[l][c * size + u];
@@ -2037,6 +2038,11 @@ static int local64_batch(const DeepNetDev& n, bool grad) {
     while (nb > 1 && deep_local64_smem(n, nb, grad) > 72 * 1024) nb /= 2;
     return nb;
 }
+// f(T) with the kernel's threads a block
+template <typename F>
+static cudaError_t local64_launch(const DeepNetDev& n, F f) {
+    return widest(n) <= 128 ? f(std::integral_constant<int, 128>()) : f(std::integral_constant<int, 512>());
+}
 
 int deep_hsd64_chunk(const rbmg_psi* psi, const rbmg_psi* pp, const rbmg_operator* op, const Chunk& c,
                      double2* d_eloc, double2* d_dlp, cudaStream_t st) {
@@ -2050,10 +2056,15 @@ int deep_hsd64_chunk(const rbmg_psi* psi, const rbmg_psi* pp, const rbmg_operato
     if (alike) {
         const int nb = local64_batch(n0, false);
         const size_t sm = deep_local64_smem(n0, nb, false);
-        RBMG_CK(set_smem(deep_local64_kernel<false>, sm));
-        deep_local64_kernel<false><<<c.count, kThreads64, sm, st>>>(n0, op->dev(), c.count, c.spins, c.enum_base,
-                                                                    c.enumerate, nb, q0, d_dlp, make_double2(0.0, 0.0),
-                                                                    d_eloc, nullptr, nullptr, 0);
+        RBMG_CK(local64_launch(n0, [&](auto t) -> cudaError_t {
+            const auto kernel = deep_local64_kernel<false, decltype(t)::value>;
+            const cudaError_t e = set_smem(kernel, sm);
+            if (e != cudaSuccess) return e;
+            kernel<<<c.count, decltype(t)::value, sm, st>>>(n0, op->dev(), c.count, c.spins, c.enum_base, c.enumerate, nb,
+                                                            q0, d_dlp, make_double2(0.0, 0.0), d_eloc, nullptr, nullptr,
+                                                            0);
+            return cudaGetLastError();
+        }));
     } else {
         const size_t sm = smem_for(n0, sizeof(double2), false) + 2 * sizeof(uint64_t) * kMaxWords;
         auto run = [&](auto kernel) -> cudaError_t {
@@ -2164,16 +2175,20 @@ int deep_gradient_chunk(const rbmg_psi* psi, const rbmg_operator* op, const Chun
     RBMG_CK(erows.ensure(sizeof(double2) * static_cast<size_t>(std::min(chunk, c.count)) * P));
     const int nb = local64_batch(net, true);
     const size_t sm = deep_local64_smem(net, nb, true);
-    RBMG_CK(set_smem(deep_local64_kernel<true>, sm));
     DevBuf& part = rows_buf(2);
     RBMG_CK(launch_coef(c.count, c.weights, nullptr, 1.0, coef1, st));
     for (int base = 0; base < c.count; base += chunk) {
         const int cnt = std::min(chunk, c.count - base);
         const uint64_t* sp = c.spins ? c.spins + static_cast<size_t>(base) * ((net.N + 63) / 64) : nullptr;
-        deep_local64_kernel<true><<<cnt, kThreads64, sm, st>>>(net, op->dev(), cnt, sp, c.enum_base + base, c.enumerate,
-                                                               nb, net, nullptr, e_shift, d_eloc + base,
-                                                               orows.as<double2>(), erows.as<double2>(), P);
-        RBMG_CK(cudaGetLastError());
+        RBMG_CK(local64_launch(net, [&](auto t) -> cudaError_t {
+            const auto kernel = deep_local64_kernel<true, decltype(t)::value>;
+            const cudaError_t e = set_smem(kernel, sm);
+            if (e != cudaSuccess) return e;
+            kernel<<<cnt, decltype(t)::value, sm, st>>>(net, op->dev(), cnt, sp, c.enum_base + base, c.enumerate, nb, net,
+                                                        nullptr, e_shift, d_eloc + base, orows.as<double2>(),
+                                                        erows.as<double2>(), P);
+            return cudaGetLastError();
+        }));
         const double* wb = c.weights ? c.weights + base : nullptr;
         RBMG_CK(launch_coef(cnt, wb, d_eloc + base, 1.0, coef2 + base, st, e_shift));
         // sum w conj(E - E0) (E_k - E0 O_k): the fluctuation gradient's covariance term

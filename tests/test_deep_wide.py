@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 import rbmongpu_gb300 as rg
+import test_deep_fp64
 from test_deep_pairs import net, with_env
 
 pytestmark = pytest.mark.gpu
@@ -59,3 +60,9 @@ def test_adjoint_threads(samples, sizes, batch):
         return rg.ExpectationValue().eloc_gradient(psi, op, rg.FixedSamples(N, words))
     (g, E), (h, F) = (with_env("RBMG_DEEP_ADJOINT_BATCH", q, gradient) for q in (batch, 1))
     assert np.array_equal(g, h) and E == F
+
+
+@pytest.mark.parametrize("sizes", [(128, 10), (129, 10), (10, 129, 3)])
+def test_estimator_threads(sizes):
+    """The FP64 estimator takes 128 threads a block up to 128 units and 512 above."""
+    test_deep_fp64.test_estimator(9, sizes, 17, False)
