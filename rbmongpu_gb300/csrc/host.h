@@ -94,7 +94,10 @@ struct HostBuf {
 class Prefault {
   public:
     Prefault(void* p, size_t bytes) : p_(static_cast<char*>(p)), bytes_(bytes) {
-        const size_t n = std::min<size_t>({16, std::max(1u, std::thread::hardware_concurrency()), bytes >> 22});
+        if (bytes < size_t(8) << 20) return;
+        // asked for once: a call reads a file, 5 to 10 us
+        static const size_t cores = std::max(1u, std::thread::hardware_concurrency());
+        const size_t n = std::min<size_t>({16, cores, bytes >> 22});
         if (n < 2) return;
         const size_t per = ((bytes + n - 1) / n + 65535) / 65536 * 65536;
         try {
