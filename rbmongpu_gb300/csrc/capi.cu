@@ -434,6 +434,18 @@ static int op_compile(rbmg_operator* op) {
             site = 1;
         }
     }
+    {
+        // more strings than one round of one item a lane, none of more than two flips, and hardly a round
+        // of 16 strings of both kinds
+        int most = 0, changes = 0, last = 0;
+        for (int n = 0; n < op->S; n++) {
+            if (op->nflip[n] == 0) continue;
+            changes += last != 0 && op->nflip[n] != last;
+            last = op->nflip[n];
+            most = std::max(most, last);
+        }
+        op->in_pairs = op->num_offdiag > 8 && most <= 2 && 16 * changes <= op->num_offdiag;
+    }
     if (op->flip_sites.empty()) op->flip_sites.push_back(0);
     auto up = [](DevBuf& d, const void* h, size_t bytes) -> cudaError_t {
         cudaError_t e = d.ensure(std::max<size_t>(bytes, 16));

@@ -263,6 +263,7 @@ struct rbmg_operator {
     int num_offdiag = 0;
     int max_site = -1;
     bool single_flips = false;   // every off-diagonal string flips one site, no two the same
+    bool in_pairs = false;       // OpDev::in_pairs
     rbmg::DevBuf d_coef, d_coef32, d_site1, d_next1, d_ypow, d_zmask, d_nflip, d_flip_off, d_flip_sites, d_slot;
     rbmg::DevBuf d_offdiag;
     // per-site CSR of the off-diagonal slots whose string flips the site (E_k term)
@@ -282,7 +283,8 @@ struct rbmg_operator {
                            d_coef32.as<float2>(),
                            d_site1.as<int>(),
                            d_next1.as<int>(),
-                           d_offdiag.as<int>()};
+                           d_offdiag.as<int>(),
+                           in_pairs ? 1 : 0};
     }
 };
 

@@ -56,6 +56,7 @@ struct OpDev {
     const int* site1;          // [S] the flipped site of a single-flip string, -1 otherwise
     const int* next1;          // [S + 1] next1[n]: first single-flip string >= n (S if none)
     const int* offdiag;        // [num_offdiag] the off-diagonal strings in order
+    int in_pairs;              // the local energies take them two a lane and round (rbm_eloc_t_kernel)
 };
 
 // Metropolis launch: one warp per walker (include/spin_ensembles/MonteCarloLoop.hpp:55-256)

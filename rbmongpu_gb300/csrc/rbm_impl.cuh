@@ -747,14 +747,20 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) rbm_grad_terms_kernel(Rbm
 // per-string reduction sits on the critical path, and each lane's loop over units is
 // independent work.
 // Bound by shared-memory reads of theta and f and the latency of W's loads beside the FP32 pipe
-// (62 to 70 %); a lane takes two items per round, which halve those reads, and four units in flight
-// at large K, where W exceeds the L1.  16384 energies, one item a round / now: N = 64, M = 128 238 /
-// 209 us; N = 75, M = 150 366 / 324; N = 100, M = 400 1061 / 1002; N = 140, M = 576 2057 / 1867; 512
-// of them 37 / 25, 76 / 37, 154 / 80, 264 / 127.  Two configurations a warp, sharing the loads of W
-// instead, took 225, 336, 1129 and 2330, and half as long again at 512.
+// (62 to 70 %).  TWO (OpDev::in_pairs): a lane takes two items per round, which halve those reads,
+// and four units in flight at large K, where W exceeds the L1.  16384 energies of a transverse field,
+// one item a round / two: N = 64, M = 128 238 / 209 us; N = 75, M = 150 366 / 324; N = 100, M = 400 1061 /
+// 1002; N = 140, M = 576 2057 / 1867; 512 of them 37 / 25, 76 / 37, 154 / 80, 264 / 127.  Two
+// configurations a warp, sharing the loads of W instead, took 225, 336, 1129 and 2330, and half as long
+// again at 512.  Strings of two flips (a Heisenberg chain) gain as much: 16384 energies at N = 64, M = 128
+// 1.23 times, 500 1.8 times.  One item a round, and the registers for ten blocks an SM instead of
+// seven, serves operators of few strings (eight: the second item is no one's), of three flips and more,
+// whose sites are looked up unit by unit (5000 energies, N = 64, M = 256, three flips: 356 us, two items 498),
+// and of kinds that alternate.  Between 4256 and 5500 configurations, a wave of ten blocks and two of
+// seven, strings of two flips lose up to 13 % by it at N = 64 and 256 and gain up to a third elsewhere.
 // ---------------------------------------------------------------------------
-template <int K, int NW>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, K >= 18 ? 4 : (K >= 13 ? 5 : 7)) rbm_eloc_t_kernel(RbmDev P, OpDev op, EstLaunch L) {
+template <int K, int NW, bool TWO>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, TWO ? (K >= 18 ? 4 : (K >= 13 ? 5 : 7)) : 0) rbm_eloc_t_kernel(RbmDev P, OpDev op, EstLaunch L) {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const long t = static_cast<long>(blockIdx.x) * kWarpsPerBlock + wib;
     if (t >= L.count) return;
@@ -815,8 +821,61 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, K >= 18 ? 4 : (K >= 13 ? 
     }
     const int items = 4 * op.num_offdiag;
     const int N = P.N;
+    // an item a lane and round
+    auto item = [&](int nf, int off, int q, pair_t& sr, pair_t& si) {
+        auto unit = [&](float4 f, pair_t xr, pair_t xi) {
+            const Pair2 g = lc_c2_approx(xr, xi);
+            sr = add2(sr, sub2(g.re, pk2(f.x, f.y)));
+            si = add2(si, sub2(g.im, pk2(f.z, f.w)));
+        };
+        // pairs p = q, q + 4, ...: units (j, j + 4), j = q, q + 8, ...
+        if (nf == 1) {
+            const int site = op.flip_sites[off];
+            const pair_t two_s = splat2(s.up(site) ? -2.0f : 2.0f);
+            const float4* wcol = P.Wt4 + site;
+#pragma unroll 2
+            for (int p = q; p < MP / 2; p += 4) {
+                const float4 w = __ldg(wcol + static_cast<long>(p) * N);
+                const float4 a = tA[p], f = tB[p];
+                unit(f, fma2(two_s, pk2(w.x, w.y), pk2(a.x, a.y)), fma2(two_s, pk2(w.z, w.w), pk2(a.z, a.w)));
+            }
+        } else {
+            for (int p = q; p < MP / 2; p += 4) {
+                const float4 a = tA[p], f = tB[p];
+                pair_t xr = pk2(a.x, a.y), xi = pk2(a.z, a.w);
+                for (int u = 0; u < nf; u++) {
+                    const int site = op.flip_sites[off + u];
+                    const pair_t two_s = splat2(s.up(site) ? -2.0f : 2.0f);
+                    const float4 w = __ldg(P.Wt4 + static_cast<long>(p) * N + site);
+                    xr = fma2(two_s, pk2(w.x, w.y), xr);
+                    xi = fma2(two_s, pk2(w.z, w.w), xi);
+                }
+                unit(f, xr, xi);
+            }
+        }
+    };
+    for (int it0 = 0; !TWO && it0 < items; it0 += 32) {
+        const int it = it0 + lane, q = it & 3;
+        const bool live = it < items;
+        const int n = live ? op.offdiag[it >> 2] : 0;
+        pair_t sr = splat2(0.0f), si = sr;
+        if (live) item(op.nflip[n], op.flip_off[n], q, sr, si);
+        float r0, r1, i0, i1;
+        up2(sr, r0, r1);
+        up2(si, i0, i1);
+        float dx = r0 + r1, dy = i0 + i1;
+        // the four quarters of a string are lanes 4m .. 4m + 3
+        dx += __shfl_xor_sync(0xffffffffu, dx, 1);
+        dy += __shfl_xor_sync(0xffffffffu, dy, 1);
+        dx += __shfl_xor_sync(0xffffffffu, dx, 2);
+        dy += __shfl_xor_sync(0xffffffffu, dy, 2);
+        if (live && q == 0) {
+            const float2 e = string_term(string_factor(op, n, s), make_float2(dx, dy));
+            acc.add(e.x, e.y);
+        }
+    }
     // rounds of 64 items, a lane's two 32 apart: they share the loads of theta and f
-    for (int it0 = 0; it0 < items; it0 += 64) {
+    for (int it0 = 0; TWO && it0 < items; it0 += 64) {
         const int q = lane & 3;
         const bool two = it0 + 32 < items;   // for the whole warp
         bool live[2];
@@ -839,59 +898,48 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, K >= 18 ? 4 : (K >= 13 ? 
             si[h] = add2(si[h], sub2(g.im, pk2(f.z, f.w)));
         };
         // pairs p = q, q + 4, ...: units (j, j + 4), j = q, q + 8, ...
-        if (two && __all_sync(0xffffffffu, nf[0] == 1 && nf[1] == 1)) {
-            const int s0 = op.flip_sites[off[0]], s1 = op.flip_sites[off[1]];
-            const pair_t t0 = splat2(s.up(s0) ? -2.0f : 2.0f), t1 = splat2(s.up(s1) ? -2.0f : 2.0f);
-            const float4* w0 = P.Wt4 + s0;
-            const float4* w1 = P.Wt4 + s1;
-#pragma unroll (K >= 13 ? 4 : 2)
+        // both items, strings of F flips each
+        auto both = [&](auto flips) {
+            constexpr int F = decltype(flips)::value;
+            const float4* w[2][F];
+            pair_t ts[2][F];
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+#pragma unroll
+                for (int u = 0; u < F; u++) {
+                    const int site = op.flip_sites[off[h] + u];
+                    ts[h][u] = splat2(s.up(site) ? -2.0f : 2.0f);
+                    w[h][u] = P.Wt4 + site;
+                }
+#pragma unroll (K >= 13 && F == 1 ? 4 : 2)
             for (int p = q; p < MP / 2; p += 4) {
-                const float4 wa = __ldg(w0 + static_cast<long>(p) * N), wb = __ldg(w1 + static_cast<long>(p) * N);
+                float4 wv[2][F];
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+#pragma unroll
+                    for (int u = 0; u < F; u++) wv[h][u] = __ldg(w[h][u] + static_cast<long>(p) * N);
                 const float4 a = tA[p], f = tB[p];
-                unit(0, f, fma2(t0, pk2(wa.x, wa.y), pk2(a.x, a.y)), fma2(t0, pk2(wa.z, wa.w), pk2(a.z, a.w)));
-                unit(1, f, fma2(t1, pk2(wb.x, wb.y), pk2(a.x, a.y)), fma2(t1, pk2(wb.z, wb.w), pk2(a.z, a.w)));
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    pair_t xr = pk2(a.x, a.y), xi = pk2(a.z, a.w);
+#pragma unroll
+                    for (int u = 0; u < F; u++) {
+                        xr = fma2(ts[h][u], pk2(wv[h][u].x, wv[h][u].y), xr);
+                        xi = fma2(ts[h][u], pk2(wv[h][u].z, wv[h][u].w), xi);
+                    }
+                    unit(h, f, xr, xi);
+                }
             }
+        };
+        if (two && __all_sync(0xffffffffu, nf[0] == 1 && nf[1] == 1)) {
+            both(std::integral_constant<int, 1>());
+        } else if (two && __all_sync(0xffffffffu, nf[0] == 2 && nf[1] == 2)) {
+            both(std::integral_constant<int, 2>());
         } else {
-            for (int h = 0; h < (two ? 2 : 1); h++) {
-                const int nfh = h ? nf[1] : nf[0], offh = h ? off[1] : off[0];
-                pair_t r = splat2(0.0f), i = r;
-                if (nfh == 1) {
-                    const int site = op.flip_sites[offh];
-                    const pair_t two_s = splat2(s.up(site) ? -2.0f : 2.0f);
-                    const float4* wcol = P.Wt4 + site;
-#pragma unroll 2
-                    for (int p = q; p < MP / 2; p += 4) {
-                        const float4 w = __ldg(wcol + static_cast<long>(p) * N);
-                        const float4 a = tA[p], f = tB[p];
-                        const Pair2 g = lc_c2_approx(fma2(two_s, pk2(w.x, w.y), pk2(a.x, a.y)),
-                                                     fma2(two_s, pk2(w.z, w.w), pk2(a.z, a.w)));
-                        r = add2(r, sub2(g.re, pk2(f.x, f.y)));
-                        i = add2(i, sub2(g.im, pk2(f.z, f.w)));
-                    }
-                } else {
-                    for (int p = q; p < MP / 2; p += 4) {
-                        const float4 a = tA[p], f = tB[p];
-                        pair_t xr = pk2(a.x, a.y), xi = pk2(a.z, a.w);
-                        for (int u = 0; u < nfh; u++) {
-                            const int site = op.flip_sites[offh + u];
-                            const pair_t two_s = splat2(s.up(site) ? -2.0f : 2.0f);
-                            const float4 w = __ldg(P.Wt4 + static_cast<long>(p) * N + site);
-                            xr = fma2(two_s, pk2(w.x, w.y), xr);
-                            xi = fma2(two_s, pk2(w.z, w.w), xi);
-                        }
-                        const Pair2 g = lc_c2_approx(xr, xi);
-                        r = add2(r, sub2(g.re, pk2(f.x, f.y)));
-                        i = add2(i, sub2(g.im, pk2(f.z, f.w)));
-                    }
-                }
-                if (h) {
-                    sr[1] = r;
-                    si[1] = i;
-                } else {
-                    sr[0] = r;
-                    si[0] = i;
-                }
-            }
+            // an item at a time, live ones only
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+                if (live[h]) item(nf[h], off[h], q, sr[h], si[h]);
         }
         // the four quarters of a string are lanes 4m .. 4m + 3, of which lane 4m + h forms the
         // term of item h
@@ -985,14 +1033,18 @@ cudaError_t rbm_est_launch_k(const RbmDev& P, const OpDev* op, const RbmDev* PP,
     const int has = op != nullptr;
     RbmDev pp = PP ? *PP : P;
     if (has && (L.flags & ~(EST_ELOC | EST_ENUMERATE)) == 0) {
-        switch (nw) {
-            case 1: rbm_eloc_t_kernel<K, 1><<<grid, block, 0, st>>>(P, o, L); break;
-            case 2: rbm_eloc_t_kernel<K, 2><<<grid, block, 0, st>>>(P, o, L); break;
-            case 3: rbm_eloc_t_kernel<K, 3><<<grid, block, 0, st>>>(P, o, L); break;
-            case 4: rbm_eloc_t_kernel<K, 4><<<grid, block, 0, st>>>(P, o, L); break;
-            default: return cudaErrorInvalidValue;
-        }
-        return cudaGetLastError();
+        auto energies = [&](auto two) {
+            constexpr bool TWO = decltype(two)::value;
+            switch (nw) {
+                case 1: rbm_eloc_t_kernel<K, 1, TWO><<<grid, block, 0, st>>>(P, o, L); break;
+                case 2: rbm_eloc_t_kernel<K, 2, TWO><<<grid, block, 0, st>>>(P, o, L); break;
+                case 3: rbm_eloc_t_kernel<K, 3, TWO><<<grid, block, 0, st>>>(P, o, L); break;
+                case 4: rbm_eloc_t_kernel<K, 4, TWO><<<grid, block, 0, st>>>(P, o, L); break;
+                default: return cudaErrorInvalidValue;
+            }
+            return cudaGetLastError();
+        };
+        return o.in_pairs ? energies(std::true_type()) : energies(std::false_type());
     }
     if (L.en) {
         switch (nw) {
