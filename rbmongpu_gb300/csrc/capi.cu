@@ -148,8 +148,10 @@ static int rbm_upload(rbmg_psi* p) {
     RBMG_CK(p->dWq.ensure(sizeof(float4) * kp * p->N));
     RBMG_CK(p->dbq.ensure(sizeof(float4) * kp));
     RBMG_CK(p->dWt.ensure(sizeof(float2) * static_cast<size_t>(p->Mpad) * p->N));
-    RBMG_CK(p->dWg.ensure(sizeof(float2) * static_cast<size_t>(p->Mpad) * p->N));
-    RBMG_CK(p->dbg.ensure(sizeof(float2) * static_cast<size_t>(p->Mpad)));
+    if (rbm_group(p->Mpad / 32) < 32) {
+        RBMG_CK(p->dWg.ensure(sizeof(float2) * static_cast<size_t>(p->Mpad) * p->N));
+        RBMG_CK(p->dbg.ensure(sizeof(float2) * static_cast<size_t>(p->Mpad)));
+    }
     RBMG_CK(launch_rbm_pairs(p->N, p->Mpad, p->dW.as<float2>(), p->db.as<float2>(), p->dWq.as<float4>(),
                              p->dbq.as<float4>(), p->dWt.as<float4>(), p->dWg.as<float4>(), p->dbg.as<float4>(),
                              stream()));

@@ -26,7 +26,7 @@ struct RbmDev {
     // Wt4 [Mpad / 2][N], entry (p, i) = (x_j, x_j+4, y_j, y_j+4) of spin i's row,
     // j = 8 (p / 4) + p % 4
     const float4* Wt4;
-    // the same for walkers on rbm_group(K) < 32 lanes each (rbm_mc_group_kernel): lane g of G,
+    // the same for walkers on rbm_group(K) < 32 lanes each, else null (rbm_mc_group_kernel): lane g of G,
     // pair k H + h (H = 16 / G): units j0 = 32 k + 2 G h + g and j0 + G, as (x, x, y, y):
     // Wg [N][K H][G], bg [K H][G]
     const float4* Wg;
@@ -34,7 +34,7 @@ struct RbmDev {
 };
 
 // lanes that share a walker in the grouped sampler
-constexpr int rbm_group(int K) { return K == 1 ? 8 : (K < 18 ? 16 : 32); }   // 32: no groups
+constexpr int rbm_group(int K) { return K == 1 ? 8 : (K < 18 && K != 10 ? 16 : 32); }   // 32: no groups
 
 // build Wq, bq, Wg, bg from W [N][Mpad], b [Mpad] (K = Mpad / 32 hidden units per lane), and Wt4
 cudaError_t launch_rbm_pairs(int N, int Mpad, const float2* W, const float2* b, float4* Wq, float4* bq,

@@ -307,11 +307,8 @@ __device__ __forceinline__ double2 warp_log_psi(const float2 (&f)[K]) {
 // and decisions are the same bit for bit.
 // Bound by the FP32 pipe with many walkers (16384: its floor is half of the time) and by one
 // proposal's latency with few; the next site is found while a proposal is evaluated, both ways
-// the test's number may or may not be used.  Microseconds a sweep at 512 / 4096 / 16384 walkers,
-// G = 32 and 16: K = 3 (N = 30): 10, 36, 130 and 13, 29, 94; K = 4 (N = 64): 21, 75, 273 and 31, 73,
-// 236; K = 8 (N = 90): 41, 172, 630 and 74, 183, 597; K = 13 (N = 100): 74, 306, 1119 and 146, 355,
-// 1096; K = 18 (N = 140): 139, 551, 1996 and 252, 652, 2250.  Before, with G = 16 throughout (32 at K = 8):
-// 14, 29, 93; 32, 72, 233; 66, 183, 595; 149, 365, 1120; 253, 667, 2281.
+// the test's number may or may not be used.  rbm_grouped has the times of both; K = 18 has no groups
+// (N = 140, 512 / 4096 / 16384 walkers 139, 551, 1996 us a sweep, in groups 252, 652, 2250).
 // Blocks of one, two or four warps and keeping the proposed angles measured alike; G = 8 at K = 2
 // and 4 was slower up to 4096 walkers.  Five blocks an SM where the registers allow it gained 3 %
 // at 16384 walkers and lost 8 % at 512.
@@ -981,15 +978,24 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, TWO ? (K >= 18 ? 4 : (K >
 // ---------------------------------------------------------------------------
 // launchers for this K (instantiated by rbm_k<K>.cu)
 // ---------------------------------------------------------------------------
-// One walker per warp or a group of lanes each (rbm_mc_group_kernel's figures).  At an odd K the
-// whole warp leaves half a pair of units empty, which tells most at K = 3; from K = 8 on the
-// groups' longer chains still cost more at 4096 walkers, where both forms fill the chip's last
-// wave alike, but not between 1536 and 3584, where only the groups' first wave has room; K = 18 has
-// no groups (1996 against 2250 us at 16384 walkers).
-constexpr bool rbm_grouped(int K, int walkers) {
+// One walker per warp or a group of lanes each (rbm_mc_group_kernel).  A sweep takes as long as the
+// blocks that the fullest SM has, with whole warps ceil(walkers / 4 SMs).  Up to one (K = 3, whose whole
+// warps leave a quarter of their pairs empty), two (K = 1) or three of them the shorter chain of a whole
+// warp's proposal wins.  From there on half as many blocks of the groups, each slower, do the same
+// work: below K = 8 they are faster at once, above, where one costs 1.9 to 2 of the others, only where
+// they are exactly half as many, or so many that the odd one is lost.  K = 10 and 18 have no groups.
+// Microseconds a sweep at N = 96, 152 SMs, whole warps / groups of lanes, walkers 1216, 1536, 2048, 3072,
+// 4096, 6144, 16384: K = 1: 31/33 38/33 47/33 70/43 78/43 119/59 275/124; K = 2: 32/31 40/40 49/40 74/53
+// 83/67 126/102 292/222; K = 3: 38/36 50/49 62/50 92/66 106/85 163/127 385/281; K = 4: 40/43 51/60
+// 64/60 96/81 110/103 169/154 400/339; K = 5: 47/48 63/70 80/70 117/95 134/121 209/180 494/399; K = 6:
+// 50/60 65/80 82/80 122/111 140/142 216/210 512/468; K = 8: 59/74 78/100 100/100 147/140 169/180 262/264
+// 620/594; K = 10: 71/111 93/138 119/138 173/182 200/232 308/336 732/754; K = 13: 91/128 122/162 165/162
+// 231/222 270/310 414/430 985/967.
+constexpr bool rbm_grouped(int K, int walkers, int sms) {
     if (rbm_group(K) == 32) return false;
-    if (walkers <= (K == 3 ? 608 : (K == 1 ? 1216 : 1536))) return false;
-    return !(K >= 8 && walkers >= 3584 && walkers <= 6144);
+    const int blocks = (walkers + 4 * sms - 1) / (4 * sms);
+    if (blocks <= (K == 3 ? 1 : (K == 1 ? 2 : 3))) return false;
+    return K < 8 || blocks % 2 == 0 || blocks > 14;
 }
 
 template <int K>
@@ -1020,7 +1026,11 @@ cudaError_t rbm_mc_launch_k(const RbmDev& P, const OpDev* op, const McLaunch& L,
         else return cudaErrorInvalidValue;
         return cudaGetLastError();
     };
-    if (rbm_grouped(K, L.B)) return sampler(std::integral_constant<int, rbm_group(K)>());
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    if (rbm_grouped(K, L.B, sms)) return sampler(std::integral_constant<int, rbm_group(K)>());
     return sampler(std::integral_constant<int, 32>());
 }
 
