@@ -1823,11 +1823,6 @@ struct DeepHost {
     DeepNetDev net[2];
 };
 
-static std::vector<std::unique_ptr<DeepHost>>& deep_registry() {
-    static std::vector<std::unique_ptr<DeepHost>> r;
-    return r;
-}
-
 template <typename T>
 static cudaError_t upload(DeepHost* h, const std::vector<T>& v, const T** out) {
     auto b = std::make_unique<DevBuf>();

@@ -125,7 +125,5 @@ cudaError_t launch_ratio_weights(int count, const double* w, const double2* lp, 
                                  double2* rwc, cudaStream_t st);
 // a[s] = exp(2 Im E + Re(E E - E)), the weight of ExpectationValue::corrected
 cudaError_t launch_corrected_terms(int count, const double2* e, double2* a, cudaStream_t st);
-cudaError_t launch_hsd_terms(int count, const double2* eloc, const double2* lp, const double2* lpp, int is_unitary,
-                             double2* omega, double2* pr, double2* nn, cudaStream_t st);
 
 }  // namespace rbmg

@@ -689,31 +689,6 @@ __global__ void abs2_kernel(int count, const double2* __restrict__ v, double2* o
         out[s] = make_double2(v[s].x * v[s].x + v[s].y * v[s].y, 0.0);
 }
 
-// Hilbert-space distance per-sample terms (source/network_functions/HilbertSpaceDistance.cu:83-106)
-__global__ void hsd_terms_kernel(int count, const double2* __restrict__ eloc, const double2* __restrict__ lp,
-                                 const double2* __restrict__ lpp, int is_unitary, double2* omega, double2* pr,
-                                 double2* nn) {
-    for (long s = blockIdx.x * 256L + threadIdx.x; s < count; s += static_cast<long>(gridDim.x) * 256) {
-        const double2 e = eloc[s];
-        const double dr = lpp[s].x - lp[s].x, di = -(lpp[s].y - lp[s].y);   // conj(log psi' - log psi)
-        double2 om;
-        double n;
-        if (is_unitary) {
-            const double m = exp(dr);
-            const double ar = m * cos(di), ai = m * sin(di);
-            om = make_double2(ar * e.x - ai * e.y, ar * e.y + ai * e.x);
-            n = e.x * e.x + e.y * e.y;
-        } else {
-            const double m = exp(e.x + dr);
-            om = make_double2(m * cos(e.y + di), m * sin(e.y + di));
-            n = exp(2.0 * e.x);
-        }
-        omega[s] = om;
-        pr[s] = make_double2(exp(2.0 * (lpp[s].x - lp[s].x)), 0.0);
-        nn[s] = make_double2(n, 0.0);
-    }
-}
-
 inline int grid_for(long count) { return static_cast<int>(min(1024L, max(1L, (count + 255) / 256))); }
 
 }  // namespace
@@ -902,12 +877,6 @@ cudaError_t launch_corrected_terms(int count, const double2* e, double2* a, cuda
 
 cudaError_t launch_abs2(int count, const double2* v, double2* out, cudaStream_t st) {
     abs2_kernel<<<grid_for(count), 256, 0, st>>>(count, v, out);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_hsd_terms(int count, const double2* eloc, const double2* lp, const double2* lpp, int is_unitary,
-                             double2* omega, double2* pr, double2* nn, cudaStream_t st) {
-    hsd_terms_kernel<<<grid_for(count), 256, 0, st>>>(count, eloc, lp, lpp, is_unitary, omega, pr, nn);
     return cudaGetLastError();
 }
 
