@@ -2214,17 +2214,29 @@ int deep_adjoint_chunk(const rbmg_psi* psi, const rbmg_operator* op, const Chunk
     static thread_local DevBuf acts, dlts, alpha, xsp, dltsO, alphaO, partial;
     const size_t per_sample = static_cast<size_t>(xs) * (2 * sizeof(float2) * net.units + sizeof(float2) + 8 * nw) +
                               sizeof(float2) * (net.units + 1);
-    // parts of the FP32 sums (AdjSplit), and as many of them per launch as fit 4 GB of the
-    // stored activations and errors
+    // parts of the FP32 sums (AdjSplit) of at most 768 MB of stored activations and errors, and as many
+    // parts per launch as fit 4 GB of them, held by the thread (N = 100, 200-100-50, 8192 samples: one
+    // part 35.3 ms, 1.6 GB 33.5, 4 GB 32.0, 8 GB 32.0); one part where the device has no room for more
     const int part = std::max(1, static_cast<int>(std::min<size_t>(c.count, (size_t(768) << 20) / per_sample)));
-    const int chunk = static_cast<int>(std::min<size_t>(
+    int chunk = static_cast<int>(std::min<size_t>(
         c.count, static_cast<size_t>(part) * std::max<size_t>(1, (size_t(4) << 30) / (per_sample * part))));
-    RBMG_CK(acts.ensure(sizeof(float2) * static_cast<size_t>(chunk) * xs * net.units));
-    RBMG_CK(dlts.ensure(sizeof(float2) * static_cast<size_t>(chunk) * xs * net.units));
-    RBMG_CK(alpha.ensure(sizeof(float2) * static_cast<size_t>(chunk) * xs));
-    RBMG_CK(xsp.ensure(sizeof(uint64_t) * static_cast<size_t>(chunk) * xs * nw));
-    RBMG_CK(dltsO.ensure(sizeof(float2) * static_cast<size_t>(chunk) * net.units));
-    RBMG_CK(alphaO.ensure(sizeof(float2) * static_cast<size_t>(chunk)));
+    auto room = [&]() {
+        cudaError_t e = acts.ensure(sizeof(float2) * static_cast<size_t>(chunk) * xs * net.units);
+        if (e == cudaSuccess) e = dlts.ensure(sizeof(float2) * static_cast<size_t>(chunk) * xs * net.units);
+        if (e == cudaSuccess) e = alpha.ensure(sizeof(float2) * static_cast<size_t>(chunk) * xs);
+        if (e == cudaSuccess) e = xsp.ensure(sizeof(uint64_t) * static_cast<size_t>(chunk) * xs * nw);
+        if (e == cudaSuccess) e = dltsO.ensure(sizeof(float2) * static_cast<size_t>(chunk) * net.units);
+        return e == cudaSuccess ? alphaO.ensure(sizeof(float2) * static_cast<size_t>(chunk)) : e;
+    };
+    cudaError_t held = room();
+    if (held == cudaErrorMemoryAllocation && chunk > part) {
+        cudaGetLastError();
+        acts.release();
+        dlts.release();
+        chunk = part;
+        held = room();
+    }
+    RBMG_CK(held);
     const size_t sm = smem_for(net, sizeof(float2), true) + 2 * sizeof(float2) * net.size[0];
     RBMG_CK(set_smem(deep_adjoint_kernel, sm));
     // neighbours per pass of the reverse kernel: eight, or as many as the widest nets leave room
