@@ -767,7 +767,16 @@ cudaError_t launch_vterm_reduce(int count, int N, int nw, int M, int Mpad, const
     return launch_split_sums(&job, 1, true, st);
 }
 
-// the blocks of a column of 32 hidden units walk its units of work, three blocks an SM in all
+static size_t grad_vectors_smem(int cap) {
+    return sizeof(float4) * kGvWarps * kGvStrings * cap + sizeof(float2) * kGvStrings * kGvWarps * 32 +
+           sizeof(pair_t) * kGvWarps * 32 * cap;
+}
+
+// the blocks of a column of 32 hidden units walk its units of work, as many in all as the SMs hold at
+// once: three each, or two where a group of more than 9700 samples (all states of 14 spins and more)
+// takes more than a third of their shared memory; three there were a second, half empty wave (the
+// gradient over all states of 16 spins, M = 128, 2.11 ms, now 2.01; 40960 samples at N = 30, M = 75
+// 1.57 / 1.50)
 struct GradVectorsShape {
     int per_group, units, rows, cap;   // units of a full group, of all groups; blocks a column of units
 };
@@ -775,7 +784,8 @@ static GradVectorsShape grad_vectors_grid(int count, int group, int Mpad, int ma
     int per_split, splits, chunks, cap;
     grad_vectors_shape(std::min(count, group), max_splits, &per_split, &splits, &chunks, &cap);
     const int per_group = splits * chunks, units = (count + group - 1) / group * per_group;
-    return {per_group, units, std::min(units, std::max(1, 3 * sms / (Mpad / 32))), cap};
+    const int fit = std::min(3, static_cast<int>((size_t(228) << 10) / (grad_vectors_smem(cap) + 1024)));
+    return {per_group, units, std::min(units, std::max(1, fit * sms / (Mpad / 32))), cap};
 }
 
 size_t grad_vectors_bytes(int count, int group, int N, int M, int Mpad, int max_splits, int sms) {
@@ -786,8 +796,7 @@ cudaError_t launch_grad_vectors(const GradVectors& g, const OpDev& op, double2* 
                                 SplitSum* job) {
     if (g.count <= 0) return cudaSuccess;
     const GradVectorsShape S = grad_vectors_grid(g.count, g.group, g.Mpad, g.max_splits, sms);
-    const size_t sm = sizeof(float4) * kGvWarps * kGvStrings * S.cap + sizeof(float2) * kGvStrings * kGvWarps * 32 +
-                      sizeof(pair_t) * kGvWarps * 32 * S.cap;
+    const size_t sm = grad_vectors_smem(S.cap);
     const auto kernel = g.Mpad == 32 ? grad_vectors_kernel<true> : grad_vectors_kernel<false>;
     if (sm > 48 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
