@@ -63,10 +63,10 @@ THERM_SWEEPS = 8000
 METRIC = "effective samples/s (ESS of E_loc) at N=100: learned-proposal MCMC (plain single-flip beside)"
 UNIT = "samples/s"
 L2_FLUSH_BYTES = 256 << 20
-# DRAM bytes of one sampler launch: dram__bytes_read.sum + dram__bytes_write.sum of an ncu
-# capture of the one-walker-per-warp sampler on these 16384 walkers (rbm_mc_group_kernel<13,16,2>
-# moves the same spins, stream positions and counts)
-SAMPLER_DRAM_BYTES = 1.059e6
+# DRAM bytes of one sampler launch, 10 sweeps of 16384 walkers: dram__bytes_read.sum +
+# dram__bytes_write.sum of rbm_mc_group_kernel<13,16,2>, mean of three launches under ncu
+# (1.59 MB read, 0.07 MB written: W and the walkers' spins, stream positions and counts)
+SAMPLER_DRAM_BYTES = 1.664e6
 # DRAM bytes of one learned_accept_kernel<13,2> launch of 16384 walkers (ncu, sigma 0.05, mean
 # of three launches: 100.3 MB read, 4.1 MB written -- accepted angles stay in L2 within a launch)
 ACCEPT_DRAM_BYTES = 104.4e6

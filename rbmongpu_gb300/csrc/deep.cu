@@ -1,6 +1,8 @@
 // PsiDeep / PsiPair kernels (include/quantum_state/PsiDeep.hpp:89-293, PsiPair.hpp:36-119).
 //
-// One CTA per configuration: thread j owns unit j of the layer being evaluated;
+// The general form has one CTA per configuration, thread j owning unit j of the layer being
+// evaluated; complex nets without translation sums take several walkers or neighbours of a sample
+// per CTA (deep_mc_pairs_kernel, deep_adjoint_pairs_kernel, deep_local64_kernel);
 // the estimator kernels (local energies, O_k and E_k rows) run in FP64 -- for these
 // nets log psi(s') - log psi(s) is the difference of two full forward passes, so FP32
 // would cost ~1e-7 |log psi| per local-energy term -- while the Metropolis sampler runs
@@ -2168,6 +2170,9 @@ int deep_gradient_chunk(const rbmg_psi* psi, const rbmg_operator* op, const Chun
     DevBuf& erows = rows_buf(1);
     RBMG_CK(orows.ensure(sizeof(double2) * static_cast<size_t>(std::min(chunk, c.count)) * P));
     RBMG_CK(erows.ensure(sizeof(double2) * static_cast<size_t>(std::min(chunk, c.count)) * P));
+    int dev = 0, sms = 0;
+    RBMG_CK(cudaGetDevice(&dev));
+    RBMG_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const int nb = local64_batch(net, true);
     const size_t sm = deep_local64_smem(net, nb, true);
     DevBuf& part = rows_buf(2);
@@ -2188,9 +2193,9 @@ int deep_gradient_chunk(const rbmg_psi* psi, const rbmg_operator* op, const Chun
         RBMG_CK(launch_coef(cnt, wb, d_eloc + base, 1.0, coef2 + base, st, e_shift));
         // sum w conj(E - E0) (E_k - E0 O_k): the fluctuation gradient's covariance term
         if (acc_B) RBMG_CK(launch_coef_conj(cnt, wb, d_eloc + base, e_shift, coef3 + base, st));
-        // enough splits of the samples to fill the GPU, of eight samples at least
-        const int cols = (P + 127) / 128;
-        const int per = std::max(8, (cnt + std::max(1, 608 / cols) - 1) / std::max(1, 608 / cols));
+        // enough splits of the samples for four blocks an SM, of eight samples at least
+        const int cols = (P + 127) / 128, want = std::max(1, 4 * sms / cols);
+        const int per = std::max(8, (cnt + want - 1) / want);
         const int splits = (cnt + per - 1) / per;
         RBMG_CK(part.ensure(sizeof(double2) * 4 * static_cast<size_t>(splits) * P));
         row_sums_kernel<<<dim3(cols, splits), 128, 0, st>>>(cnt, P, coef1 + base, coef2 + base,

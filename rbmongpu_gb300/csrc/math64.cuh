@@ -13,6 +13,13 @@ namespace rbmg {
 // reciprocal serves both parts: the hardware's estimate (at least 19 bits) and one cubic step
 // r (1 + e + e^2), e = 1 - den r, which leaves e^3 < 2^-57.  32 FP64 operations with the
 // difference and its sum, against 61 with two divisions.
+// All of it is 64 bits, but not the same roundings.  Against 113 bits (emulated, Re z and Im z normal
+// with deviation 0.1 / 0.3 / 1 / 3 / 10) the activation's rms error is 5.4e-17 / 4.7e-17 / 6.3e-17 /
+// 1.6e-16 / 4.5e-16, with Horner's scheme and divisions 4.6e-17 / 4.2e-17 / 6.9e-17 / 1.6e-16 / 4.5e-16.
+// In a whole log psi the angles' sums count for more, and these have fewer roundings by groups of
+// spins: 2.5e-16 against 2.4e-16 at N = 12, M = 24, 4.5e-16 / 5.0e-16 at 36, 75, 9.4e-16 / 1.4e-15 at 75, 150,
+// 3.0e-15 / 5.4e-15 at 140, 400.  The distance of deep nets, a difference down to the last bits, keeps
+// the other order (lc64_plain).
 constexpr double kLcC = 0.598139;
 constexpr double kLcA = 0.9003320053750442;
 

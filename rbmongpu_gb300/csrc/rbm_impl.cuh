@@ -1,9 +1,10 @@
 // Complex-RBM kernels: Metropolis sampler and per-sample estimator pass.
 //
-// Layout: one warp per walker (or per configuration).  Lane l owns hidden units
-// j = l + 32 k, k < K, and keeps their angles theta_j and Re f(theta_j) in
-// registers for the whole chain; W rows are read coalesced (one float2 per lane
-// per k) from global memory through L1/L2.  This file is included by the rbm_k*.cu
+// Layout: one warp per configuration, and per walker one warp or, where walkers fill the
+// chip, a group of 16 or 8 lanes (rbm_mc_group_kernel).  Lane l of a warp owns hidden units
+// j = l + 32 k, k < K (lane g of a group those of lanes g, g + G, ...), and the sampler keeps
+// their angles theta_j and Re f(theta_j) in registers for the whole chain; W rows are read
+// coalesced from global memory through L1/L2.  This file is included by the rbm_k*.cu
 // translation units, each instantiating one K.
 #pragma once
 #include <type_traits>

@@ -1,9 +1,10 @@
 // Deterministic reductions of per-sample quantities into the estimator sums.
 //
 // All sums over samples run in a fixed order: FP32 partial sums over chunks of at
-// most 32 samples, accumulated in FP64, then per-block partials combined by a
-// second kernel in block order.  No floating-point atomics, so results are
-// bit-reproducible run to run.
+// most 32 samples, accumulated in FP64, then the blocks' partials in a fixed order: those of the
+// outer sums by a second kernel, split by split; those of the weighted sums of series by the block
+// that arrives last, each lane its own blocks in order and the lanes by a butterfly.  No
+// floating-point atomics, so results are bit-reproducible run to run.
 #include <algorithm>
 
 #include "device_math.cuh"
