@@ -882,7 +882,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, TWO ? (K >= 18 ? 4 : (K >
         for (int h = 0; h < 2; h++) {
             const int it = it0 + 32 * h + lane;
             live[h] = it < items;
-            n[h] = op.offdiag[live[h] ? it >> 2 : 0];
+            n[h] = op.offdiag[min(it >> 2, op.num_offdiag - 1)];   // of no item: a string of this round's kind
             nf[h] = op.nflip[n[h]];
             off[h] = op.flip_off[n[h]];
         }
